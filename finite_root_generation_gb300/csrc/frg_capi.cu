@@ -390,8 +390,9 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     int bps = ctx->cfg.blocks_per_sm > 0             ? ctx->cfg.blocks_per_sm
               : (ctx->cfg.system != 0 && mode < 3)  ? plugin_bps[mode]
                                                     : (team ? ctx->team_blocks_per_sm[mode] : ctx->blocks_per_sm[mode]);
+    if (!team) return frg_thread_grid(ctx->sm_count, bps, n);
     int64_t grid = (int64_t)ctx->sm_count * bps;
-    int64_t per_block = team ? FRG_TEAM_THREADS / 8 : FRG_TRACK_THREADS;
+    int64_t per_block = FRG_TEAM_THREADS / 8;
     int64_t need = (n + per_block - 1) / per_block;
     if (grid > need) grid = need;
     return (int)(grid < 1 ? 1 : grid);

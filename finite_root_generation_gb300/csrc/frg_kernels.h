@@ -81,6 +81,18 @@ struct TrackArgs {
 
 }  // namespace frg
 
+// Grid of a thread-per-path launch over n paths with at most bps blocks per SM: one warp
+// per SM sub-partition while the paths fit there (the kernel then spreads them over the
+// warps, one path per lane at most), beyond that one path per thread.
+inline int frg_thread_grid(int sms, int bps, int64_t n) {
+  const int64_t wpb = FRG_TRACK_THREADS / 32, spread = (int64_t)sms * 4;
+  const int64_t want = n <= spread * 32 ? ((n < spread ? n : spread) + wpb - 1) / wpb
+                                        : (n + FRG_TRACK_THREADS - 1) / FRG_TRACK_THREADS;
+  const int64_t cap = (int64_t)sms * bps;
+  const int64_t grid = want < cap ? want : cap;
+  return (int)(grid < 1 ? 1 : grid);
+}
+
 // mode: 0 plain FP64, 1 FP32 stage with handoff, 2 FP64 resume of handed-off paths
 cudaError_t frg_launch_track(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream);
 cudaError_t frg_track_occupancy(int mode, int* blocks_per_sm);

@@ -34,7 +34,7 @@
 
 namespace frg {
 
-enum Phase : int { PH_FETCH = 0, PH_TANGENT0 = 1, PH_RK = 2, PH_NEWTON = 3, PH_SHARP = 4 };
+enum Phase : int { PH_FETCH = 0, PH_TANGENT0 = 1, PH_RK = 2, PH_NEWTON = 3, PH_SHARP = 4, PH_IDLE = 5 };
 enum Mode : int { MODE_PLAIN = 0, MODE_LO = 1, MODE_RESUME = 2 };
 
 // NY_ = the path state's length (homogeneous unknowns + t), NP_ = parameters.
@@ -147,53 +147,69 @@ track_kernel(TrackArgs a) {
   PathState<T, NY_, NP_> P;
   cx<T> Ye[NY_], q[NP_], dq[NP_], F[NZ_], b[NY_], x[NY_];
   cx<T> M[NY_ * LD_];
-  P.phase = PH_FETCH;
   unsigned long long fp64_solves = 0;
   const int64_t nqueue = (MODE == MODE_RESUME) ? (int64_t)*a.handoff_count : a.npaths;
+  // Paths per warp: as few as spread the queue over the launch's warps. A warp-wide FP64
+  // instruction holds its sub-partition's FP64 pipe for the same time whatever the number
+  // of active lanes, and paths in different phases of their steps make a warp run each
+  // phase's code in turn, so a short queue is tracked fastest one path per warp (64 conic2
+  // paths in mixed precision 5.7 -> 3.8 ms, 777 burmester5 paths in FP64 545 -> 495 ms, the
+  // latter one long path's latency).
+  const int64_t warps = (int64_t)gridDim.x * (FRG_TRACK_THREADS / 32);
+  P.phase = (int64_t)(threadIdx.x & 31) * warps < nqueue ? PH_FETCH : PH_IDLE;
 
   for (;;) {
     // ------------------------------------------------------------------ fetch
     if (P.phase == PH_FETCH) {
       const int64_t qi = (int64_t)atomicAdd(a.queue, 1ull);
-      if (qi >= nqueue) break;
-      const int64_t id = (MODE == MODE_RESUME) ? a.handoff_list[qi] : qi;
-      P.id = id;
-      int lo = 0, hi = a.ntasks - 1;  // task of this path
-      while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (a.task_start[mid] <= id) lo = mid; else hi = mid - 1;
-      }
-      P.task = lo;
-      // Start system (frg.cu:54): the stream of path id; TrackPath receives the same
-      // fresh state (frg.cu:57, by value), so its draws restart at index 0.
-      P.rng.seed = a.seed; P.rng.stream = (uint64_t)(id + c.path_offset); P.rng.index = 0;
-      cd spt[NV_], spm[NP_];
-      S::start(P.rng, c.start_dist, c.start_range, spt, spm);
-#pragma unroll 1
-      for (int e = 0; e < NP_; ++e) P.spm[e] = cx<T>(spm[e]);
-      P.code = 0; P.stage = 0; P.attempt = 0; P.it = 0; P.residual = T(100); P.err = T(0); P.scale = T(0);
-      if (MODE == MODE_RESUME) {
-        const Handoff& h = a.handoff[id];
-#pragma unroll 1
-        for (int e = 0; e < NY_; ++e) { P.Yc[e] = cx<T>(h.Yc[e]); P.Vc[e] = cx<T>(h.Vc[e]); P.u[e] = cx<T>(h.u[e]); }
-        P.s = T(h.s); P.rng.index = h.rng_index;
-        P.streak = h.streak; P.step = h.step; P.ministep = h.ministep; P.tstepQ = h.tstepQ;
-        P.n_ivp = h.n_ivp; P.n_newton = h.n_newton;
-        P.phase = PH_RK;
+      if (qi >= nqueue) {
+        P.phase = PH_IDLE;
       } else {
-        P.rng.index = 0;
+        const int64_t id = (MODE == MODE_RESUME) ? a.handoff_list[qi] : qi;
+        P.id = id;
+        int lo = 0, hi = a.ntasks - 1;  // task of this path
+        while (lo < hi) {
+          int mid = (lo + hi + 1) >> 1;
+          if (a.task_start[mid] <= id) lo = mid; else hi = mid - 1;
+        }
+        P.task = lo;
+        // Start system (frg.cu:54): the stream of path id; TrackPath receives the same
+        // fresh state (frg.cu:57, by value), so its draws restart at index 0.
+        P.rng.seed = a.seed; P.rng.stream = (uint64_t)(id + c.path_offset); P.rng.index = 0;
+        cd spt[NV_], spm[NP_];
+        S::start(P.rng, c.start_dist, c.start_range, spt, spm);
 #pragma unroll 1
-        for (int e = 0; e < NV_; ++e) P.Yc[e] = cx<T>(spt[e]);
-        P.Yc[NV_] = cx<T>(T(1));
-        P.Yc[NV_ + 1] = cx<T>(T(0));
-        draw_patch<T, NY_>(P.rng, c.patch_range, P.u);
-        switch_patch<T, NY_>(P.u, P.Yc, P.Yc);
-        draw_patch<T, NY_>(P.rng, c.patch_range, P.Vc);
-        P.s = T(c.s_init); P.tstepQ = 0; P.streak = c.caution_steps - 1; P.step = 0; P.ministep = 0;
-        P.n_ivp = 0; P.n_newton = 0;
-        P.phase = PH_TANGENT0;
+        for (int e = 0; e < NP_; ++e) P.spm[e] = cx<T>(spm[e]);
+        P.code = 0; P.stage = 0; P.attempt = 0; P.it = 0; P.residual = T(100); P.err = T(0); P.scale = T(0);
+        if (MODE == MODE_RESUME) {
+          const Handoff& h = a.handoff[id];
+#pragma unroll 1
+          for (int e = 0; e < NY_; ++e) { P.Yc[e] = cx<T>(h.Yc[e]); P.Vc[e] = cx<T>(h.Vc[e]); P.u[e] = cx<T>(h.u[e]); }
+          P.s = T(h.s); P.rng.index = h.rng_index;
+          P.streak = h.streak; P.step = h.step; P.ministep = h.ministep; P.tstepQ = h.tstepQ;
+          P.n_ivp = h.n_ivp; P.n_newton = h.n_newton;
+          P.phase = PH_RK;
+        } else {
+          P.rng.index = 0;
+#pragma unroll 1
+          for (int e = 0; e < NV_; ++e) P.Yc[e] = cx<T>(spt[e]);
+          P.Yc[NV_] = cx<T>(T(1));
+          P.Yc[NV_ + 1] = cx<T>(T(0));
+          draw_patch<T, NY_>(P.rng, c.patch_range, P.u);
+          switch_patch<T, NY_>(P.u, P.Yc, P.Yc);
+          draw_patch<T, NY_>(P.rng, c.patch_range, P.Vc);
+          P.s = T(c.s_init); P.tstepQ = 0; P.streak = c.caution_steps - 1; P.step = 0; P.ministep = 0;
+          P.n_ivp = 0; P.n_newton = 0;
+          P.phase = PH_TANGENT0;
+        }
       }
     }
+    // The warp's lanes meet here each trip and again before the linear step, so that the
+    // divergent control code does not leave them apart in it (262,144 conic2 paths in
+    // FP64: 267 -> 250 ms, of which the longest paths' tail is the larger part).
+    const unsigned live = __ballot_sync(0xffffffffu, P.phase != PH_IDLE);
+    if (!live) break;
+    if (P.phase == PH_IDLE) continue;
 
     // -------------------------------------------------- set up the linear step
     const cx<T>* fpmT = TaskFpm<T, NP_>::get(a, P.task);
@@ -221,32 +237,34 @@ track_kernel(TrackArgs a) {
     }
 
     // ------------------------------------------------------ the linear step
+    __syncwarp(live);
     params_at<T, NP_>(Ye[NY_ - 1].re, P.spm, fpmT, gamma, q, dq);
     if (MODE != MODE_LO) fp64_solves++;
     S::template rows<T, LD_>(Ye, q, dq, M, newton ? F : nullptr);
     // row NV_: the projective patch u (htpysupport.cu:139-142); row NV_ + 1: the velocity patch
 #pragma unroll 1
     for (int e = 0; e < NY_; ++e) { M[NV_ * LD_ + e] = P.u[e]; M[(NV_ + 1) * LD_ + e] = patch[e]; }
-    T hnorm = T(0), ratio;
+    T hnorm = T(0);
+    T tdiff = T(0);
     if (newton) {
       cx<T> d(T(0));
 #pragma unroll 1
       for (int e = 0; e < NY_; ++e) d = cfma(P.u[e], Ye[e], d);
       F[NV_] = d - cx<T>(T(1));
       hnorm = vnorm(F, NZ_);
-      row_scale<T, NY_, LD_>(M, NZ_, F);
+      tdiff = ((P.phase == PH_SHARP) ? T(1) : P.Yn[NY_ - 1].re) - Ye[NY_ - 1].re;
+    }
+    // one scaling and one elimination for both kinds of step, so that lanes in the
+    // corrector and lanes in the predictor run them together
+    row_scale<T, NY_, LD_>(M, NZ_, newton ? F : nullptr);
 #pragma unroll 1
-      for (int e = 0; e < NZ_; ++e) b[e] = -F[e];
-      b[NZ_] = cx<T>(T(0));
-      const T tgoal = (P.phase == PH_SHARP) ? T(1) : P.Yn[NY_ - 1].re;
-      ratio = lu_solve<T, NY_, LD_>(M, b, x, NZ_, true, cx<T>(tgoal - Ye[NY_ - 1].re));
+    for (int e = 0; e < NZ_; ++e) b[e] = newton ? -F[e] : cx<T>(T(0));
+    b[NY_ - 1] = newton ? cx<T>(T(0)) : cx<T>(T(1));
+    __syncwarp(live);
+    const T ratio = lu_solve<T, NY_, LD_>(M, b, x, newton ? NZ_ : NY_, newton, cx<T>(tdiff));
+    if (newton) {
       P.n_newton++;
     } else {
-      row_scale<T, NY_, LD_>(M, NZ_, nullptr);
-#pragma unroll 1
-      for (int e = 0; e < NY_; ++e) b[e] = cx<T>(T(0));
-      b[NY_ - 1] = cx<T>(T(1));
-      ratio = lu_solve<T, NY_, LD_>(M, b, x, NY_, false, cx<T>(T(0)));
       // normalise the tangent (htpysupport.cu:285-296): unit length with real
       // dt/ds, or dt = 1 when stepping in t. conj(x22)/|x22| is the reference's
       // (cos theta, -sin theta) with theta = arg(x22).
