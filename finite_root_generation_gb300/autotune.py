@@ -8,7 +8,7 @@ fresh seeds, and caches it per GPU model and workload in a JSON file.
 
 Searched dimensions (each a field of frg_config, a bundle of fields, or the rounds in
 flight of frg_track_rounds):
-  kernel_variant  paths per warp: 4 (8-lane teams) or 32 (one path per thread)
+  kernel_variant  a warp per path (team) or one path per thread
   blocks_per_sm   resident blocks per SM (0 = the occupancy maximum)
   precision       FP64, or mixed with the FP32 stage's point type lo_points 0/1
   cond_switch     the condition estimate above which a step goes to FP64

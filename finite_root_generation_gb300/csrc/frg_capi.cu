@@ -348,6 +348,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   a.gamma_df = (const cx<df>*)sl.gamma_df.p;
   a.task_start = (const int64_t*)sl.task_start.p;
   a.ntasks = ntasks;
+  a.sms = ctx->sm_count;
   a.npaths = N;
   a.seed = seed;
   unsigned long long* q = (unsigned long long*)sl.queue.p;
@@ -380,8 +381,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     cudaError_t e = frg_launch_starts(a, (cx<double>*)sl.starts.p, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "start kernel launch");
   }
-  // persistent grids: SMs x resident blocks, capped by the work (one path per thread
-  // for the thread kernels, one per 8 lanes for the team kernels)
+  // persistent grids: SMs x resident blocks, capped by the work
   int plugin_bps[3] = {0, 0, 0};  // a plug-in system's kernels have their own occupancy
   if (ctx->cfg.system != 0)
     for (int m = 0; m < (mixed ? 3 : 1); ++m)
@@ -390,12 +390,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     int bps = ctx->cfg.blocks_per_sm > 0             ? ctx->cfg.blocks_per_sm
               : (ctx->cfg.system != 0 && mode < 3)  ? plugin_bps[mode]
                                                     : (team ? ctx->team_blocks_per_sm[mode] : ctx->blocks_per_sm[mode]);
-    if (!team) return frg_thread_grid(ctx->sm_count, bps, n);
-    int64_t grid = (int64_t)ctx->sm_count * bps;
-    int64_t per_block = FRG_TEAM_THREADS / 8;
-    int64_t need = (n + per_block - 1) / per_block;
-    if (grid > need) grid = need;
-    return (int)(grid < 1 ? 1 : grid);
+    return team ? frg_team_grid(ctx->sm_count, bps, n) : frg_thread_grid(ctx->sm_count, bps, n);
   };
   auto launch = [&](int mode, int grid) {
     return team ? frg_launch_team(mode, a, grid, st) : frg_launch_track(mode, a, grid, st);
@@ -688,6 +683,7 @@ static frg_status enqueue_rounds_carry(frg_ctx* ctx, const cx<double>* d_fpm, bo
   a.gamma_df = (const cx<df>*)ctx->c_gamma_df.p;
   a.task_start = (const int64_t*)ctx->c_task_start.p;
   a.ntasks = ntasks;
+  a.sms = ctx->sm_count;
   a.npaths = N;
   a.seeds = (const uint64_t*)ctx->c_seeds.p;
   a.roots = d_roots;
@@ -696,8 +692,7 @@ static frg_status enqueue_rounds_carry(frg_ctx* ctx, const cx<double>* d_fpm, bo
   a.handoff = (frg::Handoff*)ctx->c_rec.p;
   auto grid_for = [&](int mode) {
     int bps = ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : ctx->team_blocks_per_sm[mode];
-    int64_t grid = (int64_t)ctx->sm_count * bps;
-    return (int)(grid < 1 ? 1 : grid);
+    return frg_team_grid(ctx->sm_count, bps, (int64_t)KN);
   };
   const int lo_mode = ctx->cfg.lo_points == 1 ? 3 : 1;
   auto rounds = [&]() -> frg_status {

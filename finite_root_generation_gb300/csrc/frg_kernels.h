@@ -12,9 +12,7 @@
 #ifndef FRG_TRACK_THREADS
 #define FRG_TRACK_THREADS 64
 #endif
-#ifndef FRG_TEAM_THREADS
-#define FRG_TEAM_THREADS 64
-#endif
+#define FRG_START_THREADS 64
 
 namespace frg {
 
@@ -71,6 +69,7 @@ struct TrackArgs {
   const unsigned long long* lo_count;
   int64_t* back_list;           // FP64 kernel: paths handed back to FP32 (null: none, e.g. the last round)
   unsigned long long* back_count;
+  int sms;                      // the device's SMs
   int lo_keep_ill;              // FP32 kernel: 1 = no hand-off for ill-conditioned steps (last round)
   float* feat;                  // optional: FRG_MLP_IN features per checkpoint, feat_max checkpoints per path
   int32_t* nfeat;               // checkpoints written per path (zeroed before launch)
@@ -88,6 +87,15 @@ inline int frg_thread_grid(int sms, int bps, int64_t n) {
   const int64_t wpb = FRG_TRACK_THREADS / 32, spread = (int64_t)sms * 4;
   const int64_t want = n <= spread * 32 ? ((n < spread ? n : spread) + wpb - 1) / wpb
                                         : (n + FRG_TRACK_THREADS - 1) / FRG_TRACK_THREADS;
+  const int64_t cap = (int64_t)sms * bps;
+  const int64_t grid = want < cap ? want : cap;
+  return (int)(grid < 1 ? 1 : grid);
+}
+
+// Grid of a team launch (four paths per block) over at most n paths: one block per SM
+// until every SM has its four, then as many as fit, at most bps per SM.
+inline int frg_team_grid(int sms, int bps, int64_t n) {
+  const int64_t want = n <= (int64_t)sms * 4 ? (n < sms ? n : sms) : (n + 3) / 4;
   const int64_t cap = (int64_t)sms * bps;
   const int64_t grid = want < cap ? want : cap;
   return (int)(grid < 1 ? 1 : grid);

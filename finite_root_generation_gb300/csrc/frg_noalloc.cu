@@ -168,10 +168,8 @@ extern "C" frg_status frg_track_noalloc(const frg_config* cfg, const double* fpm
   if ((team ? frg_team_occupancy(0, &bps) : frg_track_occupancy(0, &bps)) != cudaSuccess) return FRG_ERR_CUDA;
   if (cfg->blocks_per_sm > 0) bps = cfg->blocks_per_sm;
   if (bps < 1) bps = 1;
-  const int64_t per_block = FRG_TEAM_THREADS / 8;
-  int64_t grid = (int64_t)sms * bps, need = (N + per_block - 1) / per_block;
-  if (grid > need) grid = need;
-  if (!team) grid = frg_thread_grid(sms, bps, N);
-  const cudaError_t e = team ? frg_launch_team(0, a, (int)grid, st) : frg_launch_track(0, a, (int)grid, st);
+  a.sms = sms;
+  const int grid = team ? frg_team_grid(sms, bps, N) : frg_thread_grid(sms, bps, N);
+  const cudaError_t e = team ? frg_launch_team(0, a, grid, st) : frg_launch_track(0, a, grid, st);
   return e == cudaSuccess ? FRG_OK : FRG_ERR_CUDA;
 }

@@ -1,26 +1,39 @@
-// Team (8-lane) building blocks of the warp-cooperative tracker.
+// Building blocks of the warp-cooperative tracker: one path per warp, four paths per
+// block, every linear step in two parts.
 //
-// A team of 8 consecutive lanes tracks one path; a warp holds 4 teams. Lane g < 7
-// owns equation group j = g + 1 (rows j-1, j+6, j+13 of the reference's JH,
-// htpysupport.cu:89-144); lane 7 owns the two patch rows (the projective patch u,
-// row 21, and the velocity patch / t-selector, row 22).
+// Evaluation, by the block. The seven equation groups of a path (group j = rows j-1,
+// j+6, j+13 of the reference's JH, htpysupport.cu:89-144) run on seven lanes, so a warp
+// holds the groups of the block's four paths; the straight-line code of a group is cut
+// into four parts of equal cost, one per warp (frg_eval_slice, generated), and what the
+// parts share (q(t), reciprocals, the quantities of FrgEvalIn) is computed once by the
+// path's own warp (eval_prep).
 //
-// The linear system of one step (the reference's 23x23 row-scaled dense LU,
-// LinearSolve / LinearSolveNewton, htpysupport.cu:146-400) is solved with the
-// system's structure: U_j appears only in group j's three equations and in the two
-// patch rows, so each group lane pivots U_j out of its own rows (partial pivoting
-// among the group's three rows) and the eliminations are folded into the patch rows
-// with one butterfly reduction. What remains is a dense 16 x 16 system in the links
-// A..Hc, the homogenizer Z0 and t, two rows per lane, solved by LU with partial
-// pivoting across the team (argmax and pivot-row broadcast by warp shuffles), then
-// column-oriented back substitution; U_j follows from lane g's pivot row. The
-// solution is the same as the dense solve up to rounding (checked against the
-// dense LU in the tests).
+// Solve, by the path's own warp (solve_step). The reference's 23x23 row-scaled dense LU
+// (LinearSolve / LinearSolveNewton, htpysupport.cu:146-400) is solved with the system's
+// structure: U_j appears only in group j's three equations and in the two patch rows, so
+// each group pivots U_j out of its own rows (partial pivoting among its three rows; lane
+// 8 q + g holds the columns c = q mod 4 of group g + 1) and the eliminations are folded
+// into the patch rows with one butterfly reduction. What remains is a dense 16 x 16
+// system in the links A..Hc, the homogenizer Z0 and t: lane 16 h + r holds the columns
+// c = h mod 2 of row r, partial pivoting across the lanes, then column-oriented back
+// substitution; U_j follows from the group's pivot row. The solution is the same as the
+// dense solve up to rounding (checked against the dense LU in the tests). The Newton
+// variant replaces the velocity patch by the t-selector row with right-hand side
+// t_goal - t, which fixes dt exactly like LinearSolveNewton's x[22] = tdiff
+// (htpysupport.cu:374).
 //
-// Register-resident: a lane holds at most 3 rows of 18 complex values during the
-// group phase and 2 rows of 17 during the dense phase. The Newton variant replaces
-// the velocity patch by the t-selector row with right-hand side t_goal - t, which
-// fixes dt exactly like LinearSolveNewton's x[22] = tdiff (htpysupport.cu:374).
+// What bounds it: on this part a warp-wide FP64 instruction holds its sub-partition's
+// FP64 pipe for 64 cycles and answers after about 73, whatever the number of active
+// lanes, so an FP64 step takes (FP64 warp instructions on its longest warp) x 64..82
+// cycles and everything else hides behind them; the FP32 step is bound by instruction
+// issue and fetch. With one path per 8 lanes (four paths in a warp, the layout before
+// this one) an FP64 step was 5,800 FP64 instructions in one warp, 421k cycles; cut over
+// the four sub-partitions and with 32 lanes on the elimination it is 1,590 on the
+// longest warp, 131k cycles (8 to 600 paths; FP32 step 105k -> 19k). With every SM full
+// the FP64 work per path falls as well (fewer repeated sums and idle lanes: 9.3 against
+// 5.7 M FP64 steps/s, 49 against 32 M steps/s in the mixed-precision benchmark rounds).
+// Comparisons and maxima of FP64 values run on their bit patterns in the integer pipes
+// for the same reason.
 #pragma once
 
 #include "frg_device.cuh"
@@ -34,28 +47,25 @@ namespace team {
 // runs on the FP32 pipes but is ~10x more code than the FP64 form.
 template <typename T> struct PointOf { typedef double type; };
 
-constexpr int TEAM = 8;
-constexpr int NG = 16;  // links (14), Z0, t
-constexpr int VS = 24;  // shared-memory vector stride (23 used)
+constexpr int TEAM = 8;    // lanes of one path in the evaluation (7 groups)
+constexpr int PATHS = 4;   // paths (warps) per block
+constexpr int VS = 24;     // shared-memory vector stride (23 used)
+constexpr int LDU = 21;    // leading dimension of the dense system and its factor (odd: no bank conflicts)
+constexpr unsigned FULL = 0xffffffffu;
 
 // reduced-system column -> state index
 __device__ __forceinline__ constexpr int gstate(int c) { return c < 14 ? c : (c == 14 ? 21 : 22); }
 
 template <typename T>
-__device__ __forceinline__ T shfl(unsigned mask, T v, int src) { return __shfl_sync(mask, v, src, TEAM); }
-template <typename T>
 __device__ __forceinline__ T shfl_xor(unsigned mask, T v, int off) { return __shfl_xor_sync(mask, v, off, TEAM); }
-template <typename T>
-__device__ __forceinline__ cx<T> shfl(unsigned mask, cx<T> v, int src) {
-  return cx<T>(__shfl_sync(mask, v.re, src, TEAM), __shfl_sync(mask, v.im, src, TEAM));
-}
-template <typename T>
-__device__ __forceinline__ cx<T> shfl_xor(unsigned mask, cx<T> v, int off) {
-  return cx<T>(__shfl_xor_sync(mask, v.re, off, TEAM), __shfl_xor_sync(mask, v.im, off, TEAM));
-}
 __device__ __forceinline__ df shfl_xor(unsigned mask, df v, int off) {
   return df(__shfl_xor_sync(mask, v.hi, off, TEAM), __shfl_xor_sync(mask, v.lo, off, TEAM));
 }
+template <typename T>
+__device__ __forceinline__ cx<T> warp_shfl(cx<T> v, int src) {
+  return cx<T>(__shfl_sync(FULL, v.re, src), __shfl_sync(FULL, v.im, src));
+}
+// sums and maxima over each group of 8 lanes (in every lane of the group)
 template <typename T>
 __device__ __forceinline__ T team_sum(unsigned mask, T v) {
   v += shfl_xor(mask, v, 4);
@@ -70,42 +80,98 @@ __device__ __forceinline__ T team_max(unsigned mask, T v) {
   v = fmax(v, shfl_xor(mask, v, 1));
   return v;
 }
-template <typename T>
-__device__ __forceinline__ T team_min(unsigned mask, T v) {
-  v = fmin(v, shfl_xor(mask, v, 4));
-  v = fmin(v, shfl_xor(mask, v, 2));
-  v = fmin(v, shfl_xor(mask, v, 1));
-  return v;
-}
 
-// Per-team shared state of one path. The points Yc (accepted), Yn (predicted) and
-// YN (corrector iterate) are in the point type (FP64, or double-float in the FP32
-// stage, whose corrector refines on double-float residuals with an FP32 solve);
-// directions, patches and stage vectors are in the working precision T. U/Urhs hold the reduced system's
-// upper factor for the back substitution. The 32-byte tail makes the stride between
-// teams 32 bytes past a multiple of 128, so the four teams of a warp reading "the
-// same" field hit different bank groups.
-template <typename T, typename P = typename PointOf<T>::type>
-struct Smem {
-  cx<P> Yc[VS], Yn[VS], YN[VS];
-  cx<P> spm[32];
-  cx<T> Vc[VS], Vn[VS], u[VS], Ye[VS], dx[VS];
-  cx<T> k[8][VS];
-  cx<T> U[16][16];
-  cx<T> Urhs[16];
-  // Checkpoint history of the early-retirement features (lane 0 only). These 32 bytes
-  // also make the stride between teams 32 bytes past a multiple of 128.
-  double ck_t[2];   // t at the last two checkpoints
-  float ck_s[2];    // step sizes at the last two checkpoints
-  float ck_rmax;    // largest condition estimate since the last checkpoint
-  float ck_unused;
+// Largest |re| or |im| of values, NaN taking no part (as fmax drops it): FP32 directly,
+// FP64 on the bit patterns, whose order as integers is the order of the magnitudes.
+template <typename T> struct MaxAbs;
+template <> struct MaxAbs<float> {
+  float m = 0.f;
+  __device__ __forceinline__ void take(cx<float> v) { m = fmaxf(m, fmaxf(fabsf(v.re), fabsf(v.im))); }
+  __device__ __forceinline__ void across(int off) { m = fmaxf(m, __shfl_xor_sync(FULL, m, off)); }
+  __device__ __forceinline__ float value() const { return m; }
+};
+template <> struct MaxAbs<double> {
+  long long m = 0;
+  __device__ __forceinline__ void one(double x) {
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
+    if (b > m && b <= 0x7ff0000000000000ll) m = b;
+  }
+  __device__ __forceinline__ void take(cx<double> v) { one(v.re); one(v.im); }
+  __device__ __forceinline__ void across(int off) {
+    const long long o = __shfl_xor_sync(FULL, m, off);
+    if (o > m) m = o;
+  }
+  __device__ __forceinline__ double value() const { return __longlong_as_double(m); }
 };
 
-// Parameter values a lane needs for its group: index 0 P0, 1 Pc0, 2 Pj, 3 Pcj, 4 Qj, 5 Qcj.
+// running maximum and minimum of magnitudes >= 0, NaN taking no part
+__device__ __forceinline__ float max_mag(float m, float x) { return fmaxf(m, x); }
+__device__ __forceinline__ float min_mag(float m, float x) { return fminf(m, x); }
+__device__ __forceinline__ double max_mag(double m, double x) {
+  const long long b = __double_as_longlong(x);
+  return b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll ? x : m;
+}
+__device__ __forceinline__ double min_mag(double m, double x) {
+  const long long b = __double_as_longlong(x);
+  return b >= 0 && b < __double_as_longlong(m) ? x : m;
+}
+
+// 1 / b when |b|^2 is at hand (FP64: conj(b) / |b|^2; FP32 keeps Smith's form)
+__device__ __forceinline__ cx<double> cinv_norm(cx<double> b, double n2) {
+  const double r = 1.0 / n2;
+  return cx<double>(b.re * r, -b.im * r);
+}
+__device__ __forceinline__ cx<float> cinv_norm(cx<float> b, float) { return cinv(b); }
+
+// products that no later addition may absorb into a fused multiply-add
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 template <typename T>
-struct LaneParams {
-  cx<T> sp[6], fp[6];
-  cx<T> gamma;
+__device__ __forceinline__ cx<T> mul_rn(T s, cx<T> a) { return cx<T>(mul_rn(s, a.re), mul_rn(s, a.im)); }
+// s * a + b, fused
+template <typename T>
+__device__ __forceinline__ cx<T> axpy(T s, cx<T> a, cx<T> b) { return cx<T>(fma(s, a.re, b.re), fma(s, a.im, b.im)); }
+
+// Task and start parameters in the working precision, when it is not the point type's.
+template <typename T, typename P> struct LowTask { cx<T> sp[32], fp[32]; };
+template <typename T> struct LowTask<T, T> {};
+template <typename T, typename P> struct HighEval { FrgEvalIn<P> in; };
+template <typename T> struct HighEval<T, T> {};
+
+// Shared state of one path. The points Yc (accepted), Yn (predicted) and YN (corrector
+// iterate) are in the point type (FP64, or double-float in the FP32 stage, whose
+// corrector refines on double-float residuals with an FP32 solve); directions, patches
+// and stage vectors are in the working precision T. `M` holds the group rows
+// (frg_eval_slice's layout; its structural zeros are written once). The evaluation's
+// inputs and the dense system with its factor share memory: the block's barriers keep
+// them apart.
+template <typename T, typename P = typename PointOf<T>::type>
+struct Smem {
+  struct Inputs {
+    FrgEvalIn<T> in;
+    cx<T> dq[32];
+    HighEval<T, P> hi;
+  };
+  static constexpr size_t kWork =
+      sizeof(Inputs) > sizeof(cx<T>) * 16 * LDU ? sizeof(Inputs) : sizeof(cx<T>) * 16 * LDU;
+  cx<P> Yc[VS], Yn[VS], YN[VS];
+  cx<P> sp[32], fp[32];
+  cx<P> gamma;
+  LowTask<T, P> lo;
+  cx<T> Vc[VS], Vn[VS], u[VS], Ye[VS], dx[VS];
+  cx<T> k[8][VS];
+  cx<T> M[3 * 18 * 8];
+  cx<T> piv[17 * 8];  // pivot rows of the groups: [column][group], right-hand side at 16
+  cx<T> X[16], XU[8], R[3][8], Rd;  // solution; refined residuals and patch residual
+  T cn[16];
+  alignas(16) unsigned char work[kWork];
+  int active, refine;
+  double ck_t[2];  // checkpoint history of the early-retirement features: t at the last two
+  float ck_s[2];   // checkpoints, step sizes there, largest condition estimate since
+  float ck_rmax;
+  unsigned long long cyc[8];  // cycle accounting (lane 0)
+  __device__ __forceinline__ Inputs& inputs() { return *reinterpret_cast<Inputs*>(work); }
+  __device__ __forceinline__ cx<T>* U() { return reinterpret_cast<cx<T>*>(work); }
 };
 
 __device__ __forceinline__ int param_index(int slot, int j) {
@@ -122,326 +188,405 @@ __device__ __forceinline__ int param_index(int slot, int j) {
 template <typename T>
 struct StepOut {
   T ratio;   // condition estimate (pivot ratios of the elimination), +inf if not finite
-  T xnorm2;  // |x|^2 of the (normalised, for tangents) solution
-  T hnorm;   // |H| at the evaluation point (Newton)
-  long long res_cycles;  // cycles the warp spent in the refinement residual (FP32 stage)
+  T xnorm2;  // |x|^2 of the solution (Newton)
+  T hnorm;   // |H| at the evaluation point (Newton, when asked for)
 };
 
-// The team's residual F_j (its three equations) at the point Yd with q(t), all in
-// the point type P (htpysupport.cu:37-48, :64-86): the FP32 stage's corrector uses it
-// as the right-hand side, so its iterates converge in double-float although J and
-// the LU are FP32.
-template <typename P>
-__device__ __forceinline__ void residual_hi(const cx<P>* Yd, const cx<P>* spm, const cx<P>* fpm, cx<P> gamma,
-                                            int j, cx<P>& fI, cx<P>& fII, cx<P>& fIII) {
-  typedef cx<P> cp;
-  const P t = Yd[22].re;
-  const cp g1t = gamma * (P(1) - t);
-  const cp iden = cinv(g1t + cp(t));
-  cp q[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    const int pi = param_index(i, j);
-    q[i] = (g1t * spm[pi] + t * fpm[pi]) * iden;
+// What the evaluation of one path at Y needs: q(t) (and dq/dt, htpysupport.cu:37-62), one
+// parameter per lane; the reciprocals, one per lane; then the hoisted quantities, lane
+// 8 s + g for side s and group g. RESID: frg_group_f's forms (the refinement residual).
+template <bool RESID, typename V>
+__device__ __forceinline__ void eval_prep(const cx<V>* Y, const cx<V>* sp, const cx<V>* fp, cx<V> gamma,
+                                          FrgEvalIn<V>& in, cx<V>* dq, int lane) {
+  const V t = Y[22].re;
+  const cx<V> g1t = gamma * (V(1) - t);
+  const cx<V> iden = cinv(g1t + cx<V>(t));
+  if (lane < NP) {
+    const cx<V> s = sp[lane], f = fp[lane];
+    in.q[lane] = (g1t * s + t * f) * iden;
+    if constexpr (!RESID) dq[lane] = (f - s) * (gamma * (iden * iden));
   }
-  const cp z = Yd[21], z2 = z * z, z3 = z2 * z, U = Yd[13 + j];
-  frg_group_f<P>(Yd[0], Yd[1], Yd[2], Yd[3], Yd[4], Yd[5], Yd[6], Yd[7], Yd[8], Yd[9], Yd[10], Yd[11],
-                      Yd[12], Yd[13], z, cinv(Yd[4] - Yd[1]), cinv(Yd[6] - Yd[2]), cinv(Yd[11] - Yd[8]),
-                      cinv(Yd[13] - Yd[9]), z2, z3, q[0], q[1], U, cinv(U), q[2], q[3], q[4], q[5], fI, fII, fIII);
+  const int ea = lane == 8 ? 4 : lane == 9 ? 6 : lane == 10 ? 11 : 13;   // F, H, Fc, Hc
+  const int eb = lane == 8 ? 1 : lane == 9 ? 2 : lane == 10 ? 8 : 9;     // B, C, Bc, Cc
+  if (lane < 7 || (lane >= 8 && lane < 12)) {
+    const cx<V> b = lane < 7 ? Y[14 + lane] : Y[ea] - Y[eb];
+    const cx<V> ib = cinv(b);
+    if (lane < 7) in.iU[lane] = ib; else in.e[lane - 8] = ib;
+  }
+  const cx<V> z = Y[21];
+  const cx<V> z2 = z * z;
+  const cx<V> z3 = z2 * z;
+  if (lane == 0) { in.z2 = z2; in.z3 = z3; }
+  __syncwarp();
+  if (lane < 16 && (lane & 7) < 7) {
+    const int s = lane >> 3, g = lane & 7;
+    const cx<V>* L = Y + 7 * s;  // A, B, C, D, F, G, H of this side
+    const cx<V> e1 = in.e[2 * s], e2 = in.e[2 * s + 1];
+    const cx<V> P0 = in.q[8 * s], Pj = in.q[8 * s + 1 + g], Qj = in.q[15 + 7 * s + 1 + g];
+    const cx<V> pz = P0 * z, fpz = L[4] - pz, hpz = L[6] - pz;
+    const cx<V> bd = L[1] - L[3], ebd = e1 * bd, cg = L[2] - L[5], ecg = e2 * cg;
+    const cx<V> v = fpz * ebd - hpz * ecg, ac = L[0] - L[2];
+    const cx<V> pjz = Pj * z, ap = L[0] - pjz, bp = L[1] - pjz, qa = Qj * ac, aq = ap - qa;
+    in.sb[s][FRG_IN_PJZ][g] = pjz;
+    in.sb[s][FRG_IN_AP][g] = ap;
+    in.sb[s][FRG_IN_BP][g] = bp;
+    in.sb[s][FRG_IN_QA][g] = qa;
+    in.sb[s][FRG_IN_AQ][g] = aq;
+    if constexpr (RESID) {
+      in.sb[s][FRG_IN_W][g] = L[1] + qa - L[0] + bp * ebd - ecg * aq;
+    } else {
+      const cx<V> eaq = e2 * aq;
+      in.sb[s][FRG_IN_EAQ][g] = eaq;
+      in.sb[s][FRG_IN_W][g] = L[1] - L[0] + qa + bp * ebd - cg * eaq;
+    }
+    if (g == 0) {
+      cx<V>* o = in.sa[s];
+      o[FRG_IN_PZ] = pz;   o[FRG_IN_FP] = fpz;  o[FRG_IN_HP] = hpz;
+      o[FRG_IN_BD] = bd;   o[FRG_IN_EBD] = ebd; o[FRG_IN_CG] = cg;
+      o[FRG_IN_ECG] = ecg; o[FRG_IN_V] = v;     o[FRG_IN_AC] = ac;
+    }
+  }
 }
 
-// One step of the dense phase over a window of W columns: the current pivot column
-// is index 0; rows shift one column left as they are eliminated, so a rolled loop
-// needs no dynamic register indexing. The pivot row (final once chosen) goes to S.U.
-template <typename T, int W, typename P>
-__device__ __forceinline__ void lu_window_step(Smem<T, P>& S, int k, int g, cx<T>* R0, cx<T>& R0r, cx<T>* R1,
-                                               cx<T>& R1r, bool& used0, bool& used1, T& pmax, T& pmin) {
-  const unsigned FULL = 0xffffffffu;
-  const cx<T> zero(T(0));
-  const T v0 = used0 ? T(-1) : cnorm2(R0[0]);
-  const T v1 = used1 ? T(-1) : cnorm2(R1[0]);
+// u . Y over the first n entries in the point type: lane g of each group of 8 adds its
+// entries g, g + 8, g + 16 in turn, then the group sums (htpysupport.cu:9-34, :446).
+template <typename T, typename P>
+__device__ __forceinline__ cx<P> patch_dot(const cx<T>* u, const cx<P>* Y, int n, int g, unsigned mask) {
+  cx<P> d(P(0));
+  for (int e = g; e < n; e += TEAM) d = cfma(cx<P>(u[e]), Y[e], d);
+  return cx<P>(team_sum(mask, d.re), team_sum(mask, d.im));
+}
+
+// 1 / max(|re|, |im|) of the projective patch, its row's scale in every step
+template <typename T>
+__device__ __forceinline__ T patch_scale(const cx<T>* u, int lane) {
+  MaxAbs<T> m;
+  if (lane < NY) m.take(u[lane]);
+  for (int off = 16; off >= 1; off >>= 1) m.across(off);
+  return T(1) / m.value();
+}
+
+// Row with the largest v (ties: the lowest), v >= 0 or -1 for used rows; lanes 16 h + r
+// hold row r's value for h = 0 and 1. Infinite and NaN candidates take the comparisons one
+// by one, as lane 0 sees them.
+template <typename T>
+__device__ __noinline__ int pivot_row_nonfinite(T v, int r) {
+  const T v0 = __shfl_sync(FULL, v, r & ~1), v1 = __shfl_sync(FULL, v, r | 1);
   T bv = v0 >= v1 ? v0 : v1;
-  int bk = 2 * g + (v0 >= v1 ? 0 : 1);
-#pragma unroll
-  for (int off = 4; off >= 1; off >>= 1) {
-    const T ov = shfl_xor(FULL, bv, off);
-    const int ok = shfl_xor(FULL, bk, off);
+  int bk = (r & ~1) + (v0 >= v1 ? 0 : 1);
+  for (int off = 8; off >= 2; off >>= 1) {
+    const T ov = __shfl_xor_sync(FULL, bv, off);
+    const int ok = __shfl_xor_sync(FULL, bk, off);
     if (ov > bv || (ov == bv && ok < bk)) { bv = ov; bk = ok; }
   }
-  const int pl = bk >> 1, ps = bk & 1;
-  if (g == pl) { if (ps) used1 = true; else used0 = true; }
-  cx<T> prow[W];
-#pragma unroll
-  for (int c = 0; c < W; ++c) prow[c] = shfl(FULL, ps ? R1[c] : R0[c], pl);
-  const cx<T> prhs = shfl(FULL, ps ? R1r : R0r, pl);
-  const cx<T> ip = cinv(prow[0]);
-  if (g == 0) {  // the diagonal keeps the pivot's reciprocal for the back substitution
-    S.U[k][k] = ip;
-#pragma unroll
-    for (int c = 1; c < W; ++c)
-      if (k + c < 16) S.U[k][k + c] = prow[c];
-    S.Urhs[k] = prhs;
+  return __shfl_sync(FULL, bk, 0);
+}
+__device__ __forceinline__ int pivot_row(float v, int r) {
+  const int key = __float_as_int(v);
+  const int m = __reduce_max_sync(FULL, key);
+  if (m >= 0x7f800000) return pivot_row_nonfinite(v, r);
+  return __ffs(__ballot_sync(FULL, key == m) & 0xffffu) - 1;
+}
+__device__ __forceinline__ int pivot_row(double v, int r) {
+  const int hi = __double2hiint(v);
+  const unsigned lo = (unsigned)__double2loint(v);
+  const int m = __reduce_max_sync(FULL, hi);
+  if (m >= 0x7ff00000) return pivot_row_nonfinite(v, r);
+  unsigned cand = __ballot_sync(FULL, hi == m) & 0xffffu;
+  if (cand & (cand - 1)) {
+    const unsigned ml = __reduce_max_sync(FULL, hi == m ? lo : 0u);
+    cand = __ballot_sync(FULL, hi == m && lo == ml) & 0xffffu;
   }
-  const T pa = cnorm2(prow[0]);  // squared pivot magnitude
-  pmax = fmax(pmax, pa);
-  pmin = fmin(pmin, pa);
-  const cx<T> l0 = used0 ? zero : R0[0] * ip;
-  const cx<T> l1 = used1 ? zero : R1[0] * ip;
-#pragma unroll
-  for (int c = 0; c + 1 < W; ++c) {
-    R0[c] = cfms(R0[c + 1], l0, prow[c + 1]);
-    R1[c] = cfms(R1[c + 1], l1, prow[c + 1]);
-  }
-  R0[W - 1] = zero;
-  R1[W - 1] = zero;
-  R0r = cfms(R0r, l0, prhs);
-  R1r = cfms(R1r, l1, prhs);
+  return __ffs(cand) - 1;
 }
 
-// One linear-system step, executed convergently by the whole warp (full-mask
-// shuffles inside). Each team evaluates at its S.Ye:
+// Four steps k0..k0 + 3 of the dense elimination, W columns per lane. Lane 16 h + r holds
+// row r's remaining columns c = h mod 2 (the right-hand side is column 16) from index 0;
+// a step drops the pivot column, so the lanes that held it move their window up one. The
+// pivot row goes to U and every lane reads it back from there; U[k][k] keeps the pivot's
+// reciprocal. Windows of 8, 6, 4 and 2 columns for four steps each: 80 complex updates per
+// lane where 72 are needed, in code that stays small.
+template <int W, typename T>
+__device__ __forceinline__ void lu_stage(cx<T>* U, int k0, int lane, cx<T>* R, bool& used, T& pmax, T& pmin) {
+  const int h = lane >> 4, r = lane & 15;
+#pragma unroll 1
+  for (int k = k0; k < k0 + 4; ++k) {
+    const bool own = h == (k & 1);
+    const cx<T> e = warp_shfl(R[0], ((k & 1) << 4) + r);  // this row's entry in column k
+    const T v = used ? T(-1) : cnorm2(e);
+    const int pr = pivot_row(v, r);
+    cx<T>* Uk = U + k * LDU + k + 1 + ((h ^ (k + 1)) & 1);
+    cx<T> X[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) X[i] = own ? R[i + 1] : R[i];
+    if (r == pr) {
+      used = true;
+#pragma unroll
+      for (int i = 0; i < W; ++i) Uk[2 * i] = X[i];
+    }
+    const T pa = __shfl_sync(FULL, v, pr);
+    const cx<T> ip = cinv_norm(warp_shfl(e, pr), pa);
+    if (lane == 0) U[k * LDU + k] = ip;
+    pmax = max_mag(pmax, pa);
+    pmin = min_mag(pmin, pa);
+    const cx<T> l = used ? cx<T>(T(0)) : e * ip;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < W; ++i) R[i] = cfms(X[i], l, Uk[2 * i]);
+  }
+}
+
+// Back substitution, column by column; lane r holds the right-hand side of pivot row r.
+// FP32: both halves of the warp do the same.
+__device__ __forceinline__ void back_substitute(const cx<float>* U, cx<float>* X, int lane) {
+  const int r = lane & 15;
+  cx<float> rb = U[r * LDU + 16];
+  const cx<float> ip = U[r * LDU + r];
+#pragma unroll 1
+  for (int k = 15; k >= 0; --k) {
+    const cx<float> xk = warp_shfl(rb * ip, k);
+    if (lane == 0) X[k] = xk;
+    if (r < k) rb = cfms(rb, U[r * LDU + k], xk);
+  }
+}
+// FP64: lanes 0..15 hold the real parts, lanes 16..31 the imaginary parts, which halves
+// the FP64 instructions of the chain (4 per column; the operations and their order are
+// those of the complex product and cfms).
+__device__ __forceinline__ void back_substitute(const cx<double>* U, cx<double>* X, int lane) {
+  const int r = lane & 15;
+  const bool im = lane >= 16;
+  double rb = im ? U[r * LDU + 16].im : U[r * LDU + 16].re;
+  const cx<double> ip = U[r * LDU + r];
+  const double pa = im ? ip.im : ip.re, pb = im ? ip.re : -ip.im;
+#pragma unroll 1
+  for (int k = 15; k >= 0; --k) {
+    const cx<double> u = U[r * LDU + k];
+    const double ot = __shfl_xor_sync(FULL, rb, 16);
+    const double are = im ? ot : rb, aim = im ? rb : ot;
+    const double m = fma(are, pa, __dmul_rn(aim, pb));
+    const double xr = __shfl_sync(FULL, m, k), xi = __shfl_sync(FULL, m, 16 + k);
+    if (lane == 0) X[k] = cx<double>(xr, xi);
+    if (r < k) rb = fma(im ? -u.im : u.im, im ? xr : xi, fma(-u.re, im ? xi : xr, rb));
+  }
+}
+
+// U_j from the group's pivot row, lane g of each group of 8 (every such lane returns it)
+__device__ __forceinline__ cx<float> solve_u(const cx<float>* piv, const cx<float>* X, cx<float> ipu, int lane) {
+  const int g = lane & 7;
+  cx<float> xu = piv[16 * 8 + g];
+#pragma unroll 4
+  for (int c = 0; c < 16; ++c) xu = cfms(xu, piv[c * 8 + g], X[c]);
+  return xu * ipu;
+}
+__device__ __forceinline__ cx<double> solve_u(const cx<double>* piv, const cx<double>* X, cx<double> ipu, int lane) {
+  const int g = lane & 7;
+  const bool im = lane & 8;
+  double xu = im ? piv[16 * 8 + g].im : piv[16 * 8 + g].re;
+#pragma unroll 4
+  for (int c = 0; c < 16; ++c) {
+    const cx<double> p = piv[c * 8 + g], x = X[c];
+    xu = fma(im ? -p.im : p.im, im ? x.re : x.im, fma(-p.re, im ? x.im : x.re, xu));
+  }
+  const double ot = __shfl_xor_sync(FULL, xu, 8);
+  return (im ? cx<double>(ot, xu) : cx<double>(xu, ot)) * ipu;
+}
+
+// One linear-system solve of the warp's path from the group rows in S.M, evaluated at
+// S.Ye:
 //   tangent (newton = false): [JH; W] x = e_23 with W = the velocity patch Wsrc,
 //     then normalised to unit length with real dt/ds (or dt = 1 when tstep),
 //     Im(dt) = 0 (htpysupport.cu:237-299);
 //   Newton (newton = true): [JH; e_t] x = [-H; tgoal - t] (htpysupport.cu:427-477),
-//     H at the FP64 point S.YN; when T is float, H is evaluated in FP64 if `hires`
-//     and in FP32 (at the rounded point) otherwise.
-// The solution is written to dst[0..22] (shared memory).
+//     H from S.M, or from the refined residuals S.R, S.Rd at S.YN when `hires`.
+// su = patch_scale(S.u). The solution is written to dst[0..22]. `newton`, `tstep`,
+// `hires` and the results are the same in every lane.
 template <typename T, typename P>
-__device__ __forceinline__ StepOut<T> linear_step(Smem<T, P>& S, const cx<T>* Wsrc, cx<T>* dst, bool newton,
-                                                  bool tstep, T tgoal, const LaneParams<T>& lp,
-                                                  const cx<P>* fpm_hi, cx<P> gamma_hi, int g, bool hires) {
-  const unsigned FULL = 0xffffffffu;
+__device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsrc, cx<T>* dst, bool newton,
+                                                 bool tstep, T tgoal, T su, bool hires, bool want_ratio,
+                                                 bool want_hnorm, int lane) {
+  const int g = lane & 7, q = lane >> 3;
   const bool grp = g < 7;
-  const int j = grp ? g + 1 : 7;
+  const int jj = grp ? g : 6;
   const cx<T> zero(T(0));
-  constexpr bool LOWP = sizeof(T) < sizeof(P);
-  // `newton` and `hires` are per team, so reductions inside branches on them use the
-  // team's own mask; everything outside such branches runs on the full warp
-  const unsigned tmask = 0xffu << (threadIdx.x & 24);
+  StepOut<T> out;
 
-  // ---- FP64 residual of the corrector (FP32 stage only)
-  cx<T> hF0 = zero, hF1 = zero, hF2 = zero, hU = zero;
-  T hsq = T(0);
-  long long res_cycles = 0;
-  const long long t_res0 = LOWP ? clock64() : 0;
-  if (LOWP && newton && hires) {
-    cx<P> fI, fII, fIII;
-    residual_hi<P>(S.YN, S.spm, fpm_hi, gamma_hi, j, fI, fII, fIII);
-    // patch residual u . YN - 1, its 23 terms spread over the team
-    cx<P> d(P(0));
-    for (int e = g; e < 23; e += TEAM) d = cfma(cx<P>(S.u[e]), S.YN[e], d);
-    d = cx<P>(team_sum(tmask, d.re), team_sum(tmask, d.im)) - cx<P>(P(1));
-    hF0 = cx<T>(fI); hF1 = cx<T>(fII); hF2 = cx<T>(fIII); hU = cx<T>(d);
-    hsq = grp ? T(cnorm2(hF0) + cnorm2(hF1) + cnorm2(hF2)) : T(cnorm2(hU));
-  }
-  if (LOWP) res_cycles = clock64() - t_res0;
-
-  // ---- evaluation point and parameters q(t), dq/dt (htpysupport.cu:37-62)
-  const cx<T> A = S.Ye[0], B = S.Ye[1], C = S.Ye[2], D = S.Ye[3], F = S.Ye[4], G = S.Ye[5], H = S.Ye[6];
-  const cx<T> Ac = S.Ye[7], Bc = S.Ye[8], Cc = S.Ye[9], Dc = S.Ye[10], Fc = S.Ye[11], Gc = S.Ye[12],
-              Hc = S.Ye[13];
-  const cx<T> z = S.Ye[21];
-  const T t = S.Ye[22].re;
-  const cx<T> U = S.Ye[13 + j];
-  cx<T> q[6], dq[6];
-  {
-    const cx<T> g1t = lp.gamma * (T(1) - t);
-    const cx<T> iden = cinv(g1t + cx<T>(t));
-    const cx<T> gid2 = lp.gamma * (iden * iden);
+  // ---- the group's three rows, columns q, q + 4, q + 8, q + 12, then U_j and the rhs
+  cx<T> r0[6], r1[6], r2[6];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      q[i] = (g1t * lp.sp[i] + t * lp.fp[i]) * iden;
-      dq[i] = (lp.fp[i] - lp.sp[i]) * gid2;
+  for (int i = 0; i < 5; ++i) {
+    const int c = i < 4 ? q + 4 * i : 16;
+    r0[i] = S.M[c * 8 + jj];
+    r1[i] = S.M[(18 + c) * 8 + jj];
+    r2[i] = S.M[(36 + c) * 8 + jj];
+  }
+  r0[5] = r1[5] = r2[5] = zero;
+  cx<T> hU = zero;
+  out.hnorm = T(0);
+  if (newton) {
+    cx<T> f0, f1, f2;
+    if (hires) {
+      f0 = S.R[0][jj]; f1 = S.R[1][jj]; f2 = S.R[2][jj];
+      hU = S.Rd;
+    } else {
+      f0 = S.M[17 * 8 + jj]; f1 = S.M[(18 + 17) * 8 + jj]; f2 = S.M[(36 + 17) * 8 + jj];
+      hU = patch_dot<T, T>(S.u, S.Ye, NY, g, FULL) - cx<T>(T(1));
+    }
+    r0[5] = -f0; r1[5] = -f1; r2[5] = -f2;
+    if (want_hnorm) {
+      const T hsq = grp ? cnorm2(f0) + cnorm2(f1) + cnorm2(f2) : cnorm2(hU);
+      out.hnorm = sqrt(team_sum(FULL, hsq));
     }
   }
-  // ---- the group's equations, derivatives and t-column (generated code)
-  FrgGroupOut<T> o;
+  // ---- row scaling by 1/max(|re|,|im|) (htpysupport.cu:259-277, :446-471); the three
+  //      reciprocals in one division, row q on lane 8 q + g
   {
-    const cx<T> z2 = z * z, z3 = z2 * z;
-    frg_group_eval<T>(A, B, C, D, F, G, H, Ac, Bc, Cc, Dc, Fc, Gc, Hc, z, cinv(F - B), cinv(H - C),
-                      cinv(Fc - Bc), cinv(Hc - Cc), z2, z3, q[0], q[1], dq[0], dq[1], U, cinv(U), q[2], q[3],
-                      q[4], q[5], dq[2], dq[3], dq[4], dq[5], o);
-  }
-  const bool lores_h = !LOWP || !hires;  // H from the working-precision evaluation
-  if (lores_h) {
-    hF0 = o.fI; hF1 = o.fII; hF2 = o.fIII;
-    hsq = grp ? cnorm2(o.fI) + cnorm2(o.fII) + cnorm2(o.fIII) : T(0);
-  }
-  // rows in local column order: 0..13 links, 14 Z0, 15 t, 16 U_j, 17 rhs
-  cx<T> r0[18], r1[18], r2[18];
+    MaxAbs<T> m0, m1, m2;
 #pragma unroll
-  for (int c = 0; c < 18; ++c) { r0[c] = zero; r1[c] = zero; r2[c] = zero; }
-  r0[0] = o.dI[0]; r0[2] = o.dI[1]; r0[6] = o.dI[2]; r0[7] = o.dI[3]; r0[9] = o.dI[4]; r0[13] = o.dI[5];
-  r0[16] = o.dI[6]; r0[14] = o.dI[7]; r0[15] = o.tI;
-  r1[1] = o.dII[0]; r1[4] = o.dII[1]; r1[8] = o.dII[2]; r1[11] = o.dII[3];
-  r1[16] = o.dII[4]; r1[14] = o.dII[5]; r1[15] = o.tII;
+    for (int i = 0; i < 5; ++i) { m0.take(r0[i]); m1.take(r1[i]); m2.take(r2[i]); }
+    m0.across(8); m1.across(8); m2.across(8);
+    m0.across(16); m1.across(16); m2.across(16);
+    const T s = T(1) / (q == 0 ? m0.value() : (q == 1 ? m1.value() : m2.value()));
+    const T s0 = __shfl_sync(FULL, s, g), s1 = __shfl_sync(FULL, s, 8 + g), s2 = __shfl_sync(FULL, s, 16 + g);
 #pragma unroll
-  for (int c = 0; c < 14; ++c) r2[c] = o.dIII[c];
-  r2[16] = o.dIII[14]; r2[14] = o.dIII[15]; r2[15] = o.tIII;
-  if (newton) { r0[17] = -hF0; r1[17] = -hF1; r2[17] = -hF2; }
-  // row scaling by 1/max(|re|,|im|) (htpysupport.cu:259-277, :446-471)
-  {
-    T m0 = T(0), m1 = T(0), m2 = T(0);
-#pragma unroll
-    for (int c = 0; c < 17; ++c) {
-      m0 = fmax(m0, fmax(tabs(r0[c].re), tabs(r0[c].im)));
-      m1 = fmax(m1, fmax(tabs(r1[c].re), tabs(r1[c].im)));
-      m2 = fmax(m2, fmax(tabs(r2[c].re), tabs(r2[c].im)));
-    }
-    const T s0 = T(1) / m0, s1 = T(1) / m1, s2 = T(1) / m2;
-#pragma unroll
-    for (int c = 0; c < 18; ++c) { r0[c] = s0 * r0[c]; r1[c] = s1 * r1[c]; r2[c] = s2 * r2[c]; }
+    for (int i = 0; i < 6; ++i) { r0[i] = s0 * r0[i]; r1[i] = s1 * r1[i]; r2[i] = s2 * r2[i]; }
   }
   // ---- eliminate U_j inside the group: partial pivoting among its three rows
-  const T a0 = cnorm2(r0[16]), a1 = cnorm2(r1[16]), a2 = cnorm2(r2[16]);
+  const T a0 = cnorm2(r0[4]), a1 = cnorm2(r1[4]), a2 = cnorm2(r2[4]);
   const int p = (a0 >= a1 && a0 >= a2) ? 0 : (a1 >= a2 ? 1 : 2);
-  cx<T> piv[18], R0[16], R1[16], R0r, R1r;
+  const T ap = p == 0 ? a0 : (p == 1 ? a1 : a2);
+  cx<T> piv[6], R0[5], R1[5];  // [4] of R0, R1: the right-hand side
 #pragma unroll
-  for (int c = 0; c < 18; ++c) piv[c] = p == 0 ? r0[c] : (p == 1 ? r1[c] : r2[c]);
-  cx<T> ipu = cinv(piv[16]);
+  for (int i = 0; i < 6; ++i) piv[i] = p == 0 ? r0[i] : (p == 1 ? r1[i] : r2[i]);
+  cx<T> ipu = cinv_norm(piv[4], ap);
   {
-    const cx<T> la = (p == 0 ? r1[16] : r0[16]) * ipu;
-    const cx<T> lb = (p == 2 ? r1[16] : r2[16]) * ipu;
+    const cx<T> la = (p == 0 ? r1[4] : r0[4]) * ipu;
+    const cx<T> lb = (p == 2 ? r1[4] : r2[4]) * ipu;
 #pragma unroll
-    for (int c = 0; c < 17; ++c) {
-      const int cc = c < 16 ? c : 17;
+    for (int i = 0; i < 5; ++i) {
+      const int cc = i < 4 ? i : 5;
       const cx<T> xa = p == 0 ? r1[cc] : r0[cc];
       const cx<T> xb = p == 2 ? r1[cc] : r2[cc];
-      const cx<T> ya = cfms(xa, la, piv[cc]);
-      const cx<T> yb = cfms(xb, lb, piv[cc]);
-      if (c < 16) { R0[c] = ya; R1[c] = yb; } else { R0r = ya; R1r = yb; }
+      R0[i] = cfms(xa, la, piv[cc]);
+      R1[i] = cfms(xb, lb, piv[cc]);
     }
   }
-  // ---- patch rows (lane 7) and the folding of every group's pivot row into them
-  const cx<T>* u = S.u;
-  T su = T(0);
-  for (int e = g; e < 23; e += TEAM) su = fmax(su, fmax(tabs(u[e].re), tabs(u[e].im)));
-  su = T(1) / team_max(FULL, su);
-  const T tdiff = tgoal - t;
-  if (lores_h && newton) {  // patch residual u . Ye - 1, its 23 terms spread over the team
-    cx<T> d(T(0));
-    for (int e = g; e < 23; e += TEAM) d = cfma(u[e], S.Ye[e], d);
-    hU = cx<T>(team_sum(tmask, d.re), team_sum(tmask, d.im)) - cx<T>(T(1));
-  }
-  if (!grp) {
-    if (lores_h) hsq = cnorm2(hU);
-    ipu = zero;
-  }
-  const cx<T> mu = (su * u[13 + j]) * ipu;
-  const cx<T> mw = newton ? zero : Wsrc[13 + j] * ipu;
-  cx<T> Su[17], Sw[17];
+  if (grp) {
 #pragma unroll
-  for (int c = 0; c < 17; ++c) {
-    const cx<T> pc = piv[c < 16 ? c : 17];
-    Su[c] = mu * pc;
-    Sw[c] = mw * pc;
+    for (int i = 0; i < 4; ++i) S.piv[(q + 4 * i) * 8 + g] = piv[i];
+    if (q == 0) S.piv[16 * 8 + g] = piv[5];
   }
+  // ---- the folding of every group's pivot row into the patch rows (lanes g = 7 repeat
+  //      group 7's rows with weight zero and then hold the patch rows). A Newton step's
+  //      t-selector row has no entry to fold.
+  if (!grp) ipu = zero;
+  {
+    const cx<T> mu = (su * S.u[14 + jj]) * ipu;
+    cx<T> Su[5], Sw[5];
 #pragma unroll
-  for (int c = 0; c < 17; ++c) {
+    for (int i = 0; i < 5; ++i) { Su[i] = mu * piv[i < 4 ? i : 5]; Sw[i] = zero; }
 #pragma unroll
-    for (int off = 4; off >= 1; off >>= 1) {
-      Su[c] += shfl_xor(FULL, Su[c], off);
-      Sw[c] += shfl_xor(FULL, Sw[c], off);
+    for (int i = 0; i < 5; ++i) Su[i] = cx<T>(team_sum(FULL, Su[i].re), team_sum(FULL, Su[i].im));
+    if (!newton) {
+      const cx<T> mw = Wsrc[14 + jj] * ipu;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) Sw[i] = mw * piv[i < 4 ? i : 5];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) Sw[i] = cx<T>(team_sum(FULL, Sw[i].re), team_sum(FULL, Sw[i].im));
+    }
+    if (!grp) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = q + 4 * i, st = gstate(c);
+        R0[i] = su * S.u[st] - Su[i];
+        R1[i] = (newton ? (c == 15 ? cx<T>(T(1)) : zero) : Wsrc[st]) - Sw[i];
+      }
+      R0[4] = (newton ? -mul_rn(su, hU) : zero) - Su[4];
+      R1[4] = (newton ? cx<T>(tgoal - S.Ye[22].re) : cx<T>(T(1))) - Sw[4];
     }
   }
-  if (!grp) {
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      R0[c] = su * u[gstate(c)] - Su[c];
-      R1[c] = (newton ? (c == 15 ? cx<T>(T(1)) : zero) : Wsrc[gstate(c)]) - Sw[c];
-    }
-    R0r = (newton ? -(su * hU) : zero) - Su[16];
-    R1r = (newton ? cx<T>(tdiff) : cx<T>(T(1))) - Sw[16];
-  }
-
   // ---- re-scale the 16 dense rows (max(|re|,|im|) = 1): eliminating U_j can shrink a
   //      group row by cancellation, and unequal rows would mislead both the pivot
   //      choice and the pivot-ratio condition estimate (with the re-scaling the ratio
-  //      tracks the reference's 23 x 23 row-scaled elimination)
+  //      tracks the reference's 23 x 23 row-scaled elimination). Rows 2 g and 2 g + 1 to
+  //      the dense system.
+  cx<T>* U = S.U();
   {
-    T m0 = T(0), m1 = T(0);
+    MaxAbs<T> m0, m1;
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      m0 = fmax(m0, fmax(tabs(R0[c].re), tabs(R0[c].im)));
-      m1 = fmax(m1, fmax(tabs(R1[c].re), tabs(R1[c].im)));
+    for (int i = 0; i < 4; ++i) { m0.take(R0[i]); m1.take(R1[i]); }
+    m0.across(8); m1.across(8);
+    m0.across(16); m1.across(16);
+    const T s = T(1) / ((q & 1) ? m1.value() : m0.value());
+    const T s0 = __shfl_sync(FULL, s, g), s1 = __shfl_sync(FULL, s, 8 + g);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      R0[i] = s0 * R0[i];
+      R1[i] = s1 * R1[i];
+      if (i < 4 || q == 0) {
+        const int c = i < 4 ? q + 4 * i : 16;
+        U[(2 * g) * LDU + c] = R0[i];
+        U[(2 * g + 1) * LDU + c] = R1[i];
+      }
     }
-    const T s0 = T(1) / m0, s1 = T(1) / m1;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) { R0[c] = s0 * R0[c]; R1[c] = s1 * R1[c]; }
-    R0r = s0 * R0r;
-    R1r = s1 * R1r;
   }
-  // ---- dense 16 x 16 LU with partial pivoting across the team: 8 steps over a
-  //      16-wide window, then 8 over the remaining 8 columns
-  bool used0 = false, used1 = false;
+  __syncwarp();
+  // ---- dense 16 x 16 LU with partial pivoting across the lanes
   T pmax = T(0), pmin = T(3.0e38);
-#pragma unroll 1
-  for (int k = 0; k < 8; ++k) lu_window_step<T, 16, P>(S, k, g, R0, R0r, R1, R1r, used0, used1, pmax, pmin);
   {
-    cx<T> Q0[8], Q1[8];
+    const int h = lane >> 4, r = lane & 15;
+    cx<T> R[9];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) { Q0[c] = R0[c]; Q1[c] = R1[c]; }
-#pragma unroll 1
-    for (int k = 8; k < 16; ++k) lu_window_step<T, 8, P>(S, k, g, Q0, R0r, Q1, R1r, used0, used1, pmax, pmin);
+    for (int i = 0; i < 8; ++i) R[i] = U[r * LDU + h + 2 * i];
+    R[8] = h == 0 ? U[r * LDU + 16] : zero;
+    __syncwarp();
+    bool used = false;
+    lu_stage<8>(U, 0, lane, R, used, pmax, pmin);
+    lu_stage<6>(U, 4, lane, R, used, pmax, pmin);
+    lu_stage<4>(U, 8, lane, R, used, pmax, pmin);
+    lu_stage<2>(U, 12, lane, R, used, pmax, pmin);
   }
   __syncwarp();
-  // ---- back substitution, column by column; lane g keeps the right-hand sides of
-  //      pivot rows g and g + 8
-  cx<T> rb0 = S.Urhs[g], rb1 = S.Urhs[g + 8];
+  back_substitute(U, S.X, lane);
   __syncwarp();
-#pragma unroll 1
-  for (int k = 15; k >= 0; --k) {
-    const cx<T> mine = ((k >> 3) ? rb1 : rb0) * S.U[k][k];
-    const cx<T> xk = shfl(FULL, mine, k & 7);
-    if (g == 0) S.Urhs[k] = xk;
-    if (g < k) rb0 = cfms(rb0, S.U[g][k], xk);
-    if (g + 8 < k) rb1 = cfms(rb1, S.U[g + 8][k], xk);
-  }
+  const cx<T> xu = solve_u(S.piv, S.X, ipu, lane);
+  if (lane < 16) S.cn[lane] = cnorm2(S.X[lane]);
+  if (lane < 8) S.XU[lane] = xu;
   __syncwarp();
-  cx<T> xg[16];
+  T n2 = T(0);
 #pragma unroll
-  for (int c = 0; c < 16; ++c) xg[c] = S.Urhs[c];
-  // ---- U_j from the group's pivot row
-  cx<T> xu = piv[17];
-#pragma unroll
-  for (int c = 0; c < 16; ++c) xu = cfms(xu, piv[c], xg[c]);
-  xu = xu * ipu;
+  for (int c = 0; c < 16; ++c) n2 += S.cn[c];
+  n2 += team_sum(FULL, grp ? cnorm2(xu) : T(0));
   // ---- condition estimate: the larger of the dense phase's pivot ratio and the
   //      worst group amplification 1/|u_jj| (a group's pivot row is row-scaled, so its
   //      largest entry is about 1, and U_j's error grows like eps / |u_jj|). A
   //      non-finite solution (zero or non-finite pivot) makes it infinite.
-  T ratio;
-  {
-    const T ig = grp ? T(1) / cnorm2(piv[16]) : T(0);
-    ratio = sqrt(fmax(pmax / pmin, team_max(FULL, ig)));
-  }
-  // ---- normalisation and output
-  T n2 = T(0);
-#pragma unroll
-  for (int c = 0; c < 16; ++c) n2 += cnorm2(xg[c]);
-  n2 += team_sum(FULL, grp ? cnorm2(xu) : T(0));
-  StepOut<T> out;
-  out.res_cycles = res_cycles;
-  out.hnorm = sqrt(team_sum(FULL, hsq));
-  out.ratio = (n2 - n2 == T(0)) ? ratio : T(INFINITY);  // n2 - n2 is NaN iff n2 is not finite
-  if (!newton) {
-    const cx<T> xt = xg[15];
-    cx<T> sc;
-    if (!tstep) sc = cx<T>(xt.re, -xt.im) * (T(1) / (sqrt(cnorm2(xt)) * sqrt(n2)));
-    else sc = cinv(xt);
-#pragma unroll
-    for (int c = 0; c < 16; ++c) xg[c] = sc * xg[c];
-    xu = sc * xu;
-    xg[15].im = T(0);
-    n2 = n2 * cnorm2(sc);
+  out.ratio = T(0);
+  if (want_ratio) {
+    const T ig = grp ? T(1) / ap : T(0);
+    const T ratio = sqrt(fmax(pmax / pmin, team_max(FULL, ig)));
+    out.ratio = (n2 - n2 == T(0)) ? ratio : T(INFINITY);  // n2 - n2 is NaN iff n2 is not finite
   }
   out.xnorm2 = n2;
+  // ---- normalisation and output, one entry per lane
+  cx<T> sc(T(1));
+  if (!newton) {
+    const cx<T> xt = S.X[15];
+    if (!tstep) {
+      const T nr = sqrt((lane & 1) ? n2 : cnorm2(xt));
+      sc = cx<T>(xt.re, -xt.im) * (T(1) / (__shfl_sync(FULL, nr, 0) * __shfl_sync(FULL, nr, 1)));
+    } else {
+      sc = cinv(xt);
+    }
+  }
+  if (lane < NY) {
+    cx<T> x = lane < 14 ? S.X[lane] : (lane < 21 ? S.XU[lane - 14] : S.X[lane - 7]);
+    if (!newton) {
+      x = sc * x;
+      if (lane == 22) x.im = T(0);
+    }
+    dst[lane] = x;
+  }
   __syncwarp();
-  if (grp) dst[13 + j] = xu;
-#pragma unroll
-  for (int c = 0; c < 16; ++c)
-    if ((c & 7) == g) dst[gstate(c)] = xg[c];
   return out;
 }
 

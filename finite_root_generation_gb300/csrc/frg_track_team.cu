@@ -1,14 +1,14 @@
-// Warp-cooperative path-tracking kernels: one 8-lane team per path, 4 paths per
-// warp, the linear algebra register-resident (frg_team.cuh) and the path state in
-// shared memory.
+// Warp-cooperative path-tracking kernels: one path per warp, four paths per block, the
+// system evaluated by the block and solved by the path's warp (frg_team.cuh), the path
+// state in shared memory.
 //
 // The control flow is the reference's TrackPath (htpytrack.cu:33-220) with
 // DormandPrince65 (rungekutta.cu:3-123) and Newton (htpysupport.cu:407-494),
 // restated as the same state machine as the one-thread-per-path kernel
 // (frg_track.cu), with identical decisions, tolerances, counters and random draws.
-// Every trip of the loop runs one warp-convergent linear step for all four teams
-// (the expensive part), then each team's control transitions with team-masked
-// shuffles; vector updates are spread over the team's lanes (element e on lane e % 8).
+// Every trip of the loop the four warps evaluate their four systems together (two block
+// barriers) and each warp then solves its own and makes its transition; all control
+// variables are the same in a warp's lanes, and vector entry e lives on lane e.
 //
 // Modes as in frg_track.cu: MODE_PLAIN (FP64 from start to root), MODE_LO (FP32
 // stage; every path is handed to the FP64 kernel, either to continue or, when it
@@ -112,7 +112,7 @@ template <> __device__ __forceinline__ cx<float> gamma_of<float>(const TrackArgs
 // (frg.cu:44-46, :60), canonical cognate (frgkinematics.cu:227-285, frg.cu:63-65), the
 // row-scaled residual of the target system at the root, outputs and counters. id is the
 // path's global index, ti its task-set index.
-__device__ void team_finish(const TrackArgs& a, Smem<double>& S, const cd* Yf, int64_t id, int ti, int code,
+__device__ __noinline__ void team_finish(const TrackArgs& a, Smem<double>& S, const cd* Yf, int64_t id, int ti, int code,
                             int g, unsigned tmask, int n_ivp, int n_newton, int steps) {
   const cd* fpm = a.fpm + (size_t)ti * NP;
   if (a.yfinal)
@@ -257,33 +257,49 @@ __device__ __noinline__ int checkpoint(const TrackArgs& a, const cx<P>* Yc, int6
   return retire;
 }
 
+// Blocks of a launch that take paths, and paths per block. Short queues spread over the
+// SMs: a block's warps sit on the SM's four sub-partitions, so up to four paths share one
+// block (and its evaluation) before a second block joins the SM.
+__device__ __forceinline__ void spread_queue(int64_t nqueue, int sms, int& blocks, int& paths) {
+  int64_t b = nqueue <= (int64_t)sms * PATHS ? (nqueue < sms ? nqueue : sms) : (nqueue + PATHS - 1) / PATHS;
+  b = b < 1 ? 1 : b;
+  b = b < gridDim.x ? b : gridDim.x;
+  const int64_t p = (nqueue + b - 1) / b;
+  blocks = (int)b;
+  paths = (int)(p < PATHS ? p : PATHS);
+}
+
 template <int MODE, typename T, typename P = typename PointOf<T>::type>
-__global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
+__global__ void __launch_bounds__(32 * PATHS, sizeof(T) == 8 ? 2 : 4) team_kernel(TrackArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr bool LO = (MODE == MODE_LO);
-  const unsigned FULL = 0xffffffffu;
+  constexpr bool LOWP = sizeof(T) < sizeof(P);
   const frg_config& c = a.cfg;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane & 7;
-  const unsigned tmask = 0xffu << (lane & 24);
+  const int jg = g < 7 ? g + 1 : 7;
+  const bool el = lane < NY;  // this lane's vector entry exists
   typedef cx<P> cp;
-  Smem<T, P>& S = reinterpret_cast<Smem<T, P>*>(smem_raw)[threadIdx.x >> 3];
+  Smem<T, P>* const paths = reinterpret_cast<Smem<T, P>*>(smem_raw);
+  Smem<T, P>& S = paths[warp];
   {
-    cx<T>* base = reinterpret_cast<cx<T>*>(&S);
-    for (int i = g; i < (int)(sizeof(Smem<T, P>) / sizeof(cx<T>)); i += TEAM) base[i] = cx<T>(T(0));
+    unsigned* base = reinterpret_cast<unsigned*>(&S);
+    for (int i = lane; i < (int)(sizeof(Smem<T, P>) / sizeof(unsigned)); i += 32) base[i] = 0u;
   }
   // The FP32 stage's corrector iterates on FP32 residuals until |dY| falls below
-  // newt_tol_lo (or stops shrinking), then on FP64 residuals to the reference's
-  // newt_tol: an FP32 LU with FP64 residuals converges like FP64 Newton while the
-  // pivot ratio stays below cond_switch.
+  // newt_tol_lo (or stops shrinking), then on residuals in the point type to the
+  // reference's newt_tol: an FP32 LU with accurate residuals converges like FP64 Newton
+  // while the pivot ratio stays below cond_switch.
   const T newt_tol = T(c.newt_tol);
-  const int jg = g < 7 ? g + 1 : 7;
   // what this launch works through: fresh paths, paths resumed in FP32 (lo_list),
   // or paths handed to FP64 (handoff_list)
   const bool lo_resume = LO && a.lo_list != nullptr && !a.carry;
   const int64_t ncarry = (LO && a.carry && a.lo_list != nullptr) ? (int64_t)*a.lo_count : 0;
   const int64_t nqueue = (MODE == MODE_RESUME) ? (int64_t)*a.handoff_count
                          : (lo_resume ? (int64_t)*a.lo_count : ncarry + a.npaths);
+  int use_blocks, use_warps;
+  spread_queue(nqueue, a.sms, use_blocks, use_warps);
+  if ((int)blockIdx.x >= use_blocks) return;
   // A path returns from FP64 to the next round's FP32 kernel after handback_good
   // consecutive well-conditioned solves, or after fp64_segment FP64 solves in this launch
   // (FP64 latency per solve is high on this part, so long FP64 segments set a launch's
@@ -292,35 +308,32 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
   const int kSegment = c.fp64_segment > 0 ? c.fp64_segment : 96;
   constexpr int kMaxBounces = 64;
 
-  LaneParams<T> lp;
+  cx<T> gamma(T(0));
   int64_t id = -1;      // global path index: records, lists, outputs
   int64_t lid = 0;      // index within the path's round: random stream, start values, task
   int ti = 0;           // task-set index (round * ntasks + task): parameters, gamma
   uint64_t pseed = a.seed;
-  T s = T(0), err = T(0), scale = T(0), residual = T(100);
+  T s = T(0), err = T(0), scale = T(0), residual = T(100), su = T(1);
   int tstepQ = 0, streak = 0, step = 0, ministep = 0, stage = 0, attempt = 0, it = 0, code = 0;
   int n_ivp = 0, n_newton = 0;
   uint64_t rng_index = 0;
-  int phase = PH_FETCH;
+  int phase = warp < use_warps ? PH_FETCH : PH_IDLE;
   bool hires = !LO;
   T res_prev = T(0);
   int good = 0, bounces = 0, seg = 0;
   // checkpoints of the early-retirement network (history kept in S.ck_*)
   const bool checkpoints = a.feat_every > 0 && (a.feat != nullptr || a.mlp.w != nullptr);
+  const bool want_ratio = LO || checkpoints || (MODE == MODE_RESUME && a.back_list != nullptr);
   unsigned long long fp64_solves = 0;
-  // cycle accounting (lane 0 of each warp): fetch, setup, linear step, transitions;
-  // warp steps and active-team steps
-  long long cyc[4] = {0, 0, 0, 0};
-  long long warp_steps = 0, team_steps = 0, refine_steps = 0, refine_warp = 0, res_cyc = 0;
   __syncwarp();
 
   for (;;) {
-    long long tc0 = clock64();
-    // =========================================================== fetch (per team)
+    const long long tc0 = clock64();
+    // =========================================================== fetch (per warp)
     while (phase == PH_FETCH) {
       unsigned long long qi = 0;
-      if (g == 0) qi = atomicAdd(a.queue, 1ull);
-      qi = __shfl_sync(tmask, qi, 0, TEAM);
+      if (lane == 0) qi = atomicAdd(a.queue, 1ull);
+      qi = __shfl_sync(FULL, qi, 0);
       if ((int64_t)qi >= nqueue) { phase = PH_IDLE; break; }
       const bool carried = (int64_t)qi < ncarry;
       id = (MODE == MODE_RESUME) ? a.handoff_list[qi]
@@ -336,140 +349,186 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
       }
       ti = (int)(round * a.ntasks) + lo;
       {
-        cd z[14], Uj, sp[6];
         // start values precomputed by the start kernel hold this launch's round only; a
         // path of an earlier round (carried over) regenerates them (the same code, the
-        // same values)
+        // same values), its groups on the lanes of each group of 8
         if (a.starts && round * a.npaths == a.round_base) {
           const cd* st = a.starts + (size_t)lid * FRG_START_STRIDE;
-          for (int e = g; e < 14; e += TEAM) z[e] = st[e];
-          Uj = st[13 + jg];
-#pragma unroll
-          for (int i = 0; i < 6; ++i) sp[i] = st[21 + param_index(i, jg)];
+          if (lane < NP) {
+            S.sp[lane] = cp(st[21 + lane]);
+            if constexpr (LOWP) S.lo.sp[lane] = cx<T>(st[21 + lane]);
+          }
+          if (!resumed && lane < NV) S.Yc[lane] = cp(st[lane]);
         } else {
+          cd z[14], Uj, sp[6];
           team_start(pseed, (uint64_t)(lid + c.path_offset), c.start_dist, c.start_range, jg, z, Uj, sp);
-        }
-        const cx<T>* fpmT = fpm_of<T>(a, ti);
+          if (lane < 7) {
 #pragma unroll
-        for (int i = 0; i < 6; ++i) { lp.sp[i] = cx<T>(sp[i]); lp.fp[i] = fpmT[param_index(i, jg)]; }
-        lp.gamma = gamma_of<T>(a, ti);
-        if (g < 7) {
-          S.spm[jg] = cp(sp[2]); S.spm[8 + jg] = cp(sp[3]); S.spm[15 + jg] = cp(sp[4]); S.spm[22 + jg] = cp(sp[5]);
+            for (int i = 2; i < 6; ++i) {
+              S.sp[param_index(i, jg)] = cp(sp[i]);
+              if constexpr (LOWP) S.lo.sp[param_index(i, jg)] = cx<T>(sp[i]);
+            }
+            if (!resumed) S.Yc[13 + jg] = cp(Uj);
+          }
+          if (lane == 0) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              S.sp[8 * i] = cp(sp[i]);
+              if constexpr (LOWP) S.lo.sp[8 * i] = cx<T>(sp[i]);
+            }
+            if (!resumed)
+              for (int e = 0; e < 14; ++e) S.Yc[e] = cp(z[e]);
+          }
         }
-        if (g == 0) { S.spm[0] = cp(sp[0]); S.spm[8] = cp(sp[1]); }
-        if (!resumed) {
-          for (int e = g; e < 14; e += TEAM) S.Yc[e] = cp(z[e]);
-          if (g < 7) S.Yc[13 + jg] = cp(Uj);
-          if (g == 7) { S.Yc[21] = cp(P(1)); S.Yc[22] = cp(P(0)); }
+        if (lane < NP) {
+          S.fp[lane] = fpm_hi_of<P>(a, ti)[lane];
+          if constexpr (LOWP) S.lo.fp[lane] = fpm_of<T>(a, ti)[lane];
+        }
+        gamma = gamma_of<T>(a, ti);
+        if (lane == 0) {
+          S.gamma = gamma_hi_of<P>(a, ti);
+          if (!resumed) { S.Yc[21] = cp(P(1)); S.Yc[22] = cp(P(0)); }
         }
       }
       code = 0; stage = 0; attempt = 0; it = 0; residual = T(100); err = T(0); scale = T(0);
       good = 0; bounces = 0; seg = 0;
-      if (g == 0) { S.ck_t[0] = S.ck_t[1] = 0.0; S.ck_s[0] = S.ck_s[1] = 0.f; S.ck_rmax = 0.f; }
+      if (lane == 0) { S.ck_t[0] = S.ck_t[1] = 0.0; S.ck_s[0] = S.ck_s[1] = 0.f; S.ck_rmax = 0.f; }
       if (resumed) {
         const Handoff& h = a.handoff[id];
-        for (int e = g; e < NY; e += TEAM) {
-          S.Yc[e] = cp(h.Yc[e]); S.Vc[e] = cx<T>(h.Vc[e]); S.u[e] = cx<T>(h.u[e]);
-        }
+        if (el) { S.Yc[lane] = cp(h.Yc[lane]); S.Vc[lane] = cx<T>(h.Vc[lane]); S.u[lane] = cx<T>(h.u[lane]); }
         s = T(h.s); rng_index = h.rng_index; streak = h.streak; step = h.step; ministep = h.ministep;
         tstepQ = h.tstepQ; n_ivp = h.n_ivp; n_newton = h.n_newton; bounces = h.bounces;
-        __syncwarp(tmask);
+        __syncwarp();
         if (h.reason == 6) {  // the path already ended on a step limit in the FP32 stage
           if constexpr (!LO) {
-            cd Yf[NY];
-            for (int e = 0; e < NY; ++e) Yf[e] = h.Yc[e];
-            team_finish(a, *reinterpret_cast<Smem<double>*>(&S), Yf, id, ti, h.code, g, tmask, n_ivp, n_newton,
-                        step);
+            if (lane < TEAM)
+              team_finish(a, S, h.Yc, id, ti, h.code, lane, (1u << TEAM) - 1, n_ivp, n_newton, step);
+            __syncwarp();
           }
           continue;  // next path
         }
         phase = PH_RK;
       } else {
-        __syncwarp(tmask);
         // TrackPath's patches start at draw 0 of the path's stream (by-value state,
         // frg.cu:54,57); u (htpytrack.cu:53-58) then the random velocity patch (:63-67).
         const double R = c.patch_range;
         const uint64_t stream = (uint64_t)(lid + c.path_offset);
-        for (int e = g; e < NY; e += TEAM) {
+        if (el) {
+          const int e = lane;
           S.u[e] = cx<T>(T(2.0 * R * frg_uniform01(pseed, stream, 2 * e) - R),
                          T(2.0 * R * frg_uniform01(pseed, stream, 2 * e + 1) - R));
           S.Vc[e] = cx<T>(T(2.0 * R * frg_uniform01(pseed, stream, 46 + 2 * e) - R),
                           T(2.0 * R * frg_uniform01(pseed, stream, 47 + 2 * e) - R));
         }
         rng_index = 92;
-        __syncwarp(tmask);
+        __syncwarp();
         // SwitchPatch(u, Yc, Yc) (htpytrack.cu:60), in the point type
-        cp d(P(0));
-        for (int e = g; e < NZ; e += TEAM) d = cfma(cp(S.u[e]), S.Yc[e], d);
-        d = cp(team_sum(tmask, d.re), team_sum(tmask, d.im));
+        const cp d = patch_dot<T, P>(S.u, S.Yc, NZ, g, FULL);
         const cp sc = cdiv(cp(P(1)) - cp(S.u[22]) * S.Yc[22], d);
-        __syncwarp(tmask);
-        for (int e = g; e < NZ; e += TEAM) S.Yc[e] = sc * S.Yc[e];
+        __syncwarp();
+        if (lane < NZ) S.Yc[lane] = sc * S.Yc[lane];
         s = T(c.s_init); tstepQ = 0; streak = c.caution_steps - 1; step = 0; ministep = 0;
         n_ivp = 0; n_newton = 0;
         phase = PH_TANGENT0;
       }
+      __syncwarp();
+      su = patch_scale(S.u, lane);
     }
-    if (__all_sync(FULL, phase == PH_IDLE)) break;
-    long long tc1 = clock64();
+    const long long tc1 = clock64();
 
-    // ==================================================== set up (per team)
+    // ==================================================== set up (per warp)
     const bool newton = (phase == PH_NEWTON || phase == PH_SHARP);
     bool tstep = false;
     T tgoal = T(0);
     const cx<T>* Wsrc = S.Vc;
     cx<T>* dst = S.dx;
-    if (phase == PH_TANGENT0 || phase == PH_IDLE) {
-      for (int e = g; e < NY; e += TEAM) S.Ye[e] = cx<T>(S.Yc[e]);
-    } else if (phase == PH_RK) {
-      tstep = tstepQ != 0;
-      dst = S.k[stage];
-      if (stage == 0) {
-        for (int e = g; e < NY; e += TEAM) S.Ye[e] = cx<T>(S.Yc[e]);
+    if (phase != PH_IDLE) {
+      if (phase == PH_TANGENT0) {
+        if (el) S.Ye[lane] = cx<T>(S.Yc[lane]);
+      } else if (phase == PH_RK) {
+        tstep = tstepQ != 0;
+        dst = S.k[stage];
+        if (stage == 0) {
+          if (el) S.Ye[lane] = cx<T>(S.Yc[lane]);
+        } else {
+          // stage weights times s, one per lane; then the sums from the last stage back
+          Wsrc = S.k[stage - 1];
+          const T ws = g < stage ? mul_rn(T(c_dpA[stage][g]), s) : T(0);
+          cx<T> acc = mul_rn(__shfl_sync(FULL, ws, stage - 1), S.k[stage - 1][lane < VS ? lane : 0]);
+          for (int l = stage - 2; l >= 0; --l)
+            acc = axpy(__shfl_sync(FULL, ws, l), S.k[l][lane < VS ? lane : 0], acc);
+          if (el) S.Ye[lane] = cx<T>(S.Yc[lane]) + acc;
+        }
       } else {
-        Wsrc = S.k[stage - 1];
-        const double* w = c_dpA[stage];
-        for (int e = g; e < NY; e += TEAM) {
-          cx<T> acc = T(w[stage - 1]) * s * S.k[stage - 1][e];
-          for (int l = stage - 2; l >= 0; --l) acc = T(w[l]) * s * S.k[l][e] + acc;
-          S.Ye[e] = cx<T>(S.Yc[e]) + acc;
+        tgoal = (phase == PH_SHARP) ? T(1) : T(S.Yn[22].re);
+        if (el) S.Ye[lane] = cx<T>(S.YN[lane]);
+      }
+      __syncwarp();
+      if constexpr (LOWP) {
+        eval_prep<false, T>(S.Ye, S.lo.sp, S.lo.fp, gamma, S.inputs().in, S.inputs().dq, lane);
+        if (newton && hires) eval_prep<true, P>(S.YN, S.sp, S.fp, S.gamma, S.inputs().hi.in, nullptr, lane);
+      } else {
+        eval_prep<false, T>(S.Ye, S.sp, S.fp, gamma, S.inputs().in, S.inputs().dq, lane);
+      }
+    }
+    if (lane == 0) { S.active = phase != PH_IDLE; S.refine = newton && hires; }
+    const long long tc2 = clock64();
+
+    // ============== evaluation (the block: part `warp` of every path's groups)
+    if (__syncthreads_and(phase == PH_IDLE)) break;
+    {
+      Smem<T, P>& E = paths[lane >> 3];
+      if (E.active && g < 7) {
+        auto& in = E.inputs();
+        switch (warp) {
+          case 0: frg_eval_slice<0, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
+          case 1: frg_eval_slice<1, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
+          case 2: frg_eval_slice<2, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
+          default: frg_eval_slice<3, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
         }
       }
-    } else {
-      tgoal = (phase == PH_SHARP) ? T(1) : T(S.Yn[22].re);
-      for (int e = g; e < NY; e += TEAM) S.Ye[e] = cx<T>(S.YN[e]);
-    }
-    __syncwarp();
-    long long tc2 = clock64();
-
-    // ========================================== linear step (whole warp)
-    const StepOut<T> r = linear_step<T, P>(S, Wsrc, dst, newton, tstep, tgoal, lp, fpm_hi_of<P>(a, ti),
-                                        gamma_hi_of<P>(a, ti), g, hires);
-    __syncwarp();
-    long long tc3 = clock64();
-    if (lane == 0) {
-      cyc[0] += tc1 - tc0; cyc[1] += tc2 - tc1; cyc[2] += tc3 - tc2;
-      warp_steps++;
-      res_cyc += r.res_cycles;
-    }
-    {
-      const unsigned act = __ballot_sync(FULL, phase != PH_IDLE && g == 0);
-      if (lane == 0) team_steps += __popc(act);
-      if (LO) {  // corrector iterations on double-float residuals, and warp steps that ran one
-        const unsigned ref = __ballot_sync(FULL, phase != PH_IDLE && g == 0 && newton && hires);
-        if (lane == 0) { refine_steps += __popc(ref); refine_warp += ref != 0u; }
+      if constexpr (LOWP) {
+        // the corrector's refinement residual: F_j at the point YN with q(t) in the point
+        // type (htpysupport.cu:37-48, :64-86), the right-hand side with which the FP32
+        // solves converge in double-float
+        const long long tr0 = clock64();
+        if (E.refine) {
+          const FrgEvalIn<P>& in = E.inputs().hi.in;
+          if (warp == 3) {
+            const cp d = patch_dot<T, P>(E.u, E.YN, NY, g, 0xffu << (lane & 24)) - cp(P(1));
+            if (g == 0) E.Rd = cx<T>(d);
+          } else if (g < 7) {
+            E.R[warp][g] = cx<T>(warp == 0   ? frg_residual_slice<0, P>(E.YN, in, jg)
+                                 : warp == 1 ? frg_residual_slice<1, P>(E.YN, in, jg)
+                                             : frg_residual_slice<2, P>(E.YN, in, jg));
+          }
+        }
+        if (lane == 0) S.cyc[6] += clock64() - tr0;
       }
     }
+    __syncthreads();
     if (phase == PH_IDLE) continue;
+
+    // ========================================== solve (the path's warp)
+    const int restype = (LO || phase == PH_SHARP) ? (LO ? 1 : c.sharp_residual) : c.newt_residual;
+    const StepOut<T> r = solve_step<T, P>(S, Wsrc, dst, newton, tstep, tgoal, su, LOWP && hires, want_ratio,
+                                          newton && restype == 0, lane);
+    const long long tc3 = clock64();
+    if (lane == 0) {
+      S.cyc[0] += tc1 - tc0; S.cyc[1] += tc2 - tc1; S.cyc[2] += tc3 - tc2;
+      S.cyc[4] += 1;
+      // corrector iterations on double-float residuals
+      if (LO) S.cyc[5] += newton && hires;
+    }
     if (!LO) ++fp64_solves;
-    if (checkpoints && g == 0) S.ck_rmax = fmaxf(S.ck_rmax, (float)r.ratio);
+    if (checkpoints && lane == 0) S.ck_rmax = fmaxf(S.ck_rmax, (float)r.ratio);
     if (MODE == MODE_RESUME) {
       good = (r.ratio < T(c.cond_switch * 1e-2)) ? good + 1 : 0;
       ++seg;
     }
     if (newton) ++n_newton; else ++n_ivp;
 
-    // ============================================= transitions (per team)
+    // ============================================= transitions (per warp)
     bool finished = false;
     int handoff = 0;
     bool handback = false;
@@ -480,30 +539,41 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
       code = 2;  // the FP64 budget of this path is spent: retire it as a step-limit failure
       finished = true;
     } else if (phase == PH_TANGENT0) {
-      for (int e = g; e < NY; e += TEAM) S.Vc[e] = S.dx[e];
+      if (el) S.Vc[lane] = S.dx[lane];
       if (c.max_steps == 0) { code = 1; finished = true; }
       stage = 0;
       phase = PH_RK;
     } else if (phase == PH_RK) {
       if (++stage == 8) {
         stage = 0;
-        // error estimate and step factor (rungekutta.cu:99-112), prediction (:115-122)
+        // error estimate and step factor (rungekutta.cu:99-112), prediction (:115-122);
+        // the weights times s one per lane, the second stage has weight zero in both
         T es = T(0);
-        for (int e = g; e < NY; e += TEAM) {
-          cx<T> le = T(c_dpE[7]) * s * S.k[7][e];
-          cx<T> yb = T(c_dpB[7]) * s * S.k[7][e];
+        {
+          const T we = mul_rn(T(c_dpE[g]), s), wb = mul_rn(T(c_dpB[g]), s);
+          const cx<T> k7 = S.k[7][lane < VS ? lane : 0];
+          cx<T> le = mul_rn(__shfl_sync(FULL, we, 7), k7);
+          cx<T> yb = mul_rn(__shfl_sync(FULL, wb, 7), k7);
+#pragma unroll
           for (int l = 6; l >= 0; --l) {
-            if (c_dpE[l] != 0.0) le = T(c_dpE[l]) * s * S.k[l][e] + le;
-            if (c_dpB[l] != 0.0) yb = T(c_dpB[l]) * s * S.k[l][e] + yb;
+            if (l == 1) continue;
+            const cx<T> kl = S.k[l][lane < VS ? lane : 0];
+            le = axpy(__shfl_sync(FULL, we, l), kl, le);
+            yb = axpy(__shfl_sync(FULL, wb, l), kl, yb);
           }
-          es += cnorm2(le);
-          S.Yn[e] = S.Yc[e] + cp(yb);
-          S.Vn[e] = S.k[7][e];
+          if (el) {
+            es = cnorm2(le);
+            S.Yn[lane] = S.Yc[lane] + cp(yb);
+            S.Vn[lane] = k7;
+          }
+          // entries g, g + 8, g + 16, then the groups of 8
+          const T e1 = __shfl_sync(FULL, es, g + 8), e2 = __shfl_sync(FULL, es, g + 16);
+          es = __shfl_sync(FULL, es, g) + e1 + e2;
         }
-        err = sqrt(team_sum(tmask, es));
+        err = sqrt(team_sum(FULL, es));
         scale = (err > T(10e-17)) ? T(0.8) * pow(T(c.rk_tol) / err, T(1) / T(6)) : T(5);
         if (scale > T(5)) scale = T(5);
-        __syncwarp(tmask);
+        __syncwarp();
         if (ministep++ == c.max_ministeps) { code = 2; finished = true; }
         else if (err <= T(c.rk_tol)) {
           const double tn = double(S.Yn[22].re);
@@ -512,9 +582,8 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
           else if (fabs(1.0 - tn) < c.sharp_trigger) { attempt = 0; phase = PH_SHARP; }
           else { tstepQ = 1; s = T(1.0 - double(S.Yc[22].re)); }  // land on t = 1 (htpytrack.cu:120-123)
           if (phase == PH_NEWTON || phase == PH_SHARP) {
-            for (int e = g; e < NY; e += TEAM) S.YN[e] = S.Yn[e];
             // the FP32 stage sharpens at exactly t = 1 (its t-update is only FP32-accurate)
-            if (LO && phase == PH_SHARP && g == (22 & 7)) S.YN[22] = cp(P(1));
+            if (el) S.YN[lane] = (LO && phase == PH_SHARP && lane == 22) ? cp(P(1)) : S.Yn[lane];
             residual = T(100);
             it = 0;
             hires = !LO || phase == PH_SHARP;
@@ -532,14 +601,13 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
       const bool sharp = (phase == PH_SHARP);
       const int max_its = sharp ? c.sharp_its : c.newt_its;
       const T tol = sharp ? T(c.sharp_tol) : newt_tol;
-      const int restype = (LO || sharp) ? (LO ? 1 : c.sharp_residual) : c.newt_residual;
       bool done = false, predicted = false;
       if (restype == 0 && it > 0) {
         residual = r.hnorm;  // |H| at the current point: the residual of the previous update
         if (!(it < max_its && residual > tol)) done = true;
       }
       if (!done) {
-        for (int e = g; e < NY; e += TEAM) S.YN[e] += cp(S.dx[e]);
+        if (el) S.YN[lane] += cp(S.dx[lane]);
         it++;
         if (restype != 0) {
           residual = sqrt(r.xnorm2);
@@ -569,7 +637,7 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
           res_prev = residual;
         }
       }
-      __syncwarp(tmask);
+      __syncwarp();
       if (done) {
         const bool ok = predicted || ((LO && !c.lo_refine && !sharp)
                                           ? residual < T(c.newt_tol_lo) * T(100)
@@ -579,12 +647,11 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
           if (fabs(1.0 - double(S.Yn[22].re)) < c.sharp_trigger) {
             if (LO && !c.lo_endgame) handoff = 5;
             attempt = 0; phase = PH_SHARP;
-            for (int e = g; e < NY; e += TEAM) S.YN[e] = S.Yn[e];
-            if (LO && g == (22 & 7)) S.YN[22] = cp(P(1));
+            if (el) S.YN[lane] = (LO && lane == 22) ? cp(P(1)) : S.Yn[lane];
             residual = T(100); it = 0; hires = true;
           } else {
             // accept the step (htpytrack.cu:176-183)
-            for (int e = g; e < NY; e += TEAM) { S.Yc[e] = S.YN[e]; S.Vc[e] = S.Vn[e]; }
+            if (el) { S.Yc[lane] = S.YN[lane]; S.Vc[lane] = S.Vn[lane]; }
             streak++;
             if (streak < c.caution_steps && scale > T(1)) scale = T(1);
             s *= scale;
@@ -594,13 +661,13 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
             if (checkpoints && step % a.feat_every == 0) {
               // checkpoint: record the features and/or let the network retire the path
               int retire = 0;
-              __syncwarp(tmask);
-              if (g == 0)
+              __syncwarp();
+              if (lane == 0)
                 retire = checkpoint<P>(a, S.Yc, id, double(s), S.ck_rmax, step, ministep, rng_index, S.ck_t[0],
                                        S.ck_t[1], S.ck_s[0], S.ck_s[1], !LO, n_ivp, n_newton, double(residual),
                                        streak, tstepQ, bounces);
-              retire = __shfl_sync(tmask, retire, 0, TEAM);
-              if (g == 0) {
+              retire = __shfl_sync(FULL, retire, 0);
+              if (lane == 0) {
                 S.ck_t[1] = S.ck_t[0]; S.ck_t[0] = double(S.Yc[22].re);
                 S.ck_s[1] = S.ck_s[0]; S.ck_s[0] = float(s); S.ck_rmax = 0.f;
               }
@@ -620,20 +687,21 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
           // new random patch and SwitchPatch(u, Yn, Yn) (htpytrack.cu:145-151, :204-210)
           const double R = c.patch_range;
           const uint64_t stream = (uint64_t)(lid + c.path_offset);
-          for (int e = g; e < NY; e += TEAM)
+          if (el) {
+            const int e = lane;
             S.u[e] = cx<T>(T(2.0 * R * frg_uniform01(pseed, stream, rng_index + 2 * e) - R),
                            T(2.0 * R * frg_uniform01(pseed, stream, rng_index + 2 * e + 1) - R));
+          }
           rng_index += 46;
-          __syncwarp(tmask);
-          cp d(P(0));
-          for (int e = g; e < NZ; e += TEAM) d = cfma(cp(S.u[e]), S.Yn[e], d);
-          d = cp(team_sum(tmask, d.re), team_sum(tmask, d.im));
+          __syncwarp();
+          su = patch_scale(S.u, lane);
+          const cp d = patch_dot<T, P>(S.u, S.Yn, NZ, g, FULL);
           const cp sc = cdiv(cp(P(1)) - cp(S.u[22]) * S.Yn[22], d);
-          __syncwarp(tmask);
-          for (int e = g; e < NZ; e += TEAM) S.Yn[e] = sc * S.Yn[e];
+          __syncwarp();
+          if (lane < NZ) S.Yn[lane] = sc * S.Yn[lane];
           if (!sharp) {
             if (++attempt < c.newt_attempts) {
-              for (int e = g; e < NY; e += TEAM) S.YN[e] = S.Yn[e];
+              if (el) S.YN[lane] = S.Yn[lane];
               residual = T(100); it = 0; hires = !LO;
             } else if (s <= T(c.s_min)) {
               if (LO) handoff = 3; else { code = 4; finished = true; }
@@ -646,8 +714,7 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
             }
           } else {
             if (++attempt < c.sharp_attempts) {
-              for (int e = g; e < NY; e += TEAM) S.YN[e] = S.Yn[e];
-              if (LO && g == (22 & 7)) S.YN[22] = cp(P(1));
+              if (el) S.YN[lane] = (LO && lane == 22) ? cp(P(1)) : S.Yn[lane];
               residual = T(100); it = 0;
             } else if (LO) {
               handoff = 5;  // the FP32 stage could not sharpen: the FP64 kernel retries the endgame
@@ -658,10 +725,10 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
         }
       }
     }
-    __syncwarp(tmask);
-    if (lane == 0) cyc[3] += clock64() - tc3;
+    __syncwarp();
+    if (lane == 0) S.cyc[3] += clock64() - tc3;
 
-    if (MODE == MODE_RESUME && (finished || handback) && g == 0 && a.counters) {
+    if (MODE == MODE_RESUME && (finished || handback) && lane == 0 && a.counters) {
       // length of this path's FP64 segment in this launch
       const int b = seg < 100 ? 0 : seg < 300 ? 1 : seg < 1000 ? 2 : seg < 3000 ? 3 : seg < 10000 ? 4 : 5;
       atomicAdd(&a.counters[40 + b], 1ull);
@@ -672,8 +739,8 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
       // finished in FP64; an FP64 path well conditioned again returns to FP32)
       Handoff& h = a.handoff[id];
       const cp* ysrc = (finished && final_from_YN) ? S.YN : S.Yc;  // a sharpened root is in YN
-      for (int e = g; e < NY; e += TEAM) { h.Yc[e] = cd(ysrc[e]); h.Vc[e] = cd(S.Vc[e]); h.u[e] = cd(S.u[e]); }
-      if (g == 0) {
+      if (el) { h.Yc[lane] = cd(ysrc[lane]); h.Vc[lane] = cd(S.Vc[lane]); h.u[lane] = cd(S.u[lane]); }
+      if (lane == 0) {
         h.s = double(s); h.rng_index = rng_index; h.streak = streak; h.step = step; h.ministep = ministep;
         h.tstepQ = tstepQ; h.n_ivp = n_ivp; h.n_newton = n_newton;
         h.reason = finished ? 6 : handoff; h.code = code;
@@ -690,31 +757,30 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) team_kernel(TrackArgs a) {
         const unsigned long long slot = atomicAdd(cnt, 1ull);
         list[slot] = id;
       }
-      __syncwarp(tmask);
+      __syncwarp();
       phase = PH_FETCH;
       continue;
     }
     if (finished) {
       if constexpr (!LO) {
-        cd Yf[NY];
-        const cp* src = final_from_YN ? S.YN : S.Yc;
-        for (int e = 0; e < NY; ++e) Yf[e] = cd(src[e]);
-        __syncwarp(tmask);
-        team_finish(a, S, Yf, id, ti, code, g, tmask, n_ivp, n_newton, step);
+        if (lane < TEAM)
+          team_finish(a, S, final_from_YN ? S.YN : S.Yc, id, ti, code, lane, (1u << TEAM) - 1, n_ivp, n_newton,
+                      step);
+        __syncwarp();
       }
       phase = PH_FETCH;
     }
   }
-  if (a.counters && fp64_solves && g == 0) atomicAdd(&a.counters[11], fp64_solves);
   if (a.counters && lane == 0) {
+    if (fp64_solves) atomicAdd(&a.counters[11], fp64_solves);
     const int base = LO ? 24 : 30;
-    for (int i = 0; i < 4; ++i) atomicAdd(&a.counters[base + i], (unsigned long long)cyc[i]);
-    atomicAdd(&a.counters[base + 4], (unsigned long long)warp_steps);
-    atomicAdd(&a.counters[base + 5], (unsigned long long)team_steps);
+    for (int i = 0; i < 4; ++i) atomicAdd(&a.counters[base + i], S.cyc[i]);
+    atomicAdd(&a.counters[base + 4], S.cyc[4]);  // a warp step tracks one path
+    atomicAdd(&a.counters[base + 5], S.cyc[4]);
     if (LO) {
-      atomicAdd(&a.counters[22], (unsigned long long)refine_steps);
-      atomicAdd(&a.counters[23], (unsigned long long)refine_warp);
-      atomicAdd(&a.counters[37], (unsigned long long)res_cyc);
+      atomicAdd(&a.counters[22], S.cyc[5]);
+      atomicAdd(&a.counters[23], S.cyc[5]);
+      atomicAdd(&a.counters[37], S.cyc[6]);
     }
   }
 }
@@ -726,9 +792,9 @@ namespace frg {
 namespace team {
 // GenerateStart per path, one team per path (the same lane split as the tracking
 // kernels' inline generation, so the values are identical).
-__global__ void __launch_bounds__(FRG_TEAM_THREADS) start_kernel(TrackArgs a, cd* starts) {
+__global__ void __launch_bounds__(FRG_START_THREADS) start_kernel(TrackArgs a, cd* starts) {
   const int g = threadIdx.x & 7;
-  const int64_t id = ((int64_t)blockIdx.x * FRG_TEAM_THREADS + threadIdx.x) >> 3;
+  const int64_t id = ((int64_t)blockIdx.x * FRG_START_THREADS + threadIdx.x) >> 3;
   if (id >= a.npaths) return;
   const int jg = g < 7 ? g + 1 : 7;
   cd z[14], Uj, sp[6];
@@ -745,29 +811,29 @@ __global__ void __launch_bounds__(FRG_TEAM_THREADS) start_kernel(TrackArgs a, cd
 }  // namespace frg
 
 cudaError_t frg_launch_starts(const frg::TrackArgs& args, cx<double>* starts, cudaStream_t stream) {
-  const int64_t blocks = (args.npaths * 8 + FRG_TEAM_THREADS - 1) / FRG_TEAM_THREADS;
-  frg::team::start_kernel<<<(unsigned)blocks, FRG_TEAM_THREADS, 0, stream>>>(args, starts);
+  const int64_t blocks = (args.npaths * 8 + FRG_START_THREADS - 1) / FRG_START_THREADS;
+  frg::team::start_kernel<<<(unsigned)blocks, FRG_START_THREADS, 0, stream>>>(args, starts);
   return cudaGetLastError();
 }
 
 namespace {
 template <int MODE, typename T, typename P = typename frg::team::PointOf<T>::type>
 cudaError_t team_launch(const frg::TrackArgs& args, int grid, cudaStream_t stream) {
-  const size_t smem = (FRG_TEAM_THREADS / 8) * sizeof(frg::team::Smem<T, P>);
+  const size_t smem = frg::team::PATHS * sizeof(frg::team::Smem<T, P>);
   cudaError_t e = cudaFuncSetAttribute(frg::team::team_kernel<MODE, T, P>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  frg::team::team_kernel<MODE, T, P><<<grid, FRG_TEAM_THREADS, smem, stream>>>(args);
+  frg::team::team_kernel<MODE, T, P><<<grid, 32 * frg::team::PATHS, smem, stream>>>(args);
   return cudaGetLastError();
 }
 template <int MODE, typename T, typename P = typename frg::team::PointOf<T>::type>
 cudaError_t team_occ(int* bps) {
-  const size_t smem = (FRG_TEAM_THREADS / 8) * sizeof(frg::team::Smem<T, P>);
+  const size_t smem = frg::team::PATHS * sizeof(frg::team::Smem<T, P>);
   cudaError_t e = cudaFuncSetAttribute(frg::team::team_kernel<MODE, T, P>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, frg::team::team_kernel<MODE, T, P>, FRG_TEAM_THREADS,
-                                                       smem);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, frg::team::team_kernel<MODE, T, P>,
+                                                       32 * frg::team::PATHS, smem);
 }
 }  // namespace
 

@@ -22,6 +22,7 @@ from __future__ import annotations
 
 import os
 
+import numpy as np
 import sympy as sp
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -162,6 +163,163 @@ class Printer:
         raise TypeError(type(e), e)
 
 
+# ---- the evaluation split over a block's four warps -------------------------------
+# Quantities that a path's own warp computes once per step and every slice reads. Each
+# has a plain form (side 0) and its conjugate partner (side 1), computed by the same
+# instructions on different lanes; `pj` marks those that differ per group. The printed
+# forms are what the kernel's preparation evaluates: the generator checks them.
+HOISTED = [
+    # name, per group, side 0 (symbol form), side 1
+    ("pz", False, "P0*z", "Pc0*z"),
+    ("fp", False, "F - pz0", "Fc - pz1"),
+    ("hp", False, "H - pz0", "Hc - pz1"),
+    ("bd", False, "B - D", "Bc - Dc"),
+    ("ebd", False, "e1*bd0", "ec1*bd1"),
+    ("cg", False, "C - G", "Cc - Gc"),
+    ("ecg", False, "e2*cg0", "ec2*cg1"),
+    ("v", False, "fp0*ebd0 - hp0*ecg0", "fp1*ebd1 - hp1*ecg1"),
+    ("ac", False, "A - C", "Ac - Cc"),
+    ("pjz", True, "Pj*z", "Pcj*z"),
+    ("ap", True, "A - pjz0", "Ac - pjz1"),
+    ("bp", True, "B - pjz0", "Bc - pjz1"),
+    ("qa", True, "Qj*ac0", "Qcj*ac1"),
+    ("aq", True, "ap0 - qa0", "ap1 - qa1"),
+    ("eaq", True, "e2*aq0", "ec2*aq1"),
+    ("w", True, "B - A + qa0 + bp0*ebd0 - cg0*eaq0", "Bc - Ac + qa1 + bp1*ebd1 - cg1*eaq1"),
+]
+# frg_group_f's own order of the same sum
+RESIDUAL_FORMS = {"w": ("B + qa0 - A + bp0*ebd0 - ecg0*aq0", "Bc + qa1 - Ac + bp1*ebd1 - ecg1*aq1")}
+# Which warp evaluates which outputs: 4 parts of equal cost (492 real FMA-pipe operations
+# each, found by a local search over the outputs' closures; the whole group is 1,770).
+EVAL_SLICES = [
+    ["dI[5]", "dIII[1]", "dIII[2]", "dIII[3]", "dIII[4]", "dIII[5]", "dIII[6]", "dIII[15]"],
+    ["fI", "dI[0]", "dI[1]", "dI[2]", "dI[6]", "tI", "fII", "dII[0]", "dII[1]", "dII[4]", "tII", "dIII[14]"],
+    ["fIII", "dIII[0]", "dIII[7]", "dIII[8]", "dIII[9]", "dIII[11]", "tIII"],
+    ["dI[3]", "dI[4]", "dI[7]", "dII[2]", "dII[3]", "dII[5]", "dIII[10]", "dIII[12]", "dIII[13]"],
+]
+RESIDUAL_SLICES = [["fI"], ["fII"], ["fIII"]]
+# column of each derivative slot in the group's row: links 0..13, Z0 14, t 15, U_j 16, F 17
+ROW_COLS = {"I": [0, 2, 6, 7, 9, 13, 16, 14], "II": [1, 4, 8, 11, 16, 14], "III": list(range(14)) + [16, 14]}
+
+
+def hoisted_symbols(repl, pr, other={}):
+    """{temporary's name: hoisted quantity} of the temporaries that have a hoisted quantity's
+    value, after checking in single precision on random inputs that both forms round alike
+    (a - b, a + (-b) and -((-a) + b) do; another order of a sum does not)."""
+    base = {n: sp.Symbol(n) for n in ("z e1 e2 ec1 ec2 P0 Pc0 Pj Pcj Qj Qcj A B C D F G H "
+                                      "Ac Bc Cc Dc Fc Gc Hc").split()}
+    forms = {f"{name}{side}": other.get(name, (f0, f1))[side] for name, _, f0, f1 in HOISTED for side in (0, 1)}
+    values = {}
+    for key, form in forms.items():
+        values[key] = sp.sympify(form, locals={**base, **values})
+    full, found = {}, {}
+    for s_, e in repl:
+        full[s_] = sp.expand(e.subs(full))
+        for key, val in values.items():
+            if sp.expand(full[s_] - val) == 0:
+                found[s_.name] = key
+    rng = np.random.default_rng(1)
+    names = set(base) | {y.name for _, e in repl for y in e.free_symbols}
+    for _ in range(200):
+        env = {n: np.complex64(complex(*rng.normal(size=2))) for n in sorted(names)}
+        env.update(cx=lambda v: v, T=np.float32)
+        for key, form in forms.items():
+            env[key] = eval(form, {}, env)
+        for s_, e in repl:
+            env[s_.name] = eval(pr.expr(e).replace("cx<T>", "cx"), {}, env)
+            if s_.name in found:
+                assert env[s_.name] == env[found[s_.name]], (s_.name, found[s_.name])
+    return found
+
+
+def slice_lines(repl, wanted, found, loads, pr):
+    """Straight-line code of the outputs `wanted` (expr, statement) from the hoisted quantities."""
+    defs = {s_.name: e for s_, e in repl}
+    need, stack = set(), [x.name for e, _ in wanted for x in e.free_symbols]
+    used = set()
+    while stack:
+        x = stack.pop()
+        if x in found or x not in defs:
+            used.add(x)
+        elif x not in need:
+            need.add(x)
+            stack += [y.name for y in defs[x].free_symbols]
+    out = [f"    const cx<T> {x} = {loads(x, found.get(x))};" for x in sorted(used)]
+    out += [f"    const cx<T> {s_} = {pr.expr(e)};" for s_, e in repl if s_.name in need]
+    out += ["    " + st.format(pr.expr(e)) for e, st in wanted]
+    return out
+
+
+INDEP = [h[0] for h in HOISTED if not h[1]]
+PERJ = [h[0] for h in HOISTED if h[1]]
+
+
+def load_of(x, key):
+    """Where a slice reads the value named x (a hoisted quantity `key` if it is one)."""
+    links = ["A", "B", "C", "D", "F", "G", "H", "Ac", "Bc", "Cc", "Dc", "Fc", "Gc", "Hc"]
+    if key:
+        name, side = key[:-1], key[-1]
+        if name in INDEP:
+            return f"in.sa[{side}][FRG_IN_{name.upper()}]"
+        return f"in.sb[{side}][FRG_IN_{name.upper()}][j - 1]"
+    if x in links:
+        return f"Y[{links.index(x)}]"
+    q = {"P0": "0", "Pc0": "8", "Pj": "j", "Pcj": "8 + j", "Qj": "15 + j", "Qcj": "22 + j"}
+    e = {"e1": "0", "e2": "1", "ec1": "2", "ec2": "3"}
+    if x in q:
+        return f"in.q[{q[x]}]"
+    if x[0] == "d" and x[1:] in q:
+        return f"dq[{q[x[1:]]}]"
+    if x in e:
+        return f"in.e[{e[x]}]"
+    return {"z": "Y[21]", "z2": "in.z2", "z3": "in.z3", "U": "Y[13 + j]", "iU": "in.iU[j - 1]"}[x]
+
+
+def emit_slices(lines, names, repl, reduced, frepl, fred, pr):
+    found, ffound = hoisted_symbols(repl, pr), hoisted_symbols(frepl, pr, RESIDUAL_FORMS)
+    by, slot = {}, {"I": 0, "II": 0, "III": 0}
+    row = {"I": 0, "II": 1, "III": 2}
+    for (kind, fam, v), e in zip(names, reduced):
+        if kind in "ft":
+            by[f"{kind}{fam}"] = (e, row[fam], 17 if kind == "f" else 15)
+        else:
+            by[f"d{fam}[{slot[fam]}]"] = (e, row[fam], ROW_COLS[fam][slot[fam]])
+            slot[fam] += 1
+    assert sorted(by) == sorted(n for s_ in EVAL_SLICES for n in s_)
+    lines += ["",
+              "// What one path's step needs besides its point: computed by the path's own warp, read by",
+              "// the slices below. Side 0 holds a quantity's plain form, side 1 its conjugate partner.",
+              "//   sa: " + ", ".join(INDEP) + "   (the same for every group)",
+              "//   sb: " + ", ".join(PERJ) + "   (per group j)"]
+    for name, pj, f0, _ in HOISTED:
+        r = f"; for the residual alone {RESIDUAL_FORMS[name][0]}" if name in RESIDUAL_FORMS else ""
+        lines.append(f"//   {name:4s} = {f0}{r}")
+    for name in INDEP + PERJ:
+        lines.append(f"#define FRG_IN_{name.upper()} {(INDEP + PERJ).index(name) - (len(INDEP) if name in PERJ else 0)}")
+    lines += ["template <typename T>", "struct FrgEvalIn {",
+              "  cx<T> z2, z3, e[4], q[32], iU[8];  // e: e1, e2, ec1, ec2; q(t); 1 / U_j at [j - 1]",
+              f"  cx<T> sa[2][{len(INDEP)}], sb[2][{len(PERJ)}][8];", "};", "",
+              "// One quarter of group j's evaluation (frg_group_eval's operations in its order): rows of",
+              "// the group into M[(row * 18 + column) * 8 + g], columns 0..13 links, 14 Z0, 15 t, 16 U_j, 17 F.",
+              "template <int SLICE, typename T>",
+              "__device__ __forceinline__ void frg_eval_slice(const cx<T>* Y, const FrgEvalIn<T>& in, const cx<T>* dq, int j,",
+              "                                               int g, cx<T>* M) {"]
+    for k, outs in enumerate(EVAL_SLICES):
+        lines.append(f"  if constexpr (SLICE == {k}) {{")
+        wanted = [(by[n][0], f"M[{(by[n][1] * 18 + by[n][2]) * 8} + g] = {{}};") for n in outs]
+        lines += slice_lines(repl, wanted, found, load_of, pr)
+        lines.append("  }")
+    lines += ["}", "",
+              "// One of the three equations at the point Y (frg_group_f's operations in its order).",
+              "template <int SLICE, typename T>",
+              "__device__ __forceinline__ cx<T> frg_residual_slice(const cx<T>* Y, const FrgEvalIn<T>& in, int j) {"]
+    for k in range(3):
+        lines.append(f"  if constexpr (SLICE == {k}) {{")
+        lines += slice_lines(frepl, [(fred[k], "return {};")], ffound, load_of, pr)
+        lines.append("  }")
+    lines += ["}"]
+
+
 def main():
     names, outs = outputs()
     # hoist shared quantities: substitute them by symbols
@@ -251,6 +409,7 @@ def main():
     lines.append(f"  fII = {pr.expr(fred[1])};")
     lines.append(f"  fIII = {pr.expr(fred[2])};")
     lines.append("}")
+    emit_slices(lines, names, repl, reduced, frepl, fred, pr)
     used = set()
     for _, e in repl:
         used |= {s.name for s in e.free_symbols}

@@ -89,7 +89,7 @@ typedef struct frg_config {
   int threads_per_block; /* 0 = tuned default */
   int blocks_per_sm;     /* 0 = tuned default */
   double newt_tol_lo;    /* mixed: corrector tolerance of the FP32 stage */
-  int kernel_variant;    /* FRG_KERNEL_TEAM (8 lanes per path, default) or FRG_KERNEL_THREAD */
+  int kernel_variant;    /* FRG_KERNEL_TEAM (a warp per path, default) or FRG_KERNEL_THREAD */
   int mixed_rounds;      /* mixed, team kernels: FP32/FP64 rounds; a path well conditioned again in
                             FP64 returns to FP32 in the next round (1 = no return) */
   int lo_refine;         /* mixed: 1 = the FP32 corrector refines on residuals in the point type
@@ -156,10 +156,11 @@ typedef struct frg_stats {
                                 predictor at s_min, endgame entry, ended on a step limit */
   int64_t kernel_cycles[12]; /* team kernels, summed over warps: [0..5] FP32 stage, [6..11] FP64
                                 kernel; per kernel the cycles in path fetch, step set-up, linear steps
-                                and transitions, then warp steps and active-team steps */
+                                and transitions, then warp steps and path steps (the same: a warp
+                                tracks one path) */
   int64_t handbacks;       /* mixed: returns from FP64 to FP32 once well conditioned again */
   int64_t refine_solves;   /* mixed: FP32-stage corrector iterations on double-float residuals */
-  int64_t refine_warp_steps; /* mixed: FP32-stage warp steps in which at least one path refined */
+  int64_t refine_warp_steps; /* mixed: FP32-stage warp steps whose path refined */
   double round_ms[32];     /* mixed: FP32-stage and FP64-stage times, interleaved, of mixed rounds
                               0..15 (frg_track) or of rounds 0..15 of the call (frg_track_rounds) */
   int64_t fp64_segment_hist[6]; /* mixed: paths leaving an FP64 launch after <100, <300, <1000, <3000,
