@@ -3,6 +3,7 @@
 // InitRandStates/Homotopy launches and copies back (frg.cu:201-236, :351-404).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -56,11 +57,11 @@ struct Slot {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   DevBuf gamma, gamma_lo, gamma_df, fpm_lo, fpm_df, task_start, queue, counters, starts;
-  DevBuf handoff, handoff_list, lo_lists;
+  DevBuf handoff, handoff_list, lo_lists, tail;
   DevBuf roots, codes, resid;  // staging of host outputs (frg_track_rounds)
   void release() {
     for (DevBuf* b : {&gamma, &gamma_lo, &gamma_df, &fpm_lo, &fpm_df, &task_start, &queue, &counters, &starts,
-                      &handoff, &handoff_list, &lo_lists, &roots, &codes, &resid})
+                      &handoff, &handoff_list, &lo_lists, &tail, &roots, &codes, &resid})
       b->release();
     if (own_stream && stream) cudaStreamDestroy(stream);
     stream = nullptr;
@@ -324,7 +325,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   FRG_CUDA(ctx, sl.fpm_df.ensure(sizeof(cx<df>) * np * ntasks));
   FRG_CUDA(ctx, sl.gamma_df.ensure(sizeof(cx<df>) * ntasks));
   FRG_CUDA(ctx, sl.task_start.ensure(sizeof(int64_t) * (ntasks + 1)));
-  FRG_CUDA(ctx, sl.queue.ensure(sizeof(unsigned long long) * 8));
+  FRG_CUDA(ctx, sl.queue.ensure(sizeof(unsigned long long) * FRG_NQUEUE));
   FRG_CUDA(ctx, sl.counters.ensure(sizeof(unsigned long long) * FRG_NCOUNTERS));
   // (host-to-device copies from pageable memory are staged before these calls return)
   FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma_df.p, g_df.data(), sizeof(cx<df>) * ntasks, cudaMemcpyHostToDevice, st));
@@ -332,7 +333,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma_lo.p, g_lo.data(), sizeof(cx<float>) * ntasks, cudaMemcpyHostToDevice, st));
   FRG_CUDA(ctx, cudaMemcpyAsync(sl.task_start.p, starts.data(), sizeof(int64_t) * (ntasks + 1),
                                 cudaMemcpyHostToDevice, st));
-  FRG_CUDA(ctx, cudaMemsetAsync(sl.queue.p, 0, sizeof(unsigned long long) * 8, st));
+  FRG_CUDA(ctx, cudaMemsetAsync(sl.queue.p, 0, sizeof(unsigned long long) * FRG_NQUEUE, st));
   FRG_CUDA(ctx, cudaMemsetAsync(sl.counters.p, 0, sizeof(unsigned long long) * FRG_NCOUNTERS, st));
   FRG_CUDA(ctx, frg_launch_to_float(d_fpm, (cx<float>*)sl.fpm_lo.p, np * ntasks, st));
   FRG_CUDA(ctx, frg_launch_to_df(d_fpm, (cx<df>*)sl.fpm_df.p, np * ntasks, st));
@@ -382,21 +383,42 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     if (e != cudaSuccess) return cuda_fail(ctx, e, "start kernel launch");
   }
   // persistent grids: SMs x resident blocks, capped by the work
-  int plugin_bps[3] = {0, 0, 0};  // a plug-in system's kernels have their own occupancy
-  if (ctx->cfg.system != 0)
-    for (int m = 0; m < (mixed ? 3 : 1); ++m)
+  const bool plugin = ctx->cfg.system != 0;
+  int plugin_bps[3] = {0, 0, 0}, warp_bps[3] = {0, 0, 0};  // a plug-in system's kernels have their own occupancy
+  if (plugin)
+    for (int m = 0; m < (mixed ? 3 : 1); ++m) {
       FRG_CUDA(ctx, frg_track_occupancy_system(ctx->cfg.system, m, &plugin_bps[m]));
+      FRG_CUDA(ctx, frg_warp_occupancy(ctx->cfg.system, m, &warp_bps[m]));
+    }
   auto grid_for = [&](int mode, int64_t n) {
     int bps = ctx->cfg.blocks_per_sm > 0             ? ctx->cfg.blocks_per_sm
               : (ctx->cfg.system != 0 && mode < 3)  ? plugin_bps[mode]
                                                     : (team ? ctx->team_blocks_per_sm[mode] : ctx->blocks_per_sm[mode]);
     return team ? frg_team_grid(ctx->sm_count, bps, n) : frg_thread_grid(ctx->sm_count, bps, n);
   };
-  auto launch = [&](int mode, int grid) {
-    return team ? frg_launch_team(mode, a, grid, st) : frg_launch_track(mode, a, grid, st);
+  // A plug-in's launch of up to FRG_WARP_PATHS paths per SM sub-partition takes a warp
+  // per path; a larger one a thread per path, and then a warp for each of its last paths.
+  const bool by_warp = plugin && N <= (int64_t)ctx->sm_count * 4 * FRG_WARP_PATHS;
+  auto launch = [&](int mode) -> cudaError_t {
+    const int grid = grid_for(mode, N);
+    if (team) return frg_launch_team(mode, a, grid, st);
+    const int wcap = plugin ? ctx->sm_count * (ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : warp_bps[mode])
+                            : 0;
+    if (by_warp) return frg_launch_warp(mode, a, (int)std::min<int64_t>(wcap, (N + 3) / 4), st);
+    if (!plugin) return frg_launch_track(mode, a, grid, st);
+    frg::TrackArgs b = a;
+    b.tail_cap = (int64_t)grid * (FRG_TRACK_THREADS / 32) * frg_tail_lanes(mode == 1);
+    cudaError_t e = sl.tail.ensure(sizeof(frg::Handoff) * (size_t)b.tail_cap);
+    if (e != cudaSuccess) return e;
+    b.tail = (frg::Handoff*)sl.tail.p;
+    b.tail_count = q + 8 + 2 * mode;  // and the tail's queue head beside it
+    if ((e = frg_launch_track(mode, b, grid, st)) != cudaSuccess) return e;
+    b.from_tail = 1;
+    b.queue = q + 9 + 2 * mode;
+    return frg_launch_warp(mode, b, (int)std::min<int64_t>(wcap, (b.tail_cap + 3) / 4), st);
   };
   if (!mixed) {
-    cudaError_t e = launch(0, grid_for(0, N));
+    cudaError_t e = launch(0);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "track kernel launch (FP64)");
     return FRG_OK;
   }
@@ -423,7 +445,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     a.back_count = nullptr;
     a.lo_keep_ill = (ctx->cfg.lo_final && rounds > 1 && r + 1 == rounds) ? 1 : 0;
     const int lo_mode = (team && ctx->cfg.lo_points == 1) ? 3 : 1;
-    cudaError_t e = launch(lo_mode, grid_for(lo_mode, N));
+    cudaError_t e = launch(lo_mode);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "track kernel launch (FP32 stage)");
     FRG_CUDA(ctx, cudaEventRecord(evs[2 * r + 1], st));
     a.queue = q + 1;
@@ -431,7 +453,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     a.lo_count = nullptr;
     a.back_list = (team && r + 1 < rounds) ? lo + (size_t)(r & 1) * N : nullptr;
     a.back_count = q + 3 + (r & 1);
-    e = launch(2, grid_for(2, N));
+    e = launch(2);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "track kernel launch (FP64 stage)");
     FRG_CUDA(ctx, cudaEventRecord(evs[2 * r + 2], st));
   }
@@ -631,7 +653,7 @@ static frg_status enqueue_rounds_carry(frg_ctx* ctx, const cx<double>* d_fpm, bo
   for (int d = 0; d < depth; ++d) {
     Slot& sl = *ctx->slots[d];
     FRG_CUDA(ctx, sl.lo_lists.ensure(sizeof(int64_t) * 3 * KN));
-    FRG_CUDA(ctx, sl.queue.ensure(sizeof(unsigned long long) * 8));
+    FRG_CUDA(ctx, sl.queue.ensure(sizeof(unsigned long long) * FRG_NQUEUE));
     FRG_CUDA(ctx, sl.counters.ensure(sizeof(unsigned long long) * FRG_NCOUNTERS));
     FRG_CUDA(ctx, sl.starts.ensure(sizeof(cx<double>) * frg::FRG_START_STRIDE * (size_t)N));
   }

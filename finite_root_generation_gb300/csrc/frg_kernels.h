@@ -24,6 +24,7 @@ struct Handoff {
   uint64_t rng_index;
   int streak, step, ministep, tstepQ, n_ivp, n_newton, reason, code;  // reason 6: finished with code
   int bounces, pad;  // times the path returned from FP64 to FP32
+  int64_t id;        // the path (tail records)
 };
 
 // Device-side arguments of one tracking launch. All arrays are device memory.
@@ -70,6 +71,10 @@ struct TrackArgs {
   int64_t* back_list;           // FP64 kernel: paths handed back to FP32 (null: none, e.g. the last round)
   unsigned long long* back_count;
   int sms;                      // the device's SMs
+  Handoff* tail;                // thread kernel: where a launch leaves its last paths (tail_cap records, 0 = none);
+  unsigned long long* tail_count;  // warp kernel with from_tail: the paths it continues
+  int64_t tail_cap;
+  int from_tail;
   int lo_keep_ill;              // FP32 kernel: 1 = no hand-off for ill-conditioned steps (last round)
   float* feat;                  // optional: FRG_MLP_IN features per checkpoint, feat_max checkpoints per path
   int32_t* nfeat;               // checkpoints written per path (zeroed before launch)
@@ -100,6 +105,27 @@ inline int frg_team_grid(int sms, int bps, int64_t n) {
   const int64_t grid = want < cap ? want : cap;
   return (int)(grid < 1 ? 1 : grid);
 }
+
+// A plug-in launch of at most this many paths per SM sub-partition tracks a path per warp,
+// a larger one a path per thread. FP64, GB300 (152 SMs), warp / thread: conic2 2,432 paths
+// 10.0 / 15.1 ms, 4,864 20.3 / 22.0, 9,728 32.1 / 30.2, 40,000 86 / 58; burmester5 4,864
+// 67 / 107, 19,456 587 / 555. FP32 stage and resume: conic2 4,864 4.4 / 4.9, 9,728 8.0 / 5.9;
+// burmester5 9,728 487 / 506.
+constexpr int FRG_WARP_PATHS = 8;
+
+// A warp of a thread-per-path launch gives its paths up to a warp-per-path launch when the
+// queue is empty and at most this many of its lanes still track one: a warp's step costs
+// the same with few lanes as with 32, four to seven times a warp_kernel step in FP64, less
+// in FP32 (120,000 conic2 paths, FP32 stage: 4 lanes 12.6 ms, 2 lanes 11.7, never 11.4; 8,192
+// burmester5 paths: 35, 37, 58 ms).
+__host__ __device__ constexpr int frg_tail_lanes(bool fp32) { return fp32 ? 2 : 4; }
+
+#define FRG_NQUEUE 16  // queue heads and counts of a slot
+
+// Warp-per-path kernel of the plug-in systems (mode and arguments as frg_launch_track's),
+// four paths per block.
+cudaError_t frg_launch_warp(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream);
+cudaError_t frg_warp_occupancy(int system, int mode, int* blocks_per_sm);
 
 // mode: 0 plain FP64, 1 FP32 stage with handoff, 2 FP64 resume of handed-off paths
 cudaError_t frg_launch_track(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream);

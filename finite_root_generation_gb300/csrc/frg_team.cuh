@@ -38,6 +38,7 @@
 
 #include "frg_device.cuh"
 #include "frg_df.cuh"
+#include "frg_warp.cuh"
 
 namespace frg {
 namespace team {
@@ -51,7 +52,6 @@ constexpr int TEAM = 8;    // lanes of one path in the evaluation (7 groups)
 constexpr int PATHS = 4;   // paths (warps) per block
 constexpr int VS = 24;     // shared-memory vector stride (23 used)
 constexpr int LDU = 21;    // leading dimension of the dense system and its factor (odd: no bank conflicts)
-constexpr unsigned FULL = 0xffffffffu;
 
 // reduced-system column -> state index
 __device__ __forceinline__ constexpr int gstate(int c) { return c < 14 ? c : (c == 14 ? 21 : 22); }
@@ -60,10 +60,6 @@ template <typename T>
 __device__ __forceinline__ T shfl_xor(unsigned mask, T v, int off) { return __shfl_xor_sync(mask, v, off, TEAM); }
 __device__ __forceinline__ df shfl_xor(unsigned mask, df v, int off) {
   return df(__shfl_xor_sync(mask, v.hi, off, TEAM), __shfl_xor_sync(mask, v.lo, off, TEAM));
-}
-template <typename T>
-__device__ __forceinline__ cx<T> warp_shfl(cx<T> v, int src) {
-  return cx<T>(__shfl_sync(FULL, v.re, src), __shfl_sync(FULL, v.im, src));
 }
 // sums and maxima over each group of 8 lanes (in every lane of the group)
 template <typename T>
@@ -80,57 +76,6 @@ __device__ __forceinline__ T team_max(unsigned mask, T v) {
   v = fmax(v, shfl_xor(mask, v, 1));
   return v;
 }
-
-// Largest |re| or |im| of values, NaN taking no part (as fmax drops it): FP32 directly,
-// FP64 on the bit patterns, whose order as integers is the order of the magnitudes.
-template <typename T> struct MaxAbs;
-template <> struct MaxAbs<float> {
-  float m = 0.f;
-  __device__ __forceinline__ void take(cx<float> v) { m = fmaxf(m, fmaxf(fabsf(v.re), fabsf(v.im))); }
-  __device__ __forceinline__ void across(int off) { m = fmaxf(m, __shfl_xor_sync(FULL, m, off)); }
-  __device__ __forceinline__ float value() const { return m; }
-};
-template <> struct MaxAbs<double> {
-  long long m = 0;
-  __device__ __forceinline__ void one(double x) {
-    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffll;
-    if (b > m && b <= 0x7ff0000000000000ll) m = b;
-  }
-  __device__ __forceinline__ void take(cx<double> v) { one(v.re); one(v.im); }
-  __device__ __forceinline__ void across(int off) {
-    const long long o = __shfl_xor_sync(FULL, m, off);
-    if (o > m) m = o;
-  }
-  __device__ __forceinline__ double value() const { return __longlong_as_double(m); }
-};
-
-// running maximum and minimum of magnitudes >= 0, NaN taking no part
-__device__ __forceinline__ float max_mag(float m, float x) { return fmaxf(m, x); }
-__device__ __forceinline__ float min_mag(float m, float x) { return fminf(m, x); }
-__device__ __forceinline__ double max_mag(double m, double x) {
-  const long long b = __double_as_longlong(x);
-  return b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll ? x : m;
-}
-__device__ __forceinline__ double min_mag(double m, double x) {
-  const long long b = __double_as_longlong(x);
-  return b >= 0 && b < __double_as_longlong(m) ? x : m;
-}
-
-// 1 / b when |b|^2 is at hand (FP64: conj(b) / |b|^2; FP32 keeps Smith's form)
-__device__ __forceinline__ cx<double> cinv_norm(cx<double> b, double n2) {
-  const double r = 1.0 / n2;
-  return cx<double>(b.re * r, -b.im * r);
-}
-__device__ __forceinline__ cx<float> cinv_norm(cx<float> b, float) { return cinv(b); }
-
-// products that no later addition may absorb into a fused multiply-add
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-template <typename T>
-__device__ __forceinline__ cx<T> mul_rn(T s, cx<T> a) { return cx<T>(mul_rn(s, a.re), mul_rn(s, a.im)); }
-// s * a + b, fused
-template <typename T>
-__device__ __forceinline__ cx<T> axpy(T s, cx<T> a, cx<T> b) { return cx<T>(fma(s, a.re, b.re), fma(s, a.im, b.im)); }
 
 // Task and start parameters in the working precision, when it is not the point type's.
 template <typename T, typename P> struct LowTask { cx<T> sp[32], fp[32]; };

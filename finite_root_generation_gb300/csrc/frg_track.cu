@@ -115,10 +115,11 @@ template <> __device__ __forceinline__ cx<float> task_gamma<float>(const TrackAr
   return a.gamma_lo[task];
 }
 
+// The path's state at the start of a step, what the reference's tracker carries across
+// its loop (htpytrack.cu:36-77).
 template <typename T, int NY_, int NP_>
-__device__ void save_handoff(const TrackArgs& a, const PathState<T, NY_, NP_>& P, int reason) {
+__device__ void save_state(Handoff& h, const PathState<T, NY_, NP_>& P) {
   static_assert(NY_ <= NY, "hand-off records hold at most Stephenson II's 23-entry path states");
-  Handoff& h = a.handoff[P.id];
 #pragma unroll 1
   for (int e = 0; e < NY_; ++e) {
     h.Yc[e] = cd(P.Yc[e]);
@@ -128,7 +129,15 @@ __device__ void save_handoff(const TrackArgs& a, const PathState<T, NY_, NP_>& P
   h.s = double(P.s);
   h.rng_index = P.rng.index;
   h.streak = P.streak; h.step = P.step; h.ministep = P.ministep; h.tstepQ = P.tstepQ;
-  h.n_ivp = P.n_ivp; h.n_newton = P.n_newton; h.reason = reason; h.code = 0;
+  h.n_ivp = P.n_ivp; h.n_newton = P.n_newton; h.reason = 0; h.code = 0;
+  h.id = P.id;
+}
+
+template <typename T, int NY_, int NP_>
+__device__ void save_handoff(const TrackArgs& a, const PathState<T, NY_, NP_>& P, int reason) {
+  Handoff& h = a.handoff[P.id];
+  save_state(h, P);
+  h.reason = reason;
   if (a.counters) { atomicAdd(&a.counters[12], 1ull); atomicAdd(&a.counters[15 + reason], 1ull); }
   const unsigned long long slot = atomicAdd(a.handoff_count, 1ull);
   a.handoff_list[slot] = P.id;
@@ -157,6 +166,7 @@ track_kernel(TrackArgs a) {
   // latter one long path's latency).
   const int64_t warps = (int64_t)gridDim.x * (FRG_TRACK_THREADS / 32);
   P.phase = (int64_t)(threadIdx.x & 31) * warps < nqueue ? PH_FETCH : PH_IDLE;
+  bool dry = false;  // this lane found the queue empty
 
   for (;;) {
     // ------------------------------------------------------------------ fetch
@@ -164,6 +174,7 @@ track_kernel(TrackArgs a) {
       const int64_t qi = (int64_t)atomicAdd(a.queue, 1ull);
       if (qi >= nqueue) {
         P.phase = PH_IDLE;
+        dry = true;
       } else {
         const int64_t id = (MODE == MODE_RESUME) ? a.handoff_list[qi] : qi;
         P.id = id;
@@ -207,8 +218,21 @@ track_kernel(TrackArgs a) {
     // The warp's lanes meet here each trip and again before the linear step, so that the
     // divergent control code does not leave them apart in it (262,144 conic2 paths in
     // FP64: 267 -> 250 ms, of which the longest paths' tail is the larger part).
-    const unsigned live = __ballot_sync(0xffffffffu, P.phase != PH_IDLE);
+    unsigned live = __ballot_sync(0xffffffffu, P.phase != PH_IDLE);
     if (!live) break;
+    if (a.tail_cap > 0 && __any_sync(0xffffffffu, dry) && __popc(live) <= frg_tail_lanes(LO)) {
+      // The queue is empty and this warp's step serves few paths: they go on, from their
+      // next step's start, in a warp_kernel launch, where a step is that much shorter.
+      if (P.phase == PH_RK && P.stage == 0) {
+        const unsigned long long slot = atomicAdd(a.tail_count, 1ull);
+        if ((int64_t)slot < a.tail_cap) {
+          save_state(a.tail[slot], P);
+          P.phase = PH_IDLE;
+        }
+      }
+      live = __ballot_sync(0xffffffffu, P.phase != PH_IDLE);
+      if (!live) break;
+    }
     if (P.phase == PH_IDLE) continue;
 
     // -------------------------------------------------- set up the linear step
@@ -479,6 +503,8 @@ __device__ void finish_path(const TrackArgs& a, int64_t id, int task, int code, 
 
 }  // namespace frg
 
+#include "frg_track_warp.cuh"
+
 namespace {
 __global__ void to_float_kernel(const cx<double>* in, cx<float>* out, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -516,6 +542,43 @@ cudaError_t frg_launch_track(int mode, const frg::TrackArgs& args, int grid, cud
     case frg::MODE_PLAIN: return launch<frg::MODE_PLAIN, double>(args, grid, stream);
     case frg::MODE_LO: return launch<frg::MODE_LO, float>(args, grid, stream);
     case frg::MODE_RESUME: return launch<frg::MODE_RESUME, double>(args, grid, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+namespace {
+template <int MODE, typename T, class S>
+cudaError_t launch_warp(const frg::TrackArgs& args, int grid, cudaStream_t stream) {
+  frg::warp_kernel<MODE, T, S><<<grid, 32 * frg::WARP_PATHS, 0, stream>>>(args);
+  return cudaGetLastError();
+}
+template <int MODE, typename T, class S>
+cudaError_t warp_occ(int* blocks_per_sm) {
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, frg::warp_kernel<MODE, T, S>,
+                                                       32 * frg::WARP_PATHS, 0);
+}
+}  // namespace
+
+cudaError_t frg_launch_warp(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream) {
+  switch (args.cfg.system * 4 + mode) {
+#define FRG_PLUGIN_WARP(id, name, S)                                                                             \
+  case id * 4 + frg::MODE_PLAIN: return launch_warp<frg::MODE_PLAIN, double, S>(args, grid, stream);             \
+  case id * 4 + frg::MODE_LO: return launch_warp<frg::MODE_LO, float, S>(args, grid, stream);                    \
+  case id * 4 + frg::MODE_RESUME: return launch_warp<frg::MODE_RESUME, double, S>(args, grid, stream);
+    FRG_PLUGIN_LIST(FRG_PLUGIN_WARP)
+#undef FRG_PLUGIN_WARP
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t frg_warp_occupancy(int system, int mode, int* blocks_per_sm) {
+  switch (system * 4 + mode) {
+#define FRG_PLUGIN_WARP_OCC(id, name, S)                                                                         \
+  case id * 4 + frg::MODE_PLAIN: return warp_occ<frg::MODE_PLAIN, double, S>(blocks_per_sm);                     \
+  case id * 4 + frg::MODE_LO: return warp_occ<frg::MODE_LO, float, S>(blocks_per_sm);                            \
+  case id * 4 + frg::MODE_RESUME: return warp_occ<frg::MODE_RESUME, double, S>(blocks_per_sm);
+    FRG_PLUGIN_LIST(FRG_PLUGIN_WARP_OCC)
+#undef FRG_PLUGIN_WARP_OCC
     default: return cudaErrorInvalidValue;
   }
 }

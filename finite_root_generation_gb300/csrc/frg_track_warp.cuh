@@ -1,0 +1,542 @@
+// Warp-per-path tracker of the plug-in systems: the state machine, decisions, counters and
+// random draws of track_kernel (frg_track.cu, which includes this file), with one path's
+// linear step spread over a warp's lanes. The results are those of track_kernel bit for bit.
+//
+// What bounds it: one thread's step is a serial chain, for burmester5 about 2,200 FP64
+// instructions of some 75 cycles each (80 us), whatever the other lanes do, and the longest
+// of a launch's paths takes thousands of steps. Here the rows come from the generated
+// schedule (16 independent complex operations a step, one lane per real component: 29
+// FP64 instructions where the straight-line code has 834), the parameters q(t) take one
+// lane each, the elimination a lane per row and column class, the back substitution a
+// lane per real component. GB300, thread / warp: 64 burmester5 paths FP64 135 / 18 ms, 64
+// conic2 paths 16.2 / 3.3 ms, mixed 4.8 / 1.3 ms; a 3,000-step path 2,250 / 460 ms.
+//
+// Sums of products in the stage combinations and the error's squares are rounded as
+// track_kernel's compiled form rounds them (product, then sum; re * re fused onto im * im),
+// spelled out so that no compiler choice can separate the two kernels.
+#pragma once
+
+#include "frg_device.cuh"
+#include "frg_kernels.h"
+#include "frg_warp.cuh"
+
+namespace frg {
+
+constexpr int WARP_PATHS = 4;  // warps (paths) per block
+
+// Shared state of one path. `reg` is the schedule's register file: the point's homogeneous
+// unknowns, q(t), dq/dt, constants, results. Row r of the linear system: M[r * LD ...],
+// right-hand side in column NY.
+template <typename T, class S>
+struct WarpPath {
+  static constexpr int NV = S::NV, NZ = NV + 1, NY = NV + 2, NP = S::NP, LD = NY + 2;
+  cx<T> Yc[NY], Vc[NY], Yn[NY], Vn[NY], YN[NY], u[NY], x[NY];
+  cx<T> k[8][NY];
+  cx<T> sp[NP], fp[NP];
+  cx<T> reg[S::TAPE_REGS];
+  cx<T> M[NY * LD];
+  cx<T> ip[NY];
+  T t;
+  T cn[NY];
+  int row[NY];
+};
+
+template <typename T>
+struct WarpStep {
+  T ratio;  // pivot ratio (FP32 stage)
+  T xnorm;  // |x| (corrector)
+  T hnorm;  // |H| (corrector, when asked for)
+};
+
+// sum_{i < n} |v_i|^2 in index order from the magnitudes in cn
+template <typename T>
+__device__ __forceinline__ T sum_in_order(const T* cn, int n) {
+  T s = T(0);
+#pragma unroll 8
+  for (int i = 0; i < n; ++i) s += cn[i];
+  return s;
+}
+
+// One linear step at the point in W.reg[0..NZ), W.t, as track_kernel's: rows, patch rows,
+// row scaling, elimination with partial pivoting (first maximum by the rows' current
+// order, kept as a position per row instead of moving rows), back substitution; a
+// tangent is normalised. The solution goes to W.x.
+template <bool LO, typename T, class S>
+__device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32_t* tape, const uint16_t* outs,
+                                                 cx<T> gamma, const cx<T>* patch, bool newton, bool tstep, T tgoal,
+                                                 bool want_hnorm, int lane) {
+  typedef WarpPath<T, S> P;
+  constexpr int NV = P::NV, NZ = P::NZ, NY = P::NY, NP = P::NP, LD = P::LD;
+  static_assert(NY <= 32, "a lane per row");
+  constexpr int RP = NY <= 4 ? 4 : (NY <= 8 ? 8 : (NY <= 16 ? 16 : 32));  // lanes for the rows
+  constexpr int CL = 32 / RP;                                             // column classes
+  const bool im = lane & 1;
+  WarpStep<T> out;
+  out.ratio = out.xnorm = out.hnorm = T(0);
+
+  // ---- q(t), dq/dt (htpysupport.cu:37-62)
+  {
+    const T t = W.t;
+    const cx<T> g1t = gamma * (T(1) - t);
+    const cx<T> iden = cinv(g1t + cx<T>(t));
+    const cx<T> gid2 = gamma * (iden * iden);
+#pragma unroll 1
+    for (int i = lane; i < NP; i += 32) {
+      const cx<T> s = W.sp[i], f = W.fp[i];
+      W.reg[NZ + i] = (g1t * s + t * f) * iden;
+      W.reg[NZ + NP + i] = (f - s) * gid2;
+    }
+  }
+  __syncwarp();
+  // ---- the rows: lane 2 o + c computes component c of the step's operation o
+#pragma unroll 1
+  for (int st = 0; st < S::TAPE_STEPS; ++st) {
+    const uint32_t w = tape[st * 16 + (lane >> 1)];
+    const cx<T> a = W.reg[(w >> 10) & 1023], b = W.reg[(w >> 20) & 1023];
+    T r;
+    if (w >> 31) {
+      r = im ? fma(a.re, b.im, mul_rn(a.im, b.re)) : fma(a.re, b.re, mul_rn(-a.im, b.im));
+    } else {
+      const T x = im ? a.im : a.re, y = im ? b.im : b.re;
+      r = x + ((w >> 30) & 1 ? -y : y);
+    }
+    reinterpret_cast<T*>(&W.reg[w & 1023])[im] = r;
+    __syncwarp();
+  }
+  // ---- the system: rows, projective patch (htpysupport.cu:139-142), velocity patch
+#pragma unroll 1
+  for (int o = lane; o < NV * NY; o += 32) {
+    const unsigned w = outs[o];
+    const cx<T> v = W.reg[w & 1023];
+    W.M[(o / NY) * LD + o % NY] = (w >> 10) ? -v : v;
+  }
+  if (lane < NY) {
+    W.M[NV * LD + lane] = W.u[lane];
+    W.M[(NV + 1) * LD + lane] = patch[lane];
+    if (!newton) W.M[lane * LD + NY] = cx<T>(T(lane == NY - 1 ? 1 : 0));
+  }
+  if (newton) {
+    if (lane < NV) {
+      const unsigned w = outs[NV * NY + lane];
+      const cx<T> v = W.reg[w & 1023];
+      W.M[lane * LD + NY] = (w >> 10) ? -v : v;
+    }
+    // u . Y - 1, one lane per component
+    T d = T(0);
+#pragma unroll 8
+    for (int e = 0; e < NY; ++e) {
+      const cx<T> b = W.u[e], y = e < NZ ? W.reg[e] : cx<T>(W.t);
+      d = im ? fma(b.im, y.re, fma(b.re, y.im, d)) : fma(-b.im, y.im, fma(b.re, y.re, d));
+    }
+    d -= im ? T(0) : T(1);
+    if (lane < 2) reinterpret_cast<T*>(&W.M[NV * LD + NY])[im] = d;
+    __syncwarp();
+    if (want_hnorm) {
+      if (lane < NZ) W.cn[lane] = cnorm2(W.M[lane * LD + NY]);
+      __syncwarp();
+      out.hnorm = sqrt(sum_in_order(W.cn, NZ));
+    }
+  }
+  __syncwarp();
+  // ---- row scaling by 1/max(|re|,|im|) (htpysupport.cu:259-277, :446-471); b = -F
+  const int r = lane % RP, cl = lane / RP;
+  {
+    MaxAbs<T> m;
+    if (r < NZ)
+      for (int c = cl; c < NY; c += CL) m.take(W.M[r * LD + c]);
+#pragma unroll
+    for (int off = RP; off < 32; off <<= 1) m.across(off);
+    const T s = T(1) / m.value();
+    if (r < NZ)
+      for (int c = cl; c < (newton ? NY + 1 : NY); c += CL) {
+        const cx<T> v = s * W.M[r * LD + c];
+        W.M[r * LD + c] = c == NY ? -v : v;
+      }
+  }
+  __syncwarp();
+  // ---- elimination (htpysupport.cu:146-232; the corrector leaves the last row out,
+  //      :302-400)
+  const int nelim = newton ? NZ : NY;
+  int pos = r;  // current position of row r
+  T pmax = T(0), pmin = T(-1);
+#pragma unroll 1
+  for (int i = 0; i < nelim; ++i) {
+    const cx<T> e = W.M[(r < NY ? r : 0) * LD + i];
+    const bool live = r < NY && pos >= i && pos < nelim;
+    const T v = cnorm2(e);
+    int pr = -1;
+    {
+      // rows with a magnitude above zero, not NaN, compared as integers
+      unsigned cand;
+      if constexpr (sizeof(T) == 8) {
+        const long long bits = __double_as_longlong(v);
+        const bool ok = live && bits > 0 && bits <= 0x7ff0000000000000ll;
+        const int hi = ok ? (int)(bits >> 32) : -1;
+        const int mh = __reduce_max_sync(FULL, hi);
+        const unsigned lo = ok && hi == mh ? (unsigned)bits : 0u;
+        cand = __ballot_sync(FULL, ok && hi == mh);
+        if (__popc(cand) > CL) {
+          const unsigned ml = __reduce_max_sync(FULL, lo);
+          cand = __ballot_sync(FULL, ok && hi == mh && (unsigned)bits == ml);
+        }
+      } else {
+        const int bits = __float_as_int(v);
+        const bool ok = live && bits > 0 && bits <= 0x7f800000;
+        const int mh = __reduce_max_sync(FULL, ok ? bits : -1);
+        cand = __ballot_sync(FULL, ok && bits == mh);
+      }
+      if (cand) {
+        if (__popc(cand) > CL) {  // equal magnitudes: the first by position
+          const int mp = __reduce_min_sync(FULL, (cand >> lane) & 1 ? pos : 99);
+          cand = __ballot_sync(FULL, pos == mp && r < NY);
+        }
+      } else {
+        cand = __ballot_sync(FULL, pos == i && r < NY);
+      }
+      pr = (__ffs(cand) - 1) % RP;
+    }
+    const int ppos = __shfl_sync(FULL, pos, pr);
+    if (r == pr) pos = i;
+    else if (pos == i) pos = ppos;
+    const cx<T> pe = W.M[pr * LD + i];
+    const T pa = __shfl_sync(FULL, v, pr);
+    const cx<T> ip = cinv_norm(pe, pa);
+    if (lane == 0) { W.ip[i] = ip; W.row[i] = pr; }
+    if (LO) {
+      const T a = sqrt(pa);
+      pmax = fmax(pmax, a);
+      pmin = (pmin < T(0)) ? a : fmin(pmin, a);
+    }
+    if (r < NY && pos > i && pos < nelim) {
+      const cx<T> l = e * ip;
+#pragma unroll 2
+      for (int c = i + 1 + cl; c <= NY; c += CL) W.M[r * LD + c] = cfms(W.M[r * LD + c], W.M[pr * LD + c], l);
+    }
+    __syncwarp();
+  }
+  if (LO) out.ratio = pmin > T(0) ? pmax / pmin : T(1e30);
+  // ---- back substitution, row by row, one lane per component
+  int top = NY - 1;
+  if (newton) {
+    if (lane == 0) W.x[NY - 1] = cx<T>(tgoal - W.t);
+    top = NY - 2;
+    __syncwarp();
+  }
+#pragma unroll 1
+  for (int i = top; i >= 0; --i) {
+    const cx<T>* m = W.M + W.row[i] * LD;
+    T sum = T(0);
+#pragma unroll 2
+    for (int c = i + 1; c < NY; ++c) {
+      const cx<T> b = m[c], xc = W.x[c];
+      sum = im ? fma(b.im, xc.re, fma(b.re, xc.im, sum)) : fma(-b.im, xc.im, fma(b.re, xc.re, sum));
+    }
+    const T d = (im ? m[NY].im : m[NY].re) - sum, o = __shfl_xor_sync(FULL, d, 1);
+    const cx<T> ip = W.ip[i], v = im ? cx<T>(o, d) : cx<T>(d, o);
+    const T xi = im ? fma(ip.re, v.im, mul_rn(ip.im, v.re)) : fma(ip.re, v.re, mul_rn(-ip.im, v.im));
+    if (lane < 2) reinterpret_cast<T*>(&W.x[i])[im] = xi;
+    __syncwarp();
+  }
+  // ---- |x|, and the tangent's normalisation (htpysupport.cu:285-296)
+  const cx<T> xe = W.x[lane < NY ? lane : 0];
+  if (lane < NY) W.cn[lane] = cnorm2(xe);
+  __syncwarp();
+  const T n2 = sum_in_order(W.cn, NY);
+  if (newton) {
+    out.xnorm = sqrt(n2);
+  } else {
+    const cx<T> xt = W.x[NY - 1];
+    cx<T> sc;
+    if (!tstep) {
+      const T nr = sqrt((lane & 1) ? n2 : cnorm2(xt));
+      sc = cx<T>(xt.re, -xt.im) * (T(1) / (__shfl_sync(FULL, nr, 0) * __shfl_sync(FULL, nr, 1)));
+    } else {
+      sc = cinv(xt);
+    }
+    __syncwarp();
+    if (lane < NY) {
+      cx<T> v = sc * xe;
+      if (lane == NY - 1) v.im = T(0);
+      W.x[lane] = v;
+    }
+  }
+  __syncwarp();
+  return out;
+}
+
+// A new random patch (entry e from draws base + 2 e, base + 2 e + 1)
+template <typename T>
+__device__ __forceinline__ cx<T> patch_entry(uint64_t seed, uint64_t stream, uint64_t base, double range, int e) {
+  return cx<T>(T(2.0 * range * frg_uniform01(seed, stream, base + 2 * e) - range),
+               T(2.0 * range * frg_uniform01(seed, stream, base + 2 * e + 1) - range));
+}
+
+// Modes as track_kernel's. With a.from_tail the launch continues the paths that a
+// track_kernel launch of the same mode left in a.tail.
+template <int MODE, typename T, class S>
+__global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
+  typedef WarpPath<T, S> P;
+  constexpr int NV_ = P::NV, NZ_ = P::NZ, NY_ = P::NY, NP_ = P::NP;
+  constexpr bool LO = (MODE == MODE_LO);
+  __shared__ P paths[WARP_PATHS];
+  __shared__ uint32_t tape[S::TAPE_STEPS * 16];
+  __shared__ uint16_t outs[NV_ * NY_ + NV_];
+  const frg_config& c = a.cfg;
+  const int lane = threadIdx.x & 31;
+  const bool el = lane < NY_;
+  P& W = paths[threadIdx.x >> 5];
+  for (int i = threadIdx.x; i < S::TAPE_STEPS * 16; i += blockDim.x) tape[i] = S::tape()[i];
+  for (int i = threadIdx.x; i < NV_ * NY_ + NV_; i += blockDim.x) outs[i] = S::tape_out()[i];
+  for (int i = lane; i < S::TAPE_REGS; i += 32) W.reg[i] = cx<T>(T(0));
+  __syncthreads();
+  if (lane < S::TAPE_CONSTS) W.reg[NZ_ + 2 * NP_ + lane] = cx<T>(T(S::tape_const()[lane]));
+  const T newt_tol = LO ? T(c.newt_tol_lo) : T(c.newt_tol);
+  const int64_t ntail = a.from_tail ? (int64_t)*a.tail_count : 0;
+  const int64_t nqueue = a.from_tail ? (ntail < a.tail_cap ? ntail : a.tail_cap)
+                         : (MODE == MODE_RESUME) ? (int64_t)*a.handoff_count : a.npaths;
+  unsigned long long fp64_solves = 0;
+
+  for (;;) {
+    // ------------------------------------------------------------------ fetch
+    unsigned long long qi = 0;
+    if (lane == 0) qi = atomicAdd(a.queue, 1ull);
+    qi = __shfl_sync(FULL, qi, 0);
+    if ((int64_t)qi >= nqueue) break;
+    const int64_t id = a.from_tail ? a.tail[qi].id : (MODE == MODE_RESUME) ? a.handoff_list[qi] : (int64_t)qi;
+    const bool resumed = MODE == MODE_RESUME || a.from_tail;
+    int task = 0, hi = a.ntasks - 1;  // task of this path
+    while (task < hi) {
+      const int mid = (task + hi + 1) >> 1;
+      if (a.task_start[mid] <= id) task = mid; else hi = mid - 1;
+    }
+    const uint64_t stream = (uint64_t)(id + c.path_offset);
+    const cx<T> gamma = task_gamma<T>(a, task);
+    if (lane == 0) {
+      Rng rng;
+      rng.seed = a.seed; rng.stream = stream; rng.index = 0;
+      cd spt[NV_], spm[NP_];
+      S::start(rng, c.start_dist, c.start_range, spt, spm);
+#pragma unroll 1
+      for (int e = 0; e < NP_; ++e) W.sp[e] = cx<T>(spm[e]);
+      if (!resumed) {
+#pragma unroll 1
+        for (int e = 0; e < NV_; ++e) W.Yc[e] = cx<T>(spt[e]);
+        W.Yc[NV_] = cx<T>(T(1));
+        W.Yc[NV_ + 1] = cx<T>(T(0));
+      }
+    }
+    const cx<T>* fpmT = TaskFpm<T, NP_>::get(a, task);
+    for (int i = lane; i < NP_; i += 32) W.fp[i] = fpmT[i];
+    T s = T(0), err = T(0), scale = T(0), residual = T(100);
+    int tstepQ = 0, streak = 0, step = 0, ministep = 0, stage = 0, attempt = 0, it = 0, code = 0;
+    int n_ivp = 0, n_newton = 0, phase = PH_TANGENT0;
+    uint64_t rng_index = 4 * NY_;
+    if (resumed) {
+      const Handoff& h = a.from_tail ? a.tail[qi] : a.handoff[id];
+      if (el) { W.Yc[lane] = cx<T>(h.Yc[lane]); W.Vc[lane] = cx<T>(h.Vc[lane]); W.u[lane] = cx<T>(h.u[lane]); }
+      s = T(h.s); rng_index = h.rng_index; streak = h.streak; step = h.step; ministep = h.ministep;
+      tstepQ = h.tstepQ; n_ivp = h.n_ivp; n_newton = h.n_newton;
+      phase = PH_RK;
+    } else {
+      if (el) {
+        W.u[lane] = patch_entry<T>(a.seed, stream, 0, c.patch_range, lane);
+        W.Vc[lane] = patch_entry<T>(a.seed, stream, 2 * NY_, c.patch_range, lane);
+      }
+      __syncwarp();
+      if (lane == 0) switch_patch<T, NY_>(W.u, W.Yc, W.Yc);
+      s = T(c.s_init); streak = c.caution_steps - 1;
+    }
+    __syncwarp();
+
+    for (;;) {  // the path's steps
+      // ------------------------------------------------ set up the linear step
+      const bool newton = (phase == PH_NEWTON || phase == PH_SHARP);
+      const bool tstep = phase == PH_RK && tstepQ != 0;
+      const cx<T>* patch = W.Vc;
+      cx<T> y;
+      if (phase == PH_TANGENT0 || (phase == PH_RK && stage == 0)) {
+        y = W.Yc[el ? lane : 0];
+      } else if (phase == PH_RK) {
+        patch = W.k[stage - 1];
+        const T ws = lane < stage ? T(c_dpA[stage][lane]) * s : T(0);
+        cx<T> acc = mul_rn(__shfl_sync(FULL, ws, stage - 1), W.k[stage - 1][el ? lane : 0]);
+        for (int l = stage - 2; l >= 0; --l) acc = mul_rn(__shfl_sync(FULL, ws, l), W.k[l][el ? lane : 0]) + acc;
+        y = W.Yc[el ? lane : 0] + acc;
+      } else {
+        y = W.YN[el ? lane : 0];
+      }
+      if (lane < NZ_) W.reg[lane] = y;
+      if (lane == NY_ - 1) W.t = y.re;
+      const T tgoal = (phase == PH_SHARP) ? T(1) : W.Yn[NY_ - 1].re;
+      __syncwarp();
+
+      // ------------------------------------------------------ the linear step
+      const bool sharp = phase == PH_SHARP;
+      const int restype = sharp ? c.sharp_residual : c.newt_residual;
+      if (MODE != MODE_LO) fp64_solves++;
+      const WarpStep<T> r = warp_step<LO, T, S>(W, tape, outs, gamma, patch, newton, tstep, tgoal,
+                                                newton && restype == 0, lane);
+      if (newton) n_newton++; else n_ivp++;
+
+      // ------------------------------------------------------------- transitions
+      bool finished = false;
+      int handoff = 0;
+      const cx<T>* final_src = W.Yc;  // the reference's Yc aliases Yfinal (htpytrack.cu:46)
+      if (LO && !(r.ratio <= T(c.cond_switch))) {
+        handoff = 2;  // ill-conditioned (or non-finite) step: continue in FP64 from Yc
+      } else if (phase == PH_TANGENT0) {
+        if (el) W.Vc[lane] = W.x[lane];
+        if (c.max_steps == 0) { code = 1; finished = true; }
+        stage = 0;
+        phase = PH_RK;
+      } else if (phase == PH_RK) {
+        if (el) W.k[stage][lane] = W.x[lane];
+        __syncwarp();
+        if (++stage == 8) {
+          stage = 0;
+          // error estimate and step factor (rungekutta.cu:99-112), prediction (:115-122)
+          const T we = T(c_dpE[lane & 7]) * s, wb = T(c_dpB[lane & 7]) * s;
+          const cx<T> k7 = W.k[7][el ? lane : 0];
+          cx<T> le = mul_rn(__shfl_sync(FULL, we, 7), k7);
+          cx<T> yb = mul_rn(__shfl_sync(FULL, wb, 7), k7);
+#pragma unroll
+          for (int l = 6; l >= 0; --l) {
+            if (l == 1) continue;  // weight zero in both
+            const cx<T> kl = W.k[l][el ? lane : 0];
+            le = mul_rn(__shfl_sync(FULL, we, l), kl) + le;
+            yb = mul_rn(__shfl_sync(FULL, wb, l), kl) + yb;
+          }
+          if (el) {
+            W.cn[lane] = fma(le.re, le.re, mul_rn(le.im, le.im));
+            W.Yn[lane] = W.Yc[lane] + yb;
+            W.Vn[lane] = k7;
+          }
+          __syncwarp();
+          err = sqrt(sum_in_order(W.cn, NY_));
+          scale = (err > T(10e-17)) ? T(0.8) * pow(T(c.rk_tol) / err, T(1) / T(6)) : T(5);
+          if (scale > T(5)) scale = T(5);
+          if (ministep++ == c.max_ministeps) { code = 2; finished = true; }
+          else if (err <= T(c.rk_tol)) {
+            const T tn = W.Yn[NY_ - 1].re;
+            if (LO && tn > T(1.0 - c.nudge_trigger)) handoff = 5;  // the endgame runs in FP64
+            else if (tn <= T(1.0 - c.nudge_trigger)) { attempt = 0; phase = PH_NEWTON; }
+            else if (fabs(T(1) - tn) < T(c.sharp_trigger)) { attempt = 0; phase = PH_SHARP; }
+            else { tstepQ = 1; s = T(1) - W.Yc[NY_ - 1].re; }  // land on t = 1 (htpytrack.cu:120-123)
+            if (phase != PH_RK) {
+              if (el) W.YN[lane] = W.Yn[lane];
+              residual = T(100);
+              it = 0;
+            }
+          } else if (s <= T(c.s_min)) {
+            if (LO) handoff = 4; else { code = 3; finished = true; }
+          } else {
+            s *= scale;
+            if (s < T(c.s_min)) s = T(c.s_min * 0.9);
+            streak = 0;
+          }
+        }
+      } else {
+        // one corrector or sharpening iteration (htpysupport.cu:427-492)
+        const int max_its = sharp ? c.sharp_its : c.newt_its;
+        const T tol = sharp ? T(c.sharp_tol) : newt_tol;
+        bool done = false;
+        if (restype == 0 && it > 0) {
+          // |H| at the current point is the residual of the previous update
+          residual = r.hnorm;
+          if (!(it < max_its && residual > tol)) done = true;
+        }
+        if (!done) {
+          if (el) W.YN[lane] += W.x[lane];
+          it++;
+          if (restype != 0) {
+            residual = r.xnorm;
+            if (!(it < max_its && residual > tol)) done = true;
+          }
+        }
+        __syncwarp();
+        if (done) {
+          if (sharp) final_src = W.YN;
+          const bool ok = residual < (sharp ? T(c.sharp_tol) : newt_tol);
+          if (ministep++ == c.max_ministeps) { code = 2; finished = true; }
+          else if (ok && sharp) { code = 0; finished = true; }
+          else if (ok) {
+            if (fabs(T(1) - W.Yn[NY_ - 1].re) < T(c.sharp_trigger)) {
+              attempt = 0; phase = PH_SHARP; residual = T(100); it = 0;
+              if (el) W.YN[lane] = W.Yn[lane];
+            } else {
+              // accept the step (htpytrack.cu:176-183)
+              if (el) { W.Yc[lane] = W.YN[lane]; W.Vc[lane] = W.Vn[lane]; }
+              streak++;
+              if (streak < c.caution_steps && scale > T(1)) scale = T(1);
+              s *= scale;
+              if (s > T(c.s_max)) s = T(c.s_max);
+              else if (s < T(c.s_min)) s = T(c.s_min * 0.9);
+              step++;
+              if (step == c.max_steps) { code = 1; finished = true; }
+              else if (LO && W.YN[NY_ - 1].re >= T(c.t_switch)) handoff = 1;
+              else { stage = 0; phase = PH_RK; }
+            }
+          } else {
+            // new random patch and retry (htpytrack.cu:145-153, :204-213)
+            if (el) W.u[lane] = patch_entry<T>(a.seed, stream, rng_index, c.patch_range, lane);
+            rng_index += 2 * NY_;
+            __syncwarp();
+            if (lane == 0) switch_patch<T, NY_>(W.u, W.Yn, W.Yn);
+            __syncwarp();
+            if (++attempt < (sharp ? c.sharp_attempts : c.newt_attempts)) {
+              residual = T(100); it = 0;
+              if (el) W.YN[lane] = W.Yn[lane];
+            } else if (sharp) {
+              code = 5; finished = true;
+            } else if (s <= T(c.s_min)) {
+              if (LO) handoff = 3; else { code = 4; finished = true; }
+            } else {
+              s *= T(0.5);
+              if (s < T(c.s_min)) s = T(c.s_min * 0.9);
+              streak = 0;
+              stage = 0;
+              phase = PH_RK;
+            }
+          }
+        }
+      }
+      __syncwarp();
+      if (LO && handoff) {
+        Handoff& h = a.handoff[id];
+        if (el) { h.Yc[lane] = cd(W.Yc[lane]); h.Vc[lane] = cd(W.Vc[lane]); h.u[lane] = cd(W.u[lane]); }
+        if (lane == 0) {
+          h.s = double(s); h.rng_index = rng_index; h.streak = streak; h.step = step; h.ministep = ministep;
+          h.tstepQ = tstepQ; h.n_ivp = n_ivp; h.n_newton = n_newton; h.reason = handoff; h.code = 0;
+          if (a.counters) { atomicAdd(&a.counters[12], 1ull); atomicAdd(&a.counters[15 + handoff], 1ull); }
+          const unsigned long long slot = atomicAdd(a.handoff_count, 1ull);
+          a.handoff_list[slot] = id;
+        }
+        __syncwarp();
+        break;
+      }
+      if (finished) {
+        if (lane == 0) {
+          cd Yf[NY_];
+#pragma unroll 1
+          for (int e = 0; e < NY_; ++e) Yf[e] = cd(final_src[e]);
+          finish_path<S>(a, id, task, code, Yf, a.fpm + (size_t)task * NP_);
+          if (a.work) {
+            a.work[(size_t)id * 3 + 0] = n_ivp;
+            a.work[(size_t)id * 3 + 1] = n_newton;
+            a.work[(size_t)id * 3 + 2] = step;
+          }
+          if (a.counters) {
+            atomicAdd(&a.counters[8], (unsigned long long)n_ivp);
+            atomicAdd(&a.counters[9], (unsigned long long)n_newton);
+            atomicAdd(&a.counters[10], (unsigned long long)step);
+          }
+        }
+        __syncwarp();
+        break;
+      }
+    }
+  }
+  if (a.counters && fp64_solves && lane == 0) atomicAdd(&a.counters[11], fp64_solves);
+}
+
+}  // namespace frg

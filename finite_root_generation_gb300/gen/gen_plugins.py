@@ -268,17 +268,161 @@ def emit_start(mod, info, dialect):
     return lines
 
 
+class Tape:
+    """rows() as a schedule of complex operations for a warp: pairs of lanes (one per real
+    component) take one operation each, so a step is up to WIDTH products or sums that do not
+    depend on each other. Operations, operand order and the association of sums and products
+    are the printed code's; a minus sign travels with a value's use ((-a) b = -(a b) and
+    (-a) + b = -(a - b) round alike), so the results are the same bit for bit."""
+
+    WIDTH = 16
+
+    def __init__(self, info):
+        self.leaf, self.nodes, self.memo = {}, [], {}
+        nz, np_ = info["nv"] + 1, info["np"]
+        for i, x in enumerate(info["X"] + [info["z0"]]):
+            self.leaf[x] = i
+        for i, (q, d) in enumerate(zip(info["Q"], info["dq"])):
+            self.leaf[q], self.leaf[d] = nz + i, nz + np_ + i
+        self.ninputs = nz + 2 * np_
+        self.consts = [0.0]  # register ninputs + k holds constant k
+        flat = [e for row in info["jac"] for e in row] + info["Fh"]
+        repl, red = cse_block(flat, "r_")
+        self.env = {}
+        for s_, e in repl:
+            self.env[s_] = self.expr(e)
+        self.outs = [self.expr(e) if e != 0 else (("c", 0), 1) for e in red]
+        self.schedule()
+
+    def const(self, v):
+        if v not in self.consts:
+            self.consts.append(v)
+        return ("c", self.consts.index(v))
+
+    def op(self, kind, a, b, sub=0):
+        key = (kind, a, b, sub)
+        if key not in self.memo:
+            self.memo[key] = ("n", len(self.nodes))
+            self.nodes.append(key)
+        return self.memo[key]
+
+    def mul(self, x, y):
+        return self.op("mul", x[0], y[0]), x[1] * y[1]
+
+    def add(self, x, y):
+        return self.op("add", x[0], y[0], int(x[1] != y[1])), x[1]
+
+    def scale(self, c, x):
+        """|c| x as the printer's real-scalar product (exact for 2: x + x)."""
+        if c == 2.0:
+            return self.op("add", x[0], x[0], 0), x[1]
+        return self.op("mul", self.const(c), x[0]), x[1]
+
+    def expr(self, e):
+        if e.is_Symbol:
+            return self.env[e] if e in self.env else (("i", self.leaf[e]), 1)
+        if e.is_Number:
+            return self.const(abs(float(e))), 1 if e >= 0 else -1
+        if isinstance(e, sp.Pow):
+            return self.product([self.expr(e.base)] * int(e.exp))
+        if isinstance(e, sp.Mul):
+            coeff, rest = e.as_coeff_Mul()
+            body = self.product([self.expr(f) for f in sp.Mul.make_args(rest)])
+            c = float(coeff)
+            if abs(c) != 1.0:
+                body = self.scale(abs(c), body)
+            return body[0], body[1] * (1 if c > 0 else -1)
+        if isinstance(e, sp.Add):
+            out = None
+            for t in sp.Add.make_args(e):
+                v = self.expr(t)
+                out = v if out is None else self.add(out, v)
+            return out
+        raise TypeError(type(e), e)
+
+    def product(self, parts):
+        out = parts[0]
+        for v in parts[1:]:
+            out = self.mul(out, v)
+        return out
+
+    def reg(self, ref):
+        kind, k = ref
+        return {"i": 0, "c": self.ninputs, "n": self.ninputs + len(self.consts)}[kind] + k
+
+    def schedule(self):
+        """Steps of at most WIDTH ready operations of one kind, those with the longest chain
+        of FP64 instructions after them first (a product is 2 instructions, a sum 1)."""
+        users = [[] for _ in self.nodes]
+        for k, (_, a, b, _) in enumerate(self.nodes):
+            for r in (a, b):
+                if r[0] == "n":
+                    users[r[1]].append(k)
+        height = [0] * len(self.nodes)
+        for k in reversed(range(len(self.nodes))):
+            height[k] = (2 if self.nodes[k][0] == "mul" else 1) + max([height[u] for u in users[k]], default=0)
+        done, left, self.steps = set(), set(range(len(self.nodes))), []
+        while left:
+            ready = sorted((k for k in left if all(r[0] != "n" or r[1] in done for r in self.nodes[k][1:3])),
+                           key=lambda k: (-height[k], k))
+            kind = self.nodes[ready[0]][0]
+            pick = [k for k in ready if self.nodes[k][0] == kind][:self.WIDTH]
+            self.steps.append(pick)
+            done |= set(pick)
+            left -= set(pick)
+        self.nregs = self.ninputs + len(self.consts) + len(self.nodes) + 1  # the last one takes idle lanes' results
+        if self.nregs > 1024:
+            raise ValueError("too many operations for the tape's 10-bit registers")
+
+    def words(self):
+        """WIDTH words per step: dst | a << 10 | b << 20 | (b subtracted) << 30 | product << 31."""
+        out = []
+        for pick in self.steps:
+            mul = self.nodes[pick[0]][0] == "mul"
+            for k in pick:
+                _, a, b, sub = self.nodes[k]
+                out.append(self.reg(("n", k)) | self.reg(a) << 10 | self.reg(b) << 20 | sub << 30 | mul << 31)
+            out += [(self.nregs - 1) | mul << 31] * (self.WIDTH - len(pick))
+        return out
+
+    def out_words(self):
+        """Register | sign << 10 of every row entry (row by row), then of F."""
+        return [self.reg(r) | (1 if s_ < 0 else 0) << 10 for r, s_ in self.outs]
+
+
+def table(ctype, name, vals, fmt):
+    lines, row = [f"static __device__ const {ctype} {name}[{len(vals)}] = {{"], ""
+    for v in vals:
+        w = fmt(v) + ","
+        if len(row) + len(w) > 112:
+            lines.append("    " + row)
+            row = ""
+        row += w + " "
+    return lines + ["    " + row.rstrip(" ,") + "};"]
+
+
 def cuda_struct(mod, info, sid):
     cname = "Sys_" + mod.NAME
     cm, ca, sm = rows_cost(info)
+    tape = Tape(info)
     out = [f"// ---- system {sid}: {mod.NAME} ({info['nv']} unknowns, {info['np']} parameters)",
-           f"// rows(): {cm} complex mul, {ca} complex add/sub, {sm} real x complex",
+           f"// rows(): {cm} complex mul, {ca} complex add/sub, {sm} real x complex; as a warp's schedule",
+           f"// {len(tape.nodes)} operations in {len(tape.steps)} steps"]
+    out += table("uint32_t", f"tape_{mod.NAME}", tape.words(), lambda v: f"{v:#x}u")
+    out += table("uint16_t", f"tape_out_{mod.NAME}", tape.out_words(), str)
+    out += table("double", f"tape_const_{mod.NAME}", tape.consts, repr)
+    out += [
            f"struct {cname} {{",
            f"  static constexpr int ID = {sid};",
            f"  static constexpr int NV = {info['nv']};",
            f"  static constexpr int NP = {info['np']};",
            f"  static constexpr int NS = {info['ns']};",
            f"  static constexpr int ROWS_CMUL = {cm}, ROWS_CADD = {ca}, ROWS_SMUL = {sm};",
+           f"  static constexpr int TAPE_STEPS = {len(tape.steps)}, TAPE_REGS = {tape.nregs}, "
+           f"TAPE_CONSTS = {len(tape.consts)};",
+           f"  __device__ static const uint32_t* tape() {{ return tape_{mod.NAME}; }}",
+           f"  __device__ static const uint16_t* tape_out() {{ return tape_out_{mod.NAME}; }}",
+           f"  __device__ static const double* tape_const() {{ return tape_const_{mod.NAME}; }}",
            "  template <typename T, int LD>",
            "  __device__ static void rows(const cx<T>* Y, const cx<T>* q, const cx<T>* dq, cx<T>* M, cx<T>* F) {"]
     out += ["  " + ln for ln in emit_rows(mod, info, "cuda")]
@@ -313,10 +457,11 @@ def generate():
     cu = ["// GENERATED by finite_root_generation_gb300/gen/gen_plugins.py from the modules in",
           "// finite_root_generation_gb300/systems -- do not edit.",
           "//",
-          "// System plug-ins for the one-thread-per-path tracker: the homogenized equations'",
-          "// rows of the homotopy Jacobian (columns Z, Z0, then the t column dF/dq . dq/dt) and",
-          "// the finite-root-generation start (random unknowns and free parameters, then the",
-          "// parameters that make the random point an exact root).",
+          "// System plug-ins: the homogenized equations' rows of the homotopy Jacobian (columns",
+          "// Z, Z0, then the t column dF/dq . dq/dt) as straight-line code for one thread and as a",
+          "// schedule of independent operations for a warp (16 operations a step, one lane per",
+          "// real component), and the finite-root-generation start (random unknowns and free",
+          "// parameters, then the parameters that make the random point an exact root).",
           "#pragma once",
           "",
           "#include \"frg_device.cuh\"",

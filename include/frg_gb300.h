@@ -126,7 +126,8 @@ typedef struct frg_config {
   int system;            /* the polynomial system tracked: 0 = Stephenson II (the reference's
                             htpykinematics.cu, nV = 21, nP = 30); k >= 1 = generated plug-in k
                             (frg_system_info). A plug-in runs on the thread kernel
-                            (kernel_variant THREAD), in FP64 or mixed precision (the FP32
+                            (kernel_variant THREAD; short queues and a launch's last paths a
+                            warp per path, with the same results), in FP64 or mixed precision (the FP32
                             stage handing paths to FP64), through frg_track,
                             frg_track_async and frg_track_rounds; its tasks are ntasks x np
                             parameters, its roots N x nv, its yfinal N x (nv + 2), and its roots
