@@ -300,6 +300,13 @@ static void task_gammas(const frg_config& c, uint64_t seed, int ntasks, std::vec
   }
 }
 
+// Grid of a team launch in `mode` (0 FP64, 1 and 3 the FP32 stage, 2 the FP64 stage) over
+// about n paths.
+static TeamGrid team_grid(const frg_ctx* ctx, int mode, int64_t n) {
+  const int bps = ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : ctx->team_blocks_per_sm[mode];
+  return frg_team_grid(ctx->sm_count, bps, n, mode == 1 || mode == 3);
+}
+
 // One round on a slot: gammas, start values, then the tracking launches, all on `st`.
 // `evs` (2 * mixed rounds + 1 events, mixed precision only) bracket the FP32 and FP64
 // launches. Device pointers only here.
@@ -392,16 +399,16 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     }
   auto grid_for = [&](int mode, int64_t n) {
     int bps = ctx->cfg.blocks_per_sm > 0             ? ctx->cfg.blocks_per_sm
-              : (ctx->cfg.system != 0 && mode < 3)  ? plugin_bps[mode]
-                                                    : (team ? ctx->team_blocks_per_sm[mode] : ctx->blocks_per_sm[mode]);
-    return team ? frg_team_grid(ctx->sm_count, bps, n) : frg_thread_grid(ctx->sm_count, bps, n);
+              : (ctx->cfg.system != 0 && mode < 3) ? plugin_bps[mode]
+                                                   : ctx->blocks_per_sm[mode];
+    return frg_thread_grid(ctx->sm_count, bps, n);
   };
   // A plug-in's launch of up to FRG_WARP_PATHS paths per SM sub-partition takes a warp
   // per path; a larger one a thread per path, and then a warp for each of its last paths.
   const bool by_warp = plugin && N <= (int64_t)ctx->sm_count * 4 * FRG_WARP_PATHS;
   auto launch = [&](int mode) -> cudaError_t {
+    if (team) return frg_launch_team(mode, a, team_grid(ctx, mode, N), st);
     const int grid = grid_for(mode, N);
-    if (team) return frg_launch_team(mode, a, grid, st);
     const int wcap = plugin ? ctx->sm_count * (ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : warp_bps[mode])
                             : 0;
     if (by_warp) return frg_launch_warp(mode, a, (int)std::min<int64_t>(wcap, (N + 3) / 4), st);
@@ -712,10 +719,6 @@ static frg_status enqueue_rounds_carry(frg_ctx* ctx, const cx<double>* d_fpm, bo
   a.codes = d_codes;
   a.resid = d_resid;
   a.handoff = (frg::Handoff*)ctx->c_rec.p;
-  auto grid_for = [&](int mode) {
-    int bps = ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : ctx->team_blocks_per_sm[mode];
-    return frg_team_grid(ctx->sm_count, bps, (int64_t)KN);
-  };
   const int lo_mode = ctx->cfg.lo_points == 1 ? 3 : 1;
   auto rounds = [&]() -> frg_status {
     for (int r = 0; r < nrounds; ++r) {
@@ -753,7 +756,7 @@ static frg_status enqueue_rounds_carry(frg_ctx* ctx, const cx<double>* d_fpm, bo
       a.back_list = nullptr;
       a.back_count = nullptr;
       a.lo_keep_ill = 0;
-      cudaError_t e = frg_launch_team(lo_mode, a, grid_for(lo_mode), st);
+      cudaError_t e = frg_launch_team(lo_mode, a, team_grid(ctx, lo_mode, has_in ? 2 * N : N), st);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "track kernel launch (FP32 stage)");
       FRG_CUDA(ctx, record(rev[1], st));
       // FP64 stage: hand well-conditioned paths to round r + depth, or finish them all
@@ -763,7 +766,7 @@ static frg_status enqueue_rounds_carry(frg_ctx* ctx, const cx<double>* d_fpm, bo
       a.lo_count = nullptr;
       a.back_list = (r + depth < nrounds) ? lists + (size_t)(1 + pout) * KN : nullptr;
       a.back_count = q + 3 + pout;
-      e = frg_launch_team(2, a, grid_for(2), st);
+      e = frg_launch_team(2, a, team_grid(ctx, 2, (int64_t)KN), st);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "track kernel launch (FP64 stage)");
       FRG_CUDA(ctx, record(rev[2], st));
       FRG_CUDA(ctx, record(rev[per], st));

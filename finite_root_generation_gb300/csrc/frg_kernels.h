@@ -97,13 +97,18 @@ inline int frg_thread_grid(int sms, int bps, int64_t n) {
   return (int)(grid < 1 ? 1 : grid);
 }
 
-// Grid of a team launch (four paths per block) over at most n paths: one block per SM
-// until every SM has its four, then as many as fit, at most bps per SM.
-inline int frg_team_grid(int sms, int bps, int64_t n) {
-  const int64_t want = n <= (int64_t)sms * 4 ? (n < sms ? n : sms) : (n + 3) / 4;
-  const int64_t cap = (int64_t)sms * bps;
-  const int64_t grid = want < cap ? want : cap;
-  return (int)(grid < 1 ? 1 : grid);
+// Grid of a team launch (a warp per path) over at most n paths, with at most bps blocks of
+// four warps per SM: one block per SM until its warps are taken, then as many as fit. In
+// the FP32 stage (lo) a block grows with the paths per SM, from 4 warps to 16.
+struct TeamGrid { int blocks, warps; };
+inline TeamGrid frg_team_grid(int sms, int bps, int64_t n, bool lo) {
+  const int64_t most = lo ? (4 * bps < 16 ? 4 * bps : 16) : 4, per_sm = (n + sms - 1) / sms;
+  int64_t warps = (per_sm + 3) / 4 * 4;
+  warps = warps < 4 ? 4 : (warps < most ? warps : most);
+  const int64_t want = n <= sms * warps ? (n < sms ? n : sms) : (n + warps - 1) / warps;
+  const int64_t per = 4 * bps / warps, cap = sms * (per < 1 ? 1 : per);
+  const int64_t blocks = want < cap ? want : cap;
+  return {(int)(blocks < 1 ? 1 : blocks), (int)warps};
 }
 
 // A plug-in launch of at most this many paths per SM sub-partition tracks a path per warp,
@@ -130,7 +135,7 @@ cudaError_t frg_warp_occupancy(int system, int mode, int* blocks_per_sm);
 // mode: 0 plain FP64, 1 FP32 stage with handoff, 2 FP64 resume of handed-off paths
 cudaError_t frg_launch_track(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream);
 cudaError_t frg_track_occupancy(int mode, int* blocks_per_sm);
-cudaError_t frg_launch_team(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream);
+cudaError_t frg_launch_team(int mode, const frg::TrackArgs& args, TeamGrid grid, cudaStream_t stream);
 // GenerateStart for every path into args.starts (FRG_START_STRIDE complex per path:
 // the 21 start unknowns, then the 30 start parameters)
 cudaError_t frg_launch_starts(const frg::TrackArgs& args, cx<double>* starts, cudaStream_t stream);

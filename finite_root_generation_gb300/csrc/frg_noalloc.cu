@@ -169,7 +169,7 @@ extern "C" frg_status frg_track_noalloc(const frg_config* cfg, const double* fpm
   if (cfg->blocks_per_sm > 0) bps = cfg->blocks_per_sm;
   if (bps < 1) bps = 1;
   a.sms = sms;
-  const int grid = team ? frg_team_grid(sms, bps, N) : frg_thread_grid(sms, bps, N);
-  const cudaError_t e = team ? frg_launch_team(0, a, grid, st) : frg_launch_track(0, a, grid, st);
+  const cudaError_t e = team ? frg_launch_team(0, a, frg_team_grid(sms, bps, N, false), st)
+                             : frg_launch_track(0, a, frg_thread_grid(sms, bps, N), st);
   return e == cudaSuccess ? FRG_OK : FRG_ERR_CUDA;
 }

@@ -88,8 +88,8 @@ template <typename T> struct HighEval<T, T> {};
 // corrector refines on double-float residuals with an FP32 solve); directions, patches
 // and stage vectors are in the working precision T. `M` holds the group rows
 // (frg_eval_slice's layout; its structural zeros are written once). The evaluation's
-// inputs and the dense system with its factor share memory: the block's barriers keep
-// them apart.
+// inputs and what the solve writes (the dense system with its factor, the groups' pivot
+// rows) share memory: the block's barriers keep them apart.
 template <typename T, typename P = typename PointOf<T>::type>
 struct Smem {
   struct Inputs {
@@ -97,8 +97,8 @@ struct Smem {
     cx<T> dq[32];
     HighEval<T, P> hi;
   };
-  static constexpr size_t kWork =
-      sizeof(Inputs) > sizeof(cx<T>) * 16 * LDU ? sizeof(Inputs) : sizeof(cx<T>) * 16 * LDU;
+  static constexpr size_t kSolve = sizeof(cx<T>) * (16 * LDU + 17 * 8);
+  static constexpr size_t kWork = sizeof(Inputs) > kSolve ? sizeof(Inputs) : kSolve;
   cx<P> Yc[VS], Yn[VS], YN[VS];
   cx<P> sp[32], fp[32];
   cx<P> gamma;
@@ -106,7 +106,6 @@ struct Smem {
   cx<T> Vc[VS], Vn[VS], u[VS], Ye[VS], dx[VS];
   cx<T> k[8][VS];
   cx<T> M[3 * 18 * 8];
-  cx<T> piv[17 * 8];  // pivot rows of the groups: [column][group], right-hand side at 16
   cx<T> X[16], XU[8], R[3][8], Rd;  // solution; refined residuals and patch residual
   T cn[16];
   alignas(16) unsigned char work[kWork];
@@ -117,6 +116,8 @@ struct Smem {
   unsigned long long cyc[8];  // cycle accounting (lane 0)
   __device__ __forceinline__ Inputs& inputs() { return *reinterpret_cast<Inputs*>(work); }
   __device__ __forceinline__ cx<T>* U() { return reinterpret_cast<cx<T>*>(work); }
+  // pivot rows of the groups: [column][group], right-hand side at column 16
+  __device__ __forceinline__ cx<T>* piv() { return U() + 16 * LDU; }
 };
 
 __device__ __forceinline__ int param_index(int slot, int j) {
@@ -415,10 +416,11 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
       R1[i] = cfms(xb, lb, piv[cc]);
     }
   }
+  cx<T>* pivs = S.piv();
   if (grp) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) S.piv[(q + 4 * i) * 8 + g] = piv[i];
-    if (q == 0) S.piv[16 * 8 + g] = piv[5];
+    for (int i = 0; i < 4; ++i) pivs[(q + 4 * i) * 8 + g] = piv[i];
+    if (q == 0) pivs[16 * 8 + g] = piv[5];
   }
   // ---- the folding of every group's pivot row into the patch rows (lanes g = 7 repeat
   //      group 7's rows with weight zero and then hold the patch rows). A Newton step's
@@ -493,7 +495,7 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
   __syncwarp();
   back_substitute(U, S.X, lane);
   __syncwarp();
-  const cx<T> xu = solve_u(S.piv, S.X, ipu, lane);
+  const cx<T> xu = solve_u(pivs, S.X, ipu, lane);
   if (lane < 16) S.cn[lane] = cnorm2(S.X[lane]);
   if (lane < 8) S.XU[lane] = xu;
   __syncwarp();

@@ -258,19 +258,29 @@ __device__ __noinline__ int checkpoint(const TrackArgs& a, const cx<P>* Yc, int6
 }
 
 // Blocks of a launch that take paths, and paths per block. Short queues spread over the
-// SMs: a block's warps sit on the SM's four sub-partitions, so up to four paths share one
-// block (and its evaluation) before a second block joins the SM.
+// SMs: the four warps of a part sit on the SM's four sub-partitions, so paths fill one
+// block per SM (up to its warps) before a second block joins the SM.
 __device__ __forceinline__ void spread_queue(int64_t nqueue, int sms, int& blocks, int& paths) {
-  int64_t b = nqueue <= (int64_t)sms * PATHS ? (nqueue < sms ? nqueue : sms) : (nqueue + PATHS - 1) / PATHS;
+  const int warps = blockDim.x >> 5;
+  int64_t b = nqueue <= (int64_t)sms * warps ? (nqueue < sms ? nqueue : sms) : (nqueue + warps - 1) / warps;
   b = b < 1 ? 1 : b;
   b = b < gridDim.x ? b : gridDim.x;
   const int64_t p = (nqueue + b - 1) / b;
   blocks = (int)b;
-  paths = (int)(p < PATHS ? p : PATHS);
+  paths = (int)(p < warps ? p : warps);
 }
 
+// Blocks of 4 warps in FP64 (two per SM, by registers and shared memory), of 4 to 16 in
+// the FP32 stage (by the queue's length, frg_team_grid). The warps work in parts of four:
+// part k evaluates its four paths together. All warps of a block step in time, and in the
+// FP32 stage, which is bound by instruction fetch once the SM is full, that is what lets
+// them share it: 65,536-path rounds, four in flight, take 1,884 ms with four blocks of
+// 4 warps per SM, 1,701 with two of 8, 1,569 with one of 16 (9,600 paths alone: 382,
+// 354, 337 ms); with few paths the barriers of larger blocks only cost (140 paths: 126
+// against 136 ms).
 template <int MODE, typename T, typename P = typename PointOf<T>::type>
-__global__ void __launch_bounds__(32 * PATHS, sizeof(T) == 8 ? 2 : 4) team_kernel(TrackArgs a) {
+__global__ void __launch_bounds__(sizeof(T) == 8 ? 32 * PATHS : 512, sizeof(T) == 8 ? 2 : 1)
+team_kernel(TrackArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr bool LO = (MODE == MODE_LO);
   constexpr bool LOWP = sizeof(T) < sizeof(P);
@@ -474,13 +484,14 @@ __global__ void __launch_bounds__(32 * PATHS, sizeof(T) == 8 ? 2 : 4) team_kerne
     if (lane == 0) { S.active = phase != PH_IDLE; S.refine = newton && hires; }
     const long long tc2 = clock64();
 
-    // ============== evaluation (the block: part `warp` of every path's groups)
+    // ============== evaluation (the part's four warps: quarter `quarter` of every path's groups)
     if (__syncthreads_and(phase == PH_IDLE)) break;
     {
-      Smem<T, P>& E = paths[lane >> 3];
+      Smem<T, P>& E = paths[(warp & ~3) + (lane >> 3)];
+      const int quarter = warp & 3;
       if (E.active && g < 7) {
         auto& in = E.inputs();
-        switch (warp) {
+        switch (quarter) {
           case 0: frg_eval_slice<0, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
           case 1: frg_eval_slice<1, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
           case 2: frg_eval_slice<2, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
@@ -494,13 +505,13 @@ __global__ void __launch_bounds__(32 * PATHS, sizeof(T) == 8 ? 2 : 4) team_kerne
         const long long tr0 = clock64();
         if (E.refine) {
           const FrgEvalIn<P>& in = E.inputs().hi.in;
-          if (warp == 3) {
+          if (quarter == 3) {
             const cp d = patch_dot<T, P>(E.u, E.YN, NY, g, 0xffu << (lane & 24)) - cp(P(1));
             if (g == 0) E.Rd = cx<T>(d);
           } else if (g < 7) {
-            E.R[warp][g] = cx<T>(warp == 0   ? frg_residual_slice<0, P>(E.YN, in, jg)
-                                 : warp == 1 ? frg_residual_slice<1, P>(E.YN, in, jg)
-                                             : frg_residual_slice<2, P>(E.YN, in, jg));
+            E.R[quarter][g] = cx<T>(quarter == 0   ? frg_residual_slice<0, P>(E.YN, in, jg)
+                                    : quarter == 1 ? frg_residual_slice<1, P>(E.YN, in, jg)
+                                                   : frg_residual_slice<2, P>(E.YN, in, jg));
           }
         }
         if (lane == 0) S.cyc[6] += clock64() - tr0;
@@ -817,27 +828,35 @@ cudaError_t frg_launch_starts(const frg::TrackArgs& args, cx<double>* starts, cu
 }
 
 namespace {
+// The kernel's shared-memory limit, the same value from every caller (host threads may
+// launch blocks of different sizes at once).
+template <int MODE, typename T, typename P>
+cudaError_t team_limit() {
+  constexpr size_t most = (sizeof(T) == 8 ? frg::team::PATHS : 16) * sizeof(frg::team::Smem<T, P>);
+  static_assert(most <= 227 * 1024, "a block's paths must fit an SM's shared memory");
+  return cudaFuncSetAttribute(frg::team::team_kernel<MODE, T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)most);
+}
 template <int MODE, typename T, typename P = typename frg::team::PointOf<T>::type>
-cudaError_t team_launch(const frg::TrackArgs& args, int grid, cudaStream_t stream) {
-  const size_t smem = frg::team::PATHS * sizeof(frg::team::Smem<T, P>);
-  cudaError_t e = cudaFuncSetAttribute(frg::team::team_kernel<MODE, T, P>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+cudaError_t team_launch(const frg::TrackArgs& args, TeamGrid grid, cudaStream_t stream) {
+  const size_t smem = grid.warps * sizeof(frg::team::Smem<T, P>);
+  const cudaError_t e = team_limit<MODE, T, P>();
   if (e != cudaSuccess) return e;
-  frg::team::team_kernel<MODE, T, P><<<grid, 32 * frg::team::PATHS, smem, stream>>>(args);
+  frg::team::team_kernel<MODE, T, P><<<grid.blocks, 32 * grid.warps, smem, stream>>>(args);
   return cudaGetLastError();
 }
+// resident blocks of four warps per SM
 template <int MODE, typename T, typename P = typename frg::team::PointOf<T>::type>
 cudaError_t team_occ(int* bps) {
   const size_t smem = frg::team::PATHS * sizeof(frg::team::Smem<T, P>);
-  cudaError_t e = cudaFuncSetAttribute(frg::team::team_kernel<MODE, T, P>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = team_limit<MODE, T, P>();
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, frg::team::team_kernel<MODE, T, P>,
                                                        32 * frg::team::PATHS, smem);
 }
 }  // namespace
 
-cudaError_t frg_launch_team(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream) {
+cudaError_t frg_launch_team(int mode, const frg::TrackArgs& args, TeamGrid grid, cudaStream_t stream) {
   switch (mode) {
     case 0: return team_launch<frg::team::MODE_PLAIN, double>(args, grid, stream);
     case 1: return team_launch<frg::team::MODE_LO, float>(args, grid, stream);
