@@ -42,6 +42,10 @@ FRG_HD cx<T>& operator+=(cx<T>& a, cx<T> b) { a.re += b.re; a.im += b.im; return
 template <typename T>
 FRG_HD cx<T>& operator-=(cx<T>& a, cx<T> b) { a.re -= b.re; a.im -= b.im; return a; }
 
+// store a value (types that hold a complex value differently have their own)
+template <typename T>
+FRG_HD void cx_put(cx<T>* p, cx<T> v) { *p = v; }
+
 // a - b*c (one complex fused multiply-subtract: 4 FMA)
 template <typename T>
 FRG_HD cx<T> cfms(cx<T> a, cx<T> b, cx<T> c) {

@@ -309,470 +309,472 @@ struct FrgEvalIn {
 
 // One quarter of group j's evaluation (frg_group_eval's operations in its order): rows of
 // the group into M[(row * 18 + column) * 8 + g], columns 0..13 links, 14 Z0, 15 t, 16 U_j, 17 F.
-template <int SLICE, typename T>
+// CX: cx<T>, or a type with its operators whose values several lanes share.
+template <int SLICE, typename CX, typename T>
 __device__ __forceinline__ void frg_eval_slice(const cx<T>* Y, const FrgEvalIn<T>& in, const cx<T>* dq, int j,
                                                int g, cx<T>* M) {
   if constexpr (SLICE == 0) {
-    const cx<T> C = Y[2];
-    const cx<T> D = Y[3];
-    const cx<T> Dc = Y[10];
-    const cx<T> G = Y[5];
-    const cx<T> Gc = Y[12];
-    const cx<T> P0 = in.q[0];
-    const cx<T> Pc0 = in.q[8];
-    const cx<T> Pcj = in.q[8 + j];
-    const cx<T> Pj = in.q[j];
-    const cx<T> Qj = in.q[15 + j];
-    const cx<T> U = Y[13 + j];
-    const cx<T> e1 = in.e[0];
-    const cx<T> e2 = in.e[1];
-    const cx<T> iU = in.iU[j - 1];
-    const cx<T> x11 = in.sb[1][FRG_IN_PJZ][j - 1];
-    const cx<T> x16 = in.sb[0][FRG_IN_PJZ][j - 1];
-    const cx<T> x31 = in.sa[0][FRG_IN_HP];
-    const cx<T> x33 = in.sb[0][FRG_IN_AQ][j - 1];
-    const cx<T> x45 = in.sb[0][FRG_IN_AQ][j - 1];
-    const cx<T> x6 = in.sa[0][FRG_IN_PZ];
-    const cx<T> x62 = in.sa[0][FRG_IN_FP];
-    const cx<T> x63 = in.sb[0][FRG_IN_BP][j - 1];
-    const cx<T> x75 = in.sa[0][FRG_IN_BD];
-    const cx<T> x76 = in.sa[0][FRG_IN_EBD];
-    const cx<T> x77 = in.sa[0][FRG_IN_CG];
-    const cx<T> x78 = in.sa[0][FRG_IN_ECG];
-    const cx<T> x79 = in.sa[0][FRG_IN_V];
-    const cx<T> x81 = in.sa[1][FRG_IN_EBD];
-    const cx<T> x83 = in.sa[1][FRG_IN_ECG];
-    const cx<T> x84 = in.sa[1][FRG_IN_V];
-    const cx<T> x87 = in.sb[1][FRG_IN_W][j - 1];
-    const cx<T> x89 = in.sb[0][FRG_IN_EAQ][j - 1];
-    const cx<T> x90 = in.sb[0][FRG_IN_W][j - 1];
-    const cx<T> z = Y[21];
-    const cx<T> z2 = in.z2;
-    const cx<T> x7 = (-(x6));
-    const cx<T> x8 = C + x7;
-    const cx<T> x32 = U*x31;
-    const cx<T> x46 = iU*x45;
-    const cx<T> x47 = x46*z2;
-    const cx<T> x51 = iU*z2;
-    const cx<T> x67 = U*x62;
-    const cx<T> x68 = x51*x63;
-    const cx<T> x70 = (-(G));
-    const cx<T> x71 = D + x70;
-    const cx<T> x72 = (-(Gc));
-    const cx<T> x73 = Dc + x72;
-    const cx<T> x74 = x73*z;
-    const cx<T> x85 = x79*x84;
-    const cx<T> x91 = x51*x84;
-    const cx<T> x92 = x87*z;
-    const cx<T> x94 = x84*z;
-    const cx<T> x95 = e1*x63;
-    const cx<T> x96 = cx<T>(T(1.0)) + x76 + x95;
-    const cx<T> x97 = (-(x84));
-    const cx<T> x98 = x97*z;
-    const cx<T> x99 = x62*x98;
-    const cx<T> x100 = (-(x87));
-    const cx<T> x101 = x100*x67;
-    const cx<T> x102 = x100*z;
-    const cx<T> x103 = x101 - x99 + x68*x97 - x102*x63;
-    const cx<T> x104 = x32*x87;
-    const cx<T> x105 = Qj + x89 + Qj*x78;
-    const cx<T> x106 = x51*x97;
-    const cx<T> x107 = U*x100;
-    const cx<T> x108 = x100*x32;
-    const cx<T> x132 = x76 - x78;
-    const cx<T> x133 = x81 - x83;
-    const cx<T> x134 = (-(x133));
-    const cx<T> x135 = (-(x132));
-    const cx<T> x136 = U*x87;
-    const cx<T> x137 = x51*x90;
-    M[104 + g] = x47 - x8*z;
-    M[296 + g] = (-x92*x96) - e1*x62*x94 - x103*x75*(e1*e1) + U*e1*x62*x87 + iU*x84*x96*z2;
-    M[304 + g] = x105*x92 - e2*x104 - x105*x91 + e2*x31*x94 + x77*(e2*e2)*((-x104) - x33*x91 + x31*x84*z + x33*x87*z);
-    M[312 + g] = x74 + e1*x101 + x106*x95 - e1*x99 - x102*x95;
-    M[320 + g] = x76*(x98 - x107 + e1*x103);
-    M[328 + g] = (-x74) - e2*x108 - x106*x89 + e2*x100*x45*z + e2*x31*x97*z;
-    M[336 + g] = x78*(x107 - x98 - e2*(x108 + x47*x97 - x102*x45 - x31*x98));
-    M[400 + g] = (-x85) + x71*x73 - x87*x90 - P0*x132*x136 - Pc0*x133*x137 - x11*x134*x90 - x135*x16*x87 + P0*x132*x84*z + Pc0*x133*x79*z + Pcj*U*x134*x79 + (T(2.0)*(iU*x84*x90*z)) + Pj*iU*x135*x84*z2;
+    const CX C(Y[2]);
+    const CX D(Y[3]);
+    const CX Dc(Y[10]);
+    const CX G(Y[5]);
+    const CX Gc(Y[12]);
+    const CX P0(in.q[0]);
+    const CX Pc0(in.q[8]);
+    const CX Pcj(in.q[8 + j]);
+    const CX Pj(in.q[j]);
+    const CX Qj(in.q[15 + j]);
+    const CX U(Y[13 + j]);
+    const CX e1(in.e[0]);
+    const CX e2(in.e[1]);
+    const CX iU(in.iU[j - 1]);
+    const CX x11(in.sb[1][FRG_IN_PJZ][j - 1]);
+    const CX x16(in.sb[0][FRG_IN_PJZ][j - 1]);
+    const CX x31(in.sa[0][FRG_IN_HP]);
+    const CX x33(in.sb[0][FRG_IN_AQ][j - 1]);
+    const CX x45(in.sb[0][FRG_IN_AQ][j - 1]);
+    const CX x6(in.sa[0][FRG_IN_PZ]);
+    const CX x62(in.sa[0][FRG_IN_FP]);
+    const CX x63(in.sb[0][FRG_IN_BP][j - 1]);
+    const CX x75(in.sa[0][FRG_IN_BD]);
+    const CX x76(in.sa[0][FRG_IN_EBD]);
+    const CX x77(in.sa[0][FRG_IN_CG]);
+    const CX x78(in.sa[0][FRG_IN_ECG]);
+    const CX x79(in.sa[0][FRG_IN_V]);
+    const CX x81(in.sa[1][FRG_IN_EBD]);
+    const CX x83(in.sa[1][FRG_IN_ECG]);
+    const CX x84(in.sa[1][FRG_IN_V]);
+    const CX x87(in.sb[1][FRG_IN_W][j - 1]);
+    const CX x89(in.sb[0][FRG_IN_EAQ][j - 1]);
+    const CX x90(in.sb[0][FRG_IN_W][j - 1]);
+    const CX z(Y[21]);
+    const CX z2(in.z2);
+    const CX x7 = (-(x6));
+    const CX x8 = C + x7;
+    const CX x32 = U*x31;
+    const CX x46 = iU*x45;
+    const CX x47 = x46*z2;
+    const CX x51 = iU*z2;
+    const CX x67 = U*x62;
+    const CX x68 = x51*x63;
+    const CX x70 = (-(G));
+    const CX x71 = D + x70;
+    const CX x72 = (-(Gc));
+    const CX x73 = Dc + x72;
+    const CX x74 = x73*z;
+    const CX x85 = x79*x84;
+    const CX x91 = x51*x84;
+    const CX x92 = x87*z;
+    const CX x94 = x84*z;
+    const CX x95 = e1*x63;
+    const CX x96 = CX(T(1.0)) + x76 + x95;
+    const CX x97 = (-(x84));
+    const CX x98 = x97*z;
+    const CX x99 = x62*x98;
+    const CX x100 = (-(x87));
+    const CX x101 = x100*x67;
+    const CX x102 = x100*z;
+    const CX x103 = x101 - x99 + x68*x97 - x102*x63;
+    const CX x104 = x32*x87;
+    const CX x105 = Qj + x89 + Qj*x78;
+    const CX x106 = x51*x97;
+    const CX x107 = U*x100;
+    const CX x108 = x100*x32;
+    const CX x132 = x76 - x78;
+    const CX x133 = x81 - x83;
+    const CX x134 = (-(x133));
+    const CX x135 = (-(x132));
+    const CX x136 = U*x87;
+    const CX x137 = x51*x90;
+    cx_put(M + 104 + g, x47 - x8*z);
+    cx_put(M + 296 + g, (-x92*x96) - e1*x62*x94 - x103*x75*(e1*e1) + U*e1*x62*x87 + iU*x84*x96*z2);
+    cx_put(M + 304 + g, x105*x92 - e2*x104 - x105*x91 + e2*x31*x94 + x77*(e2*e2)*((-x104) - x33*x91 + x31*x84*z + x33*x87*z));
+    cx_put(M + 312 + g, x74 + e1*x101 + x106*x95 - e1*x99 - x102*x95);
+    cx_put(M + 320 + g, x76*(x98 - x107 + e1*x103));
+    cx_put(M + 328 + g, (-x74) - e2*x108 - x106*x89 + e2*x100*x45*z + e2*x31*x97*z);
+    cx_put(M + 336 + g, x78*(x107 - x98 - e2*(x108 + x47*x97 - x102*x45 - x31*x98)));
+    cx_put(M + 400 + g, (-x85) + x71*x73 - x87*x90 - P0*x132*x136 - Pc0*x133*x137 - x11*x134*x90 - x135*x16*x87 + P0*x132*x84*z + Pc0*x133*x79*z + Pcj*U*x134*x79 + (T(2.0)*(iU*x84*x90*z)) + Pj*iU*x135*x84*z2);
   }
   if constexpr (SLICE == 1) {
-    const cx<T> A = Y[0];
-    const cx<T> Ac = Y[7];
-    const cx<T> B = Y[1];
-    const cx<T> Bc = Y[8];
-    const cx<T> C = Y[2];
-    const cx<T> Cc = Y[9];
-    const cx<T> F = Y[4];
-    const cx<T> Fc = Y[11];
-    const cx<T> H = Y[6];
-    const cx<T> Hc = Y[13];
-    const cx<T> P0 = in.q[0];
-    const cx<T> Pc0 = in.q[8];
-    const cx<T> Pcj = in.q[8 + j];
-    const cx<T> Pj = in.q[j];
-    const cx<T> Qj = in.q[15 + j];
-    const cx<T> U = Y[13 + j];
-    const cx<T> dP0 = dq[0];
-    const cx<T> dPc0 = dq[8];
-    const cx<T> dPcj = dq[8 + j];
-    const cx<T> dPj = dq[j];
-    const cx<T> dQcj = dq[22 + j];
-    const cx<T> dQj = dq[15 + j];
-    const cx<T> iU = in.iU[j - 1];
-    const cx<T> x11 = in.sb[1][FRG_IN_PJZ][j - 1];
-    const cx<T> x16 = in.sb[0][FRG_IN_PJZ][j - 1];
-    const cx<T> x2 = in.sa[1][FRG_IN_PZ];
-    const cx<T> x20 = in.sa[1][FRG_IN_AC];
-    const cx<T> x21 = in.sb[1][FRG_IN_QA][j - 1];
-    const cx<T> x23 = in.sb[0][FRG_IN_AP][j - 1];
-    const cx<T> x25 = in.sa[0][FRG_IN_AC];
-    const cx<T> x26 = in.sb[0][FRG_IN_QA][j - 1];
-    const cx<T> x28 = in.sb[1][FRG_IN_AP][j - 1];
-    const cx<T> x30 = in.sb[1][FRG_IN_AQ][j - 1];
-    const cx<T> x31 = in.sa[0][FRG_IN_HP];
-    const cx<T> x33 = in.sb[0][FRG_IN_AQ][j - 1];
-    const cx<T> x34 = in.sa[1][FRG_IN_HP];
-    const cx<T> x39 = in.sb[1][FRG_IN_AQ][j - 1];
-    const cx<T> x45 = in.sb[0][FRG_IN_AQ][j - 1];
-    const cx<T> x6 = in.sa[0][FRG_IN_PZ];
-    const cx<T> x61 = in.sb[1][FRG_IN_BP][j - 1];
-    const cx<T> x62 = in.sa[0][FRG_IN_FP];
-    const cx<T> x63 = in.sb[0][FRG_IN_BP][j - 1];
-    const cx<T> x64 = in.sa[1][FRG_IN_FP];
-    const cx<T> x79 = in.sa[0][FRG_IN_V];
-    const cx<T> x84 = in.sa[1][FRG_IN_V];
-    const cx<T> x87 = in.sb[1][FRG_IN_W][j - 1];
-    const cx<T> x90 = in.sb[0][FRG_IN_W][j - 1];
-    const cx<T> z = Y[21];
-    const cx<T> z2 = in.z2;
-    const cx<T> z3 = in.z3;
-    const cx<T> x0 = P0*Pc0 + Pcj*Pj;
-    const cx<T> x1 = x0*z3;
-    const cx<T> x3 = (-(x2));
-    const cx<T> x4 = Cc + x3;
-    const cx<T> x5 = x4*z;
-    const cx<T> x7 = (-(x6));
-    const cx<T> x8 = C + x7;
-    const cx<T> x9 = Hc*z;
-    const cx<T> x10 = (-(Ac));
-    const cx<T> x12 = x10 + x11;
-    const cx<T> x13 = Cc + x12;
-    const cx<T> x14 = x13*z;
-    const cx<T> x15 = (-(A));
-    const cx<T> x17 = x15 + x16;
-    const cx<T> x18 = C + x17;
-    const cx<T> x19 = Ac*z;
-    const cx<T> x24 = x23*z;
-    const cx<T> x29 = x28*z;
-    const cx<T> x32 = U*x31;
-    const cx<T> x35 = iU*x34;
-    const cx<T> x36 = x35*z2;
-    const cx<T> x37 = Qj*x29;
-    const cx<T> x38 = (-cx<T>(T(1.0))) + Qj;
-    const cx<T> x40 = U*x39;
-    const cx<T> x46 = iU*x45;
-    const cx<T> x48 = z2*(iU*iU);
-    const cx<T> x51 = iU*z2;
-    const cx<T> x52 = Pc0*z3;
-    const cx<T> x53 = P0*z3;
-    const cx<T> x54 = Pj*z3;
-    const cx<T> x55 = Pcj*z3;
-    const cx<T> x56 = Bc + x3;
-    const cx<T> x57 = x56*z;
-    const cx<T> x58 = B + x7;
-    const cx<T> x59 = Fc*z;
-    const cx<T> x60 = B*Pcj + Bc*Pj;
-    const cx<T> x65 = x51*x64;
-    const cx<T> x66 = U*x61;
-    const cx<T> x67 = U*x62;
-    const cx<T> x69 = iU*z3;
-    const cx<T> x97 = (-(x84));
-    const cx<T> x100 = (-(x87));
-    const cx<T> x121 = (-(x79));
-    const cx<T> x123 = (-(x90));
-    M[136 + g] = (-x1) + A*x14 + x18*x19 + x21*x24 + x26*x29 + x30*x32 + x33*x36 - H*x5 - x8*x9;
-    M[0 + g] = x14 + x37 - x19 + x21*z - x36*x38;
-    M[16 + g] = x19 - x37 - x9 + Qj*x36;
-    M[48 + g] = x40 - x5;
-    M[128 + g] = x31*x39 - x34*x45*x48;
-    M[120 + g] = (-dP0*(x52 + x40*z - Hc*z2)) - dPc0*(x53 + x46*z3 - H*z2) - dPcj*(x54 + x26*z2 + x32*z - A*z2) - dPj*(x55 + x21*z2 + x35*z3 - Ac*z2) - dQcj*x20*(x32 - x24) - dQj*x25*(x36 - x29);
-    M[280 + g] = (-x1) + x60*z2 - F*x57 - x58*x59 + U*x61*x62 + iU*x63*x64*z2;
-    M[152 + g] = x65 - x59 + Pcj*z2;
-    M[176 + g] = x66 - x57;
-    M[272 + g] = x61*x62 - x48*x63*x64;
-    M[264 + g] = (-dP0*(x52 + x66*z - Fc*z2)) - dPc0*(x53 + x63*x69 - F*z2) - dPcj*(x54 + x67*z - B*z2) - dPj*(x55 + x64*x69 - Bc*z2);
-    M[416 + g] = x100*x121 - x123*x48*x97;
+    const CX A(Y[0]);
+    const CX Ac(Y[7]);
+    const CX B(Y[1]);
+    const CX Bc(Y[8]);
+    const CX C(Y[2]);
+    const CX Cc(Y[9]);
+    const CX F(Y[4]);
+    const CX Fc(Y[11]);
+    const CX H(Y[6]);
+    const CX Hc(Y[13]);
+    const CX P0(in.q[0]);
+    const CX Pc0(in.q[8]);
+    const CX Pcj(in.q[8 + j]);
+    const CX Pj(in.q[j]);
+    const CX Qj(in.q[15 + j]);
+    const CX U(Y[13 + j]);
+    const CX dP0(dq[0]);
+    const CX dPc0(dq[8]);
+    const CX dPcj(dq[8 + j]);
+    const CX dPj(dq[j]);
+    const CX dQcj(dq[22 + j]);
+    const CX dQj(dq[15 + j]);
+    const CX iU(in.iU[j - 1]);
+    const CX x11(in.sb[1][FRG_IN_PJZ][j - 1]);
+    const CX x16(in.sb[0][FRG_IN_PJZ][j - 1]);
+    const CX x2(in.sa[1][FRG_IN_PZ]);
+    const CX x20(in.sa[1][FRG_IN_AC]);
+    const CX x21(in.sb[1][FRG_IN_QA][j - 1]);
+    const CX x23(in.sb[0][FRG_IN_AP][j - 1]);
+    const CX x25(in.sa[0][FRG_IN_AC]);
+    const CX x26(in.sb[0][FRG_IN_QA][j - 1]);
+    const CX x28(in.sb[1][FRG_IN_AP][j - 1]);
+    const CX x30(in.sb[1][FRG_IN_AQ][j - 1]);
+    const CX x31(in.sa[0][FRG_IN_HP]);
+    const CX x33(in.sb[0][FRG_IN_AQ][j - 1]);
+    const CX x34(in.sa[1][FRG_IN_HP]);
+    const CX x39(in.sb[1][FRG_IN_AQ][j - 1]);
+    const CX x45(in.sb[0][FRG_IN_AQ][j - 1]);
+    const CX x6(in.sa[0][FRG_IN_PZ]);
+    const CX x61(in.sb[1][FRG_IN_BP][j - 1]);
+    const CX x62(in.sa[0][FRG_IN_FP]);
+    const CX x63(in.sb[0][FRG_IN_BP][j - 1]);
+    const CX x64(in.sa[1][FRG_IN_FP]);
+    const CX x79(in.sa[0][FRG_IN_V]);
+    const CX x84(in.sa[1][FRG_IN_V]);
+    const CX x87(in.sb[1][FRG_IN_W][j - 1]);
+    const CX x90(in.sb[0][FRG_IN_W][j - 1]);
+    const CX z(Y[21]);
+    const CX z2(in.z2);
+    const CX z3(in.z3);
+    const CX x0 = P0*Pc0 + Pcj*Pj;
+    const CX x1 = x0*z3;
+    const CX x3 = (-(x2));
+    const CX x4 = Cc + x3;
+    const CX x5 = x4*z;
+    const CX x7 = (-(x6));
+    const CX x8 = C + x7;
+    const CX x9 = Hc*z;
+    const CX x10 = (-(Ac));
+    const CX x12 = x10 + x11;
+    const CX x13 = Cc + x12;
+    const CX x14 = x13*z;
+    const CX x15 = (-(A));
+    const CX x17 = x15 + x16;
+    const CX x18 = C + x17;
+    const CX x19 = Ac*z;
+    const CX x24 = x23*z;
+    const CX x29 = x28*z;
+    const CX x32 = U*x31;
+    const CX x35 = iU*x34;
+    const CX x36 = x35*z2;
+    const CX x37 = Qj*x29;
+    const CX x38 = (-CX(T(1.0))) + Qj;
+    const CX x40 = U*x39;
+    const CX x46 = iU*x45;
+    const CX x48 = z2*(iU*iU);
+    const CX x51 = iU*z2;
+    const CX x52 = Pc0*z3;
+    const CX x53 = P0*z3;
+    const CX x54 = Pj*z3;
+    const CX x55 = Pcj*z3;
+    const CX x56 = Bc + x3;
+    const CX x57 = x56*z;
+    const CX x58 = B + x7;
+    const CX x59 = Fc*z;
+    const CX x60 = B*Pcj + Bc*Pj;
+    const CX x65 = x51*x64;
+    const CX x66 = U*x61;
+    const CX x67 = U*x62;
+    const CX x69 = iU*z3;
+    const CX x97 = (-(x84));
+    const CX x100 = (-(x87));
+    const CX x121 = (-(x79));
+    const CX x123 = (-(x90));
+    cx_put(M + 136 + g, (-x1) + A*x14 + x18*x19 + x21*x24 + x26*x29 + x30*x32 + x33*x36 - H*x5 - x8*x9);
+    cx_put(M + 0 + g, x14 + x37 - x19 + x21*z - x36*x38);
+    cx_put(M + 16 + g, x19 - x37 - x9 + Qj*x36);
+    cx_put(M + 48 + g, x40 - x5);
+    cx_put(M + 128 + g, x31*x39 - x34*x45*x48);
+    cx_put(M + 120 + g, (-dP0*(x52 + x40*z - Hc*z2)) - dPc0*(x53 + x46*z3 - H*z2) - dPcj*(x54 + x26*z2 + x32*z - A*z2) - dPj*(x55 + x21*z2 + x35*z3 - Ac*z2) - dQcj*x20*(x32 - x24) - dQj*x25*(x36 - x29));
+    cx_put(M + 280 + g, (-x1) + x60*z2 - F*x57 - x58*x59 + U*x61*x62 + iU*x63*x64*z2);
+    cx_put(M + 152 + g, x65 - x59 + Pcj*z2);
+    cx_put(M + 176 + g, x66 - x57);
+    cx_put(M + 272 + g, x61*x62 - x48*x63*x64);
+    cx_put(M + 264 + g, (-dP0*(x52 + x66*z - Fc*z2)) - dPc0*(x53 + x63*x69 - F*z2) - dPcj*(x54 + x67*z - B*z2) - dPj*(x55 + x64*x69 - Bc*z2));
+    cx_put(M + 416 + g, x100*x121 - x123*x48*x97);
   }
   if constexpr (SLICE == 2) {
-    const cx<T> A = Y[0];
-    const cx<T> B = Y[1];
-    const cx<T> D = Y[3];
-    const cx<T> Dc = Y[10];
-    const cx<T> G = Y[5];
-    const cx<T> Gc = Y[12];
-    const cx<T> Qcj = in.q[22 + j];
-    const cx<T> Qj = in.q[15 + j];
-    const cx<T> U = Y[13 + j];
-    const cx<T> dP0 = dq[0];
-    const cx<T> dPc0 = dq[8];
-    const cx<T> dPcj = dq[8 + j];
-    const cx<T> dPj = dq[j];
-    const cx<T> dQcj = dq[22 + j];
-    const cx<T> dQj = dq[15 + j];
-    const cx<T> e1 = in.e[0];
-    const cx<T> e2 = in.e[1];
-    const cx<T> ec1 = in.e[2];
-    const cx<T> ec2 = in.e[3];
-    const cx<T> iU = in.iU[j - 1];
-    const cx<T> x20 = in.sa[1][FRG_IN_AC];
-    const cx<T> x25 = in.sa[0][FRG_IN_AC];
-    const cx<T> x30 = in.sb[1][FRG_IN_AQ][j - 1];
-    const cx<T> x31 = in.sa[0][FRG_IN_HP];
-    const cx<T> x34 = in.sa[1][FRG_IN_HP];
-    const cx<T> x45 = in.sb[0][FRG_IN_AQ][j - 1];
-    const cx<T> x61 = in.sb[1][FRG_IN_BP][j - 1];
-    const cx<T> x62 = in.sa[0][FRG_IN_FP];
-    const cx<T> x63 = in.sb[0][FRG_IN_BP][j - 1];
-    const cx<T> x64 = in.sa[1][FRG_IN_FP];
-    const cx<T> x75 = in.sa[0][FRG_IN_BD];
-    const cx<T> x76 = in.sa[0][FRG_IN_EBD];
-    const cx<T> x77 = in.sa[0][FRG_IN_CG];
-    const cx<T> x78 = in.sa[0][FRG_IN_ECG];
-    const cx<T> x79 = in.sa[0][FRG_IN_V];
-    const cx<T> x80 = in.sa[1][FRG_IN_BD];
-    const cx<T> x81 = in.sa[1][FRG_IN_EBD];
-    const cx<T> x82 = in.sa[1][FRG_IN_CG];
-    const cx<T> x83 = in.sa[1][FRG_IN_ECG];
-    const cx<T> x84 = in.sa[1][FRG_IN_V];
-    const cx<T> x86 = in.sb[1][FRG_IN_EAQ][j - 1];
-    const cx<T> x87 = in.sb[1][FRG_IN_W][j - 1];
-    const cx<T> x90 = in.sb[0][FRG_IN_W][j - 1];
-    const cx<T> z = Y[21];
-    const cx<T> z2 = in.z2;
-    const cx<T> x35 = iU*x34;
-    const cx<T> x36 = x35*z2;
-    const cx<T> x38 = (-cx<T>(T(1.0))) + Qj;
-    const cx<T> x43 = (-cx<T>(T(1.0))) + Qcj;
-    const cx<T> x44 = (-(Qj*x25));
-    const cx<T> x51 = iU*z2;
-    const cx<T> x65 = x51*x64;
-    const cx<T> x70 = (-(G));
-    const cx<T> x71 = D + x70;
-    const cx<T> x72 = (-(Gc));
-    const cx<T> x73 = Dc + x72;
-    const cx<T> x74 = x73*z;
-    const cx<T> x85 = x79*x84;
-    const cx<T> x88 = U*x79;
-    const cx<T> x91 = x51*x84;
-    const cx<T> x92 = x87*z;
-    const cx<T> x93 = x91 - x92;
-    const cx<T> x97 = (-(x84));
-    const cx<T> x100 = (-(x87));
-    const cx<T> x102 = x100*z;
-    const cx<T> x106 = x51*x97;
-    const cx<T> x109 = x90*z;
-    const cx<T> x110 = x88 - x109;
-    const cx<T> x111 = (-(e2*x77));
-    const cx<T> x112 = (-x111*x31) - x62*x76;
-    const cx<T> x113 = (-(x80));
-    const cx<T> x114 = (-(x113*x61));
-    const cx<T> x115 = (-(x64*x80));
-    const cx<T> x116 = (-(e1*x75));
-    const cx<T> x117 = A + x44 - B + x116*x63 - x111*x45;
-    const cx<T> x118 = U*x112*x114 + x112*x115*z - x114*x117*z - x115*x117*x51;
-    const cx<T> x119 = ec1*x61;
-    const cx<T> x120 = cx<T>(T(1.0)) + x119 + x81;
-    const cx<T> x121 = (-(x79));
-    const cx<T> x122 = U*x121;
-    const cx<T> x123 = (-(x90));
-    const cx<T> x124 = x121*z;
-    const cx<T> x125 = ec1*x123*x65 - ec1*x124*x64;
-    const cx<T> x126 = Qcj + x86 + Qcj*x83;
-    const cx<T> x127 = x36*x90;
-    const cx<T> x129 = x123*z;
-    const cx<T> x132 = x76 - x78;
-    const cx<T> x133 = x81 - x83;
-    const cx<T> x136 = U*x87;
-    const cx<T> x137 = x51*x90;
-    M[424 + g] = x71*x74 + x87*x88 + x90*x91 - x85*z - x90*x92;
-    M[288 + g] = x93*(x38 + x38*x78);
-    M[344 + g] = x110*(x43 + x43*x83);
-    M[352 + g] = (-x125) - x118*(ec1*ec1) - x120*x122 + x120*x123*z;
-    M[360 + g] = x109*x126 - ec2*x127 - x126*x88 + x82*(ec2*ec2)*((-x127) - x30*x88 + x30*x90*z + x34*x79*z) + ec2*x34*x79*z;
-    M[376 + g] = ec1*(ec1*x118 + x124*x80 - x123*x51*x80);
-    M[408 + g] = dQcj*x110*(x20 + x20*x83) + dQj*x93*(x25 + x25*x78) + dP0*x132*z*((-x136) + x84*z) + dPc0*x133*z*((-x137) + x79*z) - dPcj*z*(x122 - x129)*(ec1*x113 + ec2*x82) - dPj*z*(x106 - x102)*(x116 - x111);
+    const CX A(Y[0]);
+    const CX B(Y[1]);
+    const CX D(Y[3]);
+    const CX Dc(Y[10]);
+    const CX G(Y[5]);
+    const CX Gc(Y[12]);
+    const CX Qcj(in.q[22 + j]);
+    const CX Qj(in.q[15 + j]);
+    const CX U(Y[13 + j]);
+    const CX dP0(dq[0]);
+    const CX dPc0(dq[8]);
+    const CX dPcj(dq[8 + j]);
+    const CX dPj(dq[j]);
+    const CX dQcj(dq[22 + j]);
+    const CX dQj(dq[15 + j]);
+    const CX e1(in.e[0]);
+    const CX e2(in.e[1]);
+    const CX ec1(in.e[2]);
+    const CX ec2(in.e[3]);
+    const CX iU(in.iU[j - 1]);
+    const CX x20(in.sa[1][FRG_IN_AC]);
+    const CX x25(in.sa[0][FRG_IN_AC]);
+    const CX x30(in.sb[1][FRG_IN_AQ][j - 1]);
+    const CX x31(in.sa[0][FRG_IN_HP]);
+    const CX x34(in.sa[1][FRG_IN_HP]);
+    const CX x45(in.sb[0][FRG_IN_AQ][j - 1]);
+    const CX x61(in.sb[1][FRG_IN_BP][j - 1]);
+    const CX x62(in.sa[0][FRG_IN_FP]);
+    const CX x63(in.sb[0][FRG_IN_BP][j - 1]);
+    const CX x64(in.sa[1][FRG_IN_FP]);
+    const CX x75(in.sa[0][FRG_IN_BD]);
+    const CX x76(in.sa[0][FRG_IN_EBD]);
+    const CX x77(in.sa[0][FRG_IN_CG]);
+    const CX x78(in.sa[0][FRG_IN_ECG]);
+    const CX x79(in.sa[0][FRG_IN_V]);
+    const CX x80(in.sa[1][FRG_IN_BD]);
+    const CX x81(in.sa[1][FRG_IN_EBD]);
+    const CX x82(in.sa[1][FRG_IN_CG]);
+    const CX x83(in.sa[1][FRG_IN_ECG]);
+    const CX x84(in.sa[1][FRG_IN_V]);
+    const CX x86(in.sb[1][FRG_IN_EAQ][j - 1]);
+    const CX x87(in.sb[1][FRG_IN_W][j - 1]);
+    const CX x90(in.sb[0][FRG_IN_W][j - 1]);
+    const CX z(Y[21]);
+    const CX z2(in.z2);
+    const CX x35 = iU*x34;
+    const CX x36 = x35*z2;
+    const CX x38 = (-CX(T(1.0))) + Qj;
+    const CX x43 = (-CX(T(1.0))) + Qcj;
+    const CX x44 = (-(Qj*x25));
+    const CX x51 = iU*z2;
+    const CX x65 = x51*x64;
+    const CX x70 = (-(G));
+    const CX x71 = D + x70;
+    const CX x72 = (-(Gc));
+    const CX x73 = Dc + x72;
+    const CX x74 = x73*z;
+    const CX x85 = x79*x84;
+    const CX x88 = U*x79;
+    const CX x91 = x51*x84;
+    const CX x92 = x87*z;
+    const CX x93 = x91 - x92;
+    const CX x97 = (-(x84));
+    const CX x100 = (-(x87));
+    const CX x102 = x100*z;
+    const CX x106 = x51*x97;
+    const CX x109 = x90*z;
+    const CX x110 = x88 - x109;
+    const CX x111 = (-(e2*x77));
+    const CX x112 = (-x111*x31) - x62*x76;
+    const CX x113 = (-(x80));
+    const CX x114 = (-(x113*x61));
+    const CX x115 = (-(x64*x80));
+    const CX x116 = (-(e1*x75));
+    const CX x117 = A + x44 - B + x116*x63 - x111*x45;
+    const CX x118 = U*x112*x114 + x112*x115*z - x114*x117*z - x115*x117*x51;
+    const CX x119 = ec1*x61;
+    const CX x120 = CX(T(1.0)) + x119 + x81;
+    const CX x121 = (-(x79));
+    const CX x122 = U*x121;
+    const CX x123 = (-(x90));
+    const CX x124 = x121*z;
+    const CX x125 = ec1*x123*x65 - ec1*x124*x64;
+    const CX x126 = Qcj + x86 + Qcj*x83;
+    const CX x127 = x36*x90;
+    const CX x129 = x123*z;
+    const CX x132 = x76 - x78;
+    const CX x133 = x81 - x83;
+    const CX x136 = U*x87;
+    const CX x137 = x51*x90;
+    cx_put(M + 424 + g, x71*x74 + x87*x88 + x90*x91 - x85*z - x90*x92);
+    cx_put(M + 288 + g, x93*(x38 + x38*x78));
+    cx_put(M + 344 + g, x110*(x43 + x43*x83));
+    cx_put(M + 352 + g, (-x125) - x118*(ec1*ec1) - x120*x122 + x120*x123*z);
+    cx_put(M + 360 + g, x109*x126 - ec2*x127 - x126*x88 + x82*(ec2*ec2)*((-x127) - x30*x88 + x30*x90*z + x34*x79*z) + ec2*x34*x79*z);
+    cx_put(M + 376 + g, ec1*(ec1*x118 + x124*x80 - x123*x51*x80));
+    cx_put(M + 408 + g, dQcj*x110*(x20 + x20*x83) + dQj*x93*(x25 + x25*x78) + dP0*x132*z*((-x136) + x84*z) + dPc0*x133*z*((-x137) + x79*z) - dPcj*z*(x122 - x129)*(ec1*x113 + ec2*x82) - dPj*z*(x106 - x102)*(x116 - x111));
   }
   if constexpr (SLICE == 3) {
-    const cx<T> A = Y[0];
-    const cx<T> Ac = Y[7];
-    const cx<T> B = Y[1];
-    const cx<T> Bc = Y[8];
-    const cx<T> C = Y[2];
-    const cx<T> Cc = Y[9];
-    const cx<T> D = Y[3];
-    const cx<T> F = Y[4];
-    const cx<T> Fc = Y[11];
-    const cx<T> G = Y[5];
-    const cx<T> H = Y[6];
-    const cx<T> Hc = Y[13];
-    const cx<T> P0 = in.q[0];
-    const cx<T> Pc0 = in.q[8];
-    const cx<T> Pcj = in.q[8 + j];
-    const cx<T> Pj = in.q[j];
-    const cx<T> Qcj = in.q[22 + j];
-    const cx<T> U = Y[13 + j];
-    const cx<T> ec1 = in.e[2];
-    const cx<T> ec2 = in.e[3];
-    const cx<T> iU = in.iU[j - 1];
-    const cx<T> x11 = in.sb[1][FRG_IN_PJZ][j - 1];
-    const cx<T> x16 = in.sb[0][FRG_IN_PJZ][j - 1];
-    const cx<T> x2 = in.sa[1][FRG_IN_PZ];
-    const cx<T> x21 = in.sb[1][FRG_IN_QA][j - 1];
-    const cx<T> x23 = in.sb[0][FRG_IN_AP][j - 1];
-    const cx<T> x26 = in.sb[0][FRG_IN_QA][j - 1];
-    const cx<T> x28 = in.sb[1][FRG_IN_AP][j - 1];
-    const cx<T> x30 = in.sb[1][FRG_IN_AQ][j - 1];
-    const cx<T> x31 = in.sa[0][FRG_IN_HP];
-    const cx<T> x33 = in.sb[0][FRG_IN_AQ][j - 1];
-    const cx<T> x34 = in.sa[1][FRG_IN_HP];
-    const cx<T> x39 = in.sb[1][FRG_IN_AQ][j - 1];
-    const cx<T> x6 = in.sa[0][FRG_IN_PZ];
-    const cx<T> x61 = in.sb[1][FRG_IN_BP][j - 1];
-    const cx<T> x62 = in.sa[0][FRG_IN_FP];
-    const cx<T> x63 = in.sb[0][FRG_IN_BP][j - 1];
-    const cx<T> x64 = in.sa[1][FRG_IN_FP];
-    const cx<T> x79 = in.sa[0][FRG_IN_V];
-    const cx<T> x83 = in.sa[1][FRG_IN_ECG];
-    const cx<T> x90 = in.sb[0][FRG_IN_W][j - 1];
-    const cx<T> z = Y[21];
-    const cx<T> z2 = in.z2;
-    const cx<T> x0 = P0*Pc0 + Pcj*Pj;
-    const cx<T> x3 = (-(x2));
-    const cx<T> x4 = Cc + x3;
-    const cx<T> x7 = (-(x6));
-    const cx<T> x8 = C + x7;
-    const cx<T> x10 = (-(Ac));
-    const cx<T> x12 = x10 + x11;
-    const cx<T> x13 = Cc + x12;
-    const cx<T> x15 = (-(A));
-    const cx<T> x17 = x15 + x16;
-    const cx<T> x18 = C + x17;
-    const cx<T> x24 = x23*z;
-    const cx<T> x32 = U*x31;
-    const cx<T> x35 = iU*x34;
-    const cx<T> x36 = x35*z2;
-    const cx<T> x40 = U*x39;
-    const cx<T> x41 = A*z;
-    const cx<T> x42 = Qcj*x24;
-    const cx<T> x43 = (-cx<T>(T(1.0))) + Qcj;
-    const cx<T> x49 = (T(3.0)*(x0*z2));
-    const cx<T> x50 = Pj*z2;
-    const cx<T> x51 = iU*z2;
-    const cx<T> x56 = Bc + x3;
-    const cx<T> x58 = B + x7;
-    const cx<T> x60 = B*Pcj + Bc*Pj;
-    const cx<T> x65 = x51*x64;
-    const cx<T> x66 = U*x61;
-    const cx<T> x67 = U*x62;
-    const cx<T> x68 = x51*x63;
-    const cx<T> x70 = (-(G));
-    const cx<T> x71 = D + x70;
-    const cx<T> x119 = ec1*x61;
-    const cx<T> x121 = (-(x79));
-    const cx<T> x123 = (-(x90));
-    const cx<T> x124 = x121*z;
-    const cx<T> x125 = ec1*x123*x65 - ec1*x124*x64;
-    const cx<T> x128 = x71*z;
-    const cx<T> x129 = x123*z;
-    const cx<T> x130 = x121*x40;
-    const cx<T> x131 = x123*x36;
-    M[56 + g] = x42 - x41 + x18*z + x26*z - x32*x43;
-    M[72 + g] = x41 - x42 + Qcj*x32 - H*z;
-    M[112 + g] = (-x49) + A*x11 + A*x13 + Ac*x16 + Ac*x18 + H*x2 + Hc*x6 + x21*x23 + x26*x28 - H*x4 - Hc*x8 - Pcj*x32 - x11*x26 - x16*x21 - x35*x50 - P0*U*x30 - Pc0*x33*x51 + (T(2.0)*(x33*x35*z));
-    M[208 + g] = x50 + x67 - F*z;
-    M[232 + g] = x68 - x58*z;
-    M[256 + g] = (-x49) - F*x56 - Fc*x58 - P0*x66 - Pc0*x68 - Pcj*x67 + (T(2.0)*(x60*z)) + F*Pc0*z + Fc*P0*z - iU*x50*x64 + (T(2.0)*(iU*x63*x64*z));
-    M[368 + g] = x125 + x128 - x119*x129 + ec1*x121*x66;
-    M[384 + g] = (-x128) - ec2*x130 - ec2*x131 + ec2*x121*x34*z + ec2*x123*x39*z;
-    M[392 + g] = x83*((-x124) - ec2*(x130 + x131 - x124*x34 - x129*x39) + iU*x123*z2);
+    const CX A(Y[0]);
+    const CX Ac(Y[7]);
+    const CX B(Y[1]);
+    const CX Bc(Y[8]);
+    const CX C(Y[2]);
+    const CX Cc(Y[9]);
+    const CX D(Y[3]);
+    const CX F(Y[4]);
+    const CX Fc(Y[11]);
+    const CX G(Y[5]);
+    const CX H(Y[6]);
+    const CX Hc(Y[13]);
+    const CX P0(in.q[0]);
+    const CX Pc0(in.q[8]);
+    const CX Pcj(in.q[8 + j]);
+    const CX Pj(in.q[j]);
+    const CX Qcj(in.q[22 + j]);
+    const CX U(Y[13 + j]);
+    const CX ec1(in.e[2]);
+    const CX ec2(in.e[3]);
+    const CX iU(in.iU[j - 1]);
+    const CX x11(in.sb[1][FRG_IN_PJZ][j - 1]);
+    const CX x16(in.sb[0][FRG_IN_PJZ][j - 1]);
+    const CX x2(in.sa[1][FRG_IN_PZ]);
+    const CX x21(in.sb[1][FRG_IN_QA][j - 1]);
+    const CX x23(in.sb[0][FRG_IN_AP][j - 1]);
+    const CX x26(in.sb[0][FRG_IN_QA][j - 1]);
+    const CX x28(in.sb[1][FRG_IN_AP][j - 1]);
+    const CX x30(in.sb[1][FRG_IN_AQ][j - 1]);
+    const CX x31(in.sa[0][FRG_IN_HP]);
+    const CX x33(in.sb[0][FRG_IN_AQ][j - 1]);
+    const CX x34(in.sa[1][FRG_IN_HP]);
+    const CX x39(in.sb[1][FRG_IN_AQ][j - 1]);
+    const CX x6(in.sa[0][FRG_IN_PZ]);
+    const CX x61(in.sb[1][FRG_IN_BP][j - 1]);
+    const CX x62(in.sa[0][FRG_IN_FP]);
+    const CX x63(in.sb[0][FRG_IN_BP][j - 1]);
+    const CX x64(in.sa[1][FRG_IN_FP]);
+    const CX x79(in.sa[0][FRG_IN_V]);
+    const CX x83(in.sa[1][FRG_IN_ECG]);
+    const CX x90(in.sb[0][FRG_IN_W][j - 1]);
+    const CX z(Y[21]);
+    const CX z2(in.z2);
+    const CX x0 = P0*Pc0 + Pcj*Pj;
+    const CX x3 = (-(x2));
+    const CX x4 = Cc + x3;
+    const CX x7 = (-(x6));
+    const CX x8 = C + x7;
+    const CX x10 = (-(Ac));
+    const CX x12 = x10 + x11;
+    const CX x13 = Cc + x12;
+    const CX x15 = (-(A));
+    const CX x17 = x15 + x16;
+    const CX x18 = C + x17;
+    const CX x24 = x23*z;
+    const CX x32 = U*x31;
+    const CX x35 = iU*x34;
+    const CX x36 = x35*z2;
+    const CX x40 = U*x39;
+    const CX x41 = A*z;
+    const CX x42 = Qcj*x24;
+    const CX x43 = (-CX(T(1.0))) + Qcj;
+    const auto x49 = (T(3.0)*(x0*z2));
+    const CX x50 = Pj*z2;
+    const CX x51 = iU*z2;
+    const CX x56 = Bc + x3;
+    const CX x58 = B + x7;
+    const CX x60 = B*Pcj + Bc*Pj;
+    const CX x65 = x51*x64;
+    const CX x66 = U*x61;
+    const CX x67 = U*x62;
+    const CX x68 = x51*x63;
+    const CX x70 = (-(G));
+    const CX x71 = D + x70;
+    const CX x119 = ec1*x61;
+    const CX x121 = (-(x79));
+    const CX x123 = (-(x90));
+    const CX x124 = x121*z;
+    const CX x125 = ec1*x123*x65 - ec1*x124*x64;
+    const CX x128 = x71*z;
+    const CX x129 = x123*z;
+    const CX x130 = x121*x40;
+    const CX x131 = x123*x36;
+    cx_put(M + 56 + g, x42 - x41 + x18*z + x26*z - x32*x43);
+    cx_put(M + 72 + g, x41 - x42 + Qcj*x32 - H*z);
+    cx_put(M + 112 + g, (-x49) + A*x11 + A*x13 + Ac*x16 + Ac*x18 + H*x2 + Hc*x6 + x21*x23 + x26*x28 - H*x4 - Hc*x8 - Pcj*x32 - x11*x26 - x16*x21 - x35*x50 - P0*U*x30 - Pc0*x33*x51 + (T(2.0)*(x33*x35*z)));
+    cx_put(M + 208 + g, x50 + x67 - F*z);
+    cx_put(M + 232 + g, x68 - x58*z);
+    cx_put(M + 256 + g, (-x49) - F*x56 - Fc*x58 - P0*x66 - Pc0*x68 - Pcj*x67 + (T(2.0)*(x60*z)) + F*Pc0*z + Fc*P0*z - iU*x50*x64 + (T(2.0)*(iU*x63*x64*z)));
+    cx_put(M + 368 + g, x125 + x128 - x119*x129 + ec1*x121*x66);
+    cx_put(M + 384 + g, (-x128) - ec2*x130 - ec2*x131 + ec2*x121*x34*z + ec2*x123*x39*z);
+    cx_put(M + 392 + g, x83*((-x124) - ec2*(x130 + x131 - x124*x34 - x129*x39) + iU*x123*z2));
   }
 }
 
 // One of the three equations at the point Y (frg_group_f's operations in its order).
 template <int SLICE, typename T>
 __device__ __forceinline__ cx<T> frg_residual_slice(const cx<T>* Y, const FrgEvalIn<T>& in, int j) {
+  typedef cx<T> CX;
   if constexpr (SLICE == 0) {
-    const cx<T> A = Y[0];
-    const cx<T> Ac = Y[7];
-    const cx<T> C = Y[2];
-    const cx<T> Cc = Y[9];
-    const cx<T> H = Y[6];
-    const cx<T> Hc = Y[13];
-    const cx<T> P0 = in.q[0];
-    const cx<T> Pc0 = in.q[8];
-    const cx<T> Pcj = in.q[8 + j];
-    const cx<T> Pj = in.q[j];
-    const cx<T> U = Y[13 + j];
-    const cx<T> iU = in.iU[j - 1];
-    const cx<T> y10 = in.sb[0][FRG_IN_AP][j - 1];
-    const cx<T> y12 = in.sb[1][FRG_IN_QA][j - 1];
-    const cx<T> y14 = in.sb[1][FRG_IN_AP][j - 1];
-    const cx<T> y16 = in.sb[0][FRG_IN_QA][j - 1];
-    const cx<T> y17 = in.sa[0][FRG_IN_HP];
-    const cx<T> y18 = in.sa[1][FRG_IN_HP];
-    const cx<T> y4 = in.sb[1][FRG_IN_PJZ][j - 1];
-    const cx<T> y7 = in.sb[0][FRG_IN_PJZ][j - 1];
-    const cx<T> z = Y[21];
-    const cx<T> z2 = in.z2;
-    const cx<T> z3 = in.z3;
-    const cx<T> y0 = z3*(P0*Pc0 + Pcj*Pj);
-    const cx<T> y1 = (-(Pc0*z));
-    const cx<T> y2 = (-(P0*z));
-    const cx<T> y3 = (-(Ac));
-    const cx<T> y5 = y3 + y4;
-    const cx<T> y6 = (-(A));
-    const cx<T> y8 = y6 + y7;
-    const cx<T> y19 = iU*z2;
+    const CX A(Y[0]);
+    const CX Ac(Y[7]);
+    const CX C(Y[2]);
+    const CX Cc(Y[9]);
+    const CX H(Y[6]);
+    const CX Hc(Y[13]);
+    const CX P0(in.q[0]);
+    const CX Pc0(in.q[8]);
+    const CX Pcj(in.q[8 + j]);
+    const CX Pj(in.q[j]);
+    const CX U(Y[13 + j]);
+    const CX iU(in.iU[j - 1]);
+    const CX y10(in.sb[0][FRG_IN_AP][j - 1]);
+    const CX y12(in.sb[1][FRG_IN_QA][j - 1]);
+    const CX y14(in.sb[1][FRG_IN_AP][j - 1]);
+    const CX y16(in.sb[0][FRG_IN_QA][j - 1]);
+    const CX y17(in.sa[0][FRG_IN_HP]);
+    const CX y18(in.sa[1][FRG_IN_HP]);
+    const CX y4(in.sb[1][FRG_IN_PJZ][j - 1]);
+    const CX y7(in.sb[0][FRG_IN_PJZ][j - 1]);
+    const CX z(Y[21]);
+    const CX z2(in.z2);
+    const CX z3(in.z3);
+    const CX y0 = z3*(P0*Pc0 + Pcj*Pj);
+    const CX y1 = (-(Pc0*z));
+    const CX y2 = (-(P0*z));
+    const CX y3 = (-(Ac));
+    const CX y5 = y3 + y4;
+    const CX y6 = (-(A));
+    const CX y8 = y6 + y7;
+    const CX y19 = iU*z2;
     return (-y0) + A*z*(Cc + y5) + Ac*z*(C + y8) + U*y17*((-y12) - y5) + y10*y12*z + y14*y16*z + y18*y19*((-y16) - y8) - H*z*(Cc + y1) - Hc*z*(C + y2);
   }
   if constexpr (SLICE == 1) {
-    const cx<T> B = Y[1];
-    const cx<T> Bc = Y[8];
-    const cx<T> F = Y[4];
-    const cx<T> Fc = Y[11];
-    const cx<T> P0 = in.q[0];
-    const cx<T> Pc0 = in.q[8];
-    const cx<T> Pcj = in.q[8 + j];
-    const cx<T> Pj = in.q[j];
-    const cx<T> U = Y[13 + j];
-    const cx<T> iU = in.iU[j - 1];
-    const cx<T> y20 = in.sb[1][FRG_IN_BP][j - 1];
-    const cx<T> y21 = in.sa[0][FRG_IN_FP];
-    const cx<T> y22 = in.sb[0][FRG_IN_BP][j - 1];
-    const cx<T> y23 = in.sa[1][FRG_IN_FP];
-    const cx<T> z = Y[21];
-    const cx<T> z2 = in.z2;
-    const cx<T> z3 = in.z3;
-    const cx<T> y0 = z3*(P0*Pc0 + Pcj*Pj);
-    const cx<T> y1 = (-(Pc0*z));
-    const cx<T> y2 = (-(P0*z));
+    const CX B(Y[1]);
+    const CX Bc(Y[8]);
+    const CX F(Y[4]);
+    const CX Fc(Y[11]);
+    const CX P0(in.q[0]);
+    const CX Pc0(in.q[8]);
+    const CX Pcj(in.q[8 + j]);
+    const CX Pj(in.q[j]);
+    const CX U(Y[13 + j]);
+    const CX iU(in.iU[j - 1]);
+    const CX y20(in.sb[1][FRG_IN_BP][j - 1]);
+    const CX y21(in.sa[0][FRG_IN_FP]);
+    const CX y22(in.sb[0][FRG_IN_BP][j - 1]);
+    const CX y23(in.sa[1][FRG_IN_FP]);
+    const CX z(Y[21]);
+    const CX z2(in.z2);
+    const CX z3(in.z3);
+    const CX y0 = z3*(P0*Pc0 + Pcj*Pj);
+    const CX y1 = (-(Pc0*z));
+    const CX y2 = (-(P0*z));
     return (-y0) + z2*(B*Pcj + Bc*Pj) + U*y20*y21 - F*z*(Bc + y1) - Fc*z*(B + y2) + iU*y22*y23*z2;
   }
   if constexpr (SLICE == 2) {
-    const cx<T> D = Y[3];
-    const cx<T> Dc = Y[10];
-    const cx<T> G = Y[5];
-    const cx<T> Gc = Y[12];
-    const cx<T> U = Y[13 + j];
-    const cx<T> iU = in.iU[j - 1];
-    const cx<T> y28 = in.sa[0][FRG_IN_V];
-    const cx<T> y31 = in.sa[1][FRG_IN_V];
-    const cx<T> y32 = in.sb[1][FRG_IN_W][j - 1];
-    const cx<T> y33 = in.sb[0][FRG_IN_W][j - 1];
-    const cx<T> z = Y[21];
-    const cx<T> z2 = in.z2;
-    const cx<T> y19 = iU*z2;
-    const cx<T> y24 = (-(G));
-    const cx<T> y25 = (-(Gc));
+    const CX D(Y[3]);
+    const CX Dc(Y[10]);
+    const CX G(Y[5]);
+    const CX Gc(Y[12]);
+    const CX U(Y[13 + j]);
+    const CX iU(in.iU[j - 1]);
+    const CX y28(in.sa[0][FRG_IN_V]);
+    const CX y31(in.sa[1][FRG_IN_V]);
+    const CX y32(in.sb[1][FRG_IN_W][j - 1]);
+    const CX y33(in.sb[0][FRG_IN_W][j - 1]);
+    const CX z(Y[21]);
+    const CX z2(in.z2);
+    const CX y19 = iU*z2;
+    const CX y24 = (-(G));
+    const CX y25 = (-(Gc));
     return U*y28*y32 + y19*y31*y33 + z*(D + y24)*(Dc + y25) - y28*y31*z - y32*y33*z;
   }
 }

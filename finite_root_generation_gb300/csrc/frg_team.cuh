@@ -24,16 +24,17 @@
 //
 // What bounds it: on this part a warp-wide FP64 instruction holds its sub-partition's
 // FP64 pipe for 64 cycles and answers after about 73, whatever the number of active
-// lanes, so an FP64 step takes (FP64 warp instructions on its longest warp) x 64..82
+// lanes, so an FP64 step takes (FP64 warp instructions on its longest warp) x 64..91
 // cycles and everything else hides behind them; the FP32 step is bound by instruction
 // issue and fetch. With one path per 8 lanes (four paths in a warp, the layout before
 // this one) an FP64 step was 5,800 FP64 instructions in one warp, 421k cycles; cut over
-// the four sub-partitions and with 32 lanes on the elimination it is 1,590 on the
-// longest warp, 131k cycles (8 to 600 paths; FP32 step 105k -> 19k). With every SM full
-// the FP64 work per path falls as well (fewer repeated sums and idle lanes: 9.3 against
-// 5.7 M FP64 steps/s, 49 against 32 M steps/s in the mixed-precision benchmark rounds).
-// Comparisons and maxima of FP64 values run on their bit patterns in the integer pipes
-// for the same reason.
+// the four sub-partitions, with 32 lanes on the elimination and equal operations of
+// different quantities in the same instructions, it is about 1,400 on the longest warp,
+// 123k cycles, and 1,150, 106k cycles, while a block has one or two paths (PairCx). The
+// FP32 step went from 105k to 19k. With every SM full the FP64 work per path falls as
+// well (fewer repeated sums and idle lanes): FP64 rounds of 32,768 paths, three in flight,
+// 6,815 to 3,696 ms a round. Comparisons, maxima and stored negations of FP64 values run
+// on their bit patterns in the integer pipes for the same reason.
 #pragma once
 
 #include "frg_device.cuh"
@@ -41,6 +42,13 @@
 #include "frg_warp.cuh"
 
 namespace frg {
+
+__device__ __forceinline__ df neg_if(df x, bool neg) { return neg ? -x : x; }
+__device__ __forceinline__ cx<df> warp_shfl(cx<df> v, int src) {
+  return cx<df>(df(__shfl_sync(FULL, v.re.hi, src), __shfl_sync(FULL, v.re.lo, src)),
+                df(__shfl_sync(FULL, v.im.hi, src), __shfl_sync(FULL, v.im.lo, src)));
+}
+
 namespace team {
 
 // Type of the path's points (Yc, Yn, YN) and of the FP32 stage's refinement residual:
@@ -76,6 +84,9 @@ __device__ __forceinline__ T team_max(unsigned mask, T v) {
   v = fmax(v, shfl_xor(mask, v, 1));
   return v;
 }
+
+template <typename T>
+__device__ __forceinline__ cx<T> neg(cx<T> a) { return cx<T>(neg_if(a.re, true), neg_if(a.im, true)); }
 
 // Task and start parameters in the working precision, when it is not the point type's.
 template <typename T, typename P> struct LowTask { cx<T> sp[32], fp[32]; };
@@ -138,58 +149,82 @@ struct StepOut {
   T hnorm;   // |H| at the evaluation point (Newton, when asked for)
 };
 
-// What the evaluation of one path at Y needs: q(t) (and dq/dt, htpysupport.cu:37-62), one
-// parameter per lane; the reciprocals, one per lane; then the hoisted quantities, lane
-// 8 s + g for side s and group g. RESID: frg_group_f's forms (the refinement residual).
+// What the evaluation of one path at Y needs: the reciprocals, one per lane (1 / U_j on
+// lanes 0..6, e on 8..11, q's denominator on 12); q(t) (and dq/dt, htpysupport.cu:37-62),
+// one parameter per lane, with z^2 and z^3 on lane 31 in the same products; then the
+// hoisted quantities, lanes 8 s + g those of side s and group g, lanes 16 + s those that
+// are the same for every group, again in the same instructions. RESID: frg_group_f's forms
+// (the refinement residual). 81 FP64 instructions; with each quantity in instructions of
+// its own it was 143.
 template <bool RESID, typename V>
 __device__ __forceinline__ void eval_prep(const cx<V>* Y, const cx<V>* sp, const cx<V>* fp, cx<V> gamma,
                                           FrgEvalIn<V>& in, cx<V>* dq, int lane) {
   const V t = Y[22].re;
-  const cx<V> g1t = gamma * (V(1) - t);
-  const cx<V> iden = cinv(g1t + cx<V>(t));
-  if (lane < NP) {
-    const cx<V> s = sp[lane], f = fp[lane];
-    in.q[lane] = (g1t * s + t * f) * iden;
-    if constexpr (!RESID) dq[lane] = (f - s) * (gamma * (iden * iden));
-  }
-  const int ea = lane == 8 ? 4 : lane == 9 ? 6 : lane == 10 ? 11 : 13;   // F, H, Fc, Hc
-  const int eb = lane == 8 ? 1 : lane == 9 ? 2 : lane == 10 ? 8 : 9;     // B, C, Bc, Cc
-  if (lane < 7 || (lane >= 8 && lane < 12)) {
-    const cx<V> b = lane < 7 ? Y[14 + lane] : Y[ea] - Y[eb];
-    const cx<V> ib = cinv(b);
-    if (lane < 7) in.iU[lane] = ib; else in.e[lane - 8] = ib;
-  }
   const cx<V> z = Y[21];
-  const cx<V> z2 = z * z;
-  const cx<V> z3 = z2 * z;
-  if (lane == 0) { in.z2 = z2; in.z3 = z3; }
-  __syncwarp();
-  if (lane < 16 && (lane & 7) < 7) {
-    const int s = lane >> 3, g = lane & 7;
-    const cx<V>* L = Y + 7 * s;  // A, B, C, D, F, G, H of this side
-    const cx<V> e1 = in.e[2 * s], e2 = in.e[2 * s + 1];
-    const cx<V> P0 = in.q[8 * s], Pj = in.q[8 * s + 1 + g], Qj = in.q[15 + 7 * s + 1 + g];
-    const cx<V> pz = P0 * z, fpz = L[4] - pz, hpz = L[6] - pz;
-    const cx<V> bd = L[1] - L[3], ebd = e1 * bd, cg = L[2] - L[5], ecg = e2 * cg;
-    const cx<V> v = fpz * ebd - hpz * ecg, ac = L[0] - L[2];
-    const cx<V> pjz = Pj * z, ap = L[0] - pjz, bp = L[1] - pjz, qa = Qj * ac, aq = ap - qa;
-    in.sb[s][FRG_IN_PJZ][g] = pjz;
-    in.sb[s][FRG_IN_AP][g] = ap;
-    in.sb[s][FRG_IN_BP][g] = bp;
-    in.sb[s][FRG_IN_QA][g] = qa;
-    in.sb[s][FRG_IN_AQ][g] = aq;
-    if constexpr (RESID) {
-      in.sb[s][FRG_IN_W][g] = L[1] + qa - L[0] + bp * ebd - ecg * aq;
-    } else {
-      const cx<V> eaq = e2 * aq;
-      in.sb[s][FRG_IN_EAQ][g] = eaq;
-      in.sb[s][FRG_IN_W][g] = L[1] - L[0] + qa + bp * ebd - cg * eaq;
+  const cx<V> g1t = gamma * (V(1) - t);
+  cx<V> ib;
+  {
+    const int ea = lane == 8 ? 4 : lane == 9 ? 6 : lane == 10 ? 11 : 13;  // F, H, Fc, Hc
+    const int eb = lane == 8 ? 1 : lane == 9 ? 2 : lane == 10 ? 8 : 9;    // B, C, Bc, Cc
+    // a - b with b = -t on lane 12 (a + t and a - (-t) round alike)
+    const cx<V> x = lane == 12 ? g1t : Y[ea], y = lane == 12 ? cx<V>(neg_if(t, true)) : Y[eb];
+    const cx<V> d = x - y;
+    ib = cinv(lane < 7 ? Y[14 + lane] : d);
+  }
+  if (lane < 7) in.iU[lane] = ib;
+  if (lane >= 8 && lane < 12) in.e[lane - 8] = ib;
+  const cx<V> iden = warp_shfl(ib, 12);
+  {
+    const bool l31 = lane == 31;
+    const cx<V> a = l31 ? z : iden;
+    const cx<V> sq = a * a;
+    const cx<V> cu = (l31 ? sq : gamma) * (l31 ? z : sq);
+    if (l31) { in.z2 = sq; in.z3 = cu; }
+    const int i = lane < NP ? lane : 0;
+    const cx<V> s = sp[i], f = fp[i];
+    const cx<V> q = (g1t * s + t * f) * iden;
+    if (lane < NP) in.q[lane] = q;
+    if constexpr (!RESID) {
+      const cx<V> v = (f - s) * cu;
+      if (lane < NP) dq[lane] = v;
     }
-    if (g == 0) {
+  }
+  __syncwarp();
+  {
+    const bool all = lane >= 16;  // lanes 16, 17: the same for every group
+    const int s = all ? lane & 1 : lane >> 3, g = (lane & 7) < 7 ? lane & 7 : 6;
+    const cx<V>* L = Y + 7 * s;  // A, B, C, D, F, G, H of this side
+    const cx<V> e2 = in.e[2 * s + 1];
+    const cx<V> m0 = in.q[all ? 8 * s : 8 * s + 1 + g] * z;                  // pjz | pz
+    const cx<V> d0 = L[all ? 4 : 0] - m0, d1 = L[all ? 6 : 1] - m0;          // ap, bp | fp, hp
+    const cx<V> d2 = L[all ? 1 : 0] - L[all ? 3 : 2];                        // ac | bd
+    const cx<V> m1 = (all ? in.e[2 * s] : in.q[15 + 7 * s + 1 + g]) * d2;    // qa | ebd
+    const cx<V> d3 = (all ? L[2] : d0) - (all ? L[5] : m1);                  // aq | cg
+    const cx<V> m2 = e2 * d3;                                                // eaq | ecg
+    const cx<V> ebd = warp_shfl(m1, 16 + s);
+    const cx<V> w0 = RESID ? L[1] + m1 - L[0] : L[1] - L[0] + m1;
+    const cx<V> t0 = (all ? d0 : d1) * ebd;                                  // bp ebd | fp ebd
+    const cx<V> w1 = w0 + t0;
+    cx<V> t1;
+    if constexpr (RESID) {
+      const cx<V> ecg = warp_shfl(m2, 16 + s);
+      t1 = (all ? d1 : ecg) * (all ? m2 : d3);                               // ecg aq | hp ecg
+    } else {
+      const cx<V> cg = warp_shfl(d3, 16 + s);
+      t1 = (all ? d1 : cg) * m2;                                             // cg eaq | hp ecg
+    }
+    const cx<V> w = (all ? t0 : w1) - t1;                                    // w | v
+    if (lane < 16) {
+      cx<V>(*o)[8] = in.sb[s];
+      const int c = lane & 7;
+      o[FRG_IN_PJZ][c] = m0; o[FRG_IN_AP][c] = d0; o[FRG_IN_BP][c] = d1;
+      o[FRG_IN_QA][c] = m1;  o[FRG_IN_AQ][c] = d3; o[FRG_IN_W][c] = w;
+      if constexpr (!RESID) o[FRG_IN_EAQ][c] = m2;
+      if (c == 0) in.sa[s][FRG_IN_AC] = d2;
+    } else if (lane < 18) {
       cx<V>* o = in.sa[s];
-      o[FRG_IN_PZ] = pz;   o[FRG_IN_FP] = fpz;  o[FRG_IN_HP] = hpz;
-      o[FRG_IN_BD] = bd;   o[FRG_IN_EBD] = ebd; o[FRG_IN_CG] = cg;
-      o[FRG_IN_ECG] = ecg; o[FRG_IN_V] = v;     o[FRG_IN_AC] = ac;
+      o[FRG_IN_PZ] = m0;  o[FRG_IN_FP] = d0; o[FRG_IN_HP] = d1;  o[FRG_IN_BD] = d2;
+      o[FRG_IN_EBD] = m1; o[FRG_IN_CG] = d3; o[FRG_IN_ECG] = m2; o[FRG_IN_V] = w;
     }
   }
 }
@@ -212,74 +247,148 @@ __device__ __forceinline__ T patch_scale(const cx<T>* u, int lane) {
   return T(1) / m.value();
 }
 
-// Row with the largest v (ties: the lowest), v >= 0 or -1 for used rows; lanes 16 h + r
-// hold row r's value for h = 0 and 1. Infinite and NaN candidates take the comparisons one
-// by one, as lane 0 sees them.
-template <typename T>
+// Row with the largest v (ties: the lowest), v >= 0 or -1 for used rows; lanes h RP + r
+// hold row r's value for every h. Infinite and NaN candidates take the comparisons one by
+// one, as lane 0 sees them.
+template <int RP, typename T>
 __device__ __noinline__ int pivot_row_nonfinite(T v, int r) {
   const T v0 = __shfl_sync(FULL, v, r & ~1), v1 = __shfl_sync(FULL, v, r | 1);
   T bv = v0 >= v1 ? v0 : v1;
   int bk = (r & ~1) + (v0 >= v1 ? 0 : 1);
-  for (int off = 8; off >= 2; off >>= 1) {
+  for (int off = RP / 2; off >= 2; off >>= 1) {
     const T ov = __shfl_xor_sync(FULL, bv, off);
     const int ok = __shfl_xor_sync(FULL, bk, off);
     if (ov > bv || (ov == bv && ok < bk)) { bv = ov; bk = ok; }
   }
   return __shfl_sync(FULL, bk, 0);
 }
+template <int RP>
 __device__ __forceinline__ int pivot_row(float v, int r) {
   const int key = __float_as_int(v);
   const int m = __reduce_max_sync(FULL, key);
-  if (m >= 0x7f800000) return pivot_row_nonfinite(v, r);
-  return __ffs(__ballot_sync(FULL, key == m) & 0xffffu) - 1;
+  if (m >= 0x7f800000) return pivot_row_nonfinite<RP>(v, r);
+  return __ffs(__ballot_sync(FULL, key == m)) - 1;
 }
+template <int RP>
 __device__ __forceinline__ int pivot_row(double v, int r) {
   const int hi = __double2hiint(v);
   const unsigned lo = (unsigned)__double2loint(v);
   const int m = __reduce_max_sync(FULL, hi);
-  if (m >= 0x7ff00000) return pivot_row_nonfinite(v, r);
-  unsigned cand = __ballot_sync(FULL, hi == m) & 0xffffu;
-  if (cand & (cand - 1)) {
+  if (m >= 0x7ff00000) return pivot_row_nonfinite<RP>(v, r);
+  unsigned cand = __ballot_sync(FULL, hi == m);
+  if (__popc(cand) > 32 / RP) {
     const unsigned ml = __reduce_max_sync(FULL, hi == m ? lo : 0u);
-    cand = __ballot_sync(FULL, hi == m && lo == ml) & 0xffffu;
+    cand = __ballot_sync(FULL, hi == m && lo == ml);
   }
   return __ffs(cand) - 1;
 }
 
-// Four steps k0..k0 + 3 of the dense elimination, W columns per lane. Lane 16 h + r holds
-// row r's remaining columns c = h mod 2 (the right-hand side is column 16) from index 0;
-// a step drops the pivot column, so the lanes that held it move their window up one. The
-// pivot row goes to U and every lane reads it back from there; U[k][k] keeps the pivot's
-// reciprocal. Windows of 8, 6, 4 and 2 columns for four steps each: 80 complex updates per
-// lane where 72 are needed, in code that stays small.
-template <int W, typename T>
+// a * b where lanes that differ in `bit` hold the same operands: in FP64 each computes one
+// component (the same operations as the complex product's) and they exchange
+__device__ __forceinline__ cx<float> mul_split(cx<float> a, cx<float> b, int, int) { return a * b; }
+__device__ __forceinline__ cx<double> mul_split(cx<double> a, cx<double> b, int lane, int bit) {
+  const bool im = lane & bit;
+  const double own = fma(a.re, im ? b.im : b.re, __dmul_rn(neg_if(a.im, !im), im ? b.re : b.im));
+  const double ot = __shfl_xor_sync(FULL, own, bit);
+  return im ? cx<double>(ot, own) : cx<double>(own, ot);
+}
+
+// Four steps k0..k0 + 3 of the dense elimination of RP rows, W columns per lane. Lane
+// RP h + r holds row r's remaining columns c = h mod 32 / RP (the right-hand side is column
+// 16) from index 0; a step drops the pivot column, so the lanes that held it move their
+// window up one. The pivot row goes to U and every lane reads it back from there; U[k][k]
+// keeps the pivot's reciprocal.
+template <int W, int RP, typename T>
 __device__ __forceinline__ void lu_stage(cx<T>* U, int k0, int lane, cx<T>* R, bool& used, T& pmax, T& pmin) {
-  const int h = lane >> 4, r = lane & 15;
+  constexpr int CL = 32 / RP;
+  const int h = lane / RP, r = lane % RP;
 #pragma unroll 1
   for (int k = k0; k < k0 + 4; ++k) {
-    const bool own = h == (k & 1);
-    const cx<T> e = warp_shfl(R[0], ((k & 1) << 4) + r);  // this row's entry in column k
+    const bool own = h == (k & (CL - 1));
+    const cx<T> e = warp_shfl(R[0], (k & (CL - 1)) * RP + r);  // this row's entry in column k
     const T v = used ? T(-1) : cnorm2(e);
-    const int pr = pivot_row(v, r);
-    cx<T>* Uk = U + k * LDU + k + 1 + ((h ^ (k + 1)) & 1);
+    const int pr = pivot_row<RP>(v, r);
+    cx<T>* Uk = U + k * LDU + k + 1 + ((h - (k + 1)) & (CL - 1));
     cx<T> X[W];
 #pragma unroll
     for (int i = 0; i < W; ++i) X[i] = own ? R[i + 1] : R[i];
     if (r == pr) {
       used = true;
 #pragma unroll
-      for (int i = 0; i < W; ++i) Uk[2 * i] = X[i];
+      for (int i = 0; i < W; ++i) Uk[CL * i] = X[i];
     }
     const T pa = __shfl_sync(FULL, v, pr);
     const cx<T> ip = cinv_norm(warp_shfl(e, pr), pa);
     if (lane == 0) U[k * LDU + k] = ip;
     pmax = max_mag(pmax, pa);
     pmin = min_mag(pmin, pa);
-    const cx<T> l = used ? cx<T>(T(0)) : e * ip;
+    const cx<T> el = mul_split(e, ip, lane, RP), l = used ? cx<T>(T(0)) : el;
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < W; ++i) R[i] = cfms(X[i], l, Uk[2 * i]);
+    for (int i = 0; i < W; ++i) R[i] = cfms(X[i], l, Uk[CL * i]);
   }
+}
+
+// Dense 16 x 16 LU with partial pivoting across the lanes. Eight steps with two lanes a
+// row, then the eight remaining rows, in their order, with four lanes a row: 68 complex
+// updates per lane (80 with two lanes a row throughout; the triangle needs 64).
+template <typename T>
+__device__ __forceinline__ void dense_lu(cx<T>* U, int lane, T& pmax, T& pmin) {
+  cx<T> R[9];
+  bool used = false;
+  {
+    const int h = lane >> 4, r = lane & 15;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) R[i] = U[r * LDU + h + 2 * i];
+    R[8] = h == 0 ? U[r * LDU + 16] : cx<T>(T(0));
+    __syncwarp();
+    lu_stage<8, 16>(U, 0, lane, R, used, pmax, pmin);
+    lu_stage<6, 16>(U, 4, lane, R, used, pmax, pmin);
+    // columns 8 + h, 10 + h, ... of the unused rows to rows 8..15 of U
+    const unsigned left = ~__ballot_sync(FULL, used) & 0xffffu;
+    if (!used) {
+      cx<T>* d = U + (8 + __popc(left & ((1u << r) - 1))) * LDU + 8 + h;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d[2 * i] = R[i];
+      if (h == 0) d[8] = R[4];
+    }
+    __syncwarp();
+  }
+  const int h = lane >> 3, r = lane & 7;
+  R[0] = U[(8 + r) * LDU + 8 + h];
+  R[1] = U[(8 + r) * LDU + 12 + h];
+  R[2] = h == 0 ? U[(8 + r) * LDU + 16] : cx<T>(T(0));
+  __syncwarp();
+  used = false;
+  lu_stage<2, 8>(U, 8, lane, R, used, pmax, pmin);
+  lu_stage<1, 8>(U, 12, lane, R, used, pmax, pmin);
+}
+
+// Sums over each group of 8 lanes (g = lane & 7) of N values a lane, those of team_sum, to
+// out[0..N) in memory: the lanes halve the values among themselves three times, N - 1 or so
+// additions a lane where a butterfly per value takes 3 N.
+template <int N, typename T>
+__device__ __forceinline__ void halve(T* v, bool up, int off) {
+  constexpr int H = (N + 1) / 2;
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    const T hi = H + i < N ? v[H + i] : T(0);
+    const T keep = up ? hi : v[i], send = up ? v[i] : hi;
+    v[i] = keep + __shfl_xor_sync(FULL, send, off);
+  }
+}
+template <int N, typename T>
+__device__ __forceinline__ void team_sums(T* v, T* out, int g) {
+  constexpr int H = (N + 1) / 2, H2 = (H + 1) / 2, H3 = (H2 + 1) / 2;
+  halve<N>(v, g & 4, 4);
+  halve<H>(v, g & 2, 2);
+  halve<H2>(v, g & 1, 1);
+  const int end = (g & 4) ? N : H;  // this lane's values: first .. first + H3, within its halves
+  const int mid = (g & 4 ? H : 0) + (g & 2 ? H2 : 0), last = (g & 2) ? end : mid + H2;
+  const int first = mid + (g & 1 ? H3 : 0), stop = (g & 1) ? last : mid + H3;
+#pragma unroll
+  for (int i = 0; i < H3; ++i)
+    if (first + i < (stop < end ? stop : end)) out[first + i] = v[i];
 }
 
 // Back substitution, column by column; lane r holds the right-hand side of pivot row r.
@@ -303,7 +412,7 @@ __device__ __forceinline__ void back_substitute(const cx<double>* U, cx<double>*
   const bool im = lane >= 16;
   double rb = im ? U[r * LDU + 16].im : U[r * LDU + 16].re;
   const cx<double> ip = U[r * LDU + r];
-  const double pa = im ? ip.im : ip.re, pb = im ? ip.re : -ip.im;
+  const double pa = im ? ip.im : ip.re, pb = im ? ip.re : neg_if(ip.im, true);
 #pragma unroll 1
   for (int k = 15; k >= 0; --k) {
     const cx<double> u = U[r * LDU + k];
@@ -312,7 +421,7 @@ __device__ __forceinline__ void back_substitute(const cx<double>* U, cx<double>*
     const double m = fma(are, pa, __dmul_rn(aim, pb));
     const double xr = __shfl_sync(FULL, m, k), xi = __shfl_sync(FULL, m, 16 + k);
     if (lane == 0) X[k] = cx<double>(xr, xi);
-    if (r < k) rb = fma(im ? -u.im : u.im, im ? xr : xi, fma(-u.re, im ? xi : xr, rb));
+    if (r < k) rb = fma(neg_if(u.im, im), im ? xr : xi, fma(-u.re, im ? xi : xr, rb));
   }
 }
 
@@ -331,7 +440,7 @@ __device__ __forceinline__ cx<double> solve_u(const cx<double>* piv, const cx<do
 #pragma unroll 4
   for (int c = 0; c < 16; ++c) {
     const cx<double> p = piv[c * 8 + g], x = X[c];
-    xu = fma(im ? -p.im : p.im, im ? x.re : x.im, fma(-p.re, im ? x.im : x.re, xu));
+    xu = fma(neg_if(p.im, im), im ? x.re : x.im, fma(-p.re, im ? x.im : x.re, xu));
   }
   const double ot = __shfl_xor_sync(FULL, xu, 8);
   return (im ? cx<double>(ot, xu) : cx<double>(xu, ot)) * ipu;
@@ -377,7 +486,7 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
       f0 = S.M[17 * 8 + jj]; f1 = S.M[(18 + 17) * 8 + jj]; f2 = S.M[(36 + 17) * 8 + jj];
       hU = patch_dot<T, T>(S.u, S.Ye, NY, g, FULL) - cx<T>(T(1));
     }
-    r0[5] = -f0; r1[5] = -f1; r2[5] = -f2;
+    r0[5] = neg(f0); r1[5] = neg(f1); r2[5] = neg(f2);
     if (want_hnorm) {
       const T hsq = grp ? cnorm2(f0) + cnorm2(f1) + cnorm2(f2) : cnorm2(hU);
       out.hnorm = sqrt(team_sum(FULL, hsq));
@@ -394,9 +503,11 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
     const T s = T(1) / (q == 0 ? m0.value() : (q == 1 ? m1.value() : m2.value()));
     const T s0 = __shfl_sync(FULL, s, g), s1 = __shfl_sync(FULL, s, 8 + g), s2 = __shfl_sync(FULL, s, 16 + g);
 #pragma unroll
-    for (int i = 0; i < 6; ++i) { r0[i] = s0 * r0[i]; r1[i] = s1 * r1[i]; r2[i] = s2 * r2[i]; }
+    for (int i = 0; i < 5; ++i) { r0[i] = s0 * r0[i]; r1[i] = s1 * r1[i]; r2[i] = s2 * r2[i]; }
+    if (newton) { r0[5] = s0 * r0[5]; r1[5] = s1 * r1[5]; r2[5] = s2 * r2[5]; }
   }
-  // ---- eliminate U_j inside the group: partial pivoting among its three rows
+  // ---- eliminate U_j inside the group: partial pivoting among its three rows (a tangent's
+  //      group rows have the right-hand side zero throughout)
   const T a0 = cnorm2(r0[4]), a1 = cnorm2(r1[4]), a2 = cnorm2(r2[4]);
   const int p = (a0 >= a1 && a0 >= a2) ? 0 : (a1 >= a2 ? 1 : 2);
   const T ap = p == 0 ? a0 : (p == 1 ? a1 : a2);
@@ -408,12 +519,14 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
     const cx<T> la = (p == 0 ? r1[4] : r0[4]) * ipu;
     const cx<T> lb = (p == 2 ? r1[4] : r2[4]) * ipu;
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const int cc = i < 4 ? i : 5;
-      const cx<T> xa = p == 0 ? r1[cc] : r0[cc];
-      const cx<T> xb = p == 2 ? r1[cc] : r2[cc];
-      R0[i] = cfms(xa, la, piv[cc]);
-      R1[i] = cfms(xb, lb, piv[cc]);
+    for (int i = 0; i < 4; ++i) {
+      R0[i] = cfms(p == 0 ? r1[i] : r0[i], la, piv[i]);
+      R1[i] = cfms(p == 2 ? r1[i] : r2[i], lb, piv[i]);
+    }
+    R0[4] = R1[4] = zero;
+    if (newton) {
+      R0[4] = cfms(p == 0 ? r1[5] : r0[5], la, piv[5]);
+      R1[4] = cfms(p == 2 ? r1[5] : r2[5], lb, piv[5]);
     }
   }
   cx<T>* pivs = S.piv();
@@ -424,39 +537,53 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
   }
   // ---- the folding of every group's pivot row into the patch rows (lanes g = 7 repeat
   //      group 7's rows with weight zero and then hold the patch rows). A Newton step's
-  //      t-selector row has no entry to fold.
+  //      t-selector row has no entry to fold, a tangent's right-hand sides none either.
+  cx<T>* U = S.U();
   if (!grp) ipu = zero;
   {
+    T* sums = reinterpret_cast<T*>(U) + q * 16;  // the dense system's place, free until it is written
     const cx<T> mu = (su * S.u[14 + jj]) * ipu;
-    cx<T> Su[5], Sw[5];
+    T v[16];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) { Su[i] = mu * piv[i < 4 ? i : 5]; Sw[i] = zero; }
-#pragma unroll
-    for (int i = 0; i < 5; ++i) Su[i] = cx<T>(team_sum(FULL, Su[i].re), team_sum(FULL, Su[i].im));
-    if (!newton) {
+    for (int i = 0; i < 4; ++i) {
+      const cx<T> m = mu * piv[i];
+      v[2 * i] = m.re;
+      v[2 * i + 1] = m.im;
+    }
+    if (newton) {
+      const cx<T> m = mu * piv[5];
+      v[8] = m.re;
+      v[9] = m.im;
+      team_sums<10>(v, sums, g);
+    } else {
       const cx<T> mw = Wsrc[14 + jj] * ipu;
 #pragma unroll
-      for (int i = 0; i < 5; ++i) Sw[i] = mw * piv[i < 4 ? i : 5];
-#pragma unroll
-      for (int i = 0; i < 5; ++i) Sw[i] = cx<T>(team_sum(FULL, Sw[i].re), team_sum(FULL, Sw[i].im));
+      for (int i = 0; i < 4; ++i) {
+        const cx<T> m = mw * piv[i];
+        v[8 + 2 * i] = m.re;
+        v[9 + 2 * i] = m.im;
+      }
+      team_sums<16>(v, sums, g);
     }
+    __syncwarp();
     if (!grp) {
+      const cx<T>* Su = reinterpret_cast<const cx<T>*>(sums);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int c = q + 4 * i, st = gstate(c);
         R0[i] = su * S.u[st] - Su[i];
-        R1[i] = (newton ? (c == 15 ? cx<T>(T(1)) : zero) : Wsrc[st]) - Sw[i];
+        R1[i] = newton ? (c == 15 ? cx<T>(T(1)) : zero) : Wsrc[st] - Su[4 + i];
       }
-      R0[4] = (newton ? -mul_rn(su, hU) : zero) - Su[4];
-      R1[4] = (newton ? cx<T>(tgoal - S.Ye[22].re) : cx<T>(T(1))) - Sw[4];
+      R0[4] = newton ? -mul_rn(su, hU) - Su[4] : zero;
+      R1[4] = newton ? cx<T>(tgoal - S.Ye[22].re) : cx<T>(T(1));
     }
+    __syncwarp();
   }
   // ---- re-scale the 16 dense rows (max(|re|,|im|) = 1): eliminating U_j can shrink a
   //      group row by cancellation, and unequal rows would mislead both the pivot
   //      choice and the pivot-ratio condition estimate (with the re-scaling the ratio
   //      tracks the reference's 23 x 23 row-scaled elimination). Rows 2 g and 2 g + 1 to
   //      the dense system.
-  cx<T>* U = S.U();
   {
     MaxAbs<T> m0, m1;
 #pragma unroll
@@ -479,19 +606,7 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
   __syncwarp();
   // ---- dense 16 x 16 LU with partial pivoting across the lanes
   T pmax = T(0), pmin = T(3.0e38);
-  {
-    const int h = lane >> 4, r = lane & 15;
-    cx<T> R[9];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) R[i] = U[r * LDU + h + 2 * i];
-    R[8] = h == 0 ? U[r * LDU + 16] : zero;
-    __syncwarp();
-    bool used = false;
-    lu_stage<8>(U, 0, lane, R, used, pmax, pmin);
-    lu_stage<6>(U, 4, lane, R, used, pmax, pmin);
-    lu_stage<4>(U, 8, lane, R, used, pmax, pmin);
-    lu_stage<2>(U, 12, lane, R, used, pmax, pmin);
-  }
+  dense_lu(U, lane, pmax, pmin);
   __syncwarp();
   back_substitute(U, S.X, lane);
   __syncwarp();
@@ -520,7 +635,7 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
     const cx<T> xt = S.X[15];
     if (!tstep) {
       const T nr = sqrt((lane & 1) ? n2 : cnorm2(xt));
-      sc = cx<T>(xt.re, -xt.im) * (T(1) / (__shfl_sync(FULL, nr, 0) * __shfl_sync(FULL, nr, 1)));
+      sc = cx<T>(xt.re, neg_if(xt.im, true)) * (T(1) / (__shfl_sync(FULL, nr, 0) * __shfl_sync(FULL, nr, 1)));
     } else {
       sc = cinv(xt);
     }

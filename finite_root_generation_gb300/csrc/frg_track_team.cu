@@ -270,6 +270,18 @@ __device__ __forceinline__ void spread_queue(int64_t nqueue, int sms, int& block
   paths = (int)(p < warps ? p : warps);
 }
 
+// Quarter `quarter` of group g + 1's evaluation, in the arithmetic of C.
+template <typename C, typename T, typename P>
+__device__ __forceinline__ void eval_quarter(Smem<T, P>& E, int quarter, int g) {
+  auto& in = E.inputs();
+  switch (quarter) {
+    case 0: frg_eval_slice<0, C, T>(E.Ye, in.in, in.dq, g + 1, g, E.M); break;
+    case 1: frg_eval_slice<1, C, T>(E.Ye, in.in, in.dq, g + 1, g, E.M); break;
+    case 2: frg_eval_slice<2, C, T>(E.Ye, in.in, in.dq, g + 1, g, E.M); break;
+    default: frg_eval_slice<3, C, T>(E.Ye, in.in, in.dq, g + 1, g, E.M); break;
+  }
+}
+
 // Blocks of 4 warps in FP64 (two per SM, by registers and shared memory), of 4 to 16 in
 // the FP32 stage (by the queue's length, frg_team_grid). The warps work in parts of four:
 // part k evaluates its four paths together. All warps of a block step in time, and in the
@@ -487,17 +499,23 @@ team_kernel(TrackArgs a) {
     // ============== evaluation (the part's four warps: quarter `quarter` of every path's groups)
     if (__syncthreads_and(phase == PH_IDLE)) break;
     {
-      Smem<T, P>& E = paths[(warp & ~3) + (lane >> 3)];
+      Smem<T, P>* const part = paths + (warp & ~3);
       const int quarter = warp & 3;
-      if (E.active && g < 7) {
-        auto& in = E.inputs();
-        switch (quarter) {
-          case 0: frg_eval_slice<0, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
-          case 1: frg_eval_slice<1, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
-          case 2: frg_eval_slice<2, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
-          default: frg_eval_slice<3, T>(E.Ye, in.in, in.dq, jg, g, E.M); break;
+      Smem<T, P>& E = part[lane >> 3];
+      bool paired = false;
+      if constexpr (sizeof(T) == 8) {
+        // At most two paths left in the part: a pair of lanes per group, one per component
+        const unsigned act = (part[0].active != 0) | (part[1].active != 0) << 1 | (part[2].active != 0) << 2 |
+                             (part[3].active != 0) << 3;
+        paired = __popc(act) <= 2;
+        if (paired) {
+          const int p0 = act ? __ffs(act) - 1 : 0, p1 = act ? 31 - __clz(act) : 0;
+          Smem<T, P>& E2 = part[lane < 16 ? p0 : p1];
+          const int g2 = (lane >> 1) & 7, gg = g2 < 7 ? g2 : 6;
+          if (act) eval_quarter<PairCx>(E2, quarter, gg);
         }
       }
+      if (!paired && E.active && g < 7) eval_quarter<cx<T>>(E, quarter, g);
       if constexpr (LOWP) {
         // the corrector's refinement residual: F_j at the point YN with q(t) in the point
         // type (htpysupport.cu:37-48, :64-86), the right-hand side with which the FP32

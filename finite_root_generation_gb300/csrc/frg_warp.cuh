@@ -65,4 +65,55 @@ __device__ __forceinline__ cx<T> mul_rn(T s, cx<T> a) { return cx<T>(mul_rn(s, a
 template <typename T>
 __device__ __forceinline__ cx<T> axpy(T s, cx<T> a, cx<T> b) { return cx<T>(fma(s, a.re, b.re), fma(s, a.im, b.im)); }
 
+
+// -x when `neg`, on the sign bit: a negation that no arithmetic absorbs (a selected or
+// stored one) would be an FP64 instruction of its own
+__device__ __forceinline__ double neg_if(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+__device__ __forceinline__ float neg_if(float x, bool neg) { return neg ? -x : x; }
+
+// An FP64 complex value held by a pair of lanes (2 k, 2 k + 1): each lane computes one
+// component of every result (the even lane the real part) and the pair exchanges, so a
+// product takes 2 FP64 instructions and a sum 1 where a lane alone takes 4 and 2. The
+// operations are cx<double>'s. `re` and `ims` (the imaginary part on the odd lane, its
+// negative on the even one) serve a left factor, `own` and `oth` the rest.
+struct PairCx {
+  double re, ims, own, oth;
+  __device__ __forceinline__ static bool odd() { return threadIdx.x & 1; }
+  __device__ __forceinline__ PairCx() {}
+  __device__ __forceinline__ explicit PairCx(cx<double> v)
+      : re(v.re), ims(neg_if(v.im, !odd())), own(odd() ? v.im : v.re), oth(odd() ? v.re : v.im) {}
+  __device__ __forceinline__ explicit PairCx(double v) : PairCx(cx<double>(v)) {}
+  __device__ __forceinline__ static PairCx of(double own) {
+    PairCx r;
+    r.own = own;
+    r.oth = __shfl_xor_sync(FULL, own, 1);
+    r.re = odd() ? r.oth : own;
+    r.ims = neg_if(odd() ? own : r.oth, !odd());
+    return r;
+  }
+};
+__device__ __forceinline__ PairCx operator*(PairCx a, PairCx b) {
+  return PairCx::of(fma(a.re, b.own, __dmul_rn(a.ims, b.oth)));
+}
+__device__ __forceinline__ PairCx operator+(PairCx a, PairCx b) { return PairCx::of(a.own + b.own); }
+__device__ __forceinline__ PairCx operator-(PairCx a, PairCx b) { return PairCx::of(a.own - b.own); }
+__device__ __forceinline__ PairCx operator-(PairCx a) {
+  PairCx r;
+  r.re = -a.re; r.ims = -a.ims; r.own = -a.own; r.oth = -a.oth;
+  return r;
+}
+// a real multiple, absorbed by the sum it enters as cx<double>'s is (one fused multiply-add)
+struct PairScaled {
+  double s, own;
+};
+__device__ __forceinline__ PairScaled operator*(double s, PairCx a) { return {s, a.own}; }
+__device__ __forceinline__ PairScaled operator-(PairScaled a) { return {-a.s, a.own}; }
+__device__ __forceinline__ PairCx operator+(PairScaled a, PairCx b) { return PairCx::of(fma(a.s, a.own, b.own)); }
+__device__ __forceinline__ PairCx operator-(PairScaled a, PairCx b) { return PairCx::of(fma(a.s, a.own, -b.own)); }
+__device__ __forceinline__ PairCx operator+(PairCx b, PairScaled a) { return PairCx::of(fma(a.s, a.own, b.own)); }
+
+__device__ __forceinline__ void cx_put(cx<double>* p, PairCx v) { reinterpret_cast<double*>(p)[PairCx::odd()] = v.own; }
+
 }  // namespace frg

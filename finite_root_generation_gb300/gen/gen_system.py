@@ -244,10 +244,12 @@ def slice_lines(repl, wanted, found, loads, pr):
         elif x not in need:
             need.add(x)
             stack += [y.name for y in defs[x].free_symbols]
-    out = [f"    const cx<T> {x} = {loads(x, found.get(x))};" for x in sorted(used)]
-    out += [f"    const cx<T> {s_} = {pr.expr(e)};" for s_, e in repl if s_.name in need]
+    out = [f"    const CX {x}({loads(x, found.get(x))});" for x in sorted(used)]
+    # a real multiple stays unevaluated where CX has a type for it, to round as the fused form
+    scaled = {s_ for s_, e in repl if abs(e.as_coeff_Mul()[0]) != 1 and e.as_coeff_Mul()[0].is_Number}
+    out += [f"    const {'auto' if s_ in scaled else 'CX'} {s_} = {pr.expr(e)};" for s_, e in repl if s_.name in need]
     out += ["    " + st.format(pr.expr(e)) for e, st in wanted]
-    return out
+    return [ln.replace("cx<T>(T(", "CX(T(") for ln in out]
 
 
 INDEP = [h[0] for h in HOISTED if not h[1]]
@@ -301,18 +303,20 @@ def emit_slices(lines, names, repl, reduced, frepl, fred, pr):
               f"  cx<T> sa[2][{len(INDEP)}], sb[2][{len(PERJ)}][8];", "};", "",
               "// One quarter of group j's evaluation (frg_group_eval's operations in its order): rows of",
               "// the group into M[(row * 18 + column) * 8 + g], columns 0..13 links, 14 Z0, 15 t, 16 U_j, 17 F.",
-              "template <int SLICE, typename T>",
+              "// CX: cx<T>, or a type with its operators whose values several lanes share.",
+              "template <int SLICE, typename CX, typename T>",
               "__device__ __forceinline__ void frg_eval_slice(const cx<T>* Y, const FrgEvalIn<T>& in, const cx<T>* dq, int j,",
               "                                               int g, cx<T>* M) {"]
     for k, outs in enumerate(EVAL_SLICES):
         lines.append(f"  if constexpr (SLICE == {k}) {{")
-        wanted = [(by[n][0], f"M[{(by[n][1] * 18 + by[n][2]) * 8} + g] = {{}};") for n in outs]
+        wanted = [(by[n][0], f"cx_put(M + {(by[n][1] * 18 + by[n][2]) * 8} + g, {{}});") for n in outs]
         lines += slice_lines(repl, wanted, found, load_of, pr)
         lines.append("  }")
     lines += ["}", "",
               "// One of the three equations at the point Y (frg_group_f's operations in its order).",
               "template <int SLICE, typename T>",
-              "__device__ __forceinline__ cx<T> frg_residual_slice(const cx<T>* Y, const FrgEvalIn<T>& in, int j) {"]
+              "__device__ __forceinline__ cx<T> frg_residual_slice(const cx<T>* Y, const FrgEvalIn<T>& in, int j) {",
+              "  typedef cx<T> CX;"]
     for k in range(3):
         lines.append(f"  if constexpr (SLICE == {k}) {{")
         lines += slice_lines(frepl, [(fred[k], "return {};")], ffound, load_of, pr)
