@@ -57,11 +57,11 @@ struct Slot {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   DevBuf gamma, gamma_lo, gamma_df, fpm_lo, fpm_df, task_start, queue, counters, starts;
-  DevBuf handoff, handoff_list, lo_lists, tail;
+  DevBuf handoff, handoff_list, lo_lists, tail, finals;
   DevBuf roots, codes, resid;  // staging of host outputs (frg_track_rounds)
   void release() {
     for (DevBuf* b : {&gamma, &gamma_lo, &gamma_df, &fpm_lo, &fpm_df, &task_start, &queue, &counters, &starts,
-                      &handoff, &handoff_list, &lo_lists, &tail, &roots, &codes, &resid})
+                      &handoff, &handoff_list, &lo_lists, &tail, &finals, &roots, &codes, &resid})
       b->release();
     if (own_stream && stream) cudaStreamDestroy(stream);
     stream = nullptr;
@@ -389,6 +389,14 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     cudaError_t e = frg_launch_starts(a, (cx<double>*)sl.starts.p, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "start kernel launch");
   }
+  if (ctx->cfg.system != 0) {
+    FRG_CUDA(ctx, sl.starts.ensure(sizeof(cx<double>) * (size_t)(nv + np) * (size_t)N));
+    FRG_CUDA(ctx, sl.finals.ensure(sizeof(cx<double>) * (size_t)(nv + 2) * (size_t)N));
+    a.starts = (const cx<double>*)sl.starts.p;
+    a.finals = (cx<double>*)sl.finals.p;
+    cudaError_t e = frg_launch_plugin_starts(a, (cx<double>*)sl.starts.p, st);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "start kernel launch");
+  }
   // persistent grids: SMs x resident blocks, capped by the work
   const bool plugin = ctx->cfg.system != 0;
   int plugin_bps[3] = {0, 0, 0}, warp_bps[3] = {0, 0, 0};  // a plug-in system's kernels have their own occupancy
@@ -414,7 +422,8 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     if (by_warp) return frg_launch_warp(mode, a, (int)std::min<int64_t>(wcap, (N + 3) / 4), st);
     if (!plugin) return frg_launch_track(mode, a, grid, st);
     frg::TrackArgs b = a;
-    b.tail_cap = (int64_t)grid * (FRG_TRACK_THREADS / 32) * frg_tail_lanes(mode == 1);
+    b.tail_cap = (int64_t)grid * (FRG_TRACK_THREADS / 32) * frg_tail_lanes(mode == 1, nv);
+    if (b.tail_cap == 0) return frg_launch_track(mode, a, grid, st);
     cudaError_t e = sl.tail.ensure(sizeof(frg::Handoff) * (size_t)b.tail_cap);
     if (e != cudaSuccess) return e;
     b.tail = (frg::Handoff*)sl.tail.p;
@@ -426,6 +435,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   };
   if (!mixed) {
     cudaError_t e = launch(0);
+    if (e == cudaSuccess && plugin) e = frg_launch_plugin_finish(a, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "track kernel launch (FP64)");
     return FRG_OK;
   }
@@ -461,6 +471,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     a.back_list = (team && r + 1 < rounds) ? lo + (size_t)(r & 1) * N : nullptr;
     a.back_count = q + 3 + (r & 1);
     e = launch(2);
+    if (e == cudaSuccess && plugin) e = frg_launch_plugin_finish(a, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "track kernel launch (FP64 stage)");
     FRG_CUDA(ctx, cudaEventRecord(evs[2 * r + 2], st));
   }

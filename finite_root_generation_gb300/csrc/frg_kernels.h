@@ -62,7 +62,9 @@ struct TrackArgs {
   double* resid;                // npaths, optional
   int32_t* work;                // npaths x 3 (ivp solves, newton iterations, steps), optional
   unsigned long long* counters; // FRG_NCOUNTERS counters (layout above)
-  const cx<double>* starts;     // npaths x FRG_START_STRIDE start values (null: generated inline)
+  const cx<double>* starts;     // npaths x FRG_START_STRIDE start values (null: generated inline); plug-ins:
+                                // npaths x (unknowns + parameters)
+  cx<double>* finals;           // plug-ins: the paths' endpoints, npaths x (unknowns + 2)
   Handoff* handoff;             // npaths slots (mixed precision)
   int64_t* handoff_list;        // ids of paths handed to the FP64 kernel
   unsigned long long* handoff_count;
@@ -120,12 +122,18 @@ constexpr int FRG_WARP_PATHS = 8;
 
 // A warp of a thread-per-path launch gives its paths up to a warp-per-path launch when the
 // queue is empty and at most this many of its lanes still track one: a warp's step costs
-// the same with few lanes as with 32, four to seven times a warp_kernel step in FP64, less
-// in FP32 (120,000 conic2 paths, FP32 stage: 4 lanes 12.6 ms, 2 lanes 11.7, never 11.4; 8,192
-// burmester5 paths: 35, 37, 58 ms).
-__host__ __device__ constexpr int frg_tail_lanes(bool fp32) { return fp32 ? 2 : 4; }
+// the same with few lanes as with 32, four to seven times a warp_kernel step in FP64. In
+// FP32 a small system's step is too short for the second launch to pay (FP32 stage of
+// 120,000 conic2 paths: 4 lanes 12.6 ms, 2 lanes 11.7, never 11.4; of 8,192 burmester5
+// paths 35, 37, 58 ms).
+__host__ __device__ constexpr int frg_tail_lanes(bool fp32, int nv) { return fp32 && nv < 4 ? 0 : 4; }
 
 #define FRG_NQUEUE 16  // queue heads and counts of a slot
+
+// A plug-in call's start values (before its tracking launches) and its paths' roots, codes
+// and residuals from `finals` and the codes tracking ended with (after them).
+cudaError_t frg_launch_plugin_starts(const frg::TrackArgs& args, cx<double>* starts, cudaStream_t stream);
+cudaError_t frg_launch_plugin_finish(const frg::TrackArgs& args, cudaStream_t stream);
 
 // Warp-per-path kernel of the plug-in systems (mode and arguments as frg_launch_track's),
 // four paths per block.

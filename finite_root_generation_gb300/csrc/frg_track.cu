@@ -187,10 +187,19 @@ track_kernel(TrackArgs a) {
         // Start system (frg.cu:54): the stream of path id; TrackPath receives the same
         // fresh state (frg.cu:57, by value), so its draws restart at index 0.
         P.rng.seed = a.seed; P.rng.stream = (uint64_t)(id + c.path_offset); P.rng.index = 0;
-        cd spt[NV_], spm[NP_];
-        S::start(P.rng, c.start_dist, c.start_range, spt, spm);
+        cd spt[NV_];
+        if constexpr (S::ID == 0) {
+          cd spm[NP_];
+          S::start(P.rng, c.start_dist, c.start_range, spt, spm);
 #pragma unroll 1
-        for (int e = 0; e < NP_; ++e) P.spm[e] = cx<T>(spm[e]);
+          for (int e = 0; e < NP_; ++e) P.spm[e] = cx<T>(spm[e]);
+        } else {
+          const cd* st = a.starts + (size_t)id * (NV_ + NP_);
+#pragma unroll 1
+          for (int e = 0; e < NV_; ++e) spt[e] = st[e];
+#pragma unroll 1
+          for (int e = 0; e < NP_; ++e) P.spm[e] = cx<T>(st[NV_ + e]);
+        }
         P.code = 0; P.stage = 0; P.attempt = 0; P.it = 0; P.residual = T(100); P.err = T(0); P.scale = T(0);
         if (MODE == MODE_RESUME) {
           const Handoff& h = a.handoff[id];
@@ -220,7 +229,8 @@ track_kernel(TrackArgs a) {
     // FP64: 267 -> 250 ms, of which the longest paths' tail is the larger part).
     unsigned live = __ballot_sync(0xffffffffu, P.phase != PH_IDLE);
     if (!live) break;
-    if (a.tail_cap > 0 && __any_sync(0xffffffffu, dry) && __popc(live) <= frg_tail_lanes(LO)) {
+    constexpr int kTail = frg_tail_lanes(LO, NV_);
+    if (kTail > 0 && a.tail_cap > 0 && __any_sync(0xffffffffu, dry) && __popc(live) <= kTail) {
       // The queue is empty and this warp's step serves few paths: they go on, from their
       // next step's start, in a warp_kernel launch, where a step is that much shorter.
       if (P.phase == PH_RK && P.stage == 0) {
@@ -429,10 +439,17 @@ track_kernel(TrackArgs a) {
 
     // ---------------------------------------------------------------- finish
     if (finished) {
-      cd Yf[NY_];
+      if constexpr (S::ID == 0) {
+        cd Yf[NY_];
 #pragma unroll 1
-      for (int e = 0; e < NY_; ++e) Yf[e] = cd(final_src[e]);
-      finish_path<S>(a, P.id, P.task, P.code, Yf, a.fpm + (size_t)P.task * NP_);
+        for (int e = 0; e < NY_; ++e) Yf[e] = cd(final_src[e]);
+        finish_path<S>(a, P.id, P.task, P.code, Yf, a.fpm + (size_t)P.task * NP_);
+      } else {  // finish_kernel does the rest
+        cd* o = a.finals + (size_t)P.id * NY_;
+#pragma unroll 1
+        for (int e = 0; e < NY_; ++e) o[e] = cd(final_src[e]);
+        a.codes[P.id] = P.code;
+      }
       if (a.work) {
         a.work[(size_t)P.id * 3 + 0] = P.n_ivp;
         a.work[(size_t)P.id * 3 + 1] = P.n_newton;
@@ -471,7 +488,19 @@ __device__ void finish_path(const TrackArgs& a, int64_t id, int task, int code, 
 #pragma unroll 1
   for (int e = 0; e < NY_; ++e) ud[e] = cd(0.0);
   ud[NV_] = cd(1.0);
-  switch_patch<double, NY_>(ud, Yf, Yf);
+  if constexpr (S::ID == 0) {
+    switch_patch<double, NY_>(ud, Yf, Yf);
+  } else {
+    // SwitchPatch with its division spelled out, so that the scale rounds the same in
+    // every kernel this is compiled into
+    cd den(0.0);
+#pragma unroll 1
+    for (int e = 0; e < NZ_; ++e) den = cfma(ud[e], Yf[e], den);
+    const double r = 1.0 / fma(den.re, den.re, __dmul_rn(den.im, den.im));
+    const cd sc = (cd(1.0) - ud[NY_ - 1] * Yf[NY_ - 1]) * cd(den.re * r, -den.im * r);
+#pragma unroll 1
+    for (int e = 0; e < NZ_; ++e) Yf[e] = sc * Yf[e];
+  }
   cd root[NV_];
   S::canonical(Yf, fpm, root);
 #pragma unroll 1
@@ -499,6 +528,40 @@ __device__ void finish_path(const TrackArgs& a, int64_t id, int task, int code, 
     }
     a.resid[id] = r;
   }
+}
+
+// A plug-in launch's start values and its paths' finishes, a thread per path: inside the
+// tracking kernels a path's start (some 2,000 FP64 instructions of draws) and finish ran
+// with one lane of 32 active, as much work for conic2 as the tracking itself (262,144 paths
+// FP64: 175 -> 138 ms, mixed 59 -> 32 ms).
+template <class S>
+__global__ void __launch_bounds__(FRG_TRACK_THREADS) plugin_start_kernel(TrackArgs a, cd* starts) {
+  const int64_t id = (int64_t)blockIdx.x * FRG_TRACK_THREADS + threadIdx.x;
+  if (id >= a.npaths) return;
+  Rng rng;
+  rng.seed = a.seed; rng.stream = (uint64_t)(id + a.cfg.path_offset); rng.index = 0;
+  cd z[S::NV], q[S::NP];
+  S::start(rng, a.cfg.start_dist, a.cfg.start_range, z, q);
+  cd* st = starts + (size_t)id * (S::NV + S::NP);
+#pragma unroll 1
+  for (int e = 0; e < S::NV; ++e) st[e] = z[e];
+#pragma unroll 1
+  for (int e = 0; e < S::NP; ++e) st[S::NV + e] = q[e];
+}
+
+template <class S>
+__global__ void __launch_bounds__(FRG_TRACK_THREADS) plugin_finish_kernel(TrackArgs a) {
+  const int64_t id = (int64_t)blockIdx.x * FRG_TRACK_THREADS + threadIdx.x;
+  if (id >= a.npaths) return;
+  int lo = 0, hi = a.ntasks - 1;  // task of this path
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (a.task_start[mid] <= id) lo = mid; else hi = mid - 1;
+  }
+  cd Yf[S::NV + 2];
+#pragma unroll 1
+  for (int e = 0; e < S::NV + 2; ++e) Yf[e] = a.finals[(size_t)id * (S::NV + 2) + e];
+  finish_path<S>(a, id, lo, a.codes[id], Yf, a.fpm + (size_t)lo * S::NP);
 }
 
 }  // namespace frg
@@ -558,6 +621,39 @@ cudaError_t warp_occ(int* blocks_per_sm) {
                                                        32 * frg::WARP_PATHS, 0);
 }
 }  // namespace
+
+namespace {
+template <class S>
+cudaError_t launch_starts(const frg::TrackArgs& args, cx<double>* starts, cudaStream_t stream) {
+  const int64_t blocks = (args.npaths + FRG_TRACK_THREADS - 1) / FRG_TRACK_THREADS;
+  frg::plugin_start_kernel<S><<<(unsigned)blocks, FRG_TRACK_THREADS, 0, stream>>>(args, starts);
+  return cudaGetLastError();
+}
+template <class S>
+cudaError_t launch_finish(const frg::TrackArgs& args, cudaStream_t stream) {
+  const int64_t blocks = (args.npaths + FRG_TRACK_THREADS - 1) / FRG_TRACK_THREADS;
+  frg::plugin_finish_kernel<S><<<(unsigned)blocks, FRG_TRACK_THREADS, 0, stream>>>(args);
+  return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t frg_launch_plugin_starts(const frg::TrackArgs& args, cx<double>* starts, cudaStream_t stream) {
+  switch (args.cfg.system) {
+#define FRG_PLUGIN_STARTS(id, name, S) case id: return launch_starts<S>(args, starts, stream);
+    FRG_PLUGIN_LIST(FRG_PLUGIN_STARTS)
+#undef FRG_PLUGIN_STARTS
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t frg_launch_plugin_finish(const frg::TrackArgs& args, cudaStream_t stream) {
+  switch (args.cfg.system) {
+#define FRG_PLUGIN_FINISH(id, name, S) case id: return launch_finish<S>(args, stream);
+    FRG_PLUGIN_LIST(FRG_PLUGIN_FINISH)
+#undef FRG_PLUGIN_FINISH
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 cudaError_t frg_launch_warp(int mode, const frg::TrackArgs& args, int grid, cudaStream_t stream) {
   switch (args.cfg.system * 4 + mode) {

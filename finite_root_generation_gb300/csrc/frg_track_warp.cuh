@@ -48,6 +48,17 @@ struct WarpStep {
   T hnorm;  // |H| (corrector, when asked for)
 };
 
+// One component (im: the imaginary one) of a b and of s + a b, the operations of the complex
+// product and cfma; the operands are selected, so that both kinds of lane share them
+template <typename T>
+__device__ __forceinline__ T mul_component(cx<T> a, cx<T> b, bool im) {
+  return fma(a.re, im ? b.im : b.re, mul_rn(neg_if(a.im, !im), im ? b.re : b.im));
+}
+template <typename T>
+__device__ __forceinline__ T fma_component(cx<T> a, cx<T> b, T s, bool im) {
+  return fma(neg_if(a.im, !im), im ? b.re : b.im, fma(a.re, im ? b.im : b.re, s));
+}
+
 // sum_{i < n} |v_i|^2 in index order from the magnitudes in cn
 template <typename T>
 __device__ __forceinline__ T sum_in_order(const T* cn, int n) {
@@ -95,10 +106,10 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
     const cx<T> a = W.reg[(w >> 10) & 1023], b = W.reg[(w >> 20) & 1023];
     T r;
     if (w >> 31) {
-      r = im ? fma(a.re, b.im, mul_rn(a.im, b.re)) : fma(a.re, b.re, mul_rn(-a.im, b.im));
+      r = mul_component(a, b, im);
     } else {
       const T x = im ? a.im : a.re, y = im ? b.im : b.re;
-      r = x + ((w >> 30) & 1 ? -y : y);
+      r = x + neg_if(y, (w >> 30) & 1);
     }
     reinterpret_cast<T*>(&W.reg[w & 1023])[im] = r;
     __syncwarp();
@@ -108,7 +119,7 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
   for (int o = lane; o < NV * NY; o += 32) {
     const unsigned w = outs[o];
     const cx<T> v = W.reg[w & 1023];
-    W.M[(o / NY) * LD + o % NY] = (w >> 10) ? -v : v;
+    W.M[(o / NY) * LD + o % NY] = cx<T>(neg_if(v.re, w >> 10), neg_if(v.im, w >> 10));
   }
   if (lane < NY) {
     W.M[NV * LD + lane] = W.u[lane];
@@ -119,14 +130,14 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
     if (lane < NV) {
       const unsigned w = outs[NV * NY + lane];
       const cx<T> v = W.reg[w & 1023];
-      W.M[lane * LD + NY] = (w >> 10) ? -v : v;
+      W.M[lane * LD + NY] = cx<T>(neg_if(v.re, w >> 10), neg_if(v.im, w >> 10));
     }
     // u . Y - 1, one lane per component
     T d = T(0);
 #pragma unroll 8
     for (int e = 0; e < NY; ++e) {
       const cx<T> b = W.u[e], y = e < NZ ? W.reg[e] : cx<T>(W.t);
-      d = im ? fma(b.im, y.re, fma(b.re, y.im, d)) : fma(-b.im, y.im, fma(b.re, y.re, d));
+      d = fma_component(b, y, d, im);
     }
     d -= im ? T(0) : T(1);
     if (lane < 2) reinterpret_cast<T*>(&W.M[NV * LD + NY])[im] = d;
@@ -150,7 +161,7 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
     if (r < NZ)
       for (int c = cl; c < (newton ? NY + 1 : NY); c += CL) {
         const cx<T> v = s * W.M[r * LD + c];
-        W.M[r * LD + c] = c == NY ? -v : v;
+        W.M[r * LD + c] = cx<T>(neg_if(v.re, c == NY), neg_if(v.im, c == NY));
       }
   }
   __syncwarp();
@@ -229,11 +240,11 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
 #pragma unroll 2
     for (int c = i + 1; c < NY; ++c) {
       const cx<T> b = m[c], xc = W.x[c];
-      sum = im ? fma(b.im, xc.re, fma(b.re, xc.im, sum)) : fma(-b.im, xc.im, fma(b.re, xc.re, sum));
+      sum = fma_component(b, xc, sum, im);
     }
     const T d = (im ? m[NY].im : m[NY].re) - sum, o = __shfl_xor_sync(FULL, d, 1);
     const cx<T> ip = W.ip[i], v = im ? cx<T>(o, d) : cx<T>(d, o);
-    const T xi = im ? fma(ip.re, v.im, mul_rn(ip.im, v.re)) : fma(ip.re, v.re, mul_rn(-ip.im, v.im));
+    const T xi = mul_component(ip, v, im);
     if (lane < 2) reinterpret_cast<T*>(&W.x[i])[im] = xi;
     __syncwarp();
   }
@@ -249,7 +260,7 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
     cx<T> sc;
     if (!tstep) {
       const T nr = sqrt((lane & 1) ? n2 : cnorm2(xt));
-      sc = cx<T>(xt.re, -xt.im) * (T(1) / (__shfl_sync(FULL, nr, 0) * __shfl_sync(FULL, nr, 1)));
+      sc = cx<T>(xt.re, neg_if(xt.im, true)) * (T(1) / (__shfl_sync(FULL, nr, 0) * __shfl_sync(FULL, nr, 1)));
     } else {
       sc = cinv(xt);
     }
@@ -311,19 +322,10 @@ __global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
     }
     const uint64_t stream = (uint64_t)(id + c.path_offset);
     const cx<T> gamma = task_gamma<T>(a, task);
-    if (lane == 0) {
-      Rng rng;
-      rng.seed = a.seed; rng.stream = stream; rng.index = 0;
-      cd spt[NV_], spm[NP_];
-      S::start(rng, c.start_dist, c.start_range, spt, spm);
-#pragma unroll 1
-      for (int e = 0; e < NP_; ++e) W.sp[e] = cx<T>(spm[e]);
-      if (!resumed) {
-#pragma unroll 1
-        for (int e = 0; e < NV_; ++e) W.Yc[e] = cx<T>(spt[e]);
-        W.Yc[NV_] = cx<T>(T(1));
-        W.Yc[NV_ + 1] = cx<T>(T(0));
-      }
+    {
+      const cd* st = a.starts + (size_t)id * (NV_ + NP_);
+      for (int i = lane; i < NP_; i += 32) W.sp[i] = cx<T>(st[NV_ + i]);
+      if (!resumed && el) W.Yc[lane] = lane < NV_ ? cx<T>(st[lane]) : cx<T>(T(lane == NV_ ? 1 : 0));
     }
     const cx<T>* fpmT = TaskFpm<T, NP_>::get(a, task);
     for (int i = lane; i < NP_; i += 32) W.fp[i] = fpmT[i];
@@ -515,11 +517,9 @@ __global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
         break;
       }
       if (finished) {
+        if (el) a.finals[(size_t)id * NY_ + lane] = cd(final_src[lane]);  // finish_kernel does the rest
         if (lane == 0) {
-          cd Yf[NY_];
-#pragma unroll 1
-          for (int e = 0; e < NY_; ++e) Yf[e] = cd(final_src[e]);
-          finish_path<S>(a, id, task, code, Yf, a.fpm + (size_t)task * NP_);
+          a.codes[id] = code;
           if (a.work) {
             a.work[(size_t)id * 3 + 0] = n_ivp;
             a.work[(size_t)id * 3 + 1] = n_newton;
