@@ -22,22 +22,26 @@ constexpr int LDM = 24; // leading dimension of the 23x23 system (+ right-hand s
 typedef cx<double> cd;
 
 // Dormand-Prince 6(5) tableau (rungekutta.cu:40-122): stage weights (:40-95), error
-// weights (LTE, :99-105) and 6th-order solution weights (:115-122).
-static __constant__ double c_dpA[8][7] = {
-    {0, 0, 0, 0, 0, 0, 0},
-    {1. / 10., 0, 0, 0, 0, 0, 0},
-    {-2. / 81., 20. / 81., 0, 0, 0, 0, 0},
-    {615. / 1372., -270. / 343., 1053. / 1372., 0, 0, 0, 0},
-    {3243. / 5500., -54. / 55., 50949. / 71500., 4998. / 17875., 0, 0, 0},
-    {-26492. / 37125., 72. / 55., 2808. / 23375., -24206. / 37125., 338. / 459., 0, 0},
-    {5561. / 2376., -35. / 11., -24117. / 31603., 899983. / 200772., -5225. / 1836., 3925. / 4056., 0},
-    {465467. / 266112., -2945. / 1232., -5610201. / 14158144., 10513573. / 3212352., -424325. / 205632.,
-     376225. / 454272., 0}};
-static __constant__ double c_dpE[8] = {-13. / 2400., 0., 19683. / 618800., -2401. / 31200., 65. / 816.,
-                                -15. / 416., -521. / 5600., 1. / 10.};
-static __constant__ double c_dpB[8] = {61. / 864., 0., 98415. / 321776., 16807. / 146016., 1375. / 7344.,
-                                1375. / 5408., -37. / 1120., 1. / 10.};
-
+// weights (LTE, :99-105) and 6th-order solution weights (:115-122), in FP64 and rounded to
+// FP32 (converting a double would cost the FP32 stage an FP64 instruction).
+#define FRG_DP_TABLEAU(T, A, E, B)                                                                               \
+  static __constant__ T A[8][7] = {                                                                              \
+      {0, 0, 0, 0, 0, 0, 0},                                                                                     \
+      {T(1. / 10.), 0, 0, 0, 0, 0, 0},                                                                           \
+      {T(-2. / 81.), T(20. / 81.), 0, 0, 0, 0, 0},                                                               \
+      {T(615. / 1372.), T(-270. / 343.), T(1053. / 1372.), 0, 0, 0, 0},                                          \
+      {T(3243. / 5500.), T(-54. / 55.), T(50949. / 71500.), T(4998. / 17875.), 0, 0, 0},                         \
+      {T(-26492. / 37125.), T(72. / 55.), T(2808. / 23375.), T(-24206. / 37125.), T(338. / 459.), 0, 0},         \
+      {T(5561. / 2376.), T(-35. / 11.), T(-24117. / 31603.), T(899983. / 200772.), T(-5225. / 1836.),            \
+       T(3925. / 4056.), 0},                                                                                     \
+      {T(465467. / 266112.), T(-2945. / 1232.), T(-5610201. / 14158144.), T(10513573. / 3212352.),               \
+       T(-424325. / 205632.), T(376225. / 454272.), 0}};                                                         \
+  static __constant__ T E[8] = {T(-13. / 2400.), 0, T(19683. / 618800.), T(-2401. / 31200.), T(65. / 816.),      \
+                                T(-15. / 416.), T(-521. / 5600.), T(1. / 10.)};                                  \
+  static __constant__ T B[8] = {T(61. / 864.), 0, T(98415. / 321776.), T(16807. / 146016.), T(1375. / 7344.),    \
+                                T(1375. / 5408.), T(-37. / 1120.), T(1. / 10.)}
+FRG_DP_TABLEAU(double, c_dpA, c_dpE, c_dpB);
+FRG_DP_TABLEAU(float, c_dpA32, c_dpE32, c_dpB32);
 
 // ---------------------------------------------------------------------------
 // Random draws (the reference's curand_uniform_double, replaced by Philox).

@@ -115,10 +115,10 @@ inline TeamGrid frg_team_grid(int sms, int bps, int64_t n, bool lo) {
 
 // A plug-in launch of at most this many paths per SM sub-partition tracks a path per warp,
 // a larger one a path per thread. FP64, GB300 (152 SMs), warp / thread: conic2 2,432 paths
-// 10.0 / 15.1 ms, 4,864 20.3 / 22.0, 9,728 32.1 / 30.2, 40,000 86 / 58; burmester5 4,864
-// 67 / 107, 19,456 587 / 555. FP32 stage and resume: conic2 4,864 4.4 / 4.9, 9,728 8.0 / 5.9;
-// burmester5 9,728 487 / 506.
-constexpr int FRG_WARP_PATHS = 8;
+// 8.5 / 14.1 ms, 9,728 26.7 / 28.1, 19,456 56.9 / 49.2, 40,000 72 / 52; burmester5 4,864
+// 57 / 99, 19,456 486 / 484. Mixed: conic2 9,728 4.2 / 5.0, 19,456 7.4 / 6.1; burmester5
+// 9,728 404 / 433.
+constexpr int FRG_WARP_PATHS = 16;
 
 // A warp of a thread-per-path launch gives its paths up to a warp-per-path launch when the
 // queue is empty and at most this many of its lanes still track one: a warp's step costs

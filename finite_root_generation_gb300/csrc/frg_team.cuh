@@ -247,12 +247,12 @@ __device__ __forceinline__ T patch_scale(const cx<T>* u, int lane) {
   return T(1) / m.value();
 }
 
-// Row with the largest v (ties: the lowest), v >= 0 or -1 for used rows; lanes h RP + r
-// hold row r's value for every h. Infinite and NaN candidates take the comparisons one by
-// one, as lane 0 sees them.
+// Pivot search: the row with the largest v (ties: the lowest). Row r's value is on lane
+// base + r, v >= 0, or -1 for used rows; the other lanes hold -1. Infinite and NaN candidates take the
+// comparisons one by one, as lane 0 sees them.
 template <int RP, typename T>
-__device__ __noinline__ int pivot_row_nonfinite(T v, int r) {
-  const T v0 = __shfl_sync(FULL, v, r & ~1), v1 = __shfl_sync(FULL, v, r | 1);
+__device__ __noinline__ int pivot_row_nonfinite(T v, int base, int r) {
+  const T v0 = __shfl_sync(FULL, v, base + (r & ~1)), v1 = __shfl_sync(FULL, v, base + (r | 1));
   T bv = v0 >= v1 ? v0 : v1;
   int bk = (r & ~1) + (v0 >= v1 ? 0 : 1);
   for (int off = RP / 2; off >= 2; off >>= 1) {
@@ -262,25 +262,36 @@ __device__ __noinline__ int pivot_row_nonfinite(T v, int r) {
   }
   return __shfl_sync(FULL, bk, 0);
 }
+// The pivot's lane as a bit (the lowest of equal ones).
 template <int RP>
-__device__ __forceinline__ int pivot_row(float v, int r) {
+__device__ __forceinline__ unsigned pivot_lane(float v, int base, int r) {
   const int key = __float_as_int(v);
   const int m = __reduce_max_sync(FULL, key);
-  if (m >= 0x7f800000) return pivot_row_nonfinite<RP>(v, r);
-  return __ffs(__ballot_sync(FULL, key == m)) - 1;
+  if (m >= 0x7f800000) return 1u << (base + pivot_row_nonfinite<RP>(v, base, r));
+  const unsigned c = __ballot_sync(FULL, key == m);
+  return c & (0u - c);
 }
 template <int RP>
-__device__ __forceinline__ int pivot_row(double v, int r) {
+__device__ __forceinline__ unsigned pivot_lane(double v, int base, int r) {
   const int hi = __double2hiint(v);
   const unsigned lo = (unsigned)__double2loint(v);
   const int m = __reduce_max_sync(FULL, hi);
-  if (m >= 0x7ff00000) return pivot_row_nonfinite<RP>(v, r);
-  unsigned cand = __ballot_sync(FULL, hi == m);
-  if (__popc(cand) > 32 / RP) {
+  if (m >= 0x7ff00000) return 1u << (base + pivot_row_nonfinite<RP>(v, base, r));
+  unsigned c = __ballot_sync(FULL, hi == m);
+  if (c & (c - 1)) {
     const unsigned ml = __reduce_max_sync(FULL, hi == m ? lo : 0u);
-    cand = __ballot_sync(FULL, hi == m && lo == ml);
+    c = __ballot_sync(FULL, hi == m && lo == ml);
   }
-  return __ffs(cand) - 1;
+  return c & (0u - c);
+}
+
+// 1 / b by Smith's form with the larger part selected instead of branched on (cinv's
+// operations)
+__device__ __forceinline__ cx<float> cinv_select(cx<float> b) {
+  const bool big = tabs(b.re) >= tabs(b.im);
+  const float p = big ? b.re : b.im, q = big ? b.im : b.re;
+  const float r = q / p, id = 1.0f / fmaf(q, r, p), o = __fmul_rn(r, id);
+  return cx<float>(big ? id : o, big ? -o : -id);
 }
 
 // a * b where lanes that differ in `bit` hold the same operands: in FP64 each computes one
@@ -297,35 +308,51 @@ __device__ __forceinline__ cx<double> mul_split(cx<double> a, cx<double> b, int 
 // RP h + r holds row r's remaining columns c = h mod 32 / RP (the right-hand side is column
 // 16) from index 0; a step drops the pivot column, so the lanes that held it move their
 // window up one. The pivot row goes to U and every lane reads it back from there; U[k][k]
-// keeps the pivot's reciprocal.
+// keeps the pivot's reciprocal; pn and pv (16 entries) pass the pivot and its norm on. In
+// FP32 the steps are chains of latencies (search, reciprocal, memory), in FP64 of the
+// FP64 instructions: 9 for the reciprocal and factor, 4 per column.
 template <int W, int RP, typename T>
-__device__ __forceinline__ void lu_stage(cx<T>* U, int k0, int lane, cx<T>* R, bool& used, T& pmax, T& pmin) {
+__device__ __forceinline__ void lu_stage(cx<T>* U, T* pn, cx<T>* pv, int k0, int lane, cx<T>* R, bool& used,
+                                         T& pmax, T& pmin) {
   constexpr int CL = 32 / RP;
   const int h = lane / RP, r = lane % RP;
 #pragma unroll 1
   for (int k = k0; k < k0 + 4; ++k) {
-    const bool own = h == (k & (CL - 1));
-    const cx<T> e = warp_shfl(R[0], (k & (CL - 1)) * RP + r);  // this row's entry in column k
-    const T v = used ? T(-1) : cnorm2(e);
-    const int pr = pivot_row<RP>(v, r);
+    const int base = (k & (CL - 1)) * RP;  // the lanes that hold column k
+    const bool own = h == (k & (CL - 1)), cand = own && !used;
+    const T v = cand ? cnorm2(R[0]) : T(-1);
+    const cx<T> e = warp_shfl(R[0], base + r);  // this row's entry in column k
+    // FP32: every candidate's reciprocal is taken while the pivot is searched for
+    cx<T> ip = R[0];
+    if constexpr (sizeof(T) == 4) ip = cinv_select(cand ? R[0] : cx<T>(T(1)));
+    const unsigned pl = pivot_lane<RP>(v, base, r);
     cx<T>* Uk = U + k * LDU + k + 1 + ((h - (k + 1)) & (CL - 1));
-    cx<T> X[W];
+    cx<T> X[W], pivot[W];
 #pragma unroll
     for (int i = 0; i < W; ++i) X[i] = own ? R[i + 1] : R[i];
-    if (r == pr) {
+    if ((pl >> (base + r)) & 1) {
       used = true;
 #pragma unroll
       for (int i = 0; i < W; ++i) Uk[CL * i] = X[i];
+      if (own) {
+        (sizeof(T) == 4 ? U[k * LDU + k] : pv[k]) = ip;
+        pn[k] = v;
+      }
     }
-    const T pa = __shfl_sync(FULL, v, pr);
-    const cx<T> ip = cinv_norm(warp_shfl(e, pr), pa);
-    if (lane == 0) U[k * LDU + k] = ip;
+    __syncwarp();
+    ip = sizeof(T) == 4 ? U[k * LDU + k] : pv[k];
+    const T pa = pn[k];
+#pragma unroll
+    for (int i = 0; i < W; ++i) pivot[i] = Uk[CL * i];
+    if constexpr (sizeof(T) == 8) {
+      ip = cinv_norm(ip, pa);
+      if (lane == 0) U[k * LDU + k] = ip;
+    }
     pmax = max_mag(pmax, pa);
     pmin = min_mag(pmin, pa);
     const cx<T> el = mul_split(e, ip, lane, RP), l = used ? cx<T>(T(0)) : el;
-    __syncwarp();
 #pragma unroll
-    for (int i = 0; i < W; ++i) R[i] = cfms(X[i], l, Uk[CL * i]);
+    for (int i = 0; i < W; ++i) R[i] = cfms(X[i], l, pivot[i]);
   }
 }
 
@@ -333,7 +360,7 @@ __device__ __forceinline__ void lu_stage(cx<T>* U, int k0, int lane, cx<T>* R, b
 // row, then the eight remaining rows, in their order, with four lanes a row: 68 complex
 // updates per lane (80 with two lanes a row throughout; the triangle needs 64).
 template <typename T>
-__device__ __forceinline__ void dense_lu(cx<T>* U, int lane, T& pmax, T& pmin) {
+__device__ __forceinline__ void dense_lu(cx<T>* U, T* pn, cx<T>* pv, int lane, T& pmax, T& pmin) {
   cx<T> R[9];
   bool used = false;
   {
@@ -342,8 +369,8 @@ __device__ __forceinline__ void dense_lu(cx<T>* U, int lane, T& pmax, T& pmin) {
     for (int i = 0; i < 8; ++i) R[i] = U[r * LDU + h + 2 * i];
     R[8] = h == 0 ? U[r * LDU + 16] : cx<T>(T(0));
     __syncwarp();
-    lu_stage<8, 16>(U, 0, lane, R, used, pmax, pmin);
-    lu_stage<6, 16>(U, 4, lane, R, used, pmax, pmin);
+    lu_stage<8, 16>(U, pn, pv, 0, lane, R, used, pmax, pmin);
+    lu_stage<6, 16>(U, pn, pv, 4, lane, R, used, pmax, pmin);
     // columns 8 + h, 10 + h, ... of the unused rows to rows 8..15 of U
     const unsigned left = ~__ballot_sync(FULL, used) & 0xffffu;
     if (!used) {
@@ -360,8 +387,8 @@ __device__ __forceinline__ void dense_lu(cx<T>* U, int lane, T& pmax, T& pmin) {
   R[2] = h == 0 ? U[(8 + r) * LDU + 16] : cx<T>(T(0));
   __syncwarp();
   used = false;
-  lu_stage<2, 8>(U, 8, lane, R, used, pmax, pmin);
-  lu_stage<1, 8>(U, 12, lane, R, used, pmax, pmin);
+  lu_stage<2, 8>(U, pn, pv, 8, lane, R, used, pmax, pmin);
+  lu_stage<1, 8>(U, pn, pv, 12, lane, R, used, pmax, pmin);
 }
 
 // Sums over each group of 8 lanes (g = lane & 7) of N values a lane, those of team_sum, to
@@ -397,7 +424,7 @@ __device__ __forceinline__ void back_substitute(const cx<float>* U, cx<float>* X
   const int r = lane & 15;
   cx<float> rb = U[r * LDU + 16];
   const cx<float> ip = U[r * LDU + r];
-#pragma unroll 1
+#pragma unroll 4
   for (int k = 15; k >= 0; --k) {
     const cx<float> xk = warp_shfl(rb * ip, k);
     if (lane == 0) X[k] = xk;
@@ -606,7 +633,7 @@ __device__ __forceinline__ StepOut<T> solve_step(Smem<T, P>& S, const cx<T>* Wsr
   __syncwarp();
   // ---- dense 16 x 16 LU with partial pivoting across the lanes
   T pmax = T(0), pmin = T(3.0e38);
-  dense_lu(U, lane, pmax, pmin);
+  dense_lu(U, S.cn, S.X, lane, pmax, pmin);
   __syncwarp();
   back_substitute(U, S.X, lane);
   __syncwarp();

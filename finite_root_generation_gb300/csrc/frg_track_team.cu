@@ -308,11 +308,20 @@ team_kernel(TrackArgs a) {
     unsigned* base = reinterpret_cast<unsigned*>(&S);
     for (int i = lane; i < (int)(sizeof(Smem<T, P>) / sizeof(unsigned)); i += 32) base[i] = 0u;
   }
+  // Limits in the working precision. The FP32 stage keeps them rounded in shared memory: a
+  // conversion from the configuration's doubles at each use is an FP64 instruction.
+  enum { L_NEWT, L_NEWT_LO, L_COND, L_SHARP, L_RK, L_SMIN, L_SMIN9, L_SMAX, L_COUNT };
+  __shared__ T limits[L_COUNT];
+  if (threadIdx.x == 0) {
+    limits[L_NEWT] = T(c.newt_tol); limits[L_NEWT_LO] = T(c.newt_tol_lo); limits[L_COND] = T(c.cond_switch);
+    limits[L_SHARP] = T(c.sharp_tol); limits[L_RK] = T(c.rk_tol); limits[L_SMIN] = T(c.s_min);
+    limits[L_SMIN9] = T(c.s_min * 0.9); limits[L_SMAX] = T(c.s_max);
+  }
+  __syncthreads();
   // The FP32 stage's corrector iterates on FP32 residuals until |dY| falls below
   // newt_tol_lo (or stops shrinking), then on residuals in the point type to the
   // reference's newt_tol: an FP32 LU with accurate residuals converges like FP64 Newton
   // while the pivot ratio stays below cond_switch.
-  const T newt_tol = T(c.newt_tol);
   // what this launch works through: fresh paths, paths resumed in FP32 (lo_list),
   // or paths handed to FP64 (handoff_list)
   const bool lo_resume = LO && a.lo_list != nullptr && !a.carry;
@@ -473,12 +482,18 @@ team_kernel(TrackArgs a) {
         if (stage == 0) {
           if (el) S.Ye[lane] = cx<T>(S.Yc[lane]);
         } else {
-          // stage weights times s, one per lane; then the sums from the last stage back
+          // the weights times s (FP64: one per lane), the sums from the last stage back
           Wsrc = S.k[stage - 1];
-          const T ws = g < stage ? mul_rn(T(c_dpA[stage][g]), s) : T(0);
-          cx<T> acc = mul_rn(__shfl_sync(FULL, ws, stage - 1), S.k[stage - 1][lane < VS ? lane : 0]);
-          for (int l = stage - 2; l >= 0; --l)
-            acc = axpy(__shfl_sync(FULL, ws, l), S.k[l][lane < VS ? lane : 0], acc);
+          const int e = lane < VS ? lane : 0;
+          cx<T> acc;
+          if constexpr (sizeof(T) == 8) {
+            const T ws = g < stage ? mul_rn(c_dpA[stage][g], s) : T(0);
+            acc = mul_rn(__shfl_sync(FULL, ws, stage - 1), S.k[stage - 1][e]);
+            for (int l = stage - 2; l >= 0; --l) acc = axpy(__shfl_sync(FULL, ws, l), S.k[l][e], acc);
+          } else {
+            acc = mul_rn(mul_rn(c_dpA32[stage][stage - 1], s), S.k[stage - 1][e]);
+            for (int l = stage - 2; l >= 0; --l) acc = axpy(mul_rn(c_dpA32[stage][l], s), S.k[l][e], acc);
+          }
           if (el) S.Ye[lane] = cx<T>(S.Yc[lane]) + acc;
         }
       } else {
@@ -562,7 +577,7 @@ team_kernel(TrackArgs a) {
     int handoff = 0;
     bool handback = false;
     bool final_from_YN = false;
-    if (LO && !(r.ratio <= T(c.cond_switch)) && !(a.lo_keep_ill && r.ratio - r.ratio == T(0))) {
+    if (LO && !(r.ratio <= limits[L_COND]) && !(a.lo_keep_ill && r.ratio - r.ratio == T(0))) {
       handoff = 2;  // ill-conditioned (or non-finite) step: continue in FP64 from Yc
     } else if (MODE == MODE_RESUME && c.fp64_budget > 0 && seg >= c.fp64_budget) {
       code = 2;  // the FP64 budget of this path is spent: retire it as a step-limit failure
@@ -579,7 +594,9 @@ team_kernel(TrackArgs a) {
         // the weights times s one per lane, the second stage has weight zero in both
         T es = T(0);
         {
-          const T we = mul_rn(T(c_dpE[g]), s), wb = mul_rn(T(c_dpB[g]), s);
+          T we, wb;
+          if constexpr (sizeof(T) == 8) { we = mul_rn(c_dpE[g], s); wb = mul_rn(c_dpB[g], s); }
+          else { we = mul_rn(c_dpE32[g], s); wb = mul_rn(c_dpB32[g], s); }
           const cx<T> k7 = S.k[7][lane < VS ? lane : 0];
           cx<T> le = mul_rn(__shfl_sync(FULL, we, 7), k7);
           cx<T> yb = mul_rn(__shfl_sync(FULL, wb, 7), k7);
@@ -600,11 +617,11 @@ team_kernel(TrackArgs a) {
           es = __shfl_sync(FULL, es, g) + e1 + e2;
         }
         err = sqrt(team_sum(FULL, es));
-        scale = (err > T(10e-17)) ? T(0.8) * pow(T(c.rk_tol) / err, T(1) / T(6)) : T(5);
+        scale = (err > T(10e-17)) ? T(0.8) * pow(limits[L_RK] / err, T(1) / T(6)) : T(5);
         if (scale > T(5)) scale = T(5);
         __syncwarp();
         if (ministep++ == c.max_ministeps) { code = 2; finished = true; }
-        else if (err <= T(c.rk_tol)) {
+        else if (err <= limits[L_RK]) {
           const double tn = double(S.Yn[22].re);
           if (LO && !c.lo_endgame && tn > 1.0 - c.nudge_trigger) handoff = 5;  // the endgame runs in FP64
           else if (tn <= 1.0 - c.nudge_trigger) { attempt = 0; phase = PH_NEWTON; }
@@ -617,11 +634,11 @@ team_kernel(TrackArgs a) {
             it = 0;
             hires = !LO || phase == PH_SHARP;
           }
-        } else if (s <= T(c.s_min)) {
+        } else if (s <= limits[L_SMIN]) {
           if (LO) handoff = 4; else { code = 3; finished = true; }
         } else {
           s *= scale;
-          if (s < T(c.s_min)) s = T(c.s_min * 0.9);
+          if (s < limits[L_SMIN]) s = limits[L_SMIN9];
           streak = 0;
         }
       }
@@ -629,7 +646,7 @@ team_kernel(TrackArgs a) {
       // one corrector or sharpening iteration (htpysupport.cu:427-492)
       const bool sharp = (phase == PH_SHARP);
       const int max_its = sharp ? c.sharp_its : c.newt_its;
-      const T tol = sharp ? T(c.sharp_tol) : newt_tol;
+      const T tol = sharp ? limits[L_SHARP] : limits[L_NEWT];
       bool done = false, predicted = false;
       if (restype == 0 && it > 0) {
         residual = r.hnorm;  // |H| at the current point: the residual of the previous update
@@ -643,7 +660,7 @@ team_kernel(TrackArgs a) {
           if (LO && !hires) {
             // FP32 residuals: at the FP32 noise floor either accept (no refinement) or
             // continue on double-float residuals to the reference's tolerance
-            const bool conv = residual < T(c.newt_tol_lo);
+            const bool conv = residual < limits[L_NEWT_LO];
             const bool floor_ = conv || (it > 1 && residual > T(0.5) * res_prev);
             if (c.lo_refine == 3 && conv && !sharp) {
               // the FP32 update is already below newt_tol_lo: accept it without refining
@@ -669,8 +686,8 @@ team_kernel(TrackArgs a) {
       __syncwarp();
       if (done) {
         const bool ok = predicted || ((LO && !c.lo_refine && !sharp)
-                                          ? residual < T(c.newt_tol_lo) * T(100)
-                                          : (hires || !LO) && residual < (sharp ? T(c.sharp_tol) : newt_tol));
+                                          ? residual < limits[L_NEWT_LO] * T(100)
+                                          : (hires || !LO) && residual < (sharp ? limits[L_SHARP] : limits[L_NEWT]));
         if (ministep++ == c.max_ministeps) { code = 2; finished = true; final_from_YN = sharp; }
         else if (ok && !sharp) {
           if (fabs(1.0 - double(S.Yn[22].re)) < c.sharp_trigger) {
@@ -684,8 +701,8 @@ team_kernel(TrackArgs a) {
             streak++;
             if (streak < c.caution_steps && scale > T(1)) scale = T(1);
             s *= scale;
-            if (s > T(c.s_max)) s = T(c.s_max);
-            else if (s < T(c.s_min)) s = T(c.s_min * 0.9);
+            if (s > limits[L_SMAX]) s = limits[L_SMAX];
+            else if (s < limits[L_SMIN]) s = limits[L_SMIN9];
             step++;
             if (checkpoints && step % a.feat_every == 0) {
               // checkpoint: record the features and/or let the network retire the path
@@ -732,11 +749,11 @@ team_kernel(TrackArgs a) {
             if (++attempt < c.newt_attempts) {
               if (el) S.YN[lane] = S.Yn[lane];
               residual = T(100); it = 0; hires = !LO;
-            } else if (s <= T(c.s_min)) {
+            } else if (s <= limits[L_SMIN]) {
               if (LO) handoff = 3; else { code = 4; finished = true; }
             } else {
               s *= T(0.5);
-              if (s < T(c.s_min)) s = T(c.s_min * 0.9);
+              if (s < limits[L_SMIN]) s = limits[L_SMIN9];
               streak = 0;
               stage = 0;
               phase = PH_RK;

@@ -1,5 +1,5 @@
 """How a launch spreads its paths over the GPU: the team kernels put one to four paths in a
-block; a plug-in's launch tracks a path per warp up to eight paths per SM sub-partition and
+block; a plug-in's launch tracks a path per warp up to 16 paths per SM sub-partition and
 a path per thread beyond, whose last paths go on a warp each. So the same path runs beside
 different neighbours, and in different kernels, in different calls. A path depends on its random
 stream alone: the first n paths of a call must equal the call of n paths bit for bit, at
@@ -48,7 +48,7 @@ def test_thread_spread(precision):
                             gamma_mode=frg.GAMMA_RANDOM, inf_tol=1e-8)
     with frg.Tracker(cfg) as t:
         full = t.track(task, [20000], 43, want_resid=True)
-        for n in (1, 33, 607, 609, 4864, 4865, 19455, 19457):
+        for n in (1, 33, 607, 609, 9728, 9729, 19455, 19457):
             part = t.track(task, [n], 43, want_resid=True)
             assert np.array_equal(part.codes, full.codes[:n]), n
             assert np.array_equal(part.roots, full.roots[:n], equal_nan=True), n
