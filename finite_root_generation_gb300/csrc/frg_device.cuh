@@ -10,6 +10,7 @@
 #include "frg_complex.cuh"
 #include "frg_rng.h"
 #include "frg_system_gen.cuh"
+#include "frg_warp.cuh"
 
 namespace frg {
 
@@ -42,6 +43,17 @@ typedef cx<double> cd;
                                 T(1375. / 5408.), T(-37. / 1120.), T(1. / 10.)}
 FRG_DP_TABLEAU(double, c_dpA, c_dpE, c_dpB);
 FRG_DP_TABLEAU(float, c_dpA32, c_dpE32, c_dpB32);
+template <typename T> struct Dp;
+template <> struct Dp<double> {
+  static __device__ __forceinline__ const double* a(int stage) { return c_dpA[stage]; }
+  static __device__ __forceinline__ const double* e() { return c_dpE; }
+  static __device__ __forceinline__ const double* b() { return c_dpB; }
+};
+template <> struct Dp<float> {
+  static __device__ __forceinline__ const float* a(int stage) { return c_dpA32[stage]; }
+  static __device__ __forceinline__ const float* e() { return c_dpE32; }
+  static __device__ __forceinline__ const float* b() { return c_dpB32; }
+};
 
 // ---------------------------------------------------------------------------
 // Random draws (the reference's curand_uniform_double, replaced by Philox).
@@ -190,10 +202,10 @@ __device__ __forceinline__ void row_scale(cx<T>* M, int rows, cx<T>* rhs) {
 #pragma unroll 1
   for (int i = 0; i < rows; ++i) {
     cx<T>* r = M + i * LD;
-    T mx = T(0);
+    MaxAbs<T> mx;
 #pragma unroll
-    for (int c = 0; c < N_Y; ++c) mx = fmax(mx, fmax(tabs(r[c].re), tabs(r[c].im)));
-    const T s = T(1) / mx;
+    for (int c = 0; c < N_Y; ++c) mx.take(r[c]);
+    const T s = T(1) / mx.value();
 #pragma unroll
     for (int c = 0; c < N_Y; ++c) r[c] = s * r[c];
     if (rhs) rhs[i] = s * rhs[i];
@@ -218,7 +230,7 @@ __device__ T lu_solve(cx<T>* M, cx<T>* b, cx<T>* x, int nelim, bool fix_last, cx
 #pragma unroll 1
       for (int k = i; k < nelim; ++k) {
         T v = cnorm2(M[k * LD + i]);
-        if (v > best) { best = v; br = k; }
+        if (mag_above(v, best)) { best = v; br = k; }
       }
       if (br != i) {
         cx<T>* ri = M + i * LD;
@@ -233,8 +245,8 @@ __device__ T lu_solve(cx<T>* M, cx<T>* b, cx<T>* x, int nelim, bool fix_last, cx
     ipiv[i] = ip;
     if (i < nelim) {
       T a = sqrt(cnorm2(ri[i]));
-      pmax = fmax(pmax, a);
-      pmin = (pmin < T(0)) ? a : fmin(pmin, a);
+      pmax = max_mag(pmax, a);
+      pmin = i == 0 ? a : min_mag(pmin, a);
     }
     const cx<T> bi = b[i];
 #pragma unroll 1

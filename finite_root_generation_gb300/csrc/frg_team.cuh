@@ -85,9 +85,6 @@ __device__ __forceinline__ T team_max(unsigned mask, T v) {
   return v;
 }
 
-template <typename T>
-__device__ __forceinline__ cx<T> neg(cx<T> a) { return cx<T>(neg_if(a.re, true), neg_if(a.im, true)); }
-
 // Task and start parameters in the working precision, when it is not the point type's.
 template <typename T, typename P> struct LowTask { cx<T> sp[32], fp[32]; };
 template <typename T> struct LowTask<T, T> {};

@@ -69,17 +69,25 @@ __device__ __forceinline__ T vnorm(const cx<T>* v, int n) {
   return sqrt(s);
 }
 
-// sum_{l < n} w[l] * s * k[l][e], accumulated from the last term to the first as the
-// reference's nested .add() chains do (rungekutta.cu:40-122).
+// The tableau's weights times the step, once a stage. A product and a zero test per term
+// and element, and the maxima and pivot comparisons as FP64 compares, held the FP64 pipe
+// for an eighth of the step (GB300, 262,144 conic2 paths: FP64 137 -> 120 ms, mixed, where
+// each weight was a conversion, 31.4 -> 28.2; 131,072 burmester5 paths in FP64 734 -> 672).
+template <typename T>
+__device__ __forceinline__ void stage_weights(const T* w, T s, int n, T* ws) {
+#pragma unroll 1
+  for (int l = 0; l < n; ++l) ws[l] = mul_rn(w[l], s);
+}
+
+// sum_l ws[l] k[l][e] over the terms in m (not empty), accumulated from the last term to the first as
+// the reference's nested .add() chains do (rungekutta.cu:40-122), product then sum.
 template <typename T, int NY_>
-__device__ __forceinline__ cx<T> comb(const double* w, T s, const cx<T> (*k)[NY_], int n, int e) {
-  cx<T> acc(T(0));
-  bool first = true;
-  for (int l = n - 1; l >= 0; --l) {
-    if (w[l] == 0.0) continue;
-    cx<T> term = (T(w[l]) * s) * k[l][e];
-    acc = first ? term : term + acc;
-    first = false;
+__device__ __forceinline__ cx<T> comb(const T* ws, unsigned m, const cx<T> (*k)[NY_], int e) {
+  int l = 31 - __clz(m);
+  cx<T> acc = mul_rn(ws[l], k[l][e]);
+  for (m ^= 1u << l; m; m ^= 1u << l) {
+    l = 31 - __clz(m);
+    acc = mul_rn(ws[l], k[l][e]) + acc;
   }
   return acc;
 }
@@ -262,8 +270,10 @@ track_kernel(TrackArgs a) {
         for (int e = 0; e < NY_; ++e) Ye[e] = P.Yc[e];
       } else {
         patch = P.k[st - 1];
+        T ws[8];
+        stage_weights(Dp<T>::a(st), P.s, st, ws);
 #pragma unroll 1
-        for (int e = 0; e < NY_; ++e) Ye[e] = P.Yc[e] + comb<T, NY_>(c_dpA[st], P.s, P.k, st, e);
+        for (int e = 0; e < NY_; ++e) Ye[e] = P.Yc[e] + comb<T, NY_>(ws, (1u << st) - 1, P.k, e);
       }
     } else {
 #pragma unroll 1
@@ -292,7 +302,7 @@ track_kernel(TrackArgs a) {
     // corrector and lanes in the predictor run them together
     row_scale<T, NY_, LD_>(M, NZ_, newton ? F : nullptr);
 #pragma unroll 1
-    for (int e = 0; e < NZ_; ++e) b[e] = newton ? -F[e] : cx<T>(T(0));
+    for (int e = 0; e < NZ_; ++e) b[e] = newton ? neg(F[e]) : cx<T>(T(0));
     b[NY_ - 1] = newton ? cx<T>(T(0)) : cx<T>(T(1));
     __syncwarp(live);
     const T ratio = lu_solve<T, NY_, LD_>(M, b, x, newton ? NZ_ : NY_, newton, cx<T>(tdiff));
@@ -333,11 +343,14 @@ track_kernel(TrackArgs a) {
       if (++P.stage == 8) {
         P.stage = 0;
         // error estimate and step factor (rungekutta.cu:99-112), prediction (:115-122)
-        T es = T(0);
+        T es = T(0), we[8], wb[8];  // the weights of k[1] are zero in both
+        stage_weights(Dp<T>::e(), P.s, 8, we);
+        stage_weights(Dp<T>::b(), P.s, 8, wb);
 #pragma unroll 1
         for (int e = 0; e < NY_; ++e) {
-          es += cnorm2(comb<T, NY_>(c_dpE, P.s, P.k, 8, e));
-          P.Yn[e] = P.Yc[e] + comb<T, NY_>(c_dpB, P.s, P.k, 8, e);
+          const cx<T> d = comb<T, NY_>(we, 0xfd, P.k, e);
+          es += fma(d.re, d.re, mul_rn(d.im, d.im));
+          P.Yn[e] = P.Yc[e] + comb<T, NY_>(wb, 0xfd, P.k, e);
           P.Vn[e] = P.k[7][e];
         }
         P.err = sqrt(es);

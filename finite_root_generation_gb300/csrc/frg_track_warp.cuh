@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
         y = W.Yc[el ? lane : 0];
       } else if (phase == PH_RK) {
         patch = W.k[stage - 1];
-        const T ws = lane < stage ? T(c_dpA[stage][lane]) * s : T(0);
+        const T ws = lane < stage ? Dp<T>::a(stage)[lane] * s : T(0);
         cx<T> acc = mul_rn(__shfl_sync(FULL, ws, stage - 1), W.k[stage - 1][el ? lane : 0]);
         for (int l = stage - 2; l >= 0; --l) acc = mul_rn(__shfl_sync(FULL, ws, l), W.k[l][el ? lane : 0]) + acc;
         y = W.Yc[el ? lane : 0] + acc;
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
         if (++stage == 8) {
           stage = 0;
           // error estimate and step factor (rungekutta.cu:99-112), prediction (:115-122)
-          const T we = T(c_dpE[lane & 7]) * s, wb = T(c_dpB[lane & 7]) * s;
+          const T we = Dp<T>::e()[lane & 7] * s, wb = Dp<T>::b()[lane & 7] * s;
           const cx<T> k7 = W.k[7][el ? lane : 0];
           cx<T> le = mul_rn(__shfl_sync(FULL, we, 7), k7);
           cx<T> yb = mul_rn(__shfl_sync(FULL, wb, 7), k7);

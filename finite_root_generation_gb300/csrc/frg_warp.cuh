@@ -45,8 +45,14 @@ __device__ __forceinline__ double max_mag(double m, double x) {
   return b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll ? x : m;
 }
 __device__ __forceinline__ double min_mag(double m, double x) {
+  return (unsigned long long)__double_as_longlong(x) < (unsigned long long)__double_as_longlong(m) ? x : m;
+}
+
+// x > m for magnitudes, false for a NaN x
+__device__ __forceinline__ bool mag_above(float x, float m) { return x > m; }
+__device__ __forceinline__ bool mag_above(double x, double m) {
   const long long b = __double_as_longlong(x);
-  return b >= 0 && b < __double_as_longlong(m) ? x : m;
+  return b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll;
 }
 
 // 1 / b when |b|^2 is at hand (FP64: conj(b) / |b|^2; FP32 keeps Smith's form)
@@ -72,6 +78,8 @@ __device__ __forceinline__ double neg_if(double x, bool neg) {
   return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
 }
 __device__ __forceinline__ float neg_if(float x, bool neg) { return neg ? -x : x; }
+template <typename T>
+__device__ __forceinline__ cx<T> neg(cx<T> a) { return cx<T>(neg_if(a.re, true), neg_if(a.im, true)); }
 
 // An FP64 complex value held by a pair of lanes (2 k, 2 k + 1): each lane computes one
 // component of every result (the even lane the real part) and the pair exchanges, so a
