@@ -6,6 +6,7 @@
 // and the t-derivative dF/dq . dq/dt (JH's last column, htpysupport.cu:113-121).
 // Straight-line cost per group: 352 complex mul, 239 complex add/sub,
 // 5 real-scalar x complex.
+// The three equations alone: 62 complex mul, 57 complex add/sub, 0 real x complex.
 #pragma once
 
 #define FRG_GEN_CMUL 352
@@ -212,57 +213,6 @@ __device__ __forceinline__ void frg_group_eval(
   o.dIII[14] = x100*x121 - x123*x48*x97;
   o.dIII[15] = (-x85) + x71*x73 - x87*x90 - P0*x132*x136 - Pc0*x133*x137 - x11*x134*x90 - x135*x16*x87 + P0*x132*x84*z + Pc0*x133*x79*z + Pcj*U*x134*x79 + (T(2.0)*(iU*x84*x90*z)) + Pj*iU*x135*x84*z2;
   o.tIII = dQcj*x110*(x20 + x20*x83) + dQj*x93*(x25 + x25*x78) + dP0*x132*z*((-x136) + x84*z) + dPc0*x133*z*((-x137) + x79*z) - dPcj*z*(x122 - x129)*(ec1*x113 + ec2*x82) - dPj*z*(x106 - x102)*(x116 - x111);
-}
-
-// The three equations alone: 62 complex mul, 57 complex add/sub, 0 real x complex.
-#define FRG_GENF_CMUL 62
-#define FRG_GENF_CADD 57
-template <typename T>
-__device__ __forceinline__ void frg_group_f(
-    const cx<T> A, const cx<T> B, const cx<T> C, const cx<T> D, const cx<T> F, const cx<T> G,
-    const cx<T> H, const cx<T> Ac, const cx<T> Bc, const cx<T> Cc, const cx<T> Dc, const cx<T> Fc,
-    const cx<T> Gc, const cx<T> Hc, const cx<T> z,
-    const cx<T> e1, const cx<T> e2, const cx<T> ec1, const cx<T> ec2,
-    const cx<T> z2, const cx<T> z3, const cx<T> P0, const cx<T> Pc0,
-    const cx<T> U, const cx<T> iU, const cx<T> Pj, const cx<T> Pcj, const cx<T> Qj, const cx<T> Qcj,
-    cx<T>& fI, cx<T>& fII, cx<T>& fIII) {
-  const cx<T> y0 = z3*(P0*Pc0 + Pcj*Pj);
-  const cx<T> y1 = (-(Pc0*z));
-  const cx<T> y2 = (-(P0*z));
-  const cx<T> y3 = (-(Ac));
-  const cx<T> y4 = Pcj*z;
-  const cx<T> y5 = y3 + y4;
-  const cx<T> y6 = (-(A));
-  const cx<T> y7 = Pj*z;
-  const cx<T> y8 = y6 + y7;
-  const cx<T> y9 = (-(y7));
-  const cx<T> y10 = A + y9;
-  const cx<T> y11 = Ac - Cc;
-  const cx<T> y12 = Qcj*y11;
-  const cx<T> y13 = (-(y4));
-  const cx<T> y14 = Ac + y13;
-  const cx<T> y15 = A - C;
-  const cx<T> y16 = Qj*y15;
-  const cx<T> y17 = H + y2;
-  const cx<T> y18 = Hc + y1;
-  const cx<T> y19 = iU*z2;
-  const cx<T> y20 = Bc + y13;
-  const cx<T> y21 = F + y2;
-  const cx<T> y22 = B + y9;
-  const cx<T> y23 = Fc + y1;
-  const cx<T> y24 = (-(G));
-  const cx<T> y25 = (-(Gc));
-  const cx<T> y26 = e1*(B - D);
-  const cx<T> y27 = e2*(C + y24);
-  const cx<T> y28 = y21*y26 - y17*y27;
-  const cx<T> y29 = ec1*(Bc - Dc);
-  const cx<T> y30 = ec2*(Cc + y25);
-  const cx<T> y31 = y23*y29 - y18*y30;
-  const cx<T> y32 = Bc + y12 + y3 + y20*y29 - y30*(y14 - Qcj*y11);
-  const cx<T> y33 = B + y16 + y6 + y22*y26 - y27*(y10 - Qj*y15);
-  fI = (-y0) + A*z*(Cc + y5) + Ac*z*(C + y8) + U*y17*((-y12) - y5) + y10*y12*z + y14*y16*z + y18*y19*((-y16) - y8) - H*z*(Cc + y1) - Hc*z*(C + y2);
-  fII = (-y0) + z2*(B*Pcj + Bc*Pj) + U*y20*y21 - F*z*(Bc + y1) - Fc*z*(B + y2) + iU*y22*y23*z2;
-  fIII = U*y28*y32 + y19*y31*y33 + z*(D + y24)*(Dc + y25) - y28*y31*z - y32*y33*z;
 }
 
 // What one path's step needs besides its point: computed by the path's own warp, read by
@@ -698,83 +648,302 @@ __device__ __forceinline__ void frg_eval_slice(const cx<T>* Y, const FrgEvalIn<T
   }
 }
 
-// One of the three equations at the point Y (frg_group_f's operations in its order).
-template <int SLICE, typename T>
-__device__ __forceinline__ cx<T> frg_residual_slice(const cx<T>* Y, const FrgEvalIn<T>& in, int j) {
-  typedef cx<T> CX;
-  if constexpr (SLICE == 0) {
-    const CX A(Y[0]);
-    const CX Ac(Y[7]);
-    const CX C(Y[2]);
-    const CX Cc(Y[9]);
-    const CX H(Y[6]);
-    const CX Hc(Y[13]);
-    const CX P0(in.q[0]);
-    const CX Pc0(in.q[8]);
-    const CX Pcj(in.q[8 + j]);
-    const CX Pj(in.q[j]);
-    const CX U(Y[13 + j]);
-    const CX iU(in.iU[j - 1]);
-    const CX y10(in.sb[0][FRG_IN_AP][j - 1]);
-    const CX y12(in.sb[1][FRG_IN_QA][j - 1]);
-    const CX y14(in.sb[1][FRG_IN_AP][j - 1]);
-    const CX y16(in.sb[0][FRG_IN_QA][j - 1]);
-    const CX y17(in.sa[0][FRG_IN_HP]);
-    const CX y18(in.sa[1][FRG_IN_HP]);
-    const CX y4(in.sb[1][FRG_IN_PJZ][j - 1]);
-    const CX y7(in.sb[0][FRG_IN_PJZ][j - 1]);
-    const CX z(Y[21]);
-    const CX z2(in.z2);
-    const CX z3(in.z3);
-    const CX y0 = z3*(P0*Pc0 + Pcj*Pj);
-    const CX y1 = (-(Pc0*z));
-    const CX y2 = (-(P0*z));
-    const CX y3 = (-(Ac));
-    const CX y5 = y3 + y4;
-    const CX y6 = (-(A));
-    const CX y8 = y6 + y7;
-    const CX y19 = iU*z2;
-    return (-y0) + A*z*(Cc + y5) + Ac*z*(C + y8) + U*y17*((-y12) - y5) + y10*y12*z + y14*y16*z + y18*y19*((-y16) - y8) - H*z*(Cc + y1) - Hc*z*(C + y2);
-  }
-  if constexpr (SLICE == 1) {
-    const CX B(Y[1]);
-    const CX Bc(Y[8]);
-    const CX F(Y[4]);
-    const CX Fc(Y[11]);
-    const CX P0(in.q[0]);
-    const CX Pc0(in.q[8]);
-    const CX Pcj(in.q[8 + j]);
-    const CX Pj(in.q[j]);
-    const CX U(Y[13 + j]);
-    const CX iU(in.iU[j - 1]);
-    const CX y20(in.sb[1][FRG_IN_BP][j - 1]);
-    const CX y21(in.sa[0][FRG_IN_FP]);
-    const CX y22(in.sb[0][FRG_IN_BP][j - 1]);
-    const CX y23(in.sa[1][FRG_IN_FP]);
-    const CX z(Y[21]);
-    const CX z2(in.z2);
-    const CX z3(in.z3);
-    const CX y0 = z3*(P0*Pc0 + Pcj*Pj);
-    const CX y1 = (-(Pc0*z));
-    const CX y2 = (-(P0*z));
-    return (-y0) + z2*(B*Pcj + Bc*Pj) + U*y20*y21 - F*z*(Bc + y1) - Fc*z*(B + y2) + iU*y22*y23*z2;
-  }
-  if constexpr (SLICE == 2) {
-    const CX D(Y[3]);
-    const CX Dc(Y[10]);
-    const CX G(Y[5]);
-    const CX Gc(Y[12]);
-    const CX U(Y[13 + j]);
-    const CX iU(in.iU[j - 1]);
-    const CX y28(in.sa[0][FRG_IN_V]);
-    const CX y31(in.sa[1][FRG_IN_V]);
-    const CX y32(in.sb[1][FRG_IN_W][j - 1]);
-    const CX y33(in.sb[0][FRG_IN_W][j - 1]);
-    const CX z(Y[21]);
-    const CX z2(in.z2);
-    const CX y19 = iU*z2;
-    const CX y24 = (-(G));
-    const CX y25 = (-(Gc));
-    return U*y28*y32 + y19*y31*y33 + z*(D + y24)*(Dc + y25) - y28*y31*z - y32*y33*z;
-  }
-}
+// The three equations at a point alone (their own common subexpressions) as schedules for a
+// part's four warps, residual_slice in frg_team.cuh executes them. Warp k: steps START[k] ..
+// START[k + 1] of 16 words OP(result, a, b, b subtracted, product), in 16-byte units from
+// Y (the point), IN (FrgEvalIn) and T (temporaries; the last takes idle lanes' results), two steps
+// of padding at the end; then OUT(unit, equation, group, negated), 7 per warp.
+#define FRG_RESIDUAL_TEMPS 119
+#define FRG_RESIDUAL_START {0, 17, 33, 47, 58}
+#define FRG_RESIDUAL_CODE(OP, Y, IN, T) \
+    OP(T + 0, Y + 7, IN + 123, 1, 0), OP(T + 1, Y + 7, IN + 122, 1, 0), OP(T + 2, Y + 7, IN + 121, 1, 0), \
+    OP(T + 3, Y + 7, IN + 120, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 4, IN + 18, IN + 10, 0, 1), \
+    OP(T + 5, IN + 17, IN + 9, 0, 1), OP(T + 6, IN + 16, IN + 8, 0, 1), OP(T + 7, Y + 0, Y + 21, 0, 1), \
+    OP(T + 8, IN + 15, IN + 7, 0, 1), OP(T + 9, IN + 6, IN + 14, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 10, T + 9, T + 4, 0, 0), OP(T + 11, T + 9, T + 5, 0, 0), \
+    OP(T + 12, T + 9, T + 6, 0, 0), OP(T + 13, T + 9, T + 8, 0, 0), OP(T + 14, Y + 9, T + 0, 1, 0), \
+    OP(T + 15, Y + 9, T + 1, 1, 0), OP(T + 16, Y + 9, T + 2, 1, 0), OP(T + 17, Y + 9, T + 3, 1, 0), \
+    OP(T + 18, Y + 0, IN + 67, 1, 0), OP(T + 19, Y + 0, IN + 66, 1, 0), OP(T + 20, Y + 0, IN + 65, 1, 0), \
+    OP(T + 21, Y + 0, IN + 64, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 4, IN + 1, T + 10, 0, 1), \
+    OP(T + 5, IN + 1, T + 11, 0, 1), OP(T + 6, IN + 1, T + 12, 0, 1), OP(T + 8, IN + 1, T + 13, 0, 1), \
+    OP(T + 9, T + 7, T + 14, 0, 1), OP(T + 22, T + 7, T + 15, 0, 1), OP(T + 23, T + 7, T + 16, 0, 1), \
+    OP(T + 24, T + 7, T + 17, 0, 1), OP(T + 25, Y + 7, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 7, T + 4, T + 9, 1, 0), \
+    OP(T + 10, T + 5, T + 22, 1, 0), OP(T + 11, T + 6, T + 23, 1, 0), OP(T + 12, T + 8, T + 24, 1, 0), \
+    OP(T + 13, Y + 2, T + 18, 1, 0), OP(T + 14, Y + 2, T + 19, 1, 0), OP(T + 15, Y + 2, T + 20, 1, 0), \
+    OP(T + 16, Y + 2, T + 21, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 17, T + 25, T + 13, 0, 1), OP(T + 4, T + 25, T + 14, 0, 1), \
+    OP(T + 5, T + 25, T + 15, 0, 1), OP(T + 6, T + 25, T + 16, 0, 1), OP(T + 8, Y + 17, IN + 48, 0, 1), \
+    OP(T + 9, Y + 16, IN + 48, 0, 1), OP(T + 22, Y + 15, IN + 48, 0, 1), OP(T + 23, Y + 14, IN + 48, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 24, T + 7, T + 17, 1, 0), OP(T + 13, T + 10, T + 4, 1, 0), OP(T + 14, T + 11, T + 5, 1, 0), \
+    OP(T + 15, T + 12, T + 6, 1, 0), OP(T + 16, IN + 147, T + 0, 1, 0), OP(T + 25, IN + 146, T + 1, 1, 0), \
+    OP(T + 26, IN + 145, T + 2, 1, 0), OP(T + 27, IN + 144, T + 3, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 0, T + 8, T + 16, 0, 1), \
+    OP(T + 1, T + 9, T + 25, 0, 1), OP(T + 2, T + 22, T + 26, 0, 1), OP(T + 3, T + 23, T + 27, 0, 1), \
+    OP(T + 4, IN + 75, IN + 147, 0, 1), OP(T + 5, IN + 74, IN + 146, 0, 1), OP(T + 6, IN + 73, IN + 145, 0, 1), \
+    OP(T + 7, IN + 72, IN + 144, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 10, T + 24, T + 0, 0, 0), \
+    OP(T + 11, T + 13, T + 1, 0, 0), OP(T + 12, T + 14, T + 2, 0, 0), OP(T + 17, T + 15, T + 3, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 8, T + 4, Y + 21, 0, 1), OP(T + 9, T + 5, Y + 21, 0, 1), OP(T + 16, T + 6, Y + 21, 0, 1), \
+    OP(T + 22, T + 7, Y + 21, 0, 1), OP(T + 23, IN + 41, IN + 0, 0, 1), OP(T + 25, IN + 40, IN + 0, 0, 1), \
+    OP(T + 26, IN + 39, IN + 0, 0, 1), OP(T + 27, IN + 38, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 0, T + 10, T + 8, 1, 0), \
+    OP(T + 1, T + 11, T + 9, 1, 0), OP(T + 2, T + 12, T + 16, 1, 0), OP(T + 3, T + 17, T + 22, 1, 0), \
+    OP(T + 13, IN + 91, T + 18, 1, 0), OP(T + 14, IN + 90, T + 19, 1, 0), OP(T + 15, IN + 89, T + 20, 1, 0), \
+    OP(T + 24, IN + 88, T + 21, 1, 0), OP(T + 4, Y + 2, IN + 46, 1, 0), OP(T + 5, Y + 9, IN + 55, 1, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 6, IN + 57, T + 23, 0, 1), \
+    OP(T + 7, IN + 57, T + 25, 0, 1), OP(T + 8, IN + 57, T + 26, 0, 1), OP(T + 9, IN + 57, T + 27, 0, 1), \
+    OP(T + 10, IN + 131, IN + 91, 0, 1), OP(T + 11, IN + 130, IN + 90, 0, 1), \
+    OP(T + 12, IN + 129, IN + 89, 0, 1), OP(T + 16, Y + 13, Y + 21, 0, 1), OP(T + 17, Y + 6, Y + 21, 0, 1), \
+    OP(T + 18, IN + 128, IN + 88, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 19, T + 6, T + 13, 0, 1), OP(T + 20, T + 7, T + 14, 0, 1), OP(T + 21, T + 8, T + 15, 0, 1), \
+    OP(T + 22, T + 9, T + 24, 0, 1), OP(T + 23, T + 10, Y + 21, 0, 1), OP(T + 25, T + 11, Y + 21, 0, 1), \
+    OP(T + 26, T + 12, Y + 21, 0, 1), OP(T + 27, T + 16, T + 4, 0, 1), OP(T + 28, T + 17, T + 5, 0, 1), \
+    OP(T + 29, T + 18, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 4, T + 0, T + 23, 1, 0), OP(T + 5, T + 1, T + 25, 1, 0), OP(T + 6, T + 2, T + 26, 1, 0), \
+    OP(T + 7, T + 3, T + 29, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 8, T + 4, T + 19, 0, 0), OP(T + 9, T + 5, T + 20, 0, 0), \
+    OP(T + 10, T + 6, T + 21, 0, 0), OP(T + 11, T + 7, T + 22, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 12, T + 8, T + 28, 0, 0), \
+    OP(T + 13, T + 9, T + 28, 0, 0), OP(T + 14, T + 10, T + 28, 0, 0), OP(T + 15, T + 11, T + 28, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 16, T + 12, T + 27, 0, 0), OP(T + 17, T + 13, T + 27, 0, 0), OP(T + 18, T + 14, T + 27, 0, 0), \
+    OP(T + 24, T + 15, T + 27, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 30, Y + 7, IN + 126, 1, 0), \
+    OP(T + 31, Y + 7, IN + 125, 1, 0), OP(T + 32, Y + 7, IN + 124, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 33, IN + 21, IN + 13, 0, 1), OP(T + 34, IN + 20, IN + 12, 0, 1), OP(T + 35, Y + 0, Y + 21, 0, 1), \
+    OP(T + 36, IN + 19, IN + 11, 0, 1), OP(T + 37, IN + 6, IN + 14, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 38, T + 37, T + 33, 0, 0), \
+    OP(T + 39, T + 37, T + 34, 0, 0), OP(T + 40, T + 37, T + 36, 0, 0), OP(T + 41, Y + 9, T + 30, 1, 0), \
+    OP(T + 42, Y + 9, T + 31, 1, 0), OP(T + 43, Y + 9, T + 32, 1, 0), OP(T + 44, Y + 0, IN + 70, 1, 0), \
+    OP(T + 45, Y + 0, IN + 69, 1, 0), OP(T + 46, Y + 0, IN + 68, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 33, IN + 1, T + 38, 0, 1), \
+    OP(T + 34, IN + 1, T + 39, 0, 1), OP(T + 36, IN + 1, T + 40, 0, 1), OP(T + 37, T + 35, T + 41, 0, 1), \
+    OP(T + 47, T + 35, T + 42, 0, 1), OP(T + 48, T + 35, T + 43, 0, 1), OP(T + 49, Y + 7, Y + 21, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 35, T + 33, T + 37, 1, 0), OP(T + 38, T + 34, T + 47, 1, 0), \
+    OP(T + 39, T + 36, T + 48, 1, 0), OP(T + 40, Y + 2, T + 44, 1, 0), OP(T + 41, Y + 2, T + 45, 1, 0), \
+    OP(T + 42, Y + 2, T + 46, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 43, T + 49, T + 40, 0, 1), OP(T + 33, T + 49, T + 41, 0, 1), OP(T + 34, T + 49, T + 42, 0, 1), \
+    OP(T + 36, IN + 78, IN + 150, 0, 1), OP(T + 37, Y + 20, IN + 48, 0, 1), \
+    OP(T + 47, IN + 77, IN + 149, 0, 1), OP(T + 48, Y + 19, IN + 48, 0, 1), \
+    OP(T + 50, IN + 76, IN + 148, 0, 1), OP(T + 51, Y + 18, IN + 48, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 40, T + 35, T + 43, 1, 0), \
+    OP(T + 41, T + 38, T + 33, 1, 0), OP(T + 42, T + 39, T + 34, 1, 0), OP(T + 49, IN + 150, T + 30, 1, 0), \
+    OP(T + 52, IN + 149, T + 31, 1, 0), OP(T + 53, IN + 148, T + 32, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 30, T + 37, T + 49, 0, 1), OP(T + 31, T + 48, T + 52, 0, 1), \
+    OP(T + 32, T + 51, T + 53, 0, 1), OP(T + 33, T + 36, Y + 21, 0, 1), OP(T + 34, T + 47, Y + 21, 0, 1), \
+    OP(T + 35, T + 50, Y + 21, 0, 1), OP(T + 38, IN + 44, IN + 0, 0, 1), OP(T + 39, IN + 43, IN + 0, 0, 1), \
+    OP(T + 43, IN + 42, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 36, T + 40, T + 30, 0, 0), OP(T + 37, T + 41, T + 31, 0, 0), \
+    OP(T + 47, T + 42, T + 32, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 48, T + 36, T + 33, 1, 0), OP(T + 49, T + 37, T + 34, 1, 0), OP(T + 50, T + 47, T + 35, 1, 0), \
+    OP(T + 51, IN + 94, T + 44, 1, 0), OP(T + 52, IN + 93, T + 45, 1, 0), OP(T + 53, IN + 92, T + 46, 1, 0), \
+    OP(T + 30, Y + 2, IN + 46, 1, 0), OP(T + 31, Y + 9, IN + 55, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 32, IN + 57, T + 38, 0, 1), OP(T + 40, IN + 57, T + 39, 0, 1), OP(T + 41, IN + 57, T + 43, 0, 1), \
+    OP(T + 42, IN + 134, IN + 94, 0, 1), OP(T + 33, IN + 133, IN + 93, 0, 1), OP(T + 34, Y + 13, Y + 21, 0, 1), \
+    OP(T + 35, Y + 6, Y + 21, 0, 1), OP(T + 36, IN + 132, IN + 92, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 37, T + 32, T + 51, 0, 1), OP(T + 44, T + 40, T + 52, 0, 1), OP(T + 45, T + 41, T + 53, 0, 1), \
+    OP(T + 46, T + 42, Y + 21, 0, 1), OP(T + 47, T + 33, Y + 21, 0, 1), OP(T + 38, T + 34, T + 30, 0, 1), \
+    OP(T + 39, T + 35, T + 31, 0, 1), OP(T + 43, T + 36, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 30, T + 48, T + 46, 1, 0), OP(T + 31, T + 49, T + 47, 1, 0), OP(T + 32, T + 50, T + 43, 1, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 33, T + 30, T + 37, 0, 0), OP(T + 34, T + 31, T + 44, 0, 0), \
+    OP(T + 35, T + 32, T + 45, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 36, T + 33, T + 39, 0, 0), OP(T + 40, T + 34, T + 39, 0, 0), OP(T + 41, T + 35, T + 39, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 42, T + 36, T + 38, 0, 0), OP(T + 51, T + 40, T + 38, 0, 0), \
+    OP(T + 52, T + 41, T + 38, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 54, Y + 1, IN + 16, 0, 1), OP(T + 55, IN + 16, IN + 8, 0, 1), OP(T + 56, Y + 8, IN + 7, 0, 1), \
+    OP(T + 57, Y + 1, IN + 15, 0, 1), OP(T + 58, IN + 15, IN + 7, 0, 1), OP(T + 59, IN + 6, IN + 14, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 60, Y + 8, IN + 13, 0, 1), \
+    OP(T + 61, Y + 1, IN + 21, 0, 1), OP(T + 62, IN + 21, IN + 13, 0, 1), OP(T + 63, Y + 8, IN + 12, 0, 1), \
+    OP(T + 64, Y + 1, IN + 20, 0, 1), OP(T + 65, IN + 20, IN + 12, 0, 1), OP(T + 66, Y + 8, IN + 11, 0, 1), \
+    OP(T + 67, Y + 1, IN + 19, 0, 1), OP(T + 68, IN + 19, IN + 11, 0, 1), OP(T + 69, Y + 8, IN + 10, 0, 1), \
+    OP(T + 70, Y + 1, IN + 18, 0, 1), OP(T + 71, IN + 18, IN + 10, 0, 1), OP(T + 72, Y + 8, IN + 9, 0, 1), \
+    OP(T + 73, Y + 1, IN + 17, 0, 1), OP(T + 74, IN + 17, IN + 9, 0, 1), OP(T + 75, Y + 8, IN + 8, 0, 1), \
+    OP(T + 76, T + 61, T + 60, 0, 0), OP(T + 77, T + 59, T + 62, 0, 0), OP(T + 78, T + 64, T + 63, 0, 0), \
+    OP(T + 79, T + 59, T + 65, 0, 0), OP(T + 80, T + 67, T + 66, 0, 0), OP(T + 81, T + 59, T + 68, 0, 0), \
+    OP(T + 82, T + 70, T + 69, 0, 0), OP(T + 83, T + 59, T + 71, 0, 0), OP(T + 84, T + 73, T + 72, 0, 0), \
+    OP(T + 85, T + 59, T + 74, 0, 0), OP(T + 86, T + 54, T + 75, 0, 0), OP(T + 87, T + 59, T + 55, 0, 0), \
+    OP(T + 88, T + 57, T + 56, 0, 0), OP(T + 89, T + 59, T + 58, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 54, IN + 0, T + 76, 0, 1), OP(T + 55, IN + 1, T + 77, 0, 1), \
+    OP(T + 56, IN + 0, T + 78, 0, 1), OP(T + 57, IN + 1, T + 79, 0, 1), OP(T + 58, IN + 0, T + 80, 0, 1), \
+    OP(T + 59, IN + 1, T + 81, 0, 1), OP(T + 60, IN + 0, T + 82, 0, 1), OP(T + 61, IN + 1, T + 83, 0, 1), \
+    OP(T + 62, IN + 0, T + 84, 0, 1), OP(T + 63, IN + 1, T + 85, 0, 1), OP(T + 64, IN + 0, T + 86, 0, 1), \
+    OP(T + 65, IN + 1, T + 87, 0, 1), OP(T + 66, IN + 0, T + 88, 0, 1), OP(T + 67, IN + 1, T + 89, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 68, T + 55, T + 54, 1, 0), \
+    OP(T + 69, T + 57, T + 56, 1, 0), OP(T + 70, T + 59, T + 58, 1, 0), OP(T + 71, T + 61, T + 60, 1, 0), \
+    OP(T + 72, T + 63, T + 62, 1, 0), OP(T + 73, T + 65, T + 64, 1, 0), OP(T + 74, T + 67, T + 66, 1, 0), \
+    OP(T + 75, Y + 1, IN + 46, 1, 0), OP(T + 76, Y + 8, IN + 55, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 77, Y + 20, IN + 142, 0, 1), \
+    OP(T + 78, Y + 19, IN + 141, 0, 1), OP(T + 79, Y + 18, IN + 140, 0, 1), OP(T + 80, Y + 17, IN + 139, 0, 1), \
+    OP(T + 81, Y + 16, IN + 138, 0, 1), OP(T + 82, Y + 15, IN + 137, 0, 1), OP(T + 83, Y + 11, Y + 21, 0, 1), \
+    OP(T + 84, Y + 4, Y + 21, 0, 1), OP(T + 85, Y + 14, IN + 136, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 86, T + 77, IN + 47, 0, 1), \
+    OP(T + 87, T + 78, IN + 47, 0, 1), OP(T + 88, T + 79, IN + 47, 0, 1), OP(T + 89, T + 80, IN + 47, 0, 1), \
+    OP(T + 54, T + 81, IN + 47, 0, 1), OP(T + 55, T + 82, IN + 47, 0, 1), OP(T + 56, T + 83, T + 75, 0, 1), \
+    OP(T + 57, T + 84, T + 76, 0, 1), OP(T + 58, T + 85, IN + 47, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 59, T + 68, T + 86, 1, 0), \
+    OP(T + 60, T + 69, T + 87, 1, 0), OP(T + 61, T + 70, T + 88, 1, 0), OP(T + 62, T + 71, T + 89, 1, 0), \
+    OP(T + 63, T + 72, T + 54, 1, 0), OP(T + 64, T + 73, T + 55, 1, 0), OP(T + 65, T + 74, T + 58, 1, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 66, T + 59, T + 57, 0, 0), OP(T + 67, T + 60, T + 57, 0, 0), \
+    OP(T + 75, T + 61, T + 57, 0, 0), OP(T + 76, T + 62, T + 57, 0, 0), OP(T + 77, T + 63, T + 57, 0, 0), \
+    OP(T + 78, T + 64, T + 57, 0, 0), OP(T + 79, T + 65, T + 57, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 80, T + 66, T + 56, 0, 0), OP(T + 81, T + 67, T + 56, 0, 0), OP(T + 82, T + 75, T + 56, 0, 0), \
+    OP(T + 83, T + 76, T + 56, 0, 0), OP(T + 84, T + 77, T + 56, 0, 0), OP(T + 85, T + 78, T + 56, 0, 0), \
+    OP(T + 54, T + 79, T + 56, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 55, IN + 44, IN + 86, 0, 1), OP(T + 58, IN + 43, IN + 85, 0, 1), OP(T + 68, IN + 42, IN + 84, 0, 1), \
+    OP(T + 69, IN + 41, IN + 83, 0, 1), OP(T + 70, IN + 40, IN + 82, 0, 1), OP(T + 71, IN + 39, IN + 81, 0, 1), \
+    OP(T + 72, IN + 38, IN + 80, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 73, T + 55, IN + 56, 0, 1), OP(T + 74, T + 58, IN + 56, 0, 1), OP(T + 86, T + 68, IN + 56, 0, 1), \
+    OP(T + 87, T + 69, IN + 56, 0, 1), OP(T + 88, T + 70, IN + 56, 0, 1), OP(T + 89, T + 71, IN + 56, 0, 1), \
+    OP(T + 57, T + 72, IN + 56, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 59, T + 73, IN + 0, 0, 1), OP(T + 60, T + 74, IN + 0, 0, 1), OP(T + 61, T + 86, IN + 0, 0, 1), \
+    OP(T + 62, T + 87, IN + 0, 0, 1), OP(T + 63, T + 88, IN + 0, 0, 1), OP(T + 64, T + 89, IN + 0, 0, 1), \
+    OP(T + 65, T + 57, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 56, T + 80, T + 59, 1, 0), OP(T + 66, T + 81, T + 60, 1, 0), OP(T + 67, T + 82, T + 61, 1, 0), \
+    OP(T + 75, T + 83, T + 62, 1, 0), OP(T + 76, T + 84, T + 63, 1, 0), OP(T + 77, T + 85, T + 64, 1, 0), \
+    OP(T + 78, T + 54, T + 65, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 90, IN + 44, IN + 0, 0, 1), OP(T + 91, IN + 43, IN + 0, 0, 1), OP(T + 92, IN + 42, IN + 0, 0, 1), \
+    OP(T + 93, IN + 41, IN + 0, 0, 1), OP(T + 94, IN + 40, IN + 0, 0, 1), OP(T + 95, IN + 39, IN + 0, 0, 1), \
+    OP(T + 96, IN + 38, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 97, T + 90, IN + 62, 0, 1), OP(T + 98, T + 91, IN + 62, 0, 1), OP(T + 99, T + 92, IN + 62, 0, 1), \
+    OP(T + 100, T + 93, IN + 62, 0, 1), OP(T + 101, T + 94, IN + 62, 0, 1), OP(T + 102, T + 95, IN + 62, 0, 1), \
+    OP(T + 103, T + 96, IN + 62, 0, 1), OP(T + 104, Y + 20, IN + 53, 0, 1), OP(T + 105, Y + 19, IN + 53, 0, 1), \
+    OP(T + 106, Y + 18, IN + 53, 0, 1), OP(T + 107, Y + 17, IN + 53, 0, 1), OP(T + 108, Y + 16, IN + 53, 0, 1), \
+    OP(T + 109, Y + 15, IN + 53, 0, 1), OP(T + 110, Y + 14, IN + 53, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 90, T + 97, IN + 118, 0, 1), OP(T + 91, T + 98, IN + 117, 0, 1), \
+    OP(T + 92, T + 99, IN + 116, 0, 1), OP(T + 93, T + 100, IN + 115, 0, 1), \
+    OP(T + 94, T + 101, IN + 114, 0, 1), OP(T + 95, T + 102, IN + 113, 0, 1), \
+    OP(T + 96, T + 103, IN + 112, 0, 1), OP(T + 111, T + 104, IN + 174, 0, 1), \
+    OP(T + 112, T + 105, IN + 173, 0, 1), OP(T + 113, T + 106, IN + 172, 0, 1), \
+    OP(T + 114, T + 107, IN + 171, 0, 1), OP(T + 115, T + 108, IN + 170, 0, 1), \
+    OP(T + 116, T + 109, IN + 169, 0, 1), OP(T + 117, T + 110, IN + 168, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 97, T + 111, T + 90, 0, 0), OP(T + 98, T + 112, T + 91, 0, 0), \
+    OP(T + 99, T + 113, T + 92, 0, 0), OP(T + 100, T + 114, T + 93, 0, 0), OP(T + 101, T + 115, T + 94, 0, 0), \
+    OP(T + 102, T + 116, T + 95, 0, 0), OP(T + 103, T + 117, T + 96, 0, 0), OP(T + 104, Y + 10, Y + 12, 1, 0), \
+    OP(T + 105, Y + 3, Y + 5, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 106, Y + 21, T + 105, 0, 1), OP(T + 107, IN + 53, IN + 62, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 108, T + 106, T + 104, 0, 1), OP(T + 109, T + 107, Y + 21, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 110, T + 97, T + 108, 0, 0), \
+    OP(T + 90, T + 98, T + 108, 0, 0), OP(T + 91, T + 99, T + 108, 0, 0), OP(T + 92, T + 100, T + 108, 0, 0), \
+    OP(T + 93, T + 101, T + 108, 0, 0), OP(T + 94, T + 102, T + 108, 0, 0), OP(T + 95, T + 103, T + 108, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 96, T + 110, T + 109, 1, 0), OP(T + 111, T + 90, T + 109, 1, 0), \
+    OP(T + 112, T + 91, T + 109, 1, 0), OP(T + 113, T + 92, T + 109, 1, 0), OP(T + 114, T + 93, T + 109, 1, 0), \
+    OP(T + 115, T + 94, T + 109, 1, 0), OP(T + 116, T + 95, T + 109, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 117, IN + 174, IN + 118, 0, 1), OP(T + 105, IN + 173, IN + 117, 0, 1), \
+    OP(T + 104, IN + 172, IN + 116, 0, 1), OP(T + 106, IN + 171, IN + 115, 0, 1), \
+    OP(T + 107, IN + 170, IN + 114, 0, 1), OP(T + 97, IN + 169, IN + 113, 0, 1), \
+    OP(T + 98, IN + 168, IN + 112, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 99, T + 117, Y + 21, 0, 1), OP(T + 100, T + 105, Y + 21, 0, 1), OP(T + 101, T + 104, Y + 21, 0, 1), \
+    OP(T + 102, T + 106, Y + 21, 0, 1), OP(T + 103, T + 107, Y + 21, 0, 1), OP(T + 108, T + 97, Y + 21, 0, 1), \
+    OP(T + 90, T + 98, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
+    OP(T + 91, T + 96, T + 99, 1, 0), OP(T + 92, T + 111, T + 100, 1, 0), OP(T + 93, T + 112, T + 101, 1, 0), \
+    OP(T + 94, T + 113, T + 102, 1, 0), OP(T + 95, T + 114, T + 103, 1, 0), \
+    OP(T + 109, T + 115, T + 108, 1, 0), OP(T + 110, T + 116, T + 90, 1, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
+    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), 0, 0, \
+    0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0
+#define FRG_RESIDUAL_OUTS(OUT, T) \
+    OUT(T + 24, 0, 0, 1), OUT(T + 18, 0, 1, 1), OUT(T + 17, 0, 2, 1), OUT(T + 16, 0, 3, 1), 0xffff, 0xffff, \
+    0xffff, OUT(T + 52, 0, 4, 1), OUT(T + 51, 0, 5, 1), OUT(T + 42, 0, 6, 1), 0xffff, 0xffff, 0xffff, 0xffff, \
+    OUT(T + 78, 1, 0, 1), OUT(T + 77, 1, 1, 1), OUT(T + 76, 1, 2, 1), OUT(T + 75, 1, 3, 1), \
+    OUT(T + 67, 1, 4, 1), OUT(T + 66, 1, 5, 1), OUT(T + 56, 1, 6, 1), OUT(T + 110, 2, 0, 0), \
+    OUT(T + 109, 2, 1, 0), OUT(T + 95, 2, 2, 0), OUT(T + 94, 2, 3, 0), OUT(T + 93, 2, 4, 0), \
+    OUT(T + 92, 2, 5, 0), OUT(T + 91, 2, 6, 0)

@@ -37,6 +37,8 @@
 // on their bit patterns in the integer pipes for the same reason.
 #pragma once
 
+#include <cstddef>
+
 #include "frg_device.cuh"
 #include "frg_df.cuh"
 #include "frg_warp.cuh"
@@ -103,7 +105,7 @@ struct Smem {
   struct Inputs {
     FrgEvalIn<T> in;
     cx<T> dq[32];
-    HighEval<T, P> hi;
+    alignas(16) HighEval<T, P> hi;
   };
   static constexpr size_t kSolve = sizeof(cx<T>) * (16 * LDU + 17 * 8);
   static constexpr size_t kWork = sizeof(Inputs) > kSolve ? sizeof(Inputs) : kSolve;
@@ -111,10 +113,11 @@ struct Smem {
   cx<P> sp[32], fp[32];
   cx<P> gamma;
   LowTask<T, P> lo;
-  cx<T> Vc[VS], Vn[VS], u[VS], Ye[VS], dx[VS];
-  cx<T> k[8][VS];
+  cx<T> Vc[VS], Vn[VS], u[VS], Ye[VS];
+  alignas(16) cx<T> X[16];  // solution; X .. k are free during a corrector step's evaluation (Residual)
+  cx<T> XU[8], dx[VS], k[8][VS];
   cx<T> M[3 * 18 * 8];
-  cx<T> X[16], XU[8], R[3][8], Rd;  // solution; refined residuals and patch residual
+  cx<T> R[3][8], Rd;  // refined residuals and patch residual
   T cn[16];
   alignas(16) unsigned char work[kWork];
   int active, refine;
@@ -150,8 +153,8 @@ struct StepOut {
 // lanes 0..6, e on 8..11, q's denominator on 12); q(t) (and dq/dt, htpysupport.cu:37-62),
 // one parameter per lane, with z^2 and z^3 on lane 31 in the same products; then the
 // hoisted quantities, lanes 8 s + g those of side s and group g, lanes 16 + s those that
-// are the same for every group, again in the same instructions. RESID: frg_group_f's forms
-// (the refinement residual). 81 FP64 instructions; with each quantity in instructions of
+// are the same for every group, again in the same instructions. RESID: the forms of the
+// refinement residual. 81 FP64 instructions; with each quantity in instructions of
 // its own it was 143.
 template <bool RESID, typename V>
 __device__ __forceinline__ void eval_prep(const cx<V>* Y, const cx<V>* sp, const cx<V>* fp, cx<V> gamma,
@@ -233,6 +236,88 @@ __device__ __forceinline__ cx<P> patch_dot(const cx<T>* u, const cx<P>* Y, int n
   cx<P> d(P(0));
   for (int e = g; e < n; e += TEAM) d = cfma(cx<P>(u[e]), Y[e], d);
   return cx<P>(team_sum(mask, d.re), team_sum(mask, d.im));
+}
+
+// The corrector's refinement residual of one path (F_j at the point YN, htpysupport.cu:64-86)
+// in the point type, by the four warps of its part: warp `part` runs its generated schedule,
+// lane 2 o + c computing component c of a step's operation o, from what eval_prep<true> left
+// in the path's inputs. The temporaries take the vectors that a corrector step does not need
+// (X .. k).
+// What bounds it: the chain of operations, 200 to 250 cycles each. As straight-line code, a
+// group's three equations on a lane of three warps, it was 39 operations long in 13 % of a
+// path's steps, and of 16 paths in step nearly always one is in such a step; the schedule has
+// 17 steps (3.8k cycles). GB300, FP32 stage of 140 paths 113 -> 104 ms, of 2,400 236 -> 213, of
+// 9,600 333 -> 282; 65,536-path rounds, four in flight, 1,448 -> 1,365 ms a round.
+template <typename P>
+struct Residual {
+  typedef Smem<float, P> S;
+  static constexpr unsigned kY = offsetof(S, YN) / 16, kT = offsetof(S, X) / 16,
+                            kIn = (offsetof(S, work) + offsetof(typename S::Inputs, hi)) / 16;
+  static_assert(sizeof(cx<P>) == 16 && offsetof(S, YN) % 16 == 0 && offsetof(S, X) % 16 == 0 &&
+                offsetof(S, work) % 16 == 0 && offsetof(typename S::Inputs, hi) % 16 == 0, "16-byte units");
+  static_assert(kT + FRG_RESIDUAL_TEMPS <= (offsetof(S, k) + sizeof(S::k)) / 16, "temporaries");
+  static_assert(kIn + sizeof(FrgEvalIn<P>) / 16 <= 1024, "10-bit units");
+};
+static_assert(Residual<df>::kY == Residual<double>::kY && Residual<df>::kT == Residual<double>::kT &&
+              Residual<df>::kIn == Residual<double>::kIn, "one table for both point types");
+#define FRG_OP(r, a, b, sub, mul) (unsigned)(r) | (unsigned)(a) << 10 | (unsigned)(b) << 20 | sub##u << 30 | mul##u << 31
+#define FRG_OUT(r, eq, g, minus) (r) | (g) << 10 | (eq) << 13 | (minus) << 15
+static __device__ const unsigned residual_code[] = {FRG_RESIDUAL_CODE(FRG_OP, Residual<df>::kY, Residual<df>::kIn, Residual<df>::kT)};
+static __device__ const unsigned short residual_outs[] = {FRG_RESIDUAL_OUTS(FRG_OUT, Residual<df>::kT)};
+#undef FRG_OP
+#undef FRG_OUT
+
+// component im of a b
+__device__ __forceinline__ df mul_comp(cx<df> a, cx<df> b, bool im) {
+  return df_dot2(a.re, im ? b.im : b.re, neg_if(a.im, !im), im ? b.re : b.im, 1.f);
+}
+__device__ __forceinline__ double mul_comp(cx<double> a, cx<double> b, bool im) {
+  return fma(a.re, im ? b.im : b.re, mul_rn(neg_if(a.im, !im), im ? b.re : b.im));
+}
+__device__ __forceinline__ cx<df> load_point(const cx<df>* p) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  return cx<df>(df(v.x, v.y), df(v.z, v.w));
+}
+__device__ __forceinline__ cx<double> load_point(const cx<double>* p) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  return cx<double>(v.x, v.y);
+}
+
+__device__ __forceinline__ void put_comp(cx<df>* p, bool im, df r) {
+  reinterpret_cast<float2*>(p)[im] = make_float2(r.hi, r.lo);
+}
+__device__ __forceinline__ void put_comp(cx<double>* p, bool im, double r) { reinterpret_cast<double*>(p)[im] = r; }
+
+template <typename P>
+__device__ __forceinline__ void residual_part(Smem<float, P>& E, int part, int lane) {
+  constexpr int start[5] = FRG_RESIDUAL_START;
+  cx<P>* const base = reinterpret_cast<cx<P>*>(&E);
+  const int from = part == 0 ? start[0] : (part == 1 ? start[1] : (part == 2 ? start[2] : start[3]));
+  const int to = part == 0 ? start[1] : (part == 1 ? start[2] : (part == 2 ? start[3] : start[4]));
+  const bool im = lane & 1;
+  const unsigned* code = residual_code + from * 16 + (lane >> 1);
+  unsigned w = __ldg(code), wn = __ldg(code + 16);  // two steps ahead; two steps of padding end the list
+#pragma unroll 1
+  for (int i = from; i < to; ++i) {
+    code += 16;
+    const unsigned wm = __ldg(code + 16);
+    const cx<P> a = load_point(base + ((w >> 10) & 1023)), b = load_point(base + ((w >> 20) & 1023));
+    P r;
+    if (w >> 31) {
+      r = mul_comp(a, b, im);
+    } else {
+      r = (im ? a.im : a.re) + neg_if(im ? b.im : b.re, (w >> 30) & 1);
+    }
+    put_comp(base + (w & 1023), im, r);
+    __syncwarp();
+    w = wn;
+    wn = wm;
+  }
+  const unsigned o = lane < 7 ? residual_outs[part * 7 + lane] : 0xffffu;
+  if (o != 0xffffu) {
+    const cx<P> v = load_point(base + (o & 1023));
+    E.R[(o >> 13) & 3][(o >> 10) & 7] = cx<float>(cx<P>(neg_if(v.re, o >> 15), neg_if(v.im, o >> 15)));
+  }
 }
 
 // 1 / max(|re|, |im|) of the projective patch, its row's scale in every step

@@ -532,21 +532,15 @@ team_kernel(TrackArgs a) {
       }
       if (!paired && E.active && g < 7) eval_quarter<cx<T>>(E, quarter, g);
       if constexpr (LOWP) {
-        // the corrector's refinement residual: F_j at the point YN with q(t) in the point
-        // type (htpysupport.cu:37-48, :64-86), the right-hand side with which the FP32
-        // solves converge in double-float
+        // the corrector's refinement residual in the point type, the right-hand side with which
+        // the FP32 solves converge to its accuracy
         const long long tr0 = clock64();
-        if (E.refine) {
-          const FrgEvalIn<P>& in = E.inputs().hi.in;
-          if (quarter == 3) {
-            const cp d = patch_dot<T, P>(E.u, E.YN, NY, g, 0xffu << (lane & 24)) - cp(P(1));
-            if (g == 0) E.Rd = cx<T>(d);
-          } else if (g < 7) {
-            E.R[quarter][g] = cx<T>(quarter == 0   ? frg_residual_slice<0, P>(E.YN, in, jg)
-                                    : quarter == 1 ? frg_residual_slice<1, P>(E.YN, in, jg)
-                                                   : frg_residual_slice<2, P>(E.YN, in, jg));
-          }
+        unsigned refine = __ballot_sync(FULL, part[lane & 3].refine) & 15;
+        if (quarter == 3 && (refine >> (lane >> 3) & 1)) {
+          const cp d = patch_dot<T, P>(E.u, E.YN, NY, g, 0xffu << (lane & 24)) - cp(P(1));
+          if (g == 0) E.Rd = cx<T>(d);
         }
+        for (; refine; refine &= refine - 1) residual_part<P>(part[__ffs(refine) - 1], quarter, lane);
         if (lane == 0) S.cyc[6] += clock64() - tr0;
       }
     }

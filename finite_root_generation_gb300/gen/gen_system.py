@@ -20,6 +20,7 @@ the operation counts used for the roofline's algorithmic FLOPs per evaluation.
 """
 from __future__ import annotations
 
+import re
 import os
 
 import numpy as np
@@ -187,7 +188,7 @@ HOISTED = [
     ("eaq", True, "e2*aq0", "ec2*aq1"),
     ("w", True, "B - A + qa0 + bp0*ebd0 - cg0*eaq0", "Bc - Ac + qa1 + bp1*ebd1 - cg1*eaq1"),
 ]
-# frg_group_f's own order of the same sum
+# the equations-alone form's own order of the same sum
 RESIDUAL_FORMS = {"w": ("B + qa0 - A + bp0*ebd0 - ecg0*aq0", "Bc + qa1 - Ac + bp1*ebd1 - ecg1*aq1")}
 # Which warp evaluates which outputs: 4 parts of equal cost (492 real FMA-pipe operations
 # each, found by a local search over the outputs' closures; the whole group is 1,770).
@@ -197,7 +198,6 @@ EVAL_SLICES = [
     ["fIII", "dIII[0]", "dIII[7]", "dIII[8]", "dIII[9]", "dIII[11]", "tIII"],
     ["dI[3]", "dI[4]", "dI[7]", "dII[2]", "dII[3]", "dII[5]", "dIII[10]", "dIII[12]", "dIII[13]"],
 ]
-RESIDUAL_SLICES = [["fI"], ["fII"], ["fIII"]]
 # column of each derivative slot in the group's row: links 0..13, Z0 14, t 15, U_j 16, F 17
 ROW_COLS = {"I": [0, 2, 6, 7, 9, 13, 16, 14], "II": [1, 4, 8, 11, 16, 14], "III": list(range(14)) + [16, 14]}
 
@@ -277,8 +277,165 @@ def load_of(x, key):
     return {"z": "Y[21]", "z2": "in.z2", "z3": "in.z3", "U": "Y[13 + j]", "iU": "in.iU[j - 1]"}[x]
 
 
-def emit_slices(lines, names, repl, reduced, frepl, fred, pr):
-    found, ffound = hoisted_symbols(repl, pr), hoisted_symbols(frepl, pr, RESIDUAL_FORMS)
+def operand_of(x, key):
+    """(segment, index, 1 if one per group) of the value named x: segment 0 the point, 1 FrgEvalIn."""
+    load = load_of(x, key)
+    index = [eval(i, {"j": 1, **{f"FRG_IN_{n.upper()}": (INDEP + PERJ).index(n) - (len(INDEP) if n in PERJ else 0)
+                                 for n in INDEP + PERJ}}) for i in re.findall(r"\[(.*?)\]", load)]
+    if load.startswith("Y"):
+        return 0, index[0], int("j" in load)
+    start = {"z2": 0, "z3": 1, "e": 2, "q": 6, "iU": 38, "sa": 46, "sb": 46 + 2 * len(INDEP)}
+    name = re.match(r"in\.(\w+)", load).group(1)
+    flat = {"sa": lambda s_, k: s_ * len(INDEP) + k, "sb": lambda s_, k, g: (s_ * len(PERJ) + k) * 8 + g}
+    return 1, start[name] + flat.get(name, lambda k=0: k)(*index), int("j" in load)
+
+
+class ResidualTape:
+    """Equations of some groups as a schedule of complex operations for a warp: pairs of lanes
+    (one per real component) take one operation each, so a step is up to WIDTH products or
+    sums that do not depend on each other. Operations, operand order and association are the
+    printed code's, an operation common to several groups is done once; a minus sign travels
+    with a value's use ((-a) b = -(a b) and (-a) + b = -(a - b) round alike). A value lives in
+    a temporary until its last use; a step writes none that it reads."""
+
+    WIDTH = 16
+
+    def __init__(self, repl, reduced, found, items, products):
+        self.defs, self.found = {s_.name: d for s_, d in repl}, found
+        self.ops, self.memo = [], {}
+        for k, q in enumerate(("P0", "Pc0")):  # eval_prep's products
+            self.memo["mul", self.value(q, 0), self.value("z", 0), 0] = ("v", (1, operand_of("pz", f"pz{k}")[1]))
+        self.outs = []  # (equation, group, operation, sign)
+        for eq, g in items:
+            self.seen = {}
+            ref, sign = self.expr(reduced[eq], g)
+            self.outs.append((eq, g, ref[1], sign))
+        self.schedule(products)
+
+    def value(self, name, g):
+        seg, index, per_group = operand_of(name, self.found.get(name))
+        return "v", (seg, index + g * per_group)
+
+    def op(self, kind, x, y, sub=0):
+        key = (kind, x, y, sub)
+        if key not in self.memo:
+            self.memo[key] = ("n", len(self.ops))
+            self.ops.append(key)
+        return self.memo[key]
+
+    def expr(self, e, g):
+        if e.is_Symbol:
+            if e.name in self.found or e.name not in self.defs:
+                return self.value(e.name, g), 1
+            if e.name not in self.seen:
+                self.seen[e.name] = self.expr(self.defs[e.name], g)
+            return self.seen[e.name]
+        if isinstance(e, sp.Mul):
+            coeff, rest = e.as_coeff_Mul()
+            assert abs(coeff) == 1, e
+            parts = [self.expr(f, g) for f in sp.Mul.make_args(rest)]
+            out = parts[0]
+            for v in parts[1:]:
+                out = self.op("mul", out[0], v[0]), out[1] * v[1]
+            return out[0], out[1] * int(coeff)
+        assert isinstance(e, sp.Add), e
+        out = None
+        for t in sp.Add.make_args(e):
+            v = self.expr(t, g)
+            out = v if out is None else (self.op("add", out[0], v[0], int(out[1] != v[1])), out[1])
+        return out
+
+    def schedule(self, products):
+        """From the last step back: each step takes operations of one kind whose users are all
+        in later steps, those with the longest chain before them first. At least `products`
+        ready products go before sums: a term is then computed shortly before it is added,
+        and few temporaries are live."""
+        n = len(self.ops)
+        need = [{r[1] for r in o[1:3] if r[0] == "n"} for o in self.ops]
+        users = [{k for k in range(n) if d in need[k]} for d in range(n)]
+        depth = [0] * n
+        for k in range(n):
+            depth[k] = (3 if self.ops[k][0] == "mul" else 2) + max([depth[d] for d in need[k]], default=0)
+        done, back = set(), []
+        while len(done) < n:
+            ready = sorted((k for k in range(n) if k not in done and users[k] <= done), key=lambda k: (-depth[k], -k))
+            many = sum(self.ops[k][0] == "mul" for k in ready) >= products
+            kind = "mul" if many else self.ops[ready[0]][0]
+            pick = [k for k in ready if self.ops[k][0] == kind][:self.WIDTH]
+            back.append(pick)
+            done |= set(pick)
+        keep = {k for _, _, k, _ in self.outs}
+        free, self.where, self.steps = [], {}, []
+        self.ntemps, ran = 0, set()
+        for pick in reversed(back):
+            for k in pick:
+                if not free:
+                    free.append(self.ntemps)
+                    self.ntemps += 1
+                self.where[k] = free.pop(0)
+            self.steps.append([(self.ops[k][0] == "mul", self.ops[k][3], self.where[k],
+                                *[r[1] if r[0] == "v" else (2, self.where[r[1]]) for r in self.ops[k][1:3]])
+                               for k in pick])
+            ran |= set(pick)
+            free += sorted({self.where[d] for k in pick for d in need[k] if d not in keep and users[d] <= ran})
+
+
+# A part's four warps: equation I of the groups 1..4 and 5..7, equations II and III; the
+# least number of ready products that go before sums (18, 16, 14 and 11 steps, 118 temporaries)
+RESIDUAL_PARTS = [([(0, g) for g in range(4)], 8), ([(0, g) for g in range(4, 7)], 8),
+                  ([(1, g) for g in range(7)], 6), ([(2, g) for g in range(7)], 2)]
+
+
+def residual_system():
+    """The three equations alone: common subexpressions, equations, hoisted symbols."""
+    f_outs = [o.subs(z**3, sp.Symbol("z3")).subs(z**2, sp.Symbol("z2")) for o in (fI, fII, fIII)]
+    repl, reduced = sp.cse(f_outs, symbols=sp.numbered_symbols("y"), optimizations="basic")
+    return repl, reduced, hoisted_symbols(repl, Printer(), RESIDUAL_FORMS)
+
+
+def residual_tapes():
+    repl, reduced, found = residual_system()
+    return [ResidualTape(repl, reduced, found, items, products) for items, products in RESIDUAL_PARTS]
+
+
+def emit_residual(lines, tapes):
+    starts = [sum(len(t.steps) for t in tapes[:k]) for k in range(len(tapes) + 1)]
+    temps = [sum(t.ntemps for t in tapes[:k]) for k in range(len(tapes) + 1)]
+    seg = ["Y", "IN", "T"]
+    lines += ["",
+              "// The three equations at a point alone (their own common subexpressions) as schedules for a",
+              "// part's four warps, residual_slice in frg_team.cuh executes them. Warp k: steps START[k] ..",
+              f"// START[k + 1] of {ResidualTape.WIDTH} words OP(result, a, b, b subtracted, product), in 16-byte units from",
+              "// Y (the point), IN (FrgEvalIn) and T (temporaries; the last takes idle lanes' results), two steps",
+              "// of padding at the end; then OUT(unit, equation, group, negated), 7 per warp.",
+              f"#define FRG_RESIDUAL_TEMPS {temps[-1] + 1}",
+              f"#define FRG_RESIDUAL_START {{{', '.join(map(str, starts))}}}"]
+    words = []
+    for k, t in enumerate(tapes):
+        for step in t.steps:
+            for mul, sub, dst, a, b in step:
+                ops = [f"{seg[s_]} + {i + (temps[k] if s_ == 2 else 0)}" for s_, i in (a, b)]
+                words.append(f"OP(T + {temps[k] + dst}, {ops[0]}, {ops[1]}, {sub}, {int(mul)})")
+            words += [f"OP(T + {temps[-1]}, Y, Y, 0, {int(step[0][0])})"] * (t.WIDTH - len(step))
+    words += ["0"] * (2 * ResidualTape.WIDTH)
+    outs = []
+    for k, t in enumerate(tapes):
+        o = [f"OUT(T + {temps[k] + t.where[n]}, {eq}, {g}, {int(s_ < 0)})" for eq, g, n, s_ in t.outs]
+        outs += o + ["0xffff"] * (7 - len(o))
+    for name, items in (("CODE(OP, Y, IN, T)", words), ("OUTS(OUT, T)", outs)):
+        lines.append(f"#define FRG_RESIDUAL_{name} \\")
+        row = "   "
+        for i, w in enumerate(items):
+            w += "," if i + 1 < len(items) else ""
+            if len(row) + len(w) > 110:
+                lines.append(row + " \\")
+                row = "   "
+            row += " " + w
+        lines.append(row)
+
+
+def emit_slices(lines, names, repl, reduced, pr):
+    found = hoisted_symbols(repl, pr)
     by, slot = {}, {"I": 0, "II": 0, "III": 0}
     row = {"I": 0, "II": 1, "III": 2}
     for (kind, fam, v), e in zip(names, reduced):
@@ -312,16 +469,8 @@ def emit_slices(lines, names, repl, reduced, frepl, fred, pr):
         wanted = [(by[n][0], f"cx_put(M + {(by[n][1] * 18 + by[n][2]) * 8} + g, {{}});") for n in outs]
         lines += slice_lines(repl, wanted, found, load_of, pr)
         lines.append("  }")
-    lines += ["}", "",
-              "// One of the three equations at the point Y (frg_group_f's operations in its order).",
-              "template <int SLICE, typename T>",
-              "__device__ __forceinline__ cx<T> frg_residual_slice(const cx<T>* Y, const FrgEvalIn<T>& in, int j) {",
-              "  typedef cx<T> CX;"]
-    for k in range(3):
-        lines.append(f"  if constexpr (SLICE == {k}) {{")
-        lines += slice_lines(frepl, [(fred[k], "return {};")], ffound, load_of, pr)
-        lines.append("  }")
-    lines += ["}"]
+    lines.append("}")
+    emit_residual(lines, residual_tapes())
 
 
 def main():
@@ -389,31 +538,11 @@ def main():
             lines.append(f"  o.d{fam}[{slot[fam]}] = {pr.expr(e)};")
             slot[fam] += 1
     lines.append("}")
-    # ---- F only (the three equations), for FP64 residuals next to FP32 Jacobians
-    f_outs = [fI, fII, fIII]
-    f_outs = [o.subs(z**3, shared_syms["z3"]).subs(z**2, shared_syms["z2"]) for o in f_outs]
-    frepl, fred = sp.cse(f_outs, symbols=sp.numbered_symbols("y"), optimizations="basic")
+    # ---- F only (the three equations), for the residuals next to FP32 Jacobians
+    frepl, fred, _ = residual_system()
     fcm, fca, fsm = count_ops([r for _, r in frepl] + fred)
-    lines.append("")
-    lines.append(f"// The three equations alone: {fcm} complex mul, {fca} complex add/sub, {fsm} real x complex.")
-    lines.append(f"#define FRG_GENF_CMUL {fcm}")
-    lines.append(f"#define FRG_GENF_CADD {fca}")
-    lines.append("template <typename T>")
-    lines.append("__device__ __forceinline__ void frg_group_f(")
-    lines.append("    const cx<T> A, const cx<T> B, const cx<T> C, const cx<T> D, const cx<T> F, const cx<T> G,")
-    lines.append("    const cx<T> H, const cx<T> Ac, const cx<T> Bc, const cx<T> Cc, const cx<T> Dc, const cx<T> Fc,")
-    lines.append("    const cx<T> Gc, const cx<T> Hc, const cx<T> z,")
-    lines.append("    const cx<T> e1, const cx<T> e2, const cx<T> ec1, const cx<T> ec2,")
-    lines.append("    const cx<T> z2, const cx<T> z3, const cx<T> P0, const cx<T> Pc0,")
-    lines.append("    const cx<T> U, const cx<T> iU, const cx<T> Pj, const cx<T> Pcj, const cx<T> Qj, const cx<T> Qcj,")
-    lines.append("    cx<T>& fI, cx<T>& fII, cx<T>& fIII) {")
-    for s_, e in frepl:
-        lines.append(f"  const cx<T> {s_} = {pr.expr(e)};")
-    lines.append(f"  fI = {pr.expr(fred[0])};")
-    lines.append(f"  fII = {pr.expr(fred[1])};")
-    lines.append(f"  fIII = {pr.expr(fred[2])};")
-    lines.append("}")
-    emit_slices(lines, names, repl, reduced, frepl, fred, pr)
+    lines.insert(8, f"// The three equations alone: {fcm} complex mul, {fca} complex add/sub, {fsm} real x complex.")
+    emit_slices(lines, names, repl, reduced, pr)
     used = set()
     for _, e in repl:
         used |= {s.name for s in e.free_symbols}
