@@ -8,8 +8,9 @@
 // schedule (16 independent complex operations a step, one lane per real component: 29
 // FP64 instructions where the straight-line code has 834), the parameters q(t) take one
 // lane each, the elimination a lane per row and column class, the back substitution a
-// lane per real component. GB300, thread / warp: 64 burmester5 paths FP64 135 / 18 ms, 64
-// conic2 paths 16.2 / 3.3 ms, mixed 4.8 / 1.3 ms; a 3,000-step path 2,250 / 460 ms.
+// lane per real component. GB300, thread / warp: 64 burmester5 paths FP64 135 / 14.5 ms, 64
+// conic2 paths 16.2 / 2.9 ms, mixed 4.8 / 0.97 ms. A step: FP64 31k cycles (conic2 19k), of
+// which the elimination is a third and each FP64 instruction some 75; FP32 8.0k (5.1k).
 //
 // Sums of products in the stage combinations and the error's squares are rounded as
 // track_kernel's compiled form rounds them (product, then sum; re * re fused onto im * im),
@@ -35,10 +36,8 @@ struct WarpPath {
   cx<T> sp[NP], fp[NP];
   cx<T> reg[S::TAPE_REGS];
   cx<T> M[NY * LD];
-  cx<T> ip[NY];
   T t;
   T cn[NY];
-  int row[NY];
 };
 
 template <typename T>
@@ -100,9 +99,11 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
   }
   __syncwarp();
   // ---- the rows: lane 2 o + c computes component c of the step's operation o
+  uint32_t wn = tape[lane >> 1];  // the next step's, loaded ahead
 #pragma unroll 1
   for (int st = 0; st < S::TAPE_STEPS; ++st) {
-    const uint32_t w = tape[st * 16 + (lane >> 1)];
+    const uint32_t w = wn;
+    wn = tape[(st + 1 < S::TAPE_STEPS ? st + 1 : 0) * 16 + (lane >> 1)];
     const cx<T> a = W.reg[(w >> 10) & 1023], b = W.reg[(w >> 20) & 1023];
     T r;
     if (w >> 31) {
@@ -149,32 +150,48 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
     }
   }
   __syncwarp();
-  // ---- row scaling by 1/max(|re|,|im|) (htpysupport.cu:259-277, :446-471); b = -F
+  // ---- row scaling by 1/max(|re|,|im|) (htpysupport.cu:259-277, :446-471); b = -F. From
+  //      here the elimination keeps row r's columns cl, cl + CL, ... in registers; in shared
+  //      memory, with a load and a store per pivot on the chain, a burmester5 step was 11.4k
+  //      cycles in FP32 and 32.0k in FP64, with it 8.3k and 30.7k (64 paths mixed: 2.5 -> 1.75
+  //      and 3.3 -> 3.1 ms)
   const int r = lane % RP, cl = lane / RP;
+  constexpr int KC = (NY + CL) / CL;  // a lane's columns of NY + 1
+  cx<T> m[KC];
   {
-    MaxAbs<T> m;
-    if (r < NZ)
-      for (int c = cl; c < NY; c += CL) m.take(W.M[r * LD + c]);
+    MaxAbs<T> mx;
 #pragma unroll
-    for (int off = RP; off < 32; off <<= 1) m.across(off);
-    const T s = T(1) / m.value();
-    if (r < NZ)
-      for (int c = cl; c < (newton ? NY + 1 : NY); c += CL) {
-        const cx<T> v = s * W.M[r * LD + c];
-        W.M[r * LD + c] = cx<T>(neg_if(v.re, c == NY), neg_if(v.im, c == NY));
+    for (int k = 0; k < KC; ++k) {
+      const int c = cl + k * CL;
+      m[k] = c <= NY ? W.M[(r < NY ? r : 0) * LD + c] : cx<T>(T(0));
+      if (c < NY) mx.take(m[k]);
+    }
+#pragma unroll
+    for (int off = RP; off < 32; off <<= 1) mx.across(off);
+    const T s = T(1) / mx.value();
+#pragma unroll
+    for (int k = 0; k < KC; ++k) {
+      const int c = cl + k * CL;
+      if (r < NZ && (c < NY || newton)) {
+        const cx<T> v = s * m[k];
+        m[k] = cx<T>(neg_if(v.re, c == NY), neg_if(v.im, c == NY));
       }
+    }
   }
-  __syncwarp();
   // ---- elimination (htpysupport.cu:146-232; the corrector leaves the last row out,
   //      :302-400)
   const int nelim = newton ? NZ : NY;
   int pos = r;  // current position of row r
   T pmax = T(0), pmin = T(-1);
-#pragma unroll 1
-  for (int i = 0; i < nelim; ++i) {
-    const cx<T> e = W.M[(r < NY ? r : 0) * LD + i];
+  cx<T> ips[NY];
+#pragma unroll
+  for (int i = 0; i < NY; ++i) {
+    if (i >= nelim) continue;  // the last row of a corrector step
+    const cx<T> e = warp_shfl(m[i / CL], r + RP * (i % CL));
     const bool live = r < NY && pos >= i && pos < nelim;
     const T v = cnorm2(e);
+    cx<T> ip;
+    if constexpr (sizeof(T) == 4) ip = cinv_norm(e, v);  // every candidate's, while the search runs
     int pr = -1;
     {
       // rows with a magnitude above zero, not NaN, compared as integers
@@ -209,45 +226,59 @@ __device__ __forceinline__ WarpStep<T> warp_step(WarpPath<T, S>& W, const uint32
     const int ppos = __shfl_sync(FULL, pos, pr);
     if (r == pr) pos = i;
     else if (pos == i) pos = ppos;
-    const cx<T> pe = W.M[pr * LD + i];
     const T pa = __shfl_sync(FULL, v, pr);
-    const cx<T> ip = cinv_norm(pe, pa);
-    if (lane == 0) { W.ip[i] = ip; W.row[i] = pr; }
+    if constexpr (sizeof(T) == 4) ip = warp_shfl(ip, pr);
+    else ip = cinv_norm(warp_shfl(e, pr), pa);
+    ips[i] = ip;
     if (LO) {
       const T a = sqrt(pa);
       pmax = fmax(pmax, a);
       pmin = (pmin < T(0)) ? a : fmin(pmin, a);
     }
-    if (r < NY && pos > i && pos < nelim) {
-      const cx<T> l = e * ip;
-#pragma unroll 2
-      for (int c = i + 1 + cl; c <= NY; c += CL) W.M[r * LD + c] = cfms(W.M[r * LD + c], W.M[pr * LD + c], l);
+    cx<T> l;
+    if constexpr (sizeof(T) == 8 && CL > 1) {
+      // the two components on neighbouring column classes
+      const T own = mul_component(e, ip, cl & 1), other = __shfl_xor_sync(FULL, own, RP);
+      l = cl & 1 ? cx<T>(other, own) : cx<T>(own, other);
+    } else {
+      l = e * ip;
     }
-    __syncwarp();
+    const bool below = r < NY && pos > i && pos < nelim;
+#pragma unroll
+    for (int k = (i + 1) / CL; k < KC; ++k) {
+      const cx<T> pv = warp_shfl(m[k], pr + RP * cl);
+      if (below && cl + k * CL > i) m[k] = cfms(m[k], pv, l);
+    }
   }
   if (LO) out.ratio = pmin > T(0) ? pmax / pmin : T(1e30);
-  // ---- back substitution, row by row, one lane per component
-  int top = NY - 1;
-  if (newton) {
-    if (lane == 0) W.x[NY - 1] = cx<T>(tgoal - W.t);
-    top = NY - 2;
-    __syncwarp();
+  // the factor's rows by position, right-hand side in column NY
+  __syncwarp();
+  if (r < NY) {
+#pragma unroll
+    for (int k = 0; k < KC; ++k)
+      if (cl + k * CL <= NY) W.M[pos * LD + cl + k * CL] = m[k];
   }
-#pragma unroll 1
-  for (int i = top; i >= 0; --i) {
-    const cx<T>* m = W.M + W.row[i] * LD;
-    T sum = T(0);
-#pragma unroll 2
-    for (int c = i + 1; c < NY; ++c) {
-      const cx<T> b = m[c], xc = W.x[c];
-      sum = fma_component(b, xc, sum, im);
+  __syncwarp();
+  // ---- back substitution, row by row, one lane per component, the solution in registers
+  cx<T> x[NY];
+#pragma unroll
+  for (int i = NY - 1; i >= 0; --i) {
+    if (i == NY - 1 && newton) {
+      x[i] = cx<T>(tgoal - W.t);
+      if (lane == 0) W.x[i] = x[i];
+      continue;
     }
-    const T d = (im ? m[NY].im : m[NY].re) - sum, o = __shfl_xor_sync(FULL, d, 1);
-    const cx<T> ip = W.ip[i], v = im ? cx<T>(o, d) : cx<T>(d, o);
-    const T xi = mul_component(ip, v, im);
-    if (lane < 2) reinterpret_cast<T*>(&W.x[i])[im] = xi;
-    __syncwarp();
+    const cx<T>* mi = W.M + i * LD;
+    T sum = T(0);
+#pragma unroll
+    for (int c = i + 1; c < NY; ++c) sum = fma_component(mi[c], x[c], sum, im);
+    const T d = (im ? mi[NY].im : mi[NY].re) - sum, o = __shfl_xor_sync(FULL, d, 1);
+    const cx<T> v = im ? cx<T>(o, d) : cx<T>(d, o);
+    const T xi = mul_component(ips[i], v, im), xo = __shfl_xor_sync(FULL, xi, 1);
+    x[i] = im ? cx<T>(xo, xi) : cx<T>(xi, xo);
+    if (lane == 0) W.x[i] = x[i];
   }
+  __syncwarp();
   // ---- |x|, and the tangent's normalisation (htpysupport.cu:285-296)
   const cx<T> xe = W.x[lane < NY ? lane : 0];
   if (lane < NY) W.cn[lane] = cnorm2(xe);
@@ -361,8 +392,15 @@ __global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
       } else if (phase == PH_RK) {
         patch = W.k[stage - 1];
         const T ws = lane < stage ? Dp<T>::a(stage)[lane] * s : T(0);
-        cx<T> acc = mul_rn(__shfl_sync(FULL, ws, stage - 1), W.k[stage - 1][el ? lane : 0]);
-        for (int l = stage - 2; l >= 0; --l) acc = mul_rn(__shfl_sync(FULL, ws, l), W.k[l][el ? lane : 0]) + acc;
+        cx<T> acc(T(0));
+#pragma unroll
+        for (int l = 6; l >= 0; --l) {
+          const T wl = __shfl_sync(FULL, ws, l);
+          if (l < stage) {
+            const cx<T> term = mul_rn(wl, W.k[l][el ? lane : 0]);
+            acc = l == stage - 1 ? term : term + acc;
+          }
+        }
         y = W.Yc[el ? lane : 0] + acc;
       } else {
         y = W.YN[el ? lane : 0];
