@@ -367,15 +367,6 @@ __device__ __forceinline__ unsigned pivot_lane(double v, int base, int r) {
   return c & (0u - c);
 }
 
-// 1 / b by Smith's form with the larger part selected instead of branched on (cinv's
-// operations)
-__device__ __forceinline__ cx<float> cinv_select(cx<float> b) {
-  const bool big = tabs(b.re) >= tabs(b.im);
-  const float p = big ? b.re : b.im, q = big ? b.im : b.re;
-  const float r = q / p, id = 1.0f / fmaf(q, r, p), o = __fmul_rn(r, id);
-  return cx<float>(big ? id : o, big ? -o : -id);
-}
-
 // a * b where lanes that differ in `bit` hold the same operands: in FP64 each computes one
 // component (the same operations as the complex product's) and they exchange
 __device__ __forceinline__ cx<float> mul_split(cx<float> a, cx<float> b, int, int) { return a * b; }
@@ -406,7 +397,7 @@ __device__ __forceinline__ void lu_stage(cx<T>* U, T* pn, cx<T>* pv, int k0, int
     const cx<T> e = warp_shfl(R[0], base + r);  // this row's entry in column k
     // FP32: every candidate's reciprocal is taken while the pivot is searched for
     cx<T> ip = R[0];
-    if constexpr (sizeof(T) == 4) ip = cinv_select(cand ? R[0] : cx<T>(T(1)));
+    if constexpr (sizeof(T) == 4) ip = cinv(cand ? R[0] : cx<T>(T(1)));
     const unsigned pl = pivot_lane<RP>(v, base, r);
     cx<T>* Uk = U + k * LDU + k + 1 + ((h - (k + 1)) & (CL - 1));
     cx<T> X[W], pivot[W];
@@ -508,10 +499,10 @@ __device__ __forceinline__ void back_substitute(const cx<float>* U, cx<float>* X
   const cx<float> ip = U[r * LDU + r];
 #pragma unroll 4
   for (int k = 15; k >= 0; --k) {
-    const cx<float> xk = warp_shfl(rb * ip, k);
-    if (lane == 0) X[k] = xk;
-    if (r < k) rb = cfms(rb, U[r * LDU + k], xk);
+    const cx<float> xk = warp_shfl(rb * ip, k), next = cfms(rb, U[r * LDU + k], xk);
+    if (r < k) rb = next;
   }
+  if (lane < 16) X[lane] = rb * ip;
 }
 // FP64: lanes 0..15 hold the real parts, lanes 16..31 the imaginary parts, which halves
 // the FP64 instructions of the chain (4 per column; the operations and their order are
@@ -522,6 +513,7 @@ __device__ __forceinline__ void back_substitute(const cx<double>* U, cx<double>*
   double rb = im ? U[r * LDU + 16].im : U[r * LDU + 16].re;
   const cx<double> ip = U[r * LDU + r];
   const double pa = im ? ip.im : ip.re, pb = im ? ip.re : neg_if(ip.im, true);
+  double x = 0.0;
 #pragma unroll 1
   for (int k = 15; k >= 0; --k) {
     const cx<double> u = U[r * LDU + k];
@@ -529,9 +521,10 @@ __device__ __forceinline__ void back_substitute(const cx<double>* U, cx<double>*
     const double are = im ? ot : rb, aim = im ? rb : ot;
     const double m = fma(are, pa, __dmul_rn(aim, pb));
     const double xr = __shfl_sync(FULL, m, k), xi = __shfl_sync(FULL, m, 16 + k);
-    if (lane == 0) X[k] = cx<double>(xr, xi);
+    if (k == r) x = m;  // row k's right-hand side is final
     if (r < k) rb = fma(neg_if(u.im, im), im ? xr : xi, fma(-u.re, im ? xi : xr, rb));
   }
+  reinterpret_cast<double*>(&X[r])[im] = x;
 }
 
 // U_j from the group's pivot row, lane g of each group of 8 (every such lane returns it)
