@@ -649,301 +649,359 @@ __device__ __forceinline__ void frg_eval_slice(const cx<T>* Y, const FrgEvalIn<T
 }
 
 // The three equations at a point alone (their own common subexpressions) as schedules for a
-// part's four warps, residual_slice in frg_team.cuh executes them. Warp k: steps START[k] ..
-// START[k + 1] of 16 words OP(result, a, b, b subtracted, product), in 16-byte units from
-// Y (the point), IN (FrgEvalIn) and T (temporaries; the last takes idle lanes' results), two steps
-// of padding at the end; then OUT(unit, equation, group, negated), 7 per warp.
-#define FRG_RESIDUAL_TEMPS 119
-#define FRG_RESIDUAL_START {0, 17, 33, 47, 58}
+// part's four warps, residual_part in frg_team.cuh executes them. Warp k: steps START[k] ..
+// START[k + 1] of 16 words OP(result, a, b, b subtracted, product), values by
+// number in Y (the point), IN (FrgEvalIn) and T (temporaries; the last takes idle lanes' results), two steps
+// of padding at the end; then OUT(value, equation, group, negated), 7 per warp.
+#define FRG_RESIDUAL_TEMPS 208
+#define FRG_RESIDUAL_START {0, 17, 34, 51, 64}
 #define FRG_RESIDUAL_CODE(OP, Y, IN, T) \
-    OP(T + 0, Y + 7, IN + 123, 1, 0), OP(T + 1, Y + 7, IN + 122, 1, 0), OP(T + 2, Y + 7, IN + 121, 1, 0), \
-    OP(T + 3, Y + 7, IN + 120, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 4, IN + 18, IN + 10, 0, 1), \
-    OP(T + 5, IN + 17, IN + 9, 0, 1), OP(T + 6, IN + 16, IN + 8, 0, 1), OP(T + 7, Y + 0, Y + 21, 0, 1), \
-    OP(T + 8, IN + 15, IN + 7, 0, 1), OP(T + 9, IN + 6, IN + 14, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 10, T + 9, T + 4, 0, 0), OP(T + 11, T + 9, T + 5, 0, 0), \
-    OP(T + 12, T + 9, T + 6, 0, 0), OP(T + 13, T + 9, T + 8, 0, 0), OP(T + 14, Y + 9, T + 0, 1, 0), \
-    OP(T + 15, Y + 9, T + 1, 1, 0), OP(T + 16, Y + 9, T + 2, 1, 0), OP(T + 17, Y + 9, T + 3, 1, 0), \
-    OP(T + 18, Y + 0, IN + 67, 1, 0), OP(T + 19, Y + 0, IN + 66, 1, 0), OP(T + 20, Y + 0, IN + 65, 1, 0), \
-    OP(T + 21, Y + 0, IN + 64, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 4, IN + 1, T + 10, 0, 1), \
-    OP(T + 5, IN + 1, T + 11, 0, 1), OP(T + 6, IN + 1, T + 12, 0, 1), OP(T + 8, IN + 1, T + 13, 0, 1), \
-    OP(T + 9, T + 7, T + 14, 0, 1), OP(T + 22, T + 7, T + 15, 0, 1), OP(T + 23, T + 7, T + 16, 0, 1), \
-    OP(T + 24, T + 7, T + 17, 0, 1), OP(T + 25, Y + 7, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 7, T + 4, T + 9, 1, 0), \
-    OP(T + 10, T + 5, T + 22, 1, 0), OP(T + 11, T + 6, T + 23, 1, 0), OP(T + 12, T + 8, T + 24, 1, 0), \
-    OP(T + 13, Y + 2, T + 18, 1, 0), OP(T + 14, Y + 2, T + 19, 1, 0), OP(T + 15, Y + 2, T + 20, 1, 0), \
-    OP(T + 16, Y + 2, T + 21, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 17, T + 25, T + 13, 0, 1), OP(T + 4, T + 25, T + 14, 0, 1), \
-    OP(T + 5, T + 25, T + 15, 0, 1), OP(T + 6, T + 25, T + 16, 0, 1), OP(T + 8, Y + 17, IN + 48, 0, 1), \
-    OP(T + 9, Y + 16, IN + 48, 0, 1), OP(T + 22, Y + 15, IN + 48, 0, 1), OP(T + 23, Y + 14, IN + 48, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 24, T + 7, T + 17, 1, 0), OP(T + 13, T + 10, T + 4, 1, 0), OP(T + 14, T + 11, T + 5, 1, 0), \
-    OP(T + 15, T + 12, T + 6, 1, 0), OP(T + 16, IN + 147, T + 0, 1, 0), OP(T + 25, IN + 146, T + 1, 1, 0), \
-    OP(T + 26, IN + 145, T + 2, 1, 0), OP(T + 27, IN + 144, T + 3, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 0, T + 8, T + 16, 0, 1), \
-    OP(T + 1, T + 9, T + 25, 0, 1), OP(T + 2, T + 22, T + 26, 0, 1), OP(T + 3, T + 23, T + 27, 0, 1), \
-    OP(T + 4, IN + 75, IN + 147, 0, 1), OP(T + 5, IN + 74, IN + 146, 0, 1), OP(T + 6, IN + 73, IN + 145, 0, 1), \
-    OP(T + 7, IN + 72, IN + 144, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 10, T + 24, T + 0, 0, 0), \
-    OP(T + 11, T + 13, T + 1, 0, 0), OP(T + 12, T + 14, T + 2, 0, 0), OP(T + 17, T + 15, T + 3, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 8, T + 4, Y + 21, 0, 1), OP(T + 9, T + 5, Y + 21, 0, 1), OP(T + 16, T + 6, Y + 21, 0, 1), \
-    OP(T + 22, T + 7, Y + 21, 0, 1), OP(T + 23, IN + 41, IN + 0, 0, 1), OP(T + 25, IN + 40, IN + 0, 0, 1), \
-    OP(T + 26, IN + 39, IN + 0, 0, 1), OP(T + 27, IN + 38, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 0, T + 10, T + 8, 1, 0), \
-    OP(T + 1, T + 11, T + 9, 1, 0), OP(T + 2, T + 12, T + 16, 1, 0), OP(T + 3, T + 17, T + 22, 1, 0), \
-    OP(T + 13, IN + 91, T + 18, 1, 0), OP(T + 14, IN + 90, T + 19, 1, 0), OP(T + 15, IN + 89, T + 20, 1, 0), \
-    OP(T + 24, IN + 88, T + 21, 1, 0), OP(T + 4, Y + 2, IN + 46, 1, 0), OP(T + 5, Y + 9, IN + 55, 1, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 6, IN + 57, T + 23, 0, 1), \
-    OP(T + 7, IN + 57, T + 25, 0, 1), OP(T + 8, IN + 57, T + 26, 0, 1), OP(T + 9, IN + 57, T + 27, 0, 1), \
-    OP(T + 10, IN + 131, IN + 91, 0, 1), OP(T + 11, IN + 130, IN + 90, 0, 1), \
-    OP(T + 12, IN + 129, IN + 89, 0, 1), OP(T + 16, Y + 13, Y + 21, 0, 1), OP(T + 17, Y + 6, Y + 21, 0, 1), \
-    OP(T + 18, IN + 128, IN + 88, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 19, T + 6, T + 13, 0, 1), OP(T + 20, T + 7, T + 14, 0, 1), OP(T + 21, T + 8, T + 15, 0, 1), \
-    OP(T + 22, T + 9, T + 24, 0, 1), OP(T + 23, T + 10, Y + 21, 0, 1), OP(T + 25, T + 11, Y + 21, 0, 1), \
-    OP(T + 26, T + 12, Y + 21, 0, 1), OP(T + 27, T + 16, T + 4, 0, 1), OP(T + 28, T + 17, T + 5, 0, 1), \
-    OP(T + 29, T + 18, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 4, T + 0, T + 23, 1, 0), OP(T + 5, T + 1, T + 25, 1, 0), OP(T + 6, T + 2, T + 26, 1, 0), \
-    OP(T + 7, T + 3, T + 29, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 8, T + 4, T + 19, 0, 0), OP(T + 9, T + 5, T + 20, 0, 0), \
-    OP(T + 10, T + 6, T + 21, 0, 0), OP(T + 11, T + 7, T + 22, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 12, T + 8, T + 28, 0, 0), \
-    OP(T + 13, T + 9, T + 28, 0, 0), OP(T + 14, T + 10, T + 28, 0, 0), OP(T + 15, T + 11, T + 28, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 16, T + 12, T + 27, 0, 0), OP(T + 17, T + 13, T + 27, 0, 0), OP(T + 18, T + 14, T + 27, 0, 0), \
-    OP(T + 24, T + 15, T + 27, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 30, Y + 7, IN + 126, 1, 0), \
-    OP(T + 31, Y + 7, IN + 125, 1, 0), OP(T + 32, Y + 7, IN + 124, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 33, IN + 21, IN + 13, 0, 1), OP(T + 34, IN + 20, IN + 12, 0, 1), OP(T + 35, Y + 0, Y + 21, 0, 1), \
-    OP(T + 36, IN + 19, IN + 11, 0, 1), OP(T + 37, IN + 6, IN + 14, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 38, T + 37, T + 33, 0, 0), \
-    OP(T + 39, T + 37, T + 34, 0, 0), OP(T + 40, T + 37, T + 36, 0, 0), OP(T + 41, Y + 9, T + 30, 1, 0), \
-    OP(T + 42, Y + 9, T + 31, 1, 0), OP(T + 43, Y + 9, T + 32, 1, 0), OP(T + 44, Y + 0, IN + 70, 1, 0), \
-    OP(T + 45, Y + 0, IN + 69, 1, 0), OP(T + 46, Y + 0, IN + 68, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 33, IN + 1, T + 38, 0, 1), \
-    OP(T + 34, IN + 1, T + 39, 0, 1), OP(T + 36, IN + 1, T + 40, 0, 1), OP(T + 37, T + 35, T + 41, 0, 1), \
-    OP(T + 47, T + 35, T + 42, 0, 1), OP(T + 48, T + 35, T + 43, 0, 1), OP(T + 49, Y + 7, Y + 21, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 35, T + 33, T + 37, 1, 0), OP(T + 38, T + 34, T + 47, 1, 0), \
-    OP(T + 39, T + 36, T + 48, 1, 0), OP(T + 40, Y + 2, T + 44, 1, 0), OP(T + 41, Y + 2, T + 45, 1, 0), \
-    OP(T + 42, Y + 2, T + 46, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 43, T + 49, T + 40, 0, 1), OP(T + 33, T + 49, T + 41, 0, 1), OP(T + 34, T + 49, T + 42, 0, 1), \
-    OP(T + 36, IN + 78, IN + 150, 0, 1), OP(T + 37, Y + 20, IN + 48, 0, 1), \
-    OP(T + 47, IN + 77, IN + 149, 0, 1), OP(T + 48, Y + 19, IN + 48, 0, 1), \
-    OP(T + 50, IN + 76, IN + 148, 0, 1), OP(T + 51, Y + 18, IN + 48, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 40, T + 35, T + 43, 1, 0), \
-    OP(T + 41, T + 38, T + 33, 1, 0), OP(T + 42, T + 39, T + 34, 1, 0), OP(T + 49, IN + 150, T + 30, 1, 0), \
-    OP(T + 52, IN + 149, T + 31, 1, 0), OP(T + 53, IN + 148, T + 32, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 30, T + 37, T + 49, 0, 1), OP(T + 31, T + 48, T + 52, 0, 1), \
-    OP(T + 32, T + 51, T + 53, 0, 1), OP(T + 33, T + 36, Y + 21, 0, 1), OP(T + 34, T + 47, Y + 21, 0, 1), \
-    OP(T + 35, T + 50, Y + 21, 0, 1), OP(T + 38, IN + 44, IN + 0, 0, 1), OP(T + 39, IN + 43, IN + 0, 0, 1), \
-    OP(T + 43, IN + 42, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 36, T + 40, T + 30, 0, 0), OP(T + 37, T + 41, T + 31, 0, 0), \
-    OP(T + 47, T + 42, T + 32, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 48, T + 36, T + 33, 1, 0), OP(T + 49, T + 37, T + 34, 1, 0), OP(T + 50, T + 47, T + 35, 1, 0), \
-    OP(T + 51, IN + 94, T + 44, 1, 0), OP(T + 52, IN + 93, T + 45, 1, 0), OP(T + 53, IN + 92, T + 46, 1, 0), \
-    OP(T + 30, Y + 2, IN + 46, 1, 0), OP(T + 31, Y + 9, IN + 55, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 32, IN + 57, T + 38, 0, 1), OP(T + 40, IN + 57, T + 39, 0, 1), OP(T + 41, IN + 57, T + 43, 0, 1), \
-    OP(T + 42, IN + 134, IN + 94, 0, 1), OP(T + 33, IN + 133, IN + 93, 0, 1), OP(T + 34, Y + 13, Y + 21, 0, 1), \
-    OP(T + 35, Y + 6, Y + 21, 0, 1), OP(T + 36, IN + 132, IN + 92, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 37, T + 32, T + 51, 0, 1), OP(T + 44, T + 40, T + 52, 0, 1), OP(T + 45, T + 41, T + 53, 0, 1), \
-    OP(T + 46, T + 42, Y + 21, 0, 1), OP(T + 47, T + 33, Y + 21, 0, 1), OP(T + 38, T + 34, T + 30, 0, 1), \
-    OP(T + 39, T + 35, T + 31, 0, 1), OP(T + 43, T + 36, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 30, T + 48, T + 46, 1, 0), OP(T + 31, T + 49, T + 47, 1, 0), OP(T + 32, T + 50, T + 43, 1, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 33, T + 30, T + 37, 0, 0), OP(T + 34, T + 31, T + 44, 0, 0), \
-    OP(T + 35, T + 32, T + 45, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 36, T + 33, T + 39, 0, 0), OP(T + 40, T + 34, T + 39, 0, 0), OP(T + 41, T + 35, T + 39, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 42, T + 36, T + 38, 0, 0), OP(T + 51, T + 40, T + 38, 0, 0), \
-    OP(T + 52, T + 41, T + 38, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 54, Y + 1, IN + 16, 0, 1), OP(T + 55, IN + 16, IN + 8, 0, 1), OP(T + 56, Y + 8, IN + 7, 0, 1), \
-    OP(T + 57, Y + 1, IN + 15, 0, 1), OP(T + 58, IN + 15, IN + 7, 0, 1), OP(T + 59, IN + 6, IN + 14, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 60, Y + 8, IN + 13, 0, 1), \
-    OP(T + 61, Y + 1, IN + 21, 0, 1), OP(T + 62, IN + 21, IN + 13, 0, 1), OP(T + 63, Y + 8, IN + 12, 0, 1), \
-    OP(T + 64, Y + 1, IN + 20, 0, 1), OP(T + 65, IN + 20, IN + 12, 0, 1), OP(T + 66, Y + 8, IN + 11, 0, 1), \
-    OP(T + 67, Y + 1, IN + 19, 0, 1), OP(T + 68, IN + 19, IN + 11, 0, 1), OP(T + 69, Y + 8, IN + 10, 0, 1), \
-    OP(T + 70, Y + 1, IN + 18, 0, 1), OP(T + 71, IN + 18, IN + 10, 0, 1), OP(T + 72, Y + 8, IN + 9, 0, 1), \
-    OP(T + 73, Y + 1, IN + 17, 0, 1), OP(T + 74, IN + 17, IN + 9, 0, 1), OP(T + 75, Y + 8, IN + 8, 0, 1), \
-    OP(T + 76, T + 61, T + 60, 0, 0), OP(T + 77, T + 59, T + 62, 0, 0), OP(T + 78, T + 64, T + 63, 0, 0), \
-    OP(T + 79, T + 59, T + 65, 0, 0), OP(T + 80, T + 67, T + 66, 0, 0), OP(T + 81, T + 59, T + 68, 0, 0), \
-    OP(T + 82, T + 70, T + 69, 0, 0), OP(T + 83, T + 59, T + 71, 0, 0), OP(T + 84, T + 73, T + 72, 0, 0), \
-    OP(T + 85, T + 59, T + 74, 0, 0), OP(T + 86, T + 54, T + 75, 0, 0), OP(T + 87, T + 59, T + 55, 0, 0), \
-    OP(T + 88, T + 57, T + 56, 0, 0), OP(T + 89, T + 59, T + 58, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 54, IN + 0, T + 76, 0, 1), OP(T + 55, IN + 1, T + 77, 0, 1), \
-    OP(T + 56, IN + 0, T + 78, 0, 1), OP(T + 57, IN + 1, T + 79, 0, 1), OP(T + 58, IN + 0, T + 80, 0, 1), \
-    OP(T + 59, IN + 1, T + 81, 0, 1), OP(T + 60, IN + 0, T + 82, 0, 1), OP(T + 61, IN + 1, T + 83, 0, 1), \
-    OP(T + 62, IN + 0, T + 84, 0, 1), OP(T + 63, IN + 1, T + 85, 0, 1), OP(T + 64, IN + 0, T + 86, 0, 1), \
-    OP(T + 65, IN + 1, T + 87, 0, 1), OP(T + 66, IN + 0, T + 88, 0, 1), OP(T + 67, IN + 1, T + 89, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 68, T + 55, T + 54, 1, 0), \
-    OP(T + 69, T + 57, T + 56, 1, 0), OP(T + 70, T + 59, T + 58, 1, 0), OP(T + 71, T + 61, T + 60, 1, 0), \
-    OP(T + 72, T + 63, T + 62, 1, 0), OP(T + 73, T + 65, T + 64, 1, 0), OP(T + 74, T + 67, T + 66, 1, 0), \
-    OP(T + 75, Y + 1, IN + 46, 1, 0), OP(T + 76, Y + 8, IN + 55, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 77, Y + 20, IN + 142, 0, 1), \
-    OP(T + 78, Y + 19, IN + 141, 0, 1), OP(T + 79, Y + 18, IN + 140, 0, 1), OP(T + 80, Y + 17, IN + 139, 0, 1), \
-    OP(T + 81, Y + 16, IN + 138, 0, 1), OP(T + 82, Y + 15, IN + 137, 0, 1), OP(T + 83, Y + 11, Y + 21, 0, 1), \
-    OP(T + 84, Y + 4, Y + 21, 0, 1), OP(T + 85, Y + 14, IN + 136, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 86, T + 77, IN + 47, 0, 1), \
-    OP(T + 87, T + 78, IN + 47, 0, 1), OP(T + 88, T + 79, IN + 47, 0, 1), OP(T + 89, T + 80, IN + 47, 0, 1), \
-    OP(T + 54, T + 81, IN + 47, 0, 1), OP(T + 55, T + 82, IN + 47, 0, 1), OP(T + 56, T + 83, T + 75, 0, 1), \
-    OP(T + 57, T + 84, T + 76, 0, 1), OP(T + 58, T + 85, IN + 47, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 59, T + 68, T + 86, 1, 0), \
-    OP(T + 60, T + 69, T + 87, 1, 0), OP(T + 61, T + 70, T + 88, 1, 0), OP(T + 62, T + 71, T + 89, 1, 0), \
-    OP(T + 63, T + 72, T + 54, 1, 0), OP(T + 64, T + 73, T + 55, 1, 0), OP(T + 65, T + 74, T + 58, 1, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 66, T + 59, T + 57, 0, 0), OP(T + 67, T + 60, T + 57, 0, 0), \
-    OP(T + 75, T + 61, T + 57, 0, 0), OP(T + 76, T + 62, T + 57, 0, 0), OP(T + 77, T + 63, T + 57, 0, 0), \
-    OP(T + 78, T + 64, T + 57, 0, 0), OP(T + 79, T + 65, T + 57, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 80, T + 66, T + 56, 0, 0), OP(T + 81, T + 67, T + 56, 0, 0), OP(T + 82, T + 75, T + 56, 0, 0), \
-    OP(T + 83, T + 76, T + 56, 0, 0), OP(T + 84, T + 77, T + 56, 0, 0), OP(T + 85, T + 78, T + 56, 0, 0), \
-    OP(T + 54, T + 79, T + 56, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 55, IN + 44, IN + 86, 0, 1), OP(T + 58, IN + 43, IN + 85, 0, 1), OP(T + 68, IN + 42, IN + 84, 0, 1), \
-    OP(T + 69, IN + 41, IN + 83, 0, 1), OP(T + 70, IN + 40, IN + 82, 0, 1), OP(T + 71, IN + 39, IN + 81, 0, 1), \
-    OP(T + 72, IN + 38, IN + 80, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 73, T + 55, IN + 56, 0, 1), OP(T + 74, T + 58, IN + 56, 0, 1), OP(T + 86, T + 68, IN + 56, 0, 1), \
-    OP(T + 87, T + 69, IN + 56, 0, 1), OP(T + 88, T + 70, IN + 56, 0, 1), OP(T + 89, T + 71, IN + 56, 0, 1), \
-    OP(T + 57, T + 72, IN + 56, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 59, T + 73, IN + 0, 0, 1), OP(T + 60, T + 74, IN + 0, 0, 1), OP(T + 61, T + 86, IN + 0, 0, 1), \
-    OP(T + 62, T + 87, IN + 0, 0, 1), OP(T + 63, T + 88, IN + 0, 0, 1), OP(T + 64, T + 89, IN + 0, 0, 1), \
-    OP(T + 65, T + 57, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 56, T + 80, T + 59, 1, 0), OP(T + 66, T + 81, T + 60, 1, 0), OP(T + 67, T + 82, T + 61, 1, 0), \
-    OP(T + 75, T + 83, T + 62, 1, 0), OP(T + 76, T + 84, T + 63, 1, 0), OP(T + 77, T + 85, T + 64, 1, 0), \
-    OP(T + 78, T + 54, T + 65, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 90, IN + 44, IN + 0, 0, 1), OP(T + 91, IN + 43, IN + 0, 0, 1), OP(T + 92, IN + 42, IN + 0, 0, 1), \
-    OP(T + 93, IN + 41, IN + 0, 0, 1), OP(T + 94, IN + 40, IN + 0, 0, 1), OP(T + 95, IN + 39, IN + 0, 0, 1), \
-    OP(T + 96, IN + 38, IN + 0, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 97, T + 90, IN + 62, 0, 1), OP(T + 98, T + 91, IN + 62, 0, 1), OP(T + 99, T + 92, IN + 62, 0, 1), \
-    OP(T + 100, T + 93, IN + 62, 0, 1), OP(T + 101, T + 94, IN + 62, 0, 1), OP(T + 102, T + 95, IN + 62, 0, 1), \
-    OP(T + 103, T + 96, IN + 62, 0, 1), OP(T + 104, Y + 20, IN + 53, 0, 1), OP(T + 105, Y + 19, IN + 53, 0, 1), \
-    OP(T + 106, Y + 18, IN + 53, 0, 1), OP(T + 107, Y + 17, IN + 53, 0, 1), OP(T + 108, Y + 16, IN + 53, 0, 1), \
-    OP(T + 109, Y + 15, IN + 53, 0, 1), OP(T + 110, Y + 14, IN + 53, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 90, T + 97, IN + 118, 0, 1), OP(T + 91, T + 98, IN + 117, 0, 1), \
-    OP(T + 92, T + 99, IN + 116, 0, 1), OP(T + 93, T + 100, IN + 115, 0, 1), \
-    OP(T + 94, T + 101, IN + 114, 0, 1), OP(T + 95, T + 102, IN + 113, 0, 1), \
-    OP(T + 96, T + 103, IN + 112, 0, 1), OP(T + 111, T + 104, IN + 174, 0, 1), \
-    OP(T + 112, T + 105, IN + 173, 0, 1), OP(T + 113, T + 106, IN + 172, 0, 1), \
-    OP(T + 114, T + 107, IN + 171, 0, 1), OP(T + 115, T + 108, IN + 170, 0, 1), \
-    OP(T + 116, T + 109, IN + 169, 0, 1), OP(T + 117, T + 110, IN + 168, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 97, T + 111, T + 90, 0, 0), OP(T + 98, T + 112, T + 91, 0, 0), \
-    OP(T + 99, T + 113, T + 92, 0, 0), OP(T + 100, T + 114, T + 93, 0, 0), OP(T + 101, T + 115, T + 94, 0, 0), \
-    OP(T + 102, T + 116, T + 95, 0, 0), OP(T + 103, T + 117, T + 96, 0, 0), OP(T + 104, Y + 10, Y + 12, 1, 0), \
-    OP(T + 105, Y + 3, Y + 5, 1, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 106, Y + 21, T + 105, 0, 1), OP(T + 107, IN + 53, IN + 62, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 108, T + 106, T + 104, 0, 1), OP(T + 109, T + 107, Y + 21, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 110, T + 97, T + 108, 0, 0), \
-    OP(T + 90, T + 98, T + 108, 0, 0), OP(T + 91, T + 99, T + 108, 0, 0), OP(T + 92, T + 100, T + 108, 0, 0), \
-    OP(T + 93, T + 101, T + 108, 0, 0), OP(T + 94, T + 102, T + 108, 0, 0), OP(T + 95, T + 103, T + 108, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 96, T + 110, T + 109, 1, 0), OP(T + 111, T + 90, T + 109, 1, 0), \
-    OP(T + 112, T + 91, T + 109, 1, 0), OP(T + 113, T + 92, T + 109, 1, 0), OP(T + 114, T + 93, T + 109, 1, 0), \
-    OP(T + 115, T + 94, T + 109, 1, 0), OP(T + 116, T + 95, T + 109, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 117, IN + 174, IN + 118, 0, 1), OP(T + 105, IN + 173, IN + 117, 0, 1), \
-    OP(T + 104, IN + 172, IN + 116, 0, 1), OP(T + 106, IN + 171, IN + 115, 0, 1), \
-    OP(T + 107, IN + 170, IN + 114, 0, 1), OP(T + 97, IN + 169, IN + 113, 0, 1), \
-    OP(T + 98, IN + 168, IN + 112, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 99, T + 117, Y + 21, 0, 1), OP(T + 100, T + 105, Y + 21, 0, 1), OP(T + 101, T + 104, Y + 21, 0, 1), \
-    OP(T + 102, T + 106, Y + 21, 0, 1), OP(T + 103, T + 107, Y + 21, 0, 1), OP(T + 108, T + 97, Y + 21, 0, 1), \
-    OP(T + 90, T + 98, Y + 21, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), OP(T + 118, Y, Y, 0, 1), \
-    OP(T + 91, T + 96, T + 99, 1, 0), OP(T + 92, T + 111, T + 100, 1, 0), OP(T + 93, T + 112, T + 101, 1, 0), \
-    OP(T + 94, T + 113, T + 102, 1, 0), OP(T + 95, T + 114, T + 103, 1, 0), \
-    OP(T + 109, T + 115, T + 108, 1, 0), OP(T + 110, T + 116, T + 90, 1, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), \
-    OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), OP(T + 118, Y, Y, 0, 0), 0, 0, \
-    0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0
+    OP(T(0), IN(18), Y(21), 0, 1), OP(T(1), IN(17), Y(21), 0, 1), OP(T(2), IN(16), Y(21), 0, 1), \
+    OP(T(3), IN(15), Y(21), 0, 1), OP(T(4), Y(21), Y(21), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(5), Y(7), T(0), 1, 0), OP(T(6), Y(7), T(1), 1, 0), \
+    OP(T(7), Y(7), T(2), 1, 0), OP(T(8), Y(7), T(3), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(2), T(4), Y(21), 0, 1), \
+    OP(T(3), IN(10), Y(21), 0, 1), OP(T(9), IN(18), IN(10), 0, 1), OP(T(10), IN(9), Y(21), 0, 1), \
+    OP(T(11), IN(17), IN(9), 0, 1), OP(T(12), IN(8), Y(21), 0, 1), OP(T(13), IN(16), IN(8), 0, 1), \
+    OP(T(14), IN(14), Y(21), 0, 1), OP(T(15), IN(6), Y(21), 0, 1), OP(T(16), Y(7), Y(21), 0, 1), \
+    OP(T(17), IN(7), Y(21), 0, 1), OP(T(18), Y(0), Y(21), 0, 1), OP(T(19), IN(15), IN(7), 0, 1), \
+    OP(T(20), IN(6), IN(14), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(21), Y(9), T(5), 1, 0), OP(T(22), Y(9), T(6), 1, 0), OP(T(23), Y(9), T(7), 1, 0), \
+    OP(T(24), Y(9), T(8), 1, 0), OP(T(25), Y(0), T(3), 1, 0), OP(T(26), T(20), T(9), 0, 0), \
+    OP(T(27), Y(0), T(10), 1, 0), OP(T(28), T(20), T(11), 0, 0), OP(T(29), Y(0), T(12), 1, 0), \
+    OP(T(30), T(20), T(13), 0, 0), OP(T(31), Y(6), T(15), 1, 0), OP(T(32), Y(0), T(17), 1, 0), \
+    OP(T(33), T(20), T(19), 0, 0), OP(T(34), Y(7), Y(9), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(9), T(18), T(21), 0, 1), OP(T(11), T(18), T(22), 0, 1), \
+    OP(T(12), T(18), T(23), 0, 1), OP(T(13), T(18), T(24), 0, 1), OP(T(17), T(2), T(26), 0, 1), \
+    OP(T(19), T(2), T(28), 0, 1), OP(T(20), T(2), T(30), 0, 1), OP(T(35), T(2), T(33), 0, 1), \
+    OP(T(36), Y(17), T(31), 0, 1), OP(T(37), Y(16), T(31), 0, 1), OP(T(38), Y(15), T(31), 0, 1), \
+    OP(T(39), Y(14), T(31), 0, 1), OP(T(40), IN(32), T(34), 0, 1), OP(T(41), IN(31), T(34), 0, 1), \
+    OP(T(42), IN(30), T(34), 0, 1), OP(T(43), IN(29), T(34), 0, 1), OP(T(2), T(17), T(9), 1, 0), \
+    OP(T(18), T(19), T(11), 1, 0), OP(T(21), T(20), T(12), 1, 0), OP(T(22), T(35), T(13), 1, 0), \
+    OP(T(23), T(40), T(5), 1, 0), OP(T(24), Y(2), T(25), 1, 0), OP(T(26), T(41), T(6), 1, 0), \
+    OP(T(28), Y(2), T(27), 1, 0), OP(T(30), T(42), T(7), 1, 0), OP(T(31), Y(2), T(29), 1, 0), \
+    OP(T(33), T(43), T(8), 1, 0), OP(T(34), Y(2), T(32), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(9), T(36), T(23), 0, 1), OP(T(11), T(37), T(26), 0, 1), OP(T(12), T(38), T(30), 0, 1), \
+    OP(T(13), T(39), T(33), 0, 1), OP(T(20), T(16), T(24), 0, 1), OP(T(35), T(16), T(28), 0, 1), \
+    OP(T(44), T(16), T(31), 0, 1), OP(T(45), T(16), T(34), 0, 1), OP(T(46), T(25), T(40), 0, 1), \
+    OP(T(47), T(27), T(41), 0, 1), OP(T(48), T(29), T(42), 0, 1), OP(T(49), T(32), T(43), 0, 1), \
+    OP(T(50), Y(8), IN(10), 0, 1), OP(T(51), Y(1), IN(18), 0, 1), OP(T(52), Y(8), IN(9), 0, 1), \
+    OP(T(53), Y(1), IN(17), 0, 1), OP(T(16), T(2), T(20), 1, 0), OP(T(23), T(18), T(35), 1, 0), \
+    OP(T(24), T(21), T(44), 1, 0), OP(T(26), T(22), T(45), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(28), T(16), T(9), 0, 0), \
+    OP(T(30), T(23), T(11), 0, 0), OP(T(31), T(24), T(12), 0, 0), OP(T(33), T(26), T(13), 0, 0), \
+    OP(T(34), Y(1), T(3), 1, 0), OP(T(36), T(51), T(50), 0, 0), OP(T(37), Y(1), T(10), 1, 0), \
+    OP(T(38), T(53), T(52), 0, 0), OP(T(39), Y(2), T(15), 1, 0), OP(T(40), Y(9), T(14), 1, 0), \
+    OP(T(41), Y(13), T(14), 1, 0), OP(T(42), Y(0), Y(2), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(43), T(46), Y(21), 0, 1), OP(T(2), T(47), Y(21), 0, 1), OP(T(18), T(48), Y(21), 0, 1), \
+    OP(T(20), T(49), Y(21), 0, 1), OP(T(21), IN(41), T(34), 0, 1), OP(T(22), T(4), T(36), 0, 1), \
+    OP(T(35), IN(40), T(37), 0, 1), OP(T(44), T(4), T(38), 0, 1), OP(T(45), IN(41), T(4), 0, 1), \
+    OP(T(3), IN(40), T(4), 0, 1), OP(T(9), IN(39), T(4), 0, 1), OP(T(10), IN(38), T(4), 0, 1), \
+    OP(T(11), IN(25), T(42), 0, 1), OP(T(12), IN(24), T(42), 0, 1), OP(T(13), IN(23), T(42), 0, 1), \
+    OP(T(16), IN(22), T(42), 0, 1), OP(T(23), T(28), T(43), 1, 0), OP(T(24), T(30), T(2), 1, 0), \
+    OP(T(26), T(31), T(18), 1, 0), OP(T(50), T(33), T(20), 1, 0), OP(T(51), T(17), T(22), 1, 0), \
+    OP(T(52), T(19), T(44), 1, 0), OP(T(53), T(11), T(25), 1, 0), OP(T(34), T(12), T(27), 1, 0), \
+    OP(T(36), T(13), T(29), 1, 0), OP(T(37), T(16), T(32), 1, 0), OP(T(38), Y(8), T(0), 1, 0), \
+    OP(T(42), Y(11), T(14), 1, 0), OP(T(46), Y(1), T(15), 1, 0), OP(T(47), Y(8), T(14), 1, 0), \
+    OP(T(48), Y(4), T(15), 1, 0), OP(T(49), Y(8), T(1), 1, 0), OP(T(0), T(21), T(42), 0, 1), \
+    OP(T(1), T(35), T(42), 0, 1), OP(T(2), T(41), T(45), 0, 1), OP(T(14), T(41), T(3), 0, 1), \
+    OP(T(15), T(41), T(9), 0, 1), OP(T(17), T(41), T(10), 0, 1), OP(T(18), Y(17), T(38), 0, 1), \
+    OP(T(19), Y(16), T(49), 0, 1), OP(T(20), T(5), T(11), 0, 1), OP(T(22), T(6), T(12), 0, 1), \
+    OP(T(25), T(7), T(13), 0, 1), OP(T(27), T(8), T(16), 0, 1), OP(T(28), Y(11), Y(21), 0, 1), \
+    OP(T(29), Y(4), Y(21), 0, 1), OP(T(30), Y(13), Y(21), 0, 1), OP(T(31), Y(6), Y(21), 0, 1), \
+    OP(T(32), T(0), T(4), 0, 1), OP(T(33), T(1), T(4), 0, 1), OP(T(43), T(2), T(53), 0, 1), \
+    OP(T(44), T(14), T(34), 0, 1), OP(T(3), T(15), T(36), 0, 1), OP(T(5), T(17), T(37), 0, 1), \
+    OP(T(6), T(18), T(48), 0, 1), OP(T(7), T(19), T(48), 0, 1), OP(T(8), T(20), Y(21), 0, 1), \
+    OP(T(9), T(22), Y(21), 0, 1), OP(T(10), T(25), Y(21), 0, 1), OP(T(11), T(27), Y(21), 0, 1), \
+    OP(T(12), T(28), T(46), 0, 1), OP(T(13), T(29), T(47), 0, 1), OP(T(16), T(30), T(39), 0, 1), \
+    OP(T(21), T(31), T(40), 0, 1), OP(T(35), T(23), T(8), 1, 0), OP(T(38), T(24), T(9), 1, 0), \
+    OP(T(41), T(26), T(10), 1, 0), OP(T(42), T(50), T(11), 1, 0), OP(T(45), T(51), T(6), 1, 0), \
+    OP(T(49), T(52), T(7), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(0), T(35), T(43), 0, 0), \
+    OP(T(1), T(38), T(44), 0, 0), OP(T(2), T(41), T(3), 0, 0), OP(T(4), T(42), T(5), 0, 0), \
+    OP(T(14), T(45), T(13), 0, 0), OP(T(15), T(49), T(13), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(17), T(0), T(21), 0, 0), OP(T(18), T(1), T(21), 0, 0), OP(T(19), T(2), T(21), 0, 0), \
+    OP(T(20), T(4), T(21), 0, 0), OP(T(22), T(14), T(12), 0, 0), OP(T(25), T(15), T(12), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(27), T(17), T(16), 0, 0), OP(T(28), T(18), T(16), 0, 0), \
+    OP(T(29), T(19), T(16), 0, 0), OP(T(30), T(20), T(16), 0, 0), OP(T(31), T(22), T(32), 1, 0), \
+    OP(T(34), T(25), T(33), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(54), IN(13), Y(21), 0, 1), \
+    OP(T(55), IN(21), Y(21), 0, 1), OP(T(56), IN(12), Y(21), 0, 1), OP(T(57), IN(20), Y(21), 0, 1), \
+    OP(T(58), IN(11), Y(21), 0, 1), OP(T(59), IN(19), Y(21), 0, 1), OP(T(60), Y(21), Y(21), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(61), Y(0), T(54), 1, 0), OP(T(62), Y(7), T(55), 1, 0), OP(T(63), Y(0), T(56), 1, 0), \
+    OP(T(64), Y(7), T(57), 1, 0), OP(T(65), Y(0), T(58), 1, 0), OP(T(66), Y(7), T(59), 1, 0), \
+    OP(T(67), Y(0), Y(2), 1, 0), OP(T(68), Y(7), Y(9), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(54), T(60), Y(21), 0, 1), OP(T(55), IN(34), T(68), 0, 1), \
+    OP(T(69), IN(26), T(67), 0, 1), OP(T(70), IN(33), T(68), 0, 1), OP(T(71), IN(21), IN(13), 0, 1), \
+    OP(T(72), IN(20), IN(12), 0, 1), OP(T(73), IN(6), Y(21), 0, 1), OP(T(74), Y(7), Y(21), 0, 1), \
+    OP(T(75), Y(0), Y(21), 0, 1), OP(T(76), IN(19), IN(11), 0, 1), OP(T(77), IN(6), IN(14), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(78), Y(2), T(61), 1, 0), \
+    OP(T(79), Y(9), T(62), 1, 0), OP(T(80), Y(2), T(63), 1, 0), OP(T(81), Y(9), T(64), 1, 0), \
+    OP(T(82), Y(2), T(65), 1, 0), OP(T(83), Y(9), T(66), 1, 0), OP(T(84), T(77), T(71), 0, 0), \
+    OP(T(85), T(77), T(72), 0, 0), OP(T(86), Y(6), T(73), 1, 0), OP(T(87), T(77), T(76), 0, 0), \
+    OP(T(88), Y(8), Y(10), 1, 0), OP(T(89), Y(1), Y(3), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(71), T(74), T(78), 0, 1), OP(T(72), T(75), T(79), 0, 1), OP(T(76), T(74), T(80), 0, 1), \
+    OP(T(77), T(75), T(81), 0, 1), OP(T(90), T(74), T(82), 0, 1), OP(T(91), T(75), T(83), 0, 1), \
+    OP(T(92), T(54), T(84), 0, 1), OP(T(93), T(54), T(85), 0, 1), OP(T(94), T(54), T(87), 0, 1), \
+    OP(T(95), Y(20), T(86), 0, 1), OP(T(96), Y(19), T(86), 0, 1), OP(T(97), Y(18), T(86), 0, 1), \
+    OP(T(98), IN(4), T(88), 0, 1), OP(T(99), IN(2), T(89), 0, 1), OP(T(100), IN(35), T(68), 0, 1), \
+    OP(T(101), IN(27), T(67), 0, 1), OP(T(54), T(92), T(72), 1, 0), OP(T(68), T(93), T(77), 1, 0), \
+    OP(T(74), T(94), T(91), 1, 0), OP(T(75), Y(1), T(101), 0, 0), OP(T(78), Y(8), T(55), 0, 0), \
+    OP(T(79), Y(1), T(69), 0, 0), OP(T(80), Y(8), T(70), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(81), T(54), T(71), 1, 0), \
+    OP(T(82), T(68), T(76), 1, 0), OP(T(83), T(74), T(90), 1, 0), OP(T(84), T(75), Y(0), 1, 0), \
+    OP(T(85), T(78), Y(7), 1, 0), OP(T(87), T(79), Y(0), 1, 0), OP(T(88), T(80), Y(7), 1, 0), \
+    OP(T(89), T(100), T(62), 1, 0), OP(T(72), T(55), T(64), 1, 0), OP(T(77), T(70), T(66), 1, 0), \
+    OP(T(91), Y(1), T(56), 1, 0), OP(T(92), Y(8), T(57), 1, 0), OP(T(93), Y(1), T(58), 1, 0), \
+    OP(T(94), Y(8), T(59), 1, 0), OP(T(102), Y(9), Y(12), 1, 0), OP(T(103), Y(2), Y(5), 1, 0), \
+    OP(T(54), T(95), T(89), 0, 1), OP(T(56), T(96), T(72), 0, 1), OP(T(57), T(97), T(77), 0, 1), \
+    OP(T(58), T(91), T(99), 0, 1), OP(T(59), T(92), T(98), 0, 1), OP(T(68), T(93), T(99), 0, 1), \
+    OP(T(71), T(94), T(98), 0, 1), OP(T(74), T(61), T(100), 0, 1), OP(T(75), T(63), T(55), 0, 1), \
+    OP(T(76), T(65), T(70), 0, 1), OP(T(78), IN(5), T(102), 0, 1), OP(T(79), IN(3), T(103), 0, 1), \
+    OP(T(80), IN(14), Y(21), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(90), T(81), T(54), 0, 0), OP(T(72), T(82), T(56), 0, 0), \
+    OP(T(77), T(83), T(57), 0, 0), OP(T(89), T(84), T(58), 0, 0), OP(T(91), T(85), T(59), 0, 0), \
+    OP(T(92), T(87), T(68), 0, 0), OP(T(93), T(88), T(71), 0, 0), OP(T(94), T(63), T(101), 1, 0), \
+    OP(T(95), T(64), T(55), 1, 0), OP(T(96), T(65), T(69), 1, 0), OP(T(97), T(66), T(70), 1, 0), \
+    OP(T(100), Y(11), T(80), 1, 0), OP(T(102), Y(4), T(73), 1, 0), OP(T(103), Y(13), T(80), 1, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(54), T(74), Y(21), 0, 1), \
+    OP(T(55), T(75), Y(21), 0, 1), OP(T(56), T(76), Y(21), 0, 1), OP(T(57), T(79), T(94), 0, 1), \
+    OP(T(58), T(78), T(95), 0, 1), OP(T(59), T(79), T(96), 0, 1), OP(T(68), T(78), T(97), 0, 1), \
+    OP(T(70), T(103), T(78), 0, 1), OP(T(71), T(100), T(98), 0, 1), OP(T(81), T(86), T(79), 0, 1), \
+    OP(T(82), T(102), T(99), 0, 1), OP(T(83), IN(44), T(60), 0, 1), OP(T(84), IN(43), T(60), 0, 1), \
+    OP(T(85), IN(42), T(60), 0, 1), OP(T(87), IN(28), T(67), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(88), T(90), T(54), 1, 0), OP(T(60), T(72), T(55), 1, 0), OP(T(67), T(77), T(56), 1, 0), \
+    OP(T(74), T(89), T(57), 1, 0), OP(T(75), T(91), T(58), 1, 0), OP(T(76), T(92), T(59), 1, 0), \
+    OP(T(78), T(93), T(68), 1, 0), OP(T(79), T(71), T(70), 1, 0), OP(T(86), T(82), T(81), 1, 0), \
+    OP(T(94), T(87), T(61), 1, 0), OP(T(95), T(101), T(63), 1, 0), OP(T(96), T(69), T(65), 1, 0), \
+    OP(T(97), Y(2), T(73), 1, 0), OP(T(98), Y(9), T(80), 1, 0), OP(T(99), Y(10), Y(12), 1, 0), \
+    OP(T(100), Y(3), Y(5), 1, 0), OP(T(102), T(75), T(74), 0, 1), OP(T(54), T(78), T(76), 0, 1), \
+    OP(T(55), T(84), T(79), 0, 1), OP(T(56), Y(19), T(86), 0, 1), OP(T(57), T(86), T(79), 0, 1), \
+    OP(T(58), T(85), T(79), 0, 1), OP(T(59), Y(18), T(86), 0, 1), OP(T(61), T(103), T(83), 0, 1), \
+    OP(T(63), T(103), T(84), 0, 1), OP(T(65), T(103), T(85), 0, 1), OP(T(68), T(62), T(87), 0, 1), \
+    OP(T(70), T(64), T(101), 0, 1), OP(T(71), T(66), T(69), 0, 1), OP(T(72), Y(21), T(100), 0, 1), \
+    OP(T(73), Y(13), Y(21), 0, 1), OP(T(77), Y(6), Y(21), 0, 1), OP(T(80), T(102), Y(21), 0, 1), \
+    OP(T(81), T(54), Y(21), 0, 1), OP(T(82), T(55), T(74), 0, 1), OP(T(89), T(56), T(75), 0, 1), \
+    OP(T(90), T(57), Y(21), 0, 1), OP(T(91), T(58), T(76), 0, 1), OP(T(92), T(59), T(78), 0, 1), \
+    OP(T(93), T(61), T(94), 0, 1), OP(T(62), T(63), T(95), 0, 1), OP(T(64), T(65), T(96), 0, 1), \
+    OP(T(66), T(68), Y(21), 0, 1), OP(T(69), T(70), Y(21), 0, 1), OP(T(79), T(71), Y(21), 0, 1), \
+    OP(T(83), T(72), T(99), 0, 1), OP(T(84), T(73), T(97), 0, 1), OP(T(85), T(77), T(98), 0, 1), \
+    OP(T(86), T(88), T(66), 1, 0), OP(T(87), T(60), T(69), 1, 0), OP(T(100), T(67), T(79), 1, 0), \
+    OP(T(101), T(89), T(82), 0, 0), OP(T(103), T(92), T(91), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(54), T(86), T(93), 0, 0), OP(T(55), T(87), T(62), 0, 0), \
+    OP(T(56), T(100), T(64), 0, 0), OP(T(57), T(101), T(83), 0, 0), OP(T(58), T(103), T(83), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(59), T(54), T(85), 0, 0), \
+    OP(T(61), T(55), T(85), 0, 0), OP(T(63), T(56), T(85), 0, 0), OP(T(65), T(57), T(90), 1, 0), \
+    OP(T(68), T(58), T(90), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(70), T(59), T(84), 0, 0), OP(T(71), T(61), T(84), 0, 0), OP(T(72), T(63), T(84), 0, 0), \
+    OP(T(73), T(65), T(80), 1, 0), OP(T(74), T(68), T(81), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(104), Y(0), Y(2), 1, 0), OP(T(105), Y(9), Y(12), 1, 0), \
+    OP(T(106), Y(8), Y(10), 1, 0), OP(T(107), Y(7), Y(9), 1, 0), OP(T(108), Y(2), Y(5), 1, 0), \
+    OP(T(109), Y(1), Y(3), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(110), IN(9), Y(21), 0, 1), \
+    OP(T(111), IN(17), Y(21), 0, 1), OP(T(112), IN(8), Y(21), 0, 1), OP(T(113), IN(16), Y(21), 0, 1), \
+    OP(T(114), IN(7), Y(21), 0, 1), OP(T(115), IN(14), Y(21), 0, 1), OP(T(116), Y(21), Y(21), 0, 1), \
+    OP(T(117), IN(15), Y(21), 0, 1), OP(T(118), IN(6), Y(21), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(119), Y(0), T(110), 1, 0), OP(T(120), Y(1), T(110), 1, 0), OP(T(121), Y(7), T(111), 1, 0), \
+    OP(T(122), Y(8), T(111), 1, 0), OP(T(123), Y(0), T(112), 1, 0), OP(T(124), Y(1), T(112), 1, 0), \
+    OP(T(125), Y(7), T(113), 1, 0), OP(T(126), Y(8), T(113), 1, 0), OP(T(127), Y(0), T(114), 1, 0), \
+    OP(T(128), Y(1), T(114), 1, 0), OP(T(129), Y(13), T(115), 1, 0), OP(T(130), Y(11), T(115), 1, 0), \
+    OP(T(131), Y(7), T(117), 1, 0), OP(T(132), Y(8), T(117), 1, 0), OP(T(133), Y(6), T(118), 1, 0), \
+    OP(T(134), Y(4), T(118), 1, 0), OP(T(110), IN(28), T(104), 0, 1), OP(T(111), IN(35), T(107), 0, 1), \
+    OP(T(112), IN(25), T(104), 0, 1), OP(T(113), IN(32), T(107), 0, 1), OP(T(114), IN(24), T(104), 0, 1), \
+    OP(T(115), IN(31), T(107), 0, 1), OP(T(117), IN(23), T(104), 0, 1), OP(T(118), IN(30), T(107), 0, 1), \
+    OP(T(135), IN(22), T(104), 0, 1), OP(T(136), IN(4), T(106), 0, 1), OP(T(137), IN(29), T(107), 0, 1), \
+    OP(T(138), IN(2), T(109), 0, 1), OP(T(139), IN(13), Y(21), 0, 1), OP(T(140), IN(21), Y(21), 0, 1), \
+    OP(T(141), IN(10), Y(21), 0, 1), OP(T(142), IN(18), Y(21), 0, 1), OP(T(104), Y(1), T(110), 0, 0), \
+    OP(T(106), Y(8), T(111), 0, 0), OP(T(107), Y(1), T(112), 0, 0), OP(T(109), Y(8), T(113), 0, 0), \
+    OP(T(143), Y(1), T(114), 0, 0), OP(T(144), Y(8), T(115), 0, 0), OP(T(145), Y(1), T(117), 0, 0), \
+    OP(T(146), Y(8), T(118), 0, 0), OP(T(147), Y(1), T(135), 0, 0), OP(T(148), Y(8), T(137), 0, 0), \
+    OP(T(149), Y(7), T(140), 1, 0), OP(T(150), Y(8), T(140), 1, 0), OP(T(151), Y(0), T(141), 1, 0), \
+    OP(T(152), Y(1), T(141), 1, 0), OP(T(153), Y(7), T(142), 1, 0), OP(T(154), Y(8), T(142), 1, 0), \
+    OP(T(140), T(104), Y(0), 1, 0), OP(T(141), T(106), Y(7), 1, 0), OP(T(142), T(107), Y(0), 1, 0), \
+    OP(T(155), T(109), Y(7), 1, 0), OP(T(156), T(143), Y(0), 1, 0), OP(T(157), T(144), Y(7), 1, 0), \
+    OP(T(158), T(145), Y(0), 1, 0), OP(T(159), T(146), Y(7), 1, 0), OP(T(160), T(147), Y(0), 1, 0), \
+    OP(T(161), T(148), Y(7), 1, 0), OP(T(162), T(123), T(117), 1, 0), OP(T(163), T(125), T(118), 1, 0), \
+    OP(T(164), T(127), T(135), 1, 0), OP(T(165), T(131), T(137), 1, 0), OP(T(166), Y(0), T(139), 1, 0), \
+    OP(T(167), Y(1), T(139), 1, 0), OP(T(104), T(167), T(138), 0, 1), OP(T(106), T(150), T(136), 0, 1), \
+    OP(T(107), T(152), T(138), 0, 1), OP(T(109), T(154), T(136), 0, 1), OP(T(117), T(120), T(138), 0, 1), \
+    OP(T(118), T(122), T(136), 0, 1), OP(T(123), T(124), T(138), 0, 1), OP(T(125), T(126), T(136), 0, 1), \
+    OP(T(127), T(128), T(138), 0, 1), OP(T(131), T(132), T(136), 0, 1), OP(T(135), IN(40), T(116), 0, 1), \
+    OP(T(137), IN(39), T(116), 0, 1), OP(T(139), IN(38), T(116), 0, 1), OP(T(143), IN(5), T(105), 0, 1), \
+    OP(T(144), IN(3), T(108), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(145), T(140), T(104), 0, 0), \
+    OP(T(146), T(141), T(106), 0, 0), OP(T(147), T(142), T(107), 0, 0), OP(T(148), T(155), T(109), 0, 0), \
+    OP(T(105), T(156), T(117), 0, 0), OP(T(108), T(157), T(118), 0, 0), OP(T(120), T(158), T(123), 0, 0), \
+    OP(T(122), T(159), T(125), 0, 0), OP(T(124), T(160), T(127), 0, 0), OP(T(126), T(161), T(131), 0, 0), \
+    OP(T(128), T(166), T(110), 1, 0), OP(T(132), T(149), T(111), 1, 0), OP(T(150), T(151), T(112), 1, 0), \
+    OP(T(152), T(153), T(113), 1, 0), OP(T(154), T(119), T(114), 1, 0), OP(T(167), T(121), T(115), 1, 0), \
+    OP(T(104), T(144), T(128), 0, 1), OP(T(106), T(143), T(132), 0, 1), OP(T(107), T(144), T(150), 0, 1), \
+    OP(T(109), T(143), T(152), 0, 1), OP(T(110), T(144), T(154), 0, 1), OP(T(111), T(143), T(167), 0, 1), \
+    OP(T(112), T(144), T(162), 0, 1), OP(T(113), T(143), T(163), 0, 1), OP(T(114), T(144), T(164), 0, 1), \
+    OP(T(115), T(143), T(165), 0, 1), OP(T(117), T(129), T(143), 0, 1), OP(T(118), T(130), T(136), 0, 1), \
+    OP(T(119), T(133), T(144), 0, 1), OP(T(121), T(134), T(138), 0, 1), OP(T(123), IN(44), T(116), 0, 1), \
+    OP(T(125), IN(41), T(116), 0, 1), OP(T(127), T(145), T(104), 1, 0), OP(T(131), T(146), T(106), 1, 0), \
+    OP(T(140), T(147), T(107), 1, 0), OP(T(141), T(148), T(109), 1, 0), OP(T(142), T(105), T(110), 1, 0), \
+    OP(T(149), T(108), T(111), 1, 0), OP(T(151), T(120), T(112), 1, 0), OP(T(153), T(122), T(113), 1, 0), \
+    OP(T(155), T(124), T(114), 1, 0), OP(T(156), T(126), T(115), 1, 0), OP(T(157), T(118), T(117), 1, 0), \
+    OP(T(158), T(121), T(119), 1, 0), OP(T(159), Y(3), Y(5), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(160), T(123), T(157), 0, 1), \
+    OP(T(161), Y(20), T(158), 0, 1), OP(T(166), T(125), T(157), 0, 1), OP(T(116), Y(17), T(158), 0, 1), \
+    OP(T(128), T(135), T(157), 0, 1), OP(T(129), Y(16), T(158), 0, 1), OP(T(130), T(137), T(157), 0, 1), \
+    OP(T(132), Y(15), T(158), 0, 1), OP(T(133), T(139), T(157), 0, 1), OP(T(134), Y(14), T(158), 0, 1), \
+    OP(T(136), Y(21), T(159), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(138), T(131), T(127), 0, 1), OP(T(143), T(160), T(127), 0, 1), OP(T(144), T(161), T(131), 0, 1), \
+    OP(T(150), T(141), T(140), 0, 1), OP(T(152), T(166), T(140), 0, 1), OP(T(154), T(116), T(141), 0, 1), \
+    OP(T(162), T(149), T(142), 0, 1), OP(T(163), T(128), T(142), 0, 1), OP(T(164), T(129), T(149), 0, 1), \
+    OP(T(165), T(153), T(151), 0, 1), OP(T(167), T(130), T(151), 0, 1), OP(T(104), T(132), T(153), 0, 1), \
+    OP(T(105), T(156), T(155), 0, 1), OP(T(106), T(133), T(155), 0, 1), OP(T(107), T(134), T(156), 0, 1), \
+    OP(T(108), T(158), T(157), 0, 1), OP(T(109), T(144), T(143), 0, 0), OP(T(110), T(154), T(152), 0, 0), \
+    OP(T(111), T(164), T(163), 0, 0), OP(T(112), T(104), T(167), 0, 0), OP(T(113), T(107), T(106), 0, 0), \
+    OP(T(114), Y(10), Y(12), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(115), T(138), Y(21), 0, 1), \
+    OP(T(117), T(150), Y(21), 0, 1), OP(T(118), T(162), Y(21), 0, 1), OP(T(119), T(165), Y(21), 0, 1), \
+    OP(T(120), T(105), Y(21), 0, 1), OP(T(121), T(108), Y(21), 0, 1), OP(T(122), T(136), T(114), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(124), T(109), T(122), 0, 0), OP(T(126), T(110), T(122), 0, 0), OP(T(145), T(111), T(122), 0, 0), \
+    OP(T(146), T(112), T(122), 0, 0), OP(T(147), T(113), T(122), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(148), T(124), T(121), 1, 0), OP(T(123), T(126), T(121), 1, 0), \
+    OP(T(125), T(145), T(121), 1, 0), OP(T(135), T(146), T(121), 1, 0), OP(T(137), T(147), T(121), 1, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(139), T(148), T(115), 1, 0), \
+    OP(T(159), T(123), T(117), 1, 0), OP(T(116), T(125), T(118), 1, 0), OP(T(127), T(135), T(119), 1, 0), \
+    OP(T(128), T(137), T(120), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(168), IN(6), IN(14), 0, 1), OP(T(169), Y(21), Y(21), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(170), Y(8), IN(13), 0, 1), OP(T(171), Y(1), IN(21), 0, 1), \
+    OP(T(172), IN(21), IN(13), 0, 1), OP(T(173), Y(8), IN(12), 0, 1), OP(T(174), Y(1), IN(20), 0, 1), \
+    OP(T(175), IN(20), IN(12), 0, 1), OP(T(176), Y(8), IN(11), 0, 1), OP(T(177), Y(1), IN(19), 0, 1), \
+    OP(T(178), IN(19), IN(11), 0, 1), OP(T(179), Y(8), IN(8), 0, 1), OP(T(180), Y(1), IN(16), 0, 1), \
+    OP(T(181), IN(16), IN(8), 0, 1), OP(T(182), IN(15), Y(21), 0, 1), OP(T(183), Y(8), IN(7), 0, 1), \
+    OP(T(184), Y(1), IN(15), 0, 1), OP(T(185), IN(15), IN(7), 0, 1), OP(T(186), T(171), T(170), 0, 0), \
+    OP(T(187), T(168), T(172), 0, 0), OP(T(188), T(174), T(173), 0, 0), OP(T(189), T(168), T(175), 0, 0), \
+    OP(T(190), T(177), T(176), 0, 0), OP(T(191), T(168), T(178), 0, 0), OP(T(192), T(180), T(179), 0, 0), \
+    OP(T(193), T(168), T(181), 0, 0), OP(T(194), Y(8), T(182), 1, 0), OP(T(195), T(184), T(183), 0, 0), \
+    OP(T(196), T(168), T(185), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(168), T(169), Y(21), 0, 1), OP(T(170), IN(8), Y(21), 0, 1), OP(T(171), IN(16), Y(21), 0, 1), \
+    OP(T(172), IN(7), Y(21), 0, 1), OP(T(173), IN(14), Y(21), 0, 1), OP(T(174), IN(6), Y(21), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(175), T(168), T(187), 0, 1), OP(T(176), T(168), T(189), 0, 1), \
+    OP(T(177), T(168), T(191), 0, 1), OP(T(178), T(168), T(193), 0, 1), OP(T(179), T(168), T(196), 0, 1), \
+    OP(T(180), T(169), T(186), 0, 1), OP(T(181), T(169), T(188), 0, 1), OP(T(182), T(169), T(190), 0, 1), \
+    OP(T(183), T(169), T(192), 0, 1), OP(T(184), T(169), T(195), 0, 1), OP(T(185), IN(13), Y(21), 0, 1), \
+    OP(T(197), IN(21), Y(21), 0, 1), OP(T(198), IN(12), Y(21), 0, 1), OP(T(199), IN(20), Y(21), 0, 1), \
+    OP(T(200), IN(11), Y(21), 0, 1), OP(T(201), IN(19), Y(21), 0, 1), OP(T(168), T(175), T(180), 1, 0), \
+    OP(T(186), T(176), T(181), 1, 0), OP(T(187), T(177), T(182), 1, 0), OP(T(188), T(178), T(183), 1, 0), \
+    OP(T(189), T(179), T(184), 1, 0), OP(T(190), Y(1), T(185), 1, 0), OP(T(191), Y(8), T(197), 1, 0), \
+    OP(T(192), Y(1), T(198), 1, 0), OP(T(193), Y(8), T(199), 1, 0), OP(T(195), Y(1), T(200), 1, 0), \
+    OP(T(196), Y(8), T(201), 1, 0), OP(T(202), Y(1), T(170), 1, 0), OP(T(203), Y(8), T(171), 1, 0), \
+    OP(T(204), Y(11), T(173), 1, 0), OP(T(205), Y(1), T(172), 1, 0), OP(T(206), Y(4), T(174), 1, 0), \
+    OP(T(170), IN(44), T(190), 0, 1), OP(T(171), Y(20), T(191), 0, 1), OP(T(172), IN(43), T(192), 0, 1), \
+    OP(T(175), Y(19), T(193), 0, 1), OP(T(176), IN(42), T(195), 0, 1), OP(T(177), Y(18), T(196), 0, 1), \
+    OP(T(178), IN(39), T(202), 0, 1), OP(T(179), Y(15), T(203), 0, 1), OP(T(180), IN(38), T(205), 0, 1), \
+    OP(T(181), Y(14), T(194), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(182), T(170), T(204), 0, 1), OP(T(183), T(171), T(206), 0, 1), \
+    OP(T(184), T(172), T(204), 0, 1), OP(T(185), T(175), T(206), 0, 1), OP(T(197), T(176), T(204), 0, 1), \
+    OP(T(198), T(177), T(206), 0, 1), OP(T(199), T(178), T(204), 0, 1), OP(T(200), T(179), T(206), 0, 1), \
+    OP(T(201), T(180), T(204), 0, 1), OP(T(190), T(181), T(206), 0, 1), OP(T(191), Y(11), Y(21), 0, 1), \
+    OP(T(192), Y(4), Y(21), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(193), T(168), T(183), 1, 0), \
+    OP(T(194), T(186), T(185), 1, 0), OP(T(195), T(187), T(198), 1, 0), OP(T(196), T(188), T(200), 1, 0), \
+    OP(T(202), T(189), T(190), 1, 0), OP(T(203), Y(1), T(174), 1, 0), OP(T(205), Y(8), T(173), 1, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(170), T(182), T(169), 0, 1), OP(T(171), T(184), T(169), 0, 1), OP(T(172), T(197), T(169), 0, 1), \
+    OP(T(175), T(199), T(169), 0, 1), OP(T(176), T(201), T(169), 0, 1), OP(T(177), T(191), T(203), 0, 1), \
+    OP(T(178), T(192), T(205), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), OP(T(207), Y(0), Y(0), 0, 1), \
+    OP(T(207), Y(0), Y(0), 0, 1), OP(T(179), T(193), T(178), 0, 0), OP(T(180), T(194), T(178), 0, 0), \
+    OP(T(181), T(195), T(178), 0, 0), OP(T(204), T(196), T(178), 0, 0), OP(T(206), T(202), T(178), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(168), T(179), T(177), 0, 0), \
+    OP(T(173), T(180), T(177), 0, 0), OP(T(174), T(181), T(177), 0, 0), OP(T(183), T(204), T(177), 0, 0), \
+    OP(T(185), T(206), T(177), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(186), T(168), T(170), 1, 0), OP(T(187), T(173), T(171), 1, 0), OP(T(188), T(174), T(172), 1, 0), \
+    OP(T(189), T(183), T(175), 1, 0), OP(T(190), T(185), T(176), 1, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), OP(T(207), Y(0), Y(0), 0, 0), \
+    OP(T(207), Y(0), Y(0), 0, 0), 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, \
+    0, 0, 0, 0, 0, 0
 #define FRG_RESIDUAL_OUTS(OUT, T) \
-    OUT(T + 24, 0, 0, 1), OUT(T + 18, 0, 1, 1), OUT(T + 17, 0, 2, 1), OUT(T + 16, 0, 3, 1), 0xffff, 0xffff, \
-    0xffff, OUT(T + 52, 0, 4, 1), OUT(T + 51, 0, 5, 1), OUT(T + 42, 0, 6, 1), 0xffff, 0xffff, 0xffff, 0xffff, \
-    OUT(T + 78, 1, 0, 1), OUT(T + 77, 1, 1, 1), OUT(T + 76, 1, 2, 1), OUT(T + 75, 1, 3, 1), \
-    OUT(T + 67, 1, 4, 1), OUT(T + 66, 1, 5, 1), OUT(T + 56, 1, 6, 1), OUT(T + 110, 2, 0, 0), \
-    OUT(T + 109, 2, 1, 0), OUT(T + 95, 2, 2, 0), OUT(T + 94, 2, 3, 0), OUT(T + 93, 2, 4, 0), \
-    OUT(T + 92, 2, 5, 0), OUT(T + 91, 2, 6, 0)
+    OUT(T(30), 0, 0, 1), OUT(T(29), 0, 1, 1), OUT(T(28), 0, 2, 1), OUT(T(27), 0, 3, 1), OUT(T(34), 1, 2, 1), \
+    OUT(T(31), 1, 3, 1), 0xffff, OUT(T(72), 0, 4, 1), OUT(T(71), 0, 5, 1), OUT(T(70), 0, 6, 1), \
+    OUT(T(74), 2, 4, 0), OUT(T(73), 2, 5, 0), 0xffff, 0xffff, OUT(T(128), 2, 0, 0), OUT(T(127), 2, 1, 0), \
+    OUT(T(116), 2, 2, 0), OUT(T(159), 2, 3, 0), OUT(T(139), 2, 6, 0), 0xffff, 0xffff, OUT(T(190), 1, 0, 1), \
+    OUT(T(189), 1, 1, 1), OUT(T(188), 1, 4, 1), OUT(T(187), 1, 5, 1), OUT(T(186), 1, 6, 1), 0xffff, 0xffff

@@ -153,9 +153,9 @@ struct StepOut {
 // lanes 0..6, e on 8..11, q's denominator on 12); q(t) (and dq/dt, htpysupport.cu:37-62),
 // one parameter per lane, with z^2 and z^3 on lane 31 in the same products; then the
 // hoisted quantities, lanes 8 s + g those of side s and group g, lanes 16 + s those that
-// are the same for every group, again in the same instructions. RESID: the forms of the
-// refinement residual. 81 FP64 instructions; with each quantity in instructions of
-// its own it was 143.
+// are the same for every group, again in the same instructions. 81 FP64 instructions; with
+// each quantity in instructions of its own it was 143. RESID (the refinement residual): the
+// reciprocals and q(t) alone, as its schedules hold the rest.
 template <bool RESID, typename V>
 __device__ __forceinline__ void eval_prep(const cx<V>* Y, const cx<V>* sp, const cx<V>* fp, cx<V> gamma,
                                           FrgEvalIn<V>& in, cx<V>* dq, int lane) {
@@ -175,22 +175,22 @@ __device__ __forceinline__ void eval_prep(const cx<V>* Y, const cx<V>* sp, const
   if (lane >= 8 && lane < 12) in.e[lane - 8] = ib;
   const cx<V> iden = warp_shfl(ib, 12);
   {
-    const bool l31 = lane == 31;
-    const cx<V> a = l31 ? z : iden;
-    const cx<V> sq = a * a;
-    const cx<V> cu = (l31 ? sq : gamma) * (l31 ? z : sq);
-    if (l31) { in.z2 = sq; in.z3 = cu; }
     const int i = lane < NP ? lane : 0;
     const cx<V> s = sp[i], f = fp[i];
     const cx<V> q = (g1t * s + t * f) * iden;
     if (lane < NP) in.q[lane] = q;
     if constexpr (!RESID) {
+      const bool l31 = lane == 31;
+      const cx<V> a = l31 ? z : iden;
+      const cx<V> sq = a * a;
+      const cx<V> cu = (l31 ? sq : gamma) * (l31 ? z : sq);
+      if (l31) { in.z2 = sq; in.z3 = cu; }
       const cx<V> v = (f - s) * cu;
       if (lane < NP) dq[lane] = v;
     }
   }
   __syncwarp();
-  {
+  if constexpr (!RESID) {
     const bool all = lane >= 16;  // lanes 16, 17: the same for every group
     const int s = all ? lane & 1 : lane >> 3, g = (lane & 7) < 7 ? lane & 7 : 6;
     const cx<V>* L = Y + 7 * s;  // A, B, C, D, F, G, H of this side
@@ -202,24 +202,17 @@ __device__ __forceinline__ void eval_prep(const cx<V>* Y, const cx<V>* sp, const
     const cx<V> d3 = (all ? L[2] : d0) - (all ? L[5] : m1);                  // aq | cg
     const cx<V> m2 = e2 * d3;                                                // eaq | ecg
     const cx<V> ebd = warp_shfl(m1, 16 + s);
-    const cx<V> w0 = RESID ? L[1] + m1 - L[0] : L[1] - L[0] + m1;
+    const cx<V> w0 = L[1] - L[0] + m1;
     const cx<V> t0 = (all ? d0 : d1) * ebd;                                  // bp ebd | fp ebd
     const cx<V> w1 = w0 + t0;
-    cx<V> t1;
-    if constexpr (RESID) {
-      const cx<V> ecg = warp_shfl(m2, 16 + s);
-      t1 = (all ? d1 : ecg) * (all ? m2 : d3);                               // ecg aq | hp ecg
-    } else {
-      const cx<V> cg = warp_shfl(d3, 16 + s);
-      t1 = (all ? d1 : cg) * m2;                                             // cg eaq | hp ecg
-    }
+    const cx<V> cg = warp_shfl(d3, 16 + s);
+    const cx<V> t1 = (all ? d1 : cg) * m2;                                   // cg eaq | hp ecg
     const cx<V> w = (all ? t0 : w1) - t1;                                    // w | v
     if (lane < 16) {
       cx<V>(*o)[8] = in.sb[s];
       const int c = lane & 7;
       o[FRG_IN_PJZ][c] = m0; o[FRG_IN_AP][c] = d0; o[FRG_IN_BP][c] = d1;
-      o[FRG_IN_QA][c] = m1;  o[FRG_IN_AQ][c] = d3; o[FRG_IN_W][c] = w;
-      if constexpr (!RESID) o[FRG_IN_EAQ][c] = m2;
+      o[FRG_IN_QA][c] = m1;  o[FRG_IN_AQ][c] = d3; o[FRG_IN_W][c] = w;   o[FRG_IN_EAQ][c] = m2;
       if (c == 0) in.sa[s][FRG_IN_AC] = d2;
     } else if (lane < 18) {
       cx<V>* o = in.sa[s];
@@ -242,12 +235,14 @@ __device__ __forceinline__ cx<P> patch_dot(const cx<T>* u, const cx<P>* Y, int n
 // in the point type, by the four warps of its part: warp `part` runs its generated schedule,
 // lane 2 o + c computing component c of a step's operation o, from what eval_prep<true> left
 // in the path's inputs. The temporaries take the vectors that a corrector step does not need
-// (X .. k).
+// (X .. k), then the place of the inputs that the schedules compute themselves.
 // What bounds it: the chain of operations, 200 to 250 cycles each. As straight-line code, a
-// group's three equations on a lane of three warps, it was 39 operations long in 13 % of a
-// path's steps, and of 16 paths in step nearly always one is in such a step; the schedule has
-// 17 steps (3.8k cycles). GB300, FP32 stage of 140 paths 113 -> 104 ms, of 2,400 236 -> 213, of
-// 9,600 333 -> 282; 65,536-path rounds, four in flight, 1,448 -> 1,365 ms a round.
+// group's three equations on a lane of three warps after the hoisted quantities on one, it was
+// 52 operations long in 13 % of a path's steps, and of 16 paths in step nearly always one is
+// in such a step; the schedule has 17 steps (3.8k cycles). GB300, FP32 stage of 140 paths 113 -> 104 ms, of 2,400 236 -> 213, of
+// 9,600 333 -> 282, and with the hoisted quantities in the
+// schedules 203 -> 191 and 293 -> 256; 65,536-path rounds, four in flight, 1,448 -> 1,365 and
+// 1,349 -> 1,311 ms a round.
 template <typename P>
 struct Residual {
   typedef Smem<float, P> S;
@@ -255,15 +250,20 @@ struct Residual {
                             kIn = (offsetof(S, work) + offsetof(typename S::Inputs, hi)) / 16;
   static_assert(sizeof(cx<P>) == 16 && offsetof(S, YN) % 16 == 0 && offsetof(S, X) % 16 == 0 &&
                 offsetof(S, work) % 16 == 0 && offsetof(typename S::Inputs, hi) % 16 == 0, "16-byte units");
-  static_assert(kT + FRG_RESIDUAL_TEMPS <= (offsetof(S, k) + sizeof(S::k)) / 16, "temporaries");
+  static constexpr unsigned kFirst = (offsetof(S, k) + sizeof(S::k)) / 16 - kT,  // temporaries in X .. k
+                            kFree = kIn + offsetof(FrgEvalIn<P>, sa) / 16;
+  static_assert(FRG_RESIDUAL_TEMPS - kFirst <= sizeof(FrgEvalIn<P>) / 16 - offsetof(FrgEvalIn<P>, sa) / 16, "temporaries");
+  static constexpr unsigned y(unsigned i) { return kY + i; }
+  static constexpr unsigned in(unsigned i) { return kIn + i; }
+  static constexpr unsigned t(unsigned i) { return i < kFirst ? kT + i : kFree + (i - kFirst); }
   static_assert(kIn + sizeof(FrgEvalIn<P>) / 16 <= 1024, "10-bit units");
 };
 static_assert(Residual<df>::kY == Residual<double>::kY && Residual<df>::kT == Residual<double>::kT &&
               Residual<df>::kIn == Residual<double>::kIn, "one table for both point types");
 #define FRG_OP(r, a, b, sub, mul) (unsigned)(r) | (unsigned)(a) << 10 | (unsigned)(b) << 20 | sub##u << 30 | mul##u << 31
 #define FRG_OUT(r, eq, g, minus) (r) | (g) << 10 | (eq) << 13 | (minus) << 15
-static __device__ const unsigned residual_code[] = {FRG_RESIDUAL_CODE(FRG_OP, Residual<df>::kY, Residual<df>::kIn, Residual<df>::kT)};
-static __device__ const unsigned short residual_outs[] = {FRG_RESIDUAL_OUTS(FRG_OUT, Residual<df>::kT)};
+static __device__ const unsigned residual_code[] = {FRG_RESIDUAL_CODE(FRG_OP, Residual<df>::y, Residual<df>::in, Residual<df>::t)};
+static __device__ const unsigned short residual_outs[] = {FRG_RESIDUAL_OUTS(FRG_OUT, Residual<df>::t)};
 #undef FRG_OP
 #undef FRG_OUT
 

@@ -20,8 +20,9 @@ the operation counts used for the roofline's algorithmic FLOPs per evaluation.
 """
 from __future__ import annotations
 
-import re
+import ast
 import os
+import re
 
 import numpy as np
 import sympy as sp
@@ -290,6 +291,11 @@ def operand_of(x, key):
     return 1, start[name] + flat.get(name, lambda k=0: k)(*index), int("j" in load)
 
 
+# name and side -> form, as the residual has it
+HOISTED_FORMS = {f"{name}{side}": (RESIDUAL_FORMS.get(name, forms))[side]
+                 for name, _, *forms in HOISTED for side in (0, 1)}
+
+
 class ResidualTape:
     """Equations of some groups as a schedule of complex operations for a warp: pairs of lanes
     (one per real component) take one operation each, so a step is up to WIDTH products or
@@ -303,8 +309,6 @@ class ResidualTape:
     def __init__(self, repl, reduced, found, items, products):
         self.defs, self.found = {s_.name: d for s_, d in repl}, found
         self.ops, self.memo = [], {}
-        for k, q in enumerate(("P0", "Pc0")):  # eval_prep's products
-            self.memo["mul", self.value(q, 0), self.value("z", 0), 0] = ("v", (1, operand_of("pz", f"pz{k}")[1]))
         self.outs = []  # (equation, group, operation, sign)
         for eq, g in items:
             self.seen = {}
@@ -313,8 +317,22 @@ class ResidualTape:
         self.schedule(products)
 
     def value(self, name, g):
-        seg, index, per_group = operand_of(name, self.found.get(name))
-        return "v", (seg, index + g * per_group)
+        """A prepared value, or a hoisted quantity from the form that eval_prep evaluates."""
+        if name == "z2" or name == "z3":
+            return self.op("mul", self.value("z" if name == "z2" else "z2", g), self.value("z", g))
+        key = self.found.get(name, name)
+        form = HOISTED_FORMS.get(key)
+        if form is None:
+            seg, index, per_group = operand_of(name, None)
+            return "v", (seg, index + g * per_group)
+
+        def walk(e):
+            if isinstance(e, ast.Name):
+                return self.value(e.id, g)
+            kind = "mul" if isinstance(e.op, ast.Mult) else "add"
+            return self.op(kind, walk(e.left), walk(e.right), int(isinstance(e.op, ast.Sub)))
+
+        return walk(ast.parse(form, mode="eval").body)
 
     def op(self, kind, x, y, sub=0):
         key = (kind, x, y, sub)
@@ -380,10 +398,11 @@ class ResidualTape:
             free += sorted({self.where[d] for k in pick for d in need[k] if d not in keep and users[d] <= ran})
 
 
-# A part's four warps: equation I of the groups 1..4 and 5..7, equations II and III; the
-# least number of ready products that go before sums (18, 16, 14 and 11 steps, 118 temporaries)
-RESIDUAL_PARTS = [([(0, g) for g in range(4)], 8), ([(0, g) for g in range(4, 7)], 8),
-                  ([(1, g) for g in range(7)], 6), ([(2, g) for g in range(7)], 2)]
+# A part's four warps: (equation, group) and the least number of ready products that go
+# before sums; 17, 17, 17 and 13 steps (the last warp also takes the patch row), 207 temporaries
+RESIDUAL_PARTS = [([(0, g) for g in range(4)] + [(1, g) for g in (2, 3)], 14),
+                  ([(0, g) for g in range(4, 7)] + [(2, g) for g in (4, 5)], 12),
+                  ([(2, g) for g in (0, 1, 2, 3, 6)], 8), ([(1, g) for g in (0, 1, 4, 5, 6)], 8)]
 
 
 def residual_system():
@@ -404,23 +423,23 @@ def emit_residual(lines, tapes):
     seg = ["Y", "IN", "T"]
     lines += ["",
               "// The three equations at a point alone (their own common subexpressions) as schedules for a",
-              "// part's four warps, residual_slice in frg_team.cuh executes them. Warp k: steps START[k] ..",
-              f"// START[k + 1] of {ResidualTape.WIDTH} words OP(result, a, b, b subtracted, product), in 16-byte units from",
-              "// Y (the point), IN (FrgEvalIn) and T (temporaries; the last takes idle lanes' results), two steps",
-              "// of padding at the end; then OUT(unit, equation, group, negated), 7 per warp.",
+              "// part's four warps, residual_part in frg_team.cuh executes them. Warp k: steps START[k] ..",
+              f"// START[k + 1] of {ResidualTape.WIDTH} words OP(result, a, b, b subtracted, product), values by",
+              "// number in Y (the point), IN (FrgEvalIn) and T (temporaries; the last takes idle lanes' results), two steps",
+              "// of padding at the end; then OUT(value, equation, group, negated), 7 per warp.",
               f"#define FRG_RESIDUAL_TEMPS {temps[-1] + 1}",
               f"#define FRG_RESIDUAL_START {{{', '.join(map(str, starts))}}}"]
     words = []
     for k, t in enumerate(tapes):
         for step in t.steps:
             for mul, sub, dst, a, b in step:
-                ops = [f"{seg[s_]} + {i + (temps[k] if s_ == 2 else 0)}" for s_, i in (a, b)]
-                words.append(f"OP(T + {temps[k] + dst}, {ops[0]}, {ops[1]}, {sub}, {int(mul)})")
-            words += [f"OP(T + {temps[-1]}, Y, Y, 0, {int(step[0][0])})"] * (t.WIDTH - len(step))
+                ops = [f"{seg[s_]}({i + (temps[k] if s_ == 2 else 0)})" for s_, i in (a, b)]
+                words.append(f"OP(T({temps[k] + dst}), {ops[0]}, {ops[1]}, {sub}, {int(mul)})")
+            words += [f"OP(T({temps[-1]}), Y(0), Y(0), 0, {int(step[0][0])})"] * (t.WIDTH - len(step))
     words += ["0"] * (2 * ResidualTape.WIDTH)
     outs = []
     for k, t in enumerate(tapes):
-        o = [f"OUT(T + {temps[k] + t.where[n]}, {eq}, {g}, {int(s_ < 0)})" for eq, g, n, s_ in t.outs]
+        o = [f"OUT(T({temps[k] + t.where[n]}), {eq}, {g}, {int(s_ < 0)})" for eq, g, n, s_ in t.outs]
         outs += o + ["0xffff"] * (7 - len(o))
     for name, items in (("CODE(OP, Y, IN, T)", words), ("OUTS(OUT, T)", outs)):
         lines.append(f"#define FRG_RESIDUAL_{name} \\")

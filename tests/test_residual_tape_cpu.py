@@ -2,6 +2,8 @@
 ResidualTape) against the printed expressions: executed step by step in single precision on
 random inputs, every equation of every group must be equal bit for bit, no step may read
 what it writes, and the parts' temporaries must not overlap."""
+import re
+
 import numpy as np
 import pytest
 
@@ -21,20 +23,26 @@ def test_schedule_equals_printed_equations(part):
         def draw(n):
             return [np.complex64(complex(*rng.normal(size=2))) for _ in range(n)]
 
-        mem = [draw(23), draw(46 + 2 * len(gs.INDEP) + 16 * len(gs.PERJ)), [np.complex64(0)] * tape.ntemps]
-
-        def value(name, g):
-            seg, index, per_group = gs.operand_of(name, found.get(name))
-            return mem[seg][index + g * per_group]
-
-        for k, q in enumerate(("P0", "Pc0")):
-            mem[1][gs.operand_of("pz", f"pz{k}")[1]] = value(q, 0) * value("z", 0)
+        mem = [draw(23), draw(46), [np.complex64(0)] * tape.ntemps]  # the point, prepared values
         want = {}
         for eq, g in items:
             env = {"T": np.float32, "cx": np.complex64}
+
+            def value(name):
+                if name in env:
+                    return env[name]
+                form = {"z2": "z*z", "z3": "z2*z"}.get(name) or gs.HOISTED_FORMS.get(found.get(name, name))
+                if form:
+                    env[name] = eval(form, {}, {x: value(x) for x in re.findall(r"[A-Za-z]\w*", form)})
+                else:
+                    seg, index, per_group = gs.operand_of(name, None)
+                    env[name] = mem[seg][index + g * per_group]
+                return env[name]
+
+            defined = {s.name for s, _ in repl}
             for name in {s.name for e in [*reduced, *(d for _, d in repl)] for s in e.free_symbols}:
-                if name in found or name not in {s.name for s, _ in repl}:
-                    env[name] = value(name, g)
+                if name in found or name not in defined:
+                    value(name)
             for s, d in repl:
                 if s.name not in found:
                     env[s.name] = eval(pr.expr(d), {}, env)
