@@ -414,6 +414,11 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   // A plug-in's launch of up to FRG_WARP_PATHS paths per SM sub-partition takes a warp
   // per path; a larger one a thread per path, and then a warp for each of its last paths.
   const bool by_warp = plugin && N <= (int64_t)ctx->sm_count * 4 * FRG_WARP_PATHS;
+  auto tail_cap = [&](int mode) -> int64_t {
+    return (int64_t)grid_for(mode, N) * (FRG_TRACK_THREADS / 32) * frg_tail_lanes(mode == 1);
+  };
+  if (plugin && !by_warp)  // the stages take turns with it; sized before the first launch
+    FRG_CUDA(ctx, sl.tail.ensure(sizeof(frg::Handoff) * (size_t)(mixed ? std::max(tail_cap(1), tail_cap(2)) : tail_cap(0))));
   auto launch = [&](int mode) -> cudaError_t {
     if (team) return frg_launch_team(mode, a, team_grid(ctx, mode, N), st);
     const int grid = grid_for(mode, N);
@@ -422,13 +427,11 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     if (by_warp) return frg_launch_warp(mode, a, (int)std::min<int64_t>(wcap, (N + 3) / 4), st);
     if (!plugin) return frg_launch_track(mode, a, grid, st);
     frg::TrackArgs b = a;
-    b.tail_cap = (int64_t)grid * (FRG_TRACK_THREADS / 32) * frg_tail_lanes(mode == 1, nv);
-    if (b.tail_cap == 0) return frg_launch_track(mode, a, grid, st);
-    cudaError_t e = sl.tail.ensure(sizeof(frg::Handoff) * (size_t)b.tail_cap);
-    if (e != cudaSuccess) return e;
+    b.tail_cap = tail_cap(mode);
     b.tail = (frg::Handoff*)sl.tail.p;
     b.tail_count = q + 8 + 2 * mode;  // and the tail's queue head beside it
-    if ((e = frg_launch_track(mode, b, grid, st)) != cudaSuccess) return e;
+    const cudaError_t e = frg_launch_track(mode, b, grid, st);
+    if (e != cudaSuccess) return e;
     b.from_tail = 1;
     b.queue = q + 9 + 2 * mode;
     return frg_launch_warp(mode, b, (int)std::min<int64_t>(wcap, (b.tail_cap + 3) / 4), st);

@@ -114,19 +114,19 @@ inline TeamGrid frg_team_grid(int sms, int bps, int64_t n, bool lo) {
 }
 
 // A plug-in launch of at most this many paths per SM sub-partition tracks a path per warp,
-// a larger one a path per thread. FP64, GB300 (152 SMs), warp / thread: conic2 2,432 paths
-// 8.5 / 14.1 ms, 9,728 26.7 / 28.1, 19,456 56.9 / 49.2, 40,000 72 / 52; burmester5 4,864
-// 57 / 99, 19,456 486 / 484. Mixed: conic2 9,728 4.2 / 5.0, 19,456 7.4 / 6.1; burmester5
-// 9,728 404 / 433.
+// a larger one a path per thread. GB300 (152 SMs), warp / thread, FP64: conic2 2,432 paths
+// 8.4 / 12.5 ms, 9,728 26.9 / 25.6, 19,456 55.9 / 45.9; burmester5 4,864 52 / 87, 9,728 406 /
+// 433, 19,456 463 / 446. Mixed: conic2 4,864 2.6 / 3.4, 9,728 3.8 / 3.5; burmester5 9,728
+// 383 / 403, 19,456 391 / 411.
 constexpr int FRG_WARP_PATHS = 16;
 
 // A warp of a thread-per-path launch gives its paths up to a warp-per-path launch when the
 // queue is empty and at most this many of its lanes still track one: a warp's step costs
-// the same with few lanes as with 32, four to seven times a warp_kernel step in FP64. In
-// FP32 a small system's step is too short for the second launch to pay (FP32 stage of
-// 120,000 conic2 paths: 4 lanes 12.6 ms, 2 lanes 11.7, never 11.4; of 8,192 burmester5
-// paths 35, 37, 58 ms).
-__host__ __device__ constexpr int frg_tail_lanes(bool fp32, int nv) { return fp32 && nv < 4 ? 0 : 4; }
+// the same with few lanes as with 32, four to seven times a warp_kernel step in FP64.
+// FP64, 4 / 8 / 12 lanes: 19,456 conic2 paths 46.2 / 43.7 ms, 262,144 116.0 / 115.5 / 115.9,
+// 131,072 burmester5 paths 652 / 639 / 642. FP32 stage of 120,000 conic2 paths, never / 2 / 3
+// lanes: 8.2 / 7.7 / 7.2 ms.
+__host__ __device__ constexpr int frg_tail_lanes(bool fp32) { return fp32 ? 4 : 8; }
 
 #define FRG_NQUEUE 16  // queue heads and counts of a slot
 

@@ -239,10 +239,10 @@ __device__ __forceinline__ cx<P> patch_dot(const cx<T>* u, const cx<P>* Y, int n
 // What bounds it: the chain of operations, 200 to 250 cycles each. As straight-line code, a
 // group's three equations on a lane of three warps after the hoisted quantities on one, it was
 // 52 operations long in 13 % of a path's steps, and of 16 paths in step nearly always one is
-// in such a step; the schedule has 17 steps (3.8k cycles). GB300, FP32 stage of 140 paths 113 -> 104 ms, of 2,400 236 -> 213, of
-// 9,600 333 -> 282, and with the hoisted quantities in the
-// schedules 203 -> 191 and 293 -> 256; 65,536-path rounds, four in flight, 1,448 -> 1,365 and
-// 1,349 -> 1,311 ms a round.
+// in such a step; the schedule has 17 steps (3.8k cycles). GB300, FP32 stage of 140 paths
+// 113 -> 104 ms, of 2,400 236 -> 213, of 9,600 333 -> 282, and with the hoisted quantities in
+// the schedules 203 -> 191 and 293 -> 256; 65,536-path rounds, four in flight, 1,448 -> 1,365
+// and 1,349 -> 1,311 ms a round.
 template <typename P>
 struct Residual {
   typedef Smem<float, P> S;

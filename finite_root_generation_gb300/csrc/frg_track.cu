@@ -237,8 +237,8 @@ track_kernel(TrackArgs a) {
     // FP64: 267 -> 250 ms, of which the longest paths' tail is the larger part).
     unsigned live = __ballot_sync(0xffffffffu, P.phase != PH_IDLE);
     if (!live) break;
-    constexpr int kTail = frg_tail_lanes(LO, NV_);
-    if (kTail > 0 && a.tail_cap > 0 && __any_sync(0xffffffffu, dry) && __popc(live) <= kTail) {
+    constexpr int kTail = frg_tail_lanes(LO);
+    if (a.tail_cap > 0 && __any_sync(0xffffffffu, dry) && __popc(live) <= kTail) {
       // The queue is empty and this warp's step serves few paths: they go on, from their
       // next step's start, in a warp_kernel launch, where a step is that much shorter.
       if (P.phase == PH_RK && P.stage == 0) {
