@@ -582,8 +582,8 @@ def run_ours(args, rank, world):
                          for kk, v in kernels.items()}},
         # tracking: with carry hand-back the FP32 and double-float parameter copies once,
         # then per round the start values, the FP32-stage and the FP64-stage kernels;
-        # without it all five per round (two per mixed round); dedup: five kernels per round
-        "gpu_launches": ((2 + 3 * k) if chosen_carry else (3 + 2 * max(1, chosen_rounds)) * k) + 5 * k,
+        # without it all five per round (two per mixed round); dedup: three kernels per round
+        "gpu_launches": ((2 + 3 * k) if chosen_carry else (3 + 2 * max(1, chosen_rounds)) * k) + 3 * k,
         "clocks": clocks,
     }
     if not args.no_cpu_baseline:
@@ -823,7 +823,9 @@ def run_plugin(args):
                          "unit": "TFLOP/s", "frac": round(achieved / peaks["fp64"], 4), "traffic": None,
                          "flops_per_solve": fps, "solves": int(solves),
                          "peak_source": "of measured: bench.py's own FP64 FMA kernel"},
-            "gpu_launches": 3 * k, "clocks": clk.summary(),
+            # the parameter copies, starts, tracking (by thread, then the last paths by warp), finishes
+            "gpu_launches": (6 if N > torch.cuda.get_device_properties(0).multi_processor_count * 64 else 5) * k,
+            "clocks": clk.summary(),
             "mixed": {"value": round(k * N / (m_ms * 1e-3), 1), "unit": "paths/s",
                       "speedup_vs_plain_fp64": round(ms / m_ms, 3), "recall_vs_plain_fp64": round(hits / max(total, 1), 5),
                       "distinct_roots_per_task": {"min": min(m_distinct), "max": max(m_distinct)},

@@ -30,8 +30,8 @@
 // this one) an FP64 step was 5,800 FP64 instructions in one warp, 421k cycles; cut over
 // the four sub-partitions, with 32 lanes on the elimination and equal operations of
 // different quantities in the same instructions, it is about 1,400 on the longest warp,
-// 123k cycles, and 1,150, 106k cycles, while a block has one or two paths (PairCx). The
-// FP32 step went from 105k to 19k. With every SM full the FP64 work per path falls as
+// 123k cycles, and 1,150, 105k cycles, while a block has one or two paths (PairCx). The
+// FP32 step went from 105k to 16k. With every SM full the FP64 work per path falls as
 // well (fewer repeated sums and idle lanes): FP64 rounds of 32,768 paths, three in flight,
 // 6,815 to 3,696 ms a round. Comparisons, maxima and stored negations of FP64 values run
 // on their bit patterns in the integer pipes for the same reason.

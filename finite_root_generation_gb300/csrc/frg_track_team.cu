@@ -286,10 +286,10 @@ __device__ __forceinline__ void eval_quarter(Smem<T, P>& E, int quarter, int g) 
 // the FP32 stage (by the queue's length, frg_team_grid). The warps work in parts of four:
 // part k evaluates its four paths together. All warps of a block step in time, and in the
 // FP32 stage, which is bound by instruction fetch once the SM is full, that is what lets
-// them share it: 65,536-path rounds, four in flight, take 1,884 ms with four blocks of
-// 4 warps per SM, 1,701 with two of 8, 1,569 with one of 16 (9,600 paths alone: 382,
-// 354, 337 ms); with few paths the barriers of larger blocks only cost (140 paths: 126
-// against 136 ms).
+// them share it: 65,536-path rounds, four in flight, take 1,560 ms with four blocks of
+// 4 warps per SM, 1,416 with two of 8, 1,324 with one of 16 (9,600 paths' FP32 stage: 291,
+// 279, 257 ms); with few paths the barriers of larger blocks only cost (140 paths: 126
+// against 136 ms when this was measured).
 template <int MODE, typename T, typename P = typename PointOf<T>::type>
 __global__ void __launch_bounds__(sizeof(T) == 8 ? 32 * PATHS : 512, sizeof(T) == 8 ? 2 : 1)
 team_kernel(TrackArgs a) {
