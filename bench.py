@@ -594,9 +594,9 @@ def run_ours(args, rank, world):
 FRG_COUNTERS_BYTES = 48 * 8
 # DRAM bytes (read + write) per path of the two tracking stages, from one ncu capture of a
 # 4,096-path round of the chosen configuration (`bench.py --profile-case`, MemoryWorkloadAnalysis):
-# 11.67 MB for the FP32 stage and 29.85 MB for the FP64 stage; a round's traffic is taken to
+# 4.36 MB for the FP32 stage and 11.19 MB for the FP64 stage; a round's traffic is taken to
 # grow in proportion to its paths
-TRAFFIC_PER_PATH = {"fp32_stage": 11.67e6 / 4096, "fp64_stage": 29.85e6 / 4096}
+TRAFFIC_PER_PATH = {"fp32_stage": 4.36e6 / 4096, "fp64_stage": 11.19e6 / 4096}
 
 
 # ------------------------------------------------------------------- CPU baseline
