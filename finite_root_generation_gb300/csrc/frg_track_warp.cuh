@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
   for (int i = threadIdx.x; i < NV_ * NY_ + NV_; i += blockDim.x) outs[i] = S::tape_out()[i];
   for (int i = lane; i < S::TAPE_REGS; i += 32) W.reg[i] = cx<T>(T(0));
   __syncthreads();
-  if (lane < S::TAPE_CONSTS) W.reg[NZ_ + 2 * NP_ + lane] = cx<T>(T(S::tape_const()[lane]));
+  for (int i = lane; i < S::TAPE_CONSTS; i += 32) W.reg[NZ_ + 2 * NP_ + i] = cx<T>(T(S::tape_const()[i]));
   const T newt_tol = LO ? T(c.newt_tol_lo) : T(c.newt_tol);
   const int64_t ntail = a.from_tail ? (int64_t)*a.tail_count : 0;
   const int64_t nqueue = a.from_tail ? (ntail < a.tail_cap ? ntail : a.tail_cap)
