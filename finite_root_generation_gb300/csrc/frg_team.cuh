@@ -329,36 +329,37 @@ __device__ __forceinline__ T patch_scale(const cx<T>* u, int lane) {
   return T(1) / m.value();
 }
 
-// Pivot search: the row with the largest v (ties: the lowest). Row r's value is on lane
-// base + r, v >= 0, or -1 for used rows; the other lanes hold -1. Infinite and NaN candidates take the
-// comparisons one by one, as lane 0 sees them.
-template <int RP, typename T>
-__device__ __noinline__ int pivot_row_nonfinite(T v, int base, int r) {
-  const T v0 = __shfl_sync(FULL, v, base + (r & ~1)), v1 = __shfl_sync(FULL, v, base + (r | 1));
-  T bv = v0 >= v1 ? v0 : v1;
-  int bk = (r & ~1) + (v0 >= v1 ? 0 : 1);
-  for (int off = RP / 2; off >= 2; off >>= 1) {
-    const T ov = __shfl_xor_sync(FULL, bv, off);
-    const int ok = __shfl_xor_sync(FULL, bk, off);
-    if (ov > bv || (ov == bv && ok < bk)) { bv = ov; bk = ok; }
-  }
-  return __shfl_sync(FULL, bk, 0);
+// Pivot search: the row with the largest v (ties: the lowest), as its lane's bit. Row r's
+// value is on lane base + r, v >= 0 or NaN, or -1 for used rows; the other lanes hold -1. As
+// integers the values' bits have their order, with a NaN of negative sign between the
+// used rows and zero; one of positive sign, which would come out above infinity, is put there
+// too, in a search of its own: a used row must never win, or a later part of the elimination
+// finds more unused rows than it has room for.
+__device__ __noinline__ unsigned pivot_lane_nan(float v) {
+  const int key = v == v ? __float_as_int(v) : -1;
+  const unsigned c = __ballot_sync(FULL, key == __reduce_max_sync(FULL, key));
+  return c & (0u - c);
 }
-// The pivot's lane as a bit (the lowest of equal ones).
-template <int RP>
-__device__ __forceinline__ unsigned pivot_lane(float v, int base, int r) {
+__device__ __noinline__ unsigned pivot_lane_nan(double v) {
+  const int hi = v == v ? __double2hiint(v) : -1;
+  const unsigned lo = v == v ? (unsigned)__double2loint(v) : 0u;
+  const int m = __reduce_max_sync(FULL, hi);
+  const unsigned ml = __reduce_max_sync(FULL, hi == m ? lo : 0u);
+  const unsigned c = __ballot_sync(FULL, hi == m && lo == ml);
+  return c & (0u - c);
+}
+__device__ __forceinline__ unsigned pivot_lane(float v) {
   const int key = __float_as_int(v);
   const int m = __reduce_max_sync(FULL, key);
-  if (m >= 0x7f800000) return 1u << (base + pivot_row_nonfinite<RP>(v, base, r));
+  if (m > 0x7f800000) return pivot_lane_nan(v);
   const unsigned c = __ballot_sync(FULL, key == m);
   return c & (0u - c);
 }
-template <int RP>
-__device__ __forceinline__ unsigned pivot_lane(double v, int base, int r) {
+__device__ __forceinline__ unsigned pivot_lane(double v) {
   const int hi = __double2hiint(v);
   const unsigned lo = (unsigned)__double2loint(v);
   const int m = __reduce_max_sync(FULL, hi);
-  if (m >= 0x7ff00000) return 1u << (base + pivot_row_nonfinite<RP>(v, base, r));
+  if (m >= 0x7ff00000) return pivot_lane_nan(v);
   unsigned c = __ballot_sync(FULL, hi == m);
   if (c & (c - 1)) {
     const unsigned ml = __reduce_max_sync(FULL, hi == m ? lo : 0u);
@@ -398,7 +399,7 @@ __device__ __forceinline__ void lu_stage(cx<T>* U, T* pn, cx<T>* pv, int k0, int
     // FP32: every candidate's reciprocal is taken while the pivot is searched for
     cx<T> ip = R[0];
     if constexpr (sizeof(T) == 4) ip = cinv(cand ? R[0] : cx<T>(T(1)));
-    const unsigned pl = pivot_lane<RP>(v, base, r);
+    const unsigned pl = pivot_lane(v);
     cx<T>* Uk = U + k * LDU + k + 1 + ((h - (k + 1)) & (CL - 1));
     cx<T> X[W], pivot[W];
 #pragma unroll
