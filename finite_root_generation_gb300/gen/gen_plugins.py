@@ -48,11 +48,14 @@ def load_plugins():
 
 class Printer:
     """Straight-line printer for the two dialects: 'cuda' (cx<T> with operators) and
-    'c' (the oracle's cd struct with cadd/csub/cmul/cscal/mk)."""
+    'c' (the oracle's cd struct with cadd/csub/cmul/cscal/mk). `rounded`: a real multiple that
+    is not exact is a product of its own (mul_rn), which the compiler cannot fuse with the
+    sum it enters."""
 
-    def __init__(self, dialect, names):
+    def __init__(self, dialect, names, rounded=False):
         self.d = dialect
         self.names = names
+        self.rounded = rounded
 
     def num(self, v):
         v = float(v)
@@ -61,7 +64,9 @@ class Printer:
     def scale(self, c, body):
         c = float(c)
         if self.d == "cuda":
-            return f"(-({body}))" if c == -1.0 else f"(T({c!r}) * ({body}))"
+            if c == -1.0:
+                return f"(-({body}))"
+            return f"mul_rn(T({c!r}), {body})" if self.rounded and abs(c) != 2.0 else f"(T({c!r}) * ({body}))"
         return f"cscal({c!r}, {body})"
 
     def mul(self, parts):
@@ -181,7 +186,7 @@ def emit_rows(mod, info, dialect):
     repl, red = cse_block(flat, "r_")
     for s_, _ in repl:
         names[s_] = s_.name
-    pr = Printer(dialect, names)
+    pr = Printer(dialect, names, rounded=True)  # as the schedule has it
     used = set()
     for _, e in repl:
         used |= e.free_symbols
@@ -273,7 +278,8 @@ class Tape:
     component) take one operation each, so a step is up to WIDTH products or sums that do not
     depend on each other. Operations, operand order and the association of sums and products
     are the printed code's; a minus sign travels with a value's use ((-a) b = -(a b) and
-    (-a) + b = -(a - b) round alike), so the results are the same bit for bit."""
+    (-a) + b = -(a - b) round alike), so the results are the same bit for bit. A real multiple
+    is rounded before it enters a sum (unless it is exact), and so it is in the printed code."""
 
     WIDTH = 16
 

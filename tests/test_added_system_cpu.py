@@ -3,11 +3,12 @@ on the CPU: the two tracking kernels of a plug-in (a path per thread, a path per
 the same computation, so a path must come out of both alike, whatever kernel its call's size
 selects. The kernels' own source runs here (tests/warp_emu): each path starts, takes a few
 steps and ends on the step limit (FP64) or is still in hand at it (FP32 stage)."""
+import importlib.util
 import os
 import re
 import subprocess
-import types
 
+import numpy as np
 import pytest
 
 import finite_root_generation_gb300 as frg
@@ -20,13 +21,93 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(gen_plugins.__file__), "..", "csrc")
 
 
-def numeric_quadrics():
-    """Four quadrics in four unknowns with coefficients that are numbers, 65 of them different."""
-    x = sp.symbols("x0:4")
-    c = sp.symbols("c0:4")
-    mono = [x[i] * x[j] for i in range(4) for j in range(i, 4)] + list(x)
-    eqs = [sum(sp.Rational((m + 2) ** (k + 2) % 97, 32) * t for m, t in enumerate(mono)) + c[k] for k in range(4)]
-    return types.SimpleNamespace(NAME="numeric4", UNKNOWNS=list(x), PARAMS=list(c), EQUATIONS=eqs, SOLVED=list(c))
+def system(name):
+    """tests/added_systems/<name>.py, as a user's module."""
+    spec = importlib.util.spec_from_file_location(name, os.path.join(HERE, "added_systems", name + ".py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+class Value:
+    """A single-precision complex value."""
+
+    def __init__(self, v):
+        self.v = np.complex64(v.v if isinstance(v, Value) else v)
+
+    def __mul__(self, o):
+        return Value(self.v * Value(o).v)
+
+    def __add__(self, o):
+        return o.plus(self, 1) if isinstance(o, Multiple) else Value(self.v + o.v)
+
+    def __sub__(self, o):
+        return o.plus(self, -1) if isinstance(o, Multiple) else Value(self.v - o.v)
+
+    def __neg__(self):
+        return Value(-self.v)
+
+
+class Multiple(Value):
+    """c x, rounded where it is used; a sum that it enters may take it unrounded (fused)."""
+
+    fused = False
+
+    def __init__(self, c, x):
+        super().__init__(np.complex64(complex(c * x.v.real, c * x.v.imag)))
+        self.c, self.x = c, x
+
+    def plus(self, o, sign):
+        if not self.fused:
+            return Value(o.v + np.float32(sign) * self.v)
+        c, x = np.float64(sign * self.c), np.complex128(self.x.v)  # the product is exact in double precision
+        return Value(complex(np.float32(c * x.real + o.v.real), np.float32(c * x.imag + o.v.imag)))
+
+    def __add__(self, o):
+        return self.plus(Value(o), 1)
+
+    def __sub__(self, o):
+        return self.plus(Value(-o), 1)
+
+    def __neg__(self):
+        return Multiple(-self.c, self.x)
+
+
+class Real:
+    def __init__(self, c):
+        self.c = np.float32(c)
+
+    def __mul__(self, x):
+        return Multiple(self.c, x)
+
+
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("name", ["numeric4", "cubic2"])
+def test_schedule_rounds_as_the_code_does(name, fused, monkeypatch):
+    """Whether or not the compiler fuses the code's real multiples into the sums they enter, the
+    warp's schedule has the same values bit for bit."""
+    monkeypatch.setattr(Multiple, "fused", fused)
+    mod = system(name)
+    info = gen_plugins.analyse(mod)
+    tape = gen_plugins.Tape(info)
+    code = "\n".join(gen_plugins.emit_rows(mod, info, "cuda")).replace("cx<T>", "cx")
+    rng = np.random.default_rng(3)
+    for _ in range(10):
+        Y, q, dq = ([Value(complex(*rng.normal(size=2))) for _ in range(n)]
+                    for n in (info["nv"] + 1, info["np"], info["np"]))
+        env = dict(Y=Y, q=q, dq=dq, T=Real, mul_rn=lambda c, x: Value(Multiple(c.c, Value(x))),
+                   cx=lambda c: Value(complex(c.c)))
+        for var, e in re.findall(r"const cx (\w+) = (.*?);", code):
+            env[var] = eval(e, {}, env)
+        want = [Value(eval(e, {}, env)).v for e in re.findall(r"[MF]\[.*?\] = (.*?);", code)]
+        reg = [v.v for v in Y + q + dq] + [np.complex64(c) for c in tape.consts]
+        reg += [np.complex64(0)] * (tape.nregs - len(reg))
+        words = tape.words()
+        for s in range(0, len(words), tape.WIDTH):
+            new = [(w & 1023, reg[(w >> 10) & 1023], reg[(w >> 20) & 1023], w >> 30) for w in words[s:s + tape.WIDTH]]
+            for d, a, b, kind in new:
+                reg[d] = a * b if kind >> 1 else (a - b if kind & 1 else a + b)
+        assert [-reg[w & 1023] if w >> 10 else reg[w & 1023] for w in tape.out_words()] == want
 
 
 def kernels_agree(mod, tmp_path, monkeypatch):
@@ -49,6 +130,6 @@ def kernels_agree(mod, tmp_path, monkeypatch):
     return r.returncode == 0
 
 
-@pytest.mark.parametrize("system", [numeric_quadrics], ids=lambda s: s.__name__)
-def test_kernels_of_an_added_system_agree(system, tmp_path, monkeypatch):
-    assert kernels_agree(system(), tmp_path, monkeypatch)
+@pytest.mark.parametrize("name", ["numeric4", "cubic2"])
+def test_kernels_of_an_added_system_agree(name, tmp_path, monkeypatch):
+    assert kernels_agree(system(name), tmp_path, monkeypatch)
