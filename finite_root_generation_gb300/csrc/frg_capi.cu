@@ -400,10 +400,12 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   // persistent grids: SMs x resident blocks, capped by the work
   const bool plugin = ctx->cfg.system != 0;
   int plugin_bps[3] = {0, 0, 0}, warp_bps[3] = {0, 0, 0};  // a plug-in system's kernels have their own occupancy
+  bool warps = plugin;  // its warp kernels exist and fit an SM
   if (plugin)
     for (int m = 0; m < (mixed ? 3 : 1); ++m) {
       FRG_CUDA(ctx, frg_track_occupancy_system(ctx->cfg.system, m, &plugin_bps[m]));
       FRG_CUDA(ctx, frg_warp_occupancy(ctx->cfg.system, m, &warp_bps[m]));
+      warps = warps && warp_bps[m] > 0;
     }
   auto grid_for = [&](int mode, int64_t n) {
     int bps = ctx->cfg.blocks_per_sm > 0             ? ctx->cfg.blocks_per_sm
@@ -413,19 +415,19 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   };
   // A plug-in's launch of up to FRG_WARP_PATHS paths per SM sub-partition takes a warp
   // per path; a larger one a thread per path, and then a warp for each of its last paths.
-  const bool by_warp = plugin && N <= (int64_t)ctx->sm_count * 4 * FRG_WARP_PATHS;
+  const bool by_warp = warps && N <= (int64_t)ctx->sm_count * 4 * FRG_WARP_PATHS;
   auto tail_cap = [&](int mode) -> int64_t {
     return (int64_t)grid_for(mode, N) * (FRG_TRACK_THREADS / 32) * frg_tail_lanes(mode == 1);
   };
-  if (plugin && !by_warp)  // the stages take turns with it; sized before the first launch
+  if (warps && !by_warp)  // the stages take turns with it; sized before the first launch
     FRG_CUDA(ctx, sl.tail.ensure(sizeof(frg::Handoff) * (size_t)(mixed ? std::max(tail_cap(1), tail_cap(2)) : tail_cap(0))));
   auto launch = [&](int mode) -> cudaError_t {
     if (team) return frg_launch_team(mode, a, team_grid(ctx, mode, N), st);
     const int grid = grid_for(mode, N);
-    const int wcap = plugin ? ctx->sm_count * (ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : warp_bps[mode])
-                            : 0;
+    const int wcap = warps ? ctx->sm_count * (ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : warp_bps[mode])
+                           : 0;
     if (by_warp) return frg_launch_warp(mode, a, (int)std::min<int64_t>(wcap, (N + 3) / 4), st);
-    if (!plugin) return frg_launch_track(mode, a, grid, st);
+    if (!warps) return frg_launch_track(mode, a, grid, st);
     frg::TrackArgs b = a;
     b.tail_cap = tail_cap(mode);
     b.tail = (frg::Handoff*)sl.tail.p;

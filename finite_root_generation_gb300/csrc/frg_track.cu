@@ -623,15 +623,36 @@ cudaError_t frg_launch_track(int mode, const frg::TrackArgs& args, int grid, cud
 }
 
 namespace {
+// more than 48 KB of shared memory has to be asked for
 template <int MODE, typename T, class S>
-cudaError_t launch_warp(const frg::TrackArgs& args, int grid, cudaStream_t stream) {
-  frg::warp_kernel<MODE, T, S><<<grid, 32 * frg::WARP_PATHS, 0, stream>>>(args);
-  return cudaGetLastError();
+cudaError_t warp_limit() {
+  constexpr size_t bytes = sizeof(frg::WarpShared<T, S>);
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(frg::warp_kernel<MODE, T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 template <int MODE, typename T, class S>
+cudaError_t launch_warp(const frg::TrackArgs& args, int grid, cudaStream_t stream) {
+  if constexpr (!frg::warp_fits<S>()) {
+    return cudaErrorInvalidValue;
+  } else {
+    const cudaError_t e = warp_limit<MODE, T, S>();
+    if (e != cudaSuccess) return e;
+    frg::warp_kernel<MODE, T, S><<<grid, 32 * frg::WARP_PATHS, sizeof(frg::WarpShared<T, S>), stream>>>(args);
+    return cudaGetLastError();
+  }
+}
+// 0 for a system whose blocks do not fit an SM
+template <int MODE, typename T, class S>
 cudaError_t warp_occ(int* blocks_per_sm) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, frg::warp_kernel<MODE, T, S>,
-                                                       32 * frg::WARP_PATHS, 0);
+  *blocks_per_sm = 0;
+  if constexpr (!frg::warp_fits<S>()) {
+    return cudaSuccess;
+  } else {
+    const cudaError_t e = warp_limit<MODE, T, S>();
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, frg::warp_kernel<MODE, T, S>,
+                                                         32 * frg::WARP_PATHS, sizeof(frg::WarpShared<T, S>));
+  }
 }
 }  // namespace
 

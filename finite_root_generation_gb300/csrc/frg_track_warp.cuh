@@ -40,6 +40,19 @@ struct WarpPath {
   T cn[NY];
 };
 
+// Shared memory of a block.
+template <typename T, class S>
+struct WarpShared {
+  WarpPath<T, S> paths[WARP_PATHS];
+  uint32_t tape[S::TAPE_STEPS * 16];
+  uint16_t outs[S::NV * (S::NV + 2) + S::NV];
+};
+
+// Whether a block of system S fits an SM (FP64, the larger): the shipped systems take 15
+// and 35 KB; one that does not fit runs on track_kernel alone.
+template <class S>
+constexpr bool warp_fits() { return sizeof(WarpShared<double, S>) <= 227 * 1024; }
+
 template <typename T>
 struct WarpStep {
   T ratio;  // pivot ratio (FP32 stage)
@@ -320,13 +333,14 @@ __global__ void __launch_bounds__(32 * WARP_PATHS) warp_kernel(TrackArgs a) {
   typedef WarpPath<T, S> P;
   constexpr int NV_ = P::NV, NZ_ = P::NZ, NY_ = P::NY, NP_ = P::NP;
   constexpr bool LO = (MODE == MODE_LO);
-  __shared__ P paths[WARP_PATHS];
-  __shared__ uint32_t tape[S::TAPE_STEPS * 16];
-  __shared__ uint16_t outs[NV_ * NY_ + NV_];
+  extern __shared__ __align__(16) unsigned char warp_smem[];
+  WarpShared<T, S>& sh = *reinterpret_cast<WarpShared<T, S>*>(warp_smem);
+  uint32_t* const tape = sh.tape;
+  uint16_t* const outs = sh.outs;
   const frg_config& c = a.cfg;
   const int lane = threadIdx.x & 31;
   const bool el = lane < NY_;
-  P& W = paths[threadIdx.x >> 5];
+  P& W = sh.paths[threadIdx.x >> 5];
   for (int i = threadIdx.x; i < S::TAPE_STEPS * 16; i += blockDim.x) tape[i] = S::tape()[i];
   for (int i = threadIdx.x; i < NV_ * NY_ + NV_; i += blockDim.x) outs[i] = S::tape_out()[i];
   for (int i = lane; i < S::TAPE_REGS; i += 32) W.reg[i] = cx<T>(T(0));

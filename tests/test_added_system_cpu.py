@@ -12,8 +12,9 @@ import numpy as np
 import pytest
 
 import finite_root_generation_gb300 as frg
+from finite_root_generation_gb300 import build as frg_build
 
-sp = pytest.importorskip("sympy")
+pytest.importorskip("sympy")
 
 from finite_root_generation_gb300.gen import gen_plugins  # noqa: E402
 
@@ -110,14 +111,21 @@ def test_schedule_rounds_as_the_code_does(name, fused, monkeypatch):
         assert [-reg[w & 1023] if w >> 10 else reg[w & 1023] for w in tape.out_words()] == want
 
 
-def kernels_agree(mod, tmp_path, monkeypatch):
+def write_sources(mod, tmp_path, monkeypatch, smem):
+    """The system's generated header and the tracking kernels' sources without the calls that
+    need a GPU, shared memory being declared as `smem`."""
     monkeypatch.setattr(gen_plugins, "load_plugins", lambda: [mod])
-    with open(tmp_path / "frg_plugins_gen.cuh", "w") as f:
-        f.write(gen_plugins.generate()[0])
-    track = open(os.path.join(CSRC, "frg_track.cu")).read()
-    track = re.sub(r"[\w:]+(<[^<>;]*>)?<<<.*?>>>\(.*?\);", ";", track)
-    assert "<<<" not in track
-    (tmp_path / "track.inc").write_text(track)
+    (tmp_path / "frg_plugins_gen.cuh").write_text(gen_plugins.generate()[0])
+    for src, dst in (("frg_track.cu", "track.inc"), ("frg_track_warp.cuh", "frg_track_warp.cuh")):
+        text = open(os.path.join(CSRC, src)).read()
+        text = re.sub(r"[\w:]+(<[^<>;]*>)?<<<.*?>>>\(.*?\);", ";", text)
+        text = re.sub(r"return cuda(Occupancy|Func)[^;]*;", "return cudaSuccess;", text)
+        assert "<<<" not in text
+        (tmp_path / dst).write_text(text.replace("extern __shared__ __align__(16) unsigned char warp_smem[];", smem))
+
+
+def kernels_agree(mod, tmp_path, monkeypatch):
+    write_sources(mod, tmp_path, monkeypatch, "unsigned char* const warp_smem = emu::smem();")
     cfg = frg.plugin_config("conic2", start_dist=frg.START_NORMAL, max_steps=4)
     (tmp_path / "config").write_bytes(bytes(cfg))
     exe = tmp_path / "kernels"
@@ -130,6 +138,19 @@ def kernels_agree(mod, tmp_path, monkeypatch):
     return r.returncode == 0
 
 
-@pytest.mark.parametrize("name", ["numeric4", "cubic2"])
+@pytest.mark.parametrize("name", ["numeric4", "cubic2", "sparse12"])
 def test_kernels_of_an_added_system_agree(name, tmp_path, monkeypatch):
     assert kernels_agree(system(name), tmp_path, monkeypatch)
+
+
+def test_static_shared_memory_of_a_large_system(tmp_path, monkeypatch):
+    """At most the 48 KB that a kernel may have without asking, whatever the system's size."""
+    write_sources(system("sparse12"), tmp_path, monkeypatch, "extern __shared__ __align__(16) unsigned char warp_smem[];")
+    (tmp_path / "warp.cu").write_text(
+        '#include "track.inc"\n'
+        "template __global__ void frg::warp_kernel<frg::MODE_PLAIN, double, frg::Sys_sparse12>(frg::TrackArgs);\n")
+    r = subprocess.run([frg_build.nvcc(), *frg_build.ARCH, "-std=c++17", "--expt-relaxed-constexpr", f"-I{tmp_path}",
+                        f"-I{CSRC}", "-Xcicc", "-O1", "-Xptxas", "-O1,-v", "-c", str(tmp_path / "warp.cu"), "-o",
+                        str(tmp_path / "warp.o")], capture_output=True, text=True, check=True)
+    assert "warp_kernel" in r.stderr
+    assert all(int(n) <= 48 * 1024 for n in re.findall(r"(\d+) bytes smem", r.stderr))

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 PKG = "finite_root_generation_gb300"
-SYSTEMS = ["numeric4", "cubic2"]
+SYSTEMS = ["numeric4", "cubic2", "sparse12"]
 
 RUN = """
 import sys

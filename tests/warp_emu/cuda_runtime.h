@@ -67,6 +67,7 @@ struct Block {
 };
 inline Block* B = nullptr;
 
+inline unsigned char* smem() { return (unsigned char*)(((uintptr_t)B->smem.data() + 15) & ~(uintptr_t)15); }
 inline void yield() {
   const int from = B->cur, n = (int)B->done.size();
   for (int k = 1; k <= n; ++k) {

@@ -42,7 +42,7 @@ bool compare(const char* what, int n, const frg_config& cfg) {
     emu::launch((n + FRG_TRACK_THREADS - 1) / FRG_TRACK_THREADS, FRG_TRACK_THREADS, 0,
                 [&] { frg::plugin_start_kernel<S>(a, o.starts.data()); });
     if (k == 0) emu::launch(1, FRG_TRACK_THREADS, 0, [&] { frg::track_kernel<MODE, T, S>(a); });
-    else emu::launch(1, 32 * frg::WARP_PATHS, 0, [&] { frg::warp_kernel<MODE, T, S>(a); });
+    else emu::launch(1, 32 * frg::WARP_PATHS, sizeof(frg::WarpShared<T, S>), [&] { frg::warp_kernel<MODE, T, S>(a); });
   }
   int moved = 0;
   for (int i = 0; i < n; ++i) moved += got[0].work[3 * i + 2] > 0 || got[0].handoff[i].step > 0;
