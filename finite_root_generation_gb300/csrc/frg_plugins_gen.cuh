@@ -16,21 +16,21 @@ namespace frg {
 // rows(): 48 complex mul, 32 complex add/sub, 3 real x complex; as a warp's schedule
 // 83 operations in 8 steps
 static __device__ const uint32_t tape_conic2[128] = {
-    0x80100024u, 0x80000026u, 0x80100427u, 0x80200825u, 0x8060081cu, 0x80000822u, 0x80c00828u, 0x8010101du, 
-    0x80100823u, 0x80102829u, 0x8070081fu, 0x80d0082au, 0x8000102eu, 0x80001832u, 0x80101c33u, 0x80002845u, 
-    0x82603c37u, 0x82404038u, 0x8260544eu, 0x8240584fu, 0x82600c59u, 0x8270145au, 0x82602464u, 0x82702c65u, 
-    0x8270443au, 0x82705c51u, 0x8250205cu, 0x82503867u, 0x8220483cu, 0x82206053u, 0x8000705eu, 0x8000a069u, 
-    0x380dc39u, 0x4f13850u, 0x5a1645bu, 0x6519066u, 0x1eu, 0x100420u, 0x200821u, 0x1d0702bu, 0x2e07c2fu, 0x330c834u, 
-    0x290a042u, 0x450a846u, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x3a0e43bu, 0x5114052u, 0x5c16c5du, 0x6719868u, 0x6fu, 
-    0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x82304c3eu, 0x80003049u, 
-    0x8010344au, 0x82306455u, 0x80007460u, 0x8000a46bu, 0x81e00c2cu, 0x82001430u, 0x82102035u, 0x82505040u, 
-    0x81e02443u, 0x82002c47u, 0x8210384cu, 0x82506857u, 0x80107c62u, 0x8010a86du, 0x3c0ec3du, 0x5314854u, 
-    0x5e1745fu, 0x691a06au, 0x4a1244bu, 0x2c0ac2du, 0x300bc31u, 0x350d036u, 0x4310844u, 0x4711848u, 0x6fu, 0x6fu, 
-    0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x3e0f43fu, 0x5515056u, 0x6017c61u, 0x6b1a86cu, 0x4c12c4du, 0x6fu, 0x6fu, 0x6fu, 
-    0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x400fc41u, 0x5715858u, 0x6218463u, 0x6d1b06eu, 0x6fu, 
-    0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu, 0x6fu};
+    0x8010001cu, 0x8000001du, 0x8010041eu, 0x8020081fu, 0x80600820u, 0x80000821u, 0x80c00822u, 0x80101023u, 
+    0x80100824u, 0x80102825u, 0x80700826u, 0x80d00827u, 0x80001028u, 0x80001829u, 0x80101c2au, 0x8000282bu, 
+    0x81d03c2cu, 0x81c0402du, 0x81d0542eu, 0x81c0582fu, 0x81d00c30u, 0x81e01431u, 0x81d02432u, 0x81e02c33u, 
+    0x81e04434u, 0x81e05c35u, 0x81f02036u, 0x81f03837u, 0x82104838u, 0x82106039u, 0x8000803au, 0x8000883bu, 
+    0x2d0b01cu, 0x2f0b81du, 0x310c01eu, 0x330c821u, 0x3cu, 0x10043du, 0x20083eu, 0x230803fu, 0x2809840u, 0x2a0a441u, 
+    0x2508842u, 0x2b09c43u, 0x44u, 0x44u, 0x44u, 0x44u, 0x3407020u, 0x3507422u, 0x3607828u, 0x3708429u, 0x44u, 
+    0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x82404c2au, 0x8000302bu, 
+    0x8010342cu, 0x8240642du, 0x80008c2eu, 0x8000942fu, 0x83c00c30u, 0x83d01431u, 0x83e02032u, 0x81f05033u, 
+    0x83c0241cu, 0x83d02c1du, 0x83e0381eu, 0x81f06821u, 0x80109834u, 0x80109c35u, 0x3808036u, 0x3908837u, 
+    0x3a0a01fu, 0x3b0a423u, 0x2c0ac24u, 0x300fc25u, 0x3110026u, 0x3210427u, 0x1c1083cu, 0x1d10c3du, 0x44u, 0x44u, 
+    0x44u, 0x44u, 0x44u, 0x44u, 0x2a0d83eu, 0x2d0dc1cu, 0x2e07c1du, 0x2f08c20u, 0x1e09022u, 0x44u, 0x44u, 0x44u, 
+    0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x330f828u, 0x2107029u, 0x340742bu, 0x350802cu, 0x44u, 
+    0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u, 0x44u};
 static __device__ const uint16_t tape_out_conic2[10] = {
-    45, 49, 54, 65, 68, 72, 77, 88, 99, 110};
+    37, 38, 39, 40, 60, 61, 34, 41, 43, 44};
 static __device__ const double tape_const_conic2[1] = {
     0.0};
 struct Sys_conic2 {
@@ -39,7 +39,7 @@ struct Sys_conic2 {
   static constexpr int NP = 12;
   static constexpr int NS = 2;
   static constexpr int ROWS_CMUL = 48, ROWS_CADD = 32, ROWS_SMUL = 3;
-  static constexpr int TAPE_STEPS = 8, TAPE_REGS = 112, TAPE_CONSTS = 1;
+  static constexpr int TAPE_STEPS = 8, TAPE_REGS = 69, TAPE_CONSTS = 1;
   __device__ static const uint32_t* tape() { return tape_conic2; }
   __device__ static const uint16_t* tape_out() { return tape_out_conic2; }
   __device__ static const double* tape_const() { return tape_const_conic2; }
@@ -149,45 +149,44 @@ struct Sys_conic2 {
 // rows(): 158 complex mul, 101 complex add/sub, 5 real x complex; as a warp's schedule
 // 259 operations in 19 steps
 static __device__ const uint32_t tape_burmester5[304] = {
-    0x8030542fu, 0x80204033u, 0x80c01438u, 0x8020443bu, 0x80305c3fu, 0x80204843u, 0x80306047u, 0x80204c4bu, 
-    0x8030644fu, 0x80205053u, 0x80601434u, 0x80305837u, 0x80801444u, 0x8090144cu, 0x80a01454u, 0x80100058u, 
-    0x80501059u, 0x80b01430u, 0x8070143cu, 0x80d01440u, 0x80e01448u, 0x80f01450u, 0x8330bcddu, 0x83b0e0eeu, 
-    0x8430fcffu, 0x84b11d10u, 0x85313d21u, 0x8340bcdfu, 0x8370ecf0u, 0x8440fd01u, 0x84c11d12u, 0x85413d23u, 
-    0x4591605au, 0x42f00431u, 0x43800439u, 0x43f00441u, 0x44700449u, 0x44f00451u, 0x43300035u, 0x3c0ec3du, 
-    0x4410c45u, 0x4c12c4du, 0x5414c55u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0xdd168deu, 0xee168efu, 0xff16900u, 
-    0x11016911u, 0x12116922u, 0x4300c432u, 0x4370e43au, 0x44010442u, 0x4481244au, 0x45014452u, 0x4340d436u, 
-    0x4000f43eu, 0x40011446u, 0x4001344eu, 0x40015456u, 0x132u, 0x8330c0e1u, 0x8370f0f2u, 0x84310103u, 0x84b12114u, 
-    0x85314125u, 0x80b0005du, 0x80b04061u, 0x81a0146au, 0x81f0146cu, 0x80c00077u, 0x80c0447bu, 0x81b01484u, 
-    0x82001486u, 0x80d00091u, 0x80d04895u, 0x81c0149eu, 0x821014a0u, 0x80e000abu, 0x80e04cafu, 0x81d014b8u, 
-    0x822014bau, 0x80f000c5u, 0x80f050c9u, 0x81e014d2u, 0x823014d4u, 0x82f000e3u, 0x838000f4u, 0x83f00105u, 
-    0x84700116u, 0x84f00127u, 0x8060045fu, 0x80605464u, 0xdf378e0u, 0xf03bcf1u, 0x10140102u, 0x11244513u, 
-    0x12348924u, 0x5d0105eu, 0x7701078u, 0x9101092u, 0xab010acu, 0xc5010c6u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 
-    0x132u, 0x8320906fu, 0x80700479u, 0x8070587eu, 0x83a09489u, 0x80800493u, 0x80805c98u, 0x842098a3u, 0x809004adu, 
-    0x809060b2u, 0x84a09cbdu, 0x80a004c7u, 0x80a064ccu, 0x8520a0d7u, 0x830000e5u, 0x837000f6u, 0x84000107u, 
-    0xe1380e2u, 0xf23c4f3u, 0x10340904u, 0x11444d15u, 0x12549126u, 0x5f17860u, 0x791e07au, 0x9324894u, 0xad2b0aeu, 
-    0xc7318c8u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0x84800118u, 0x85000129u, 0x80501457u, 0x80218462u, 
-    0x8321a86bu, 0x8361b06du, 0x8360a472u, 0x8021ec7cu, 0x83a21085u, 0x83e21887u, 0x83e0a88cu, 0x80225496u, 
-    0x8422789fu, 0x846280a1u, 0x8460aca6u, 0x8022bcb0u, 0x84a2e0b9u, 0x84e2e8bbu, 0x84e0b0c0u, 0x802324cau, 
-    0x852348d3u, 0x856350d5u, 0x8560b4dau, 0x833004e7u, 0x80b018ebu, 0x83b004f8u, 0x80c01cfcu, 0x84300509u, 
-    0x80d0210du, 0x84b0051au, 0x80e0251eu, 0x8530052bu, 0x4e3388e4u, 0x4f43ccf5u, 0x50541106u, 0x51645517u, 
-    0x52749928u, 0x46218063u, 0x6d1ac6eu, 0x47c1e87du, 0x48721488u, 0x49625097u, 0x4a127ca2u, 0x4b02b8b1u, 
-    0x4bb2e4bcu, 0x4ca320cbu, 0x4d534cd6u, 0x132u, 0x80f0292fu, 0x80319065u, 0x80b0d067u, 0x8021bc70u, 0x8031f87fu, 
-    0x80c0f081u, 0x8022248au, 0x80326099u, 0x80d1109bu, 0x80228ca4u, 0x8032c8b3u, 0x80e130b5u, 0x8022f4beu, 
-    0x803330cdu, 0x80f150cfu, 0x80235cd8u, 0x4e5390e6u, 0x4f63d4f7u, 0x50741908u, 0x51845d19u, 0x5294a12au, 
-    0x46518c66u, 0x6719c68u, 0x701b871u, 0x47f1f480u, 0x8120482u, 0x8a2208bu, 0x49925c9au, 0x9b26c9cu, 0xa4288a5u, 
-    0x4b32c4b4u, 0xb52d4b6u, 0x834004e9u, 0x83c004fau, 0x8440050bu, 0x84c0051cu, 0x8540052du, 0x8031c873u, 
-    0x8032308du, 0x803298a7u, 0x803300c1u, 0x803368dbu, 0x8573acecu, 0x8573f0fdu, 0x8574350eu, 0x8574791fu, 
-    0x8574bd30u, 0x8320405bu, 0x4e7398e8u, 0x4f83dcf9u, 0x5094210au, 0x51a4651bu, 0x52b4a92cu, 0xbe2f0bfu, 
-    0x4cd32cceu, 0xcf33cd0u, 0xd8358d9u, 0x46819869u, 0x731c474u, 0x48220083u, 0x48d22c8eu, 0x49c2689du, 
-    0x4a7294a8u, 0x4b62d0b7u, 0x8360545cu, 0x83a04475u, 0x83e05876u, 0x8420488fu, 0x84605c90u, 0x84a04ca9u, 
-    0x84e060aau, 0x852050c3u, 0x856064c4u, 0x80000132u, 0x80000132u, 0x80000132u, 0x80000132u, 0x80000132u, 
-    0x80000132u, 0x80000132u, 0x4e93a0eau, 0x4fa3e4fbu, 0x50b4290cu, 0x51c46d1du, 0x52d4b12eu, 0x4c12fcc2u, 
-    0x4d0338d1u, 0x4db364dcu, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0xec3a8edu, 
-    0xfd3ecfeu, 0x10e4310fu, 0x11f47520u, 0x1304b931u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 0x132u, 
-    0x132u, 0x132u, 0x132u, 0x132u};
+    0x8030542fu, 0x80204030u, 0x80c01431u, 0x80204432u, 0x80305c33u, 0x80204834u, 0x80306035u, 0x80204c36u, 
+    0x80306437u, 0x80205038u, 0x80601439u, 0x8030583au, 0x8080143bu, 0x8090143cu, 0x80a0143du, 0x8010003eu, 
+    0x8050103fu, 0x80b01440u, 0x80701441u, 0x80d01442u, 0x80e01443u, 0x80f01444u, 0x8300bc45u, 0x8320c446u, 
+    0x8340cc47u, 0x8360d448u, 0x8380dc49u, 0x8390bc4au, 0x83a0c84bu, 0x83b0cc4cu, 0x83c0d44du, 0x83d0dc4eu, 
+    0x43f0f84fu, 0x42f00450u, 0x43100451u, 0x43300452u, 0x43500453u, 0x43700454u, 0x43000055u, 0x410c856u, 
+    0x3b0d057u, 0x3c0d858u, 0x3d0e059u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x4513c3eu, 0x4613c3fu, 0x4713c5au, 
+    0x4813c5bu, 0x4913c5cu, 0x4401405du, 0x43a1445eu, 0x4421485fu, 0x44314c60u, 0x44415061u, 0x43915462u, 
+    0x40015863u, 0x40015c64u, 0x40016065u, 0x40016466u, 0x89u, 0x83010045u, 0x83a10446u, 0x83410847u, 0x83610c48u, 
+    0x83811049u, 0x80b0004fu, 0x80b04050u, 0x81a01451u, 0x81f01452u, 0x80c00053u, 0x80c04454u, 0x81b01455u, 
+    0x82001456u, 0x80d00057u, 0x80d04858u, 0x81c01459u, 0x82101467u, 0x80e00068u, 0x80e04c69u, 0x81d0146au, 
+    0x8220146bu, 0x80f0006cu, 0x80f0506du, 0x81e0146eu, 0x8230146fu, 0x82f00070u, 0x83100071u, 0x83300072u, 
+    0x83500073u, 0x83700074u, 0x80600475u, 0x80605476u, 0x4a0f82fu, 0x4b0fc31u, 0x4c16833u, 0x4d16c35u, 0x4e17037u, 
+    0x4f01077u, 0x5301078u, 0x5701079u, 0x680107au, 0x6c0107bu, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 
+    0x85d0903eu, 0x8070043fu, 0x8070584au, 0x85e0944bu, 0x8080044cu, 0x80805c4du, 0x85f0984eu, 0x8090044fu, 
+    0x80906053u, 0x86009c57u, 0x80a0045au, 0x80a0645bu, 0x8610a05cu, 0x84000068u, 0x83a0006cu, 0x8420007cu, 
+    0x450bc3au, 0x460c440u, 0x470cc42u, 0x480d47du, 0x490dc7eu, 0x751dc7fu, 0x3f1e080u, 0x4c1e481u, 0x4f1e882u, 
+    0x5a1ec83u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x8430002fu, 0x84400031u, 0x80501433u, 0x80214035u, 
+    0x85d14437u, 0x8621483fu, 0x8620a445u, 0x80215046u, 0x85e15447u, 0x86315848u, 0x8630a849u, 0x8021604cu, 
+    0x85f1644fu, 0x86419c5au, 0x8640ac75u, 0x8021a477u, 0x8601a878u, 0x8651ac79u, 0x8650b07au, 0x8021b47bu, 
+    0x8611b843u, 0x8661bc44u, 0x8660b450u, 0x83000451u, 0x80b01852u, 0x83200454u, 0x80c01c55u, 0x83400456u, 
+    0x80d02058u, 0x83600459u, 0x80e02467u, 0x83800469u, 0x4700e830u, 0x47110032u, 0x47210834u, 0x4731f436u, 
+    0x4741f838u, 0x4351fc6au, 0x3f0dc6bu, 0x4462006du, 0x44811c6eu, 0x44c2046fu, 0x45a13c84u, 0x47720885u, 
+    0x4791e086u, 0x47b20c87u, 0x44410c88u, 0x89u, 0x80f02835u, 0x8031d837u, 0x80b0e43au, 0x8020f83fu, 0x80312840u, 
+    0x80c10442u, 0x80212c43u, 0x80313444u, 0x80d0ec46u, 0x80213847u, 0x80314c48u, 0x80e0f04cu, 0x80215c4fu, 
+    0x80316c5au, 0x80f0f470u, 0x80217071u, 0x4680c072u, 0x46c0c873u, 0x47c0d074u, 0x42f0d877u, 0x4310e078u, 
+    0x4371a879u, 0x3a0e87bu, 0x3f1ac7du, 0x4401b47eu, 0x421087fu, 0x431b880u, 0x4441bc81u, 0x4611882u, 0x4721083u, 
+    0x4482143eu, 0x4c1304au, 0x8390044bu, 0x8410044du, 0x83b0044eu, 0x83c00453u, 0x83d00457u, 0x8031145bu, 
+    0x8031245cu, 0x8031d476u, 0x8031e82fu, 0x80314030u, 0x83314831u, 0x83315432u, 0x83316034u, 0x83319c36u, 
+    0x8330d437u, 0x85d04038u, 0x4511c83au, 0x4541cc3fu, 0x4561d040u, 0x4591dc42u, 0x4691e043u, 0x4f21844u, 
+    0x45a21c46u, 0x701c047u, 0x7122048u, 0x47b1e44cu, 0x5b1f468u, 0x47f1f86au, 0x45c2006bu, 0x4822046cu, 
+    0x47620c6du, 0x44a0f86eu, 0x8620546fu, 0x85e0447cu, 0x86305884u, 0x85f04885u, 0x86405c33u, 0x86004c35u, 
+    0x86506039u, 0x8610503bu, 0x8660643cu, 0x80000089u, 0x80000089u, 0x80000089u, 0x80000089u, 0x80000089u, 
+    0x80000089u, 0x80000089u, 0x44b0e83du, 0x44d0fc41u, 0x44e10045u, 0x45310849u, 0x45710c50u, 0x42f11052u, 
+    0x44711855u, 0x43012058u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x310f467u, 0x3210475u, 
+    0x341147au, 0x361243eu, 0x371404au, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u, 0x89u};
 static __device__ const uint16_t tape_out_burmester5[40] = {
-    50, 54, 1115, 1116, 1029, 1129, 1140, 58, 1086, 1141, 118, 1029, 1155, 1166, 66, 1094, 1167, 144, 1029, 1181, 
-    1192, 74, 1102, 1193, 170, 1029, 1207, 1218, 82, 1110, 1219, 196, 1029, 1233, 1244, 237, 254, 271, 288, 305};
+    93, 98, 1080, 1135, 1029, 1100, 1128, 94, 1123, 1148, 132, 1029, 1130, 1131, 95, 1124, 1157, 51, 1029, 1132, 
+    1133, 96, 1125, 1077, 57, 1029, 1134, 1106, 97, 1126, 1083, 60, 1029, 1109, 1112, 103, 117, 122, 62, 74};
 static __device__ const double tape_const_burmester5[1] = {
     0.0};
 struct Sys_burmester5 {
@@ -196,7 +195,7 @@ struct Sys_burmester5 {
   static constexpr int NP = 20;
   static constexpr int NS = 5;
   static constexpr int ROWS_CMUL = 158, ROWS_CADD = 101, ROWS_SMUL = 5;
-  static constexpr int TAPE_STEPS = 19, TAPE_REGS = 307, TAPE_CONSTS = 1;
+  static constexpr int TAPE_STEPS = 19, TAPE_REGS = 138, TAPE_CONSTS = 1;
   __device__ static const uint32_t* tape() { return tape_burmester5; }
   __device__ static const uint16_t* tape_out() { return tape_out_burmester5; }
   __device__ static const double* tape_const() { return tape_const_burmester5; }

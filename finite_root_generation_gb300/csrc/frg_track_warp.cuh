@@ -48,10 +48,13 @@ struct WarpShared {
   uint16_t outs[S::NV * (S::NV + 2) + S::NV];
 };
 
-// Whether a block of system S fits an SM (FP64, the larger): the shipped systems take 15
-// and 35 KB; one that does not fit runs on track_kernel alone.
+// Whether system S has a schedule and a block of it fits an SM (FP64, the larger): the
+// shipped systems take 12 and 24 KB; one that does not fit runs on track_kernel alone.
 template <class S>
-constexpr bool warp_fits() { return sizeof(WarpShared<double, S>) <= 227 * 1024; }
+constexpr bool warp_fits() {
+  if constexpr (S::TAPE_STEPS == 0) return false;
+  else return sizeof(WarpShared<double, S>) <= 227 * 1024;
+}
 
 template <typename T>
 struct WarpStep {

@@ -279,9 +279,12 @@ class Tape:
     depend on each other. Operations, operand order and the association of sums and products
     are the printed code's; a minus sign travels with a value's use ((-a) b = -(a b) and
     (-a) + b = -(a - b) round alike), so the results are the same bit for bit. A real multiple
-    is rounded before it enters a sum (unless it is exact), and so it is in the printed code."""
+    is rounded before it enters a sum (unless it is exact), and so it is in the printed code.
+    A value's register is used again after its last use; a step writes none that it reads.
+    A system for which REGS registers do not suffice has no schedule (`fits` is false) and no
+    warp kernel."""
 
-    WIDTH = 16
+    WIDTH, REGS = 16, 1024  # registers are 10 bits of an operation's word
 
     def __init__(self, info):
         self.leaf, self.nodes, self.memo = {}, [], {}
@@ -354,7 +357,9 @@ class Tape:
 
     def reg(self, ref):
         kind, k = ref
-        return {"i": 0, "c": self.ninputs, "n": self.ninputs + len(self.consts)}[kind] + k
+        if kind == "n":
+            return self.ninputs + len(self.consts) + self.where[k]
+        return k + (self.ninputs if kind == "c" else 0)
 
     def schedule(self):
         """Steps of at most WIDTH ready operations of one kind, those with the longest chain
@@ -376,9 +381,22 @@ class Tape:
             self.steps.append(pick)
             done |= set(pick)
             left -= set(pick)
-        self.nregs = self.ninputs + len(self.consts) + len(self.nodes) + 1  # the last one takes idle lanes' results
-        if self.nregs > 1024:
-            raise ValueError("too many operations for the tape's 10-bit registers")
+        step_of = {k: n for n, pick in enumerate(self.steps) for k in pick}
+        ends = [[] for _ in self.steps]  # values whose last use a step is
+        kept = {r[1] for r, _ in self.outs if r[0] == "n"}
+        for k in range(len(self.nodes)):
+            if k not in kept:
+                ends[max((step_of[u] for u in users[k]), default=step_of[k])].append(k)
+        free, ntemps, self.where = [], 0, {}
+        for pick, end in zip(self.steps, ends):
+            for k in pick:
+                if not free:
+                    free.append(ntemps)
+                    ntemps += 1
+                self.where[k] = free.pop(0)
+            free += sorted(self.where[k] for k in end)
+        self.nregs = self.ninputs + len(self.consts) + ntemps + 1  # the last one takes idle lanes' results
+        self.fits = self.nregs <= self.REGS
 
     def words(self):
         """WIDTH words per step: dst | a << 10 | b << 20 | (b subtracted) << 30 | product << 31."""
@@ -409,14 +427,17 @@ def table(ctype, name, vals, fmt):
 
 def cuda_struct(mod, info, sid):
     cname = "Sys_" + mod.NAME
+    rows = emit_rows(mod, info, "cuda")
     cm, ca, sm = rows_cost(info)
     tape = Tape(info)
     out = [f"// ---- system {sid}: {mod.NAME} ({info['nv']} unknowns, {info['np']} parameters)",
            f"// rows(): {cm} complex mul, {ca} complex add/sub, {sm} real x complex; as a warp's schedule",
-           f"// {len(tape.nodes)} operations in {len(tape.steps)} steps"]
-    out += table("uint32_t", f"tape_{mod.NAME}", tape.words(), lambda v: f"{v:#x}u")
-    out += table("uint16_t", f"tape_out_{mod.NAME}", tape.out_words(), str)
-    out += table("double", f"tape_const_{mod.NAME}", tape.consts, repr)
+           f"// {len(tape.nodes)} operations in {len(tape.steps)} steps" if tape.fits else
+           f"// {len(tape.nodes)} operations in {tape.nregs} registers, too many: no warp kernel"]
+    if tape.fits:
+        out += table("uint32_t", f"tape_{mod.NAME}", tape.words(), lambda v: f"{v:#x}u")
+        out += table("uint16_t", f"tape_out_{mod.NAME}", tape.out_words(), str)
+        out += table("double", f"tape_const_{mod.NAME}", tape.consts, repr)
     out += [
            f"struct {cname} {{",
            f"  static constexpr int ID = {sid};",
@@ -425,13 +446,15 @@ def cuda_struct(mod, info, sid):
            f"  static constexpr int NS = {info['ns']};",
            f"  static constexpr int ROWS_CMUL = {cm}, ROWS_CADD = {ca}, ROWS_SMUL = {sm};",
            f"  static constexpr int TAPE_STEPS = {len(tape.steps)}, TAPE_REGS = {tape.nregs}, "
-           f"TAPE_CONSTS = {len(tape.consts)};",
+           f"TAPE_CONSTS = {len(tape.consts)};" if tape.fits else "  static constexpr int TAPE_STEPS = 0;"]
+    if tape.fits:
+        out += [
            f"  __device__ static const uint32_t* tape() {{ return tape_{mod.NAME}; }}",
            f"  __device__ static const uint16_t* tape_out() {{ return tape_out_{mod.NAME}; }}",
-           f"  __device__ static const double* tape_const() {{ return tape_const_{mod.NAME}; }}",
-           "  template <typename T, int LD>",
+           f"  __device__ static const double* tape_const() {{ return tape_const_{mod.NAME}; }}"]
+    out += ["  template <typename T, int LD>",
            "  __device__ static void rows(const cx<T>* Y, const cx<T>* q, const cx<T>* dq, cx<T>* M, cx<T>* F) {"]
-    out += ["  " + ln for ln in emit_rows(mod, info, "cuda")]
+    out += ["  " + ln for ln in rows]
     out += ["  }",
             "  __device__ static void start(Rng& rng, int dist, double range, cd* z, cd* q) {",
             "    typedef double T;"]

@@ -83,7 +83,7 @@ class Real:
 
 
 @pytest.mark.parametrize("fused", [False, True])
-@pytest.mark.parametrize("name", ["numeric4", "cubic2"])
+@pytest.mark.parametrize("name", ["numeric4", "cubic2", "products8"])
 def test_schedule_rounds_as_the_code_does(name, fused, monkeypatch):
     """Whether or not the compiler fuses the code's real multiples into the sums they enter, the
     warp's schedule has the same values bit for bit."""
@@ -105,7 +105,10 @@ def test_schedule_rounds_as_the_code_does(name, fused, monkeypatch):
         reg += [np.complex64(0)] * (tape.nregs - len(reg))
         words = tape.words()
         for s in range(0, len(words), tape.WIDTH):
-            new = [(w & 1023, reg[(w >> 10) & 1023], reg[(w >> 20) & 1023], w >> 30) for w in words[s:s + tape.WIDTH]]
+            step = words[s:s + tape.WIDTH]
+            written = {w & 1023 for w in step} - {tape.nregs - 1}
+            assert not written & {r for w in step for r in ((w >> 10) & 1023, (w >> 20) & 1023)}
+            new = [(w & 1023, reg[(w >> 10) & 1023], reg[(w >> 20) & 1023], w >> 30) for w in step]
             for d, a, b, kind in new:
                 reg[d] = a * b if kind >> 1 else (a - b if kind & 1 else a + b)
         assert [-reg[w & 1023] if w >> 10 else reg[w & 1023] for w in tape.out_words()] == want
@@ -138,9 +141,31 @@ def kernels_agree(mod, tmp_path, monkeypatch):
     return r.returncode == 0
 
 
-@pytest.mark.parametrize("name", ["numeric4", "cubic2", "sparse12"])
+@pytest.mark.parametrize("name", ["numeric4", "cubic2", "sparse12", "products8"])
 def test_kernels_of_an_added_system_agree(name, tmp_path, monkeypatch):
     assert kernels_agree(system(name), tmp_path, monkeypatch)
+
+
+def test_system_without_a_schedule_has_no_warp_kernel(tmp_path, monkeypatch):
+    """Too many values for the schedule's registers: the kernels compile, and the host is told
+    that no block of the warp kernel fits."""
+    monkeypatch.setattr(gen_plugins.Tape, "REGS", 50)
+    write_sources(system("cubic2"), tmp_path, monkeypatch, "unsigned char* const warp_smem = emu::smem();")
+    (tmp_path / "main.cpp").write_text("""#include "track.inc"
+int main() {
+  frg::TrackArgs a{};
+  a.cfg.system = 1;
+  for (int mode = 0; mode < 3; ++mode) {
+    int blocks = 7;
+    if (frg_warp_occupancy(1, mode, &blocks) != cudaSuccess || blocks != 0) return 1;
+    if (frg_launch_warp(mode, a, 1, nullptr) != cudaErrorInvalidValue) return 2;
+  }
+}
+""")
+    exe = str(tmp_path / "main")
+    subprocess.run(["g++", "-std=c++17", "-w", f"-I{tmp_path}", f"-I{os.path.join(HERE, 'warp_emu')}", f"-I{CSRC}",
+                    str(tmp_path / "main.cpp"), "-o", exe], check=True)
+    assert subprocess.run([exe]).returncode == 0
 
 
 def test_static_shared_memory_of_a_large_system(tmp_path, monkeypatch):
