@@ -41,6 +41,7 @@ namespace {
 constexpr int kReals = 2 * FRG_NV;
 constexpr unsigned long long kEmpty = ~0ull;
 constexpr int kThreads = 256;
+constexpr int64_t kMost = (int64_t)1 << 48;  // roots: more fit no GPU, and their bytes may not fit 64 bits
 
 struct DcollDev {
   double* roots;                  // capacity x 42
@@ -366,6 +367,7 @@ extern "C" frg_status frg_dcoll_create(frg_dcoll** out, int device, int64_t capa
   if (!out) return FRG_ERR_ARG;
   *out = nullptr;
   if (capacity < 1 || !(dup_tol > 0) || !std::isfinite(dup_tol)) return FRG_ERR_ARG;
+  if (capacity > kMost) return FRG_ERR_CUDA;
   frg_dcoll* c = new (std::nothrow) frg_dcoll();
   if (!c) return FRG_ERR_ALLOC;
   c->device = device;
@@ -402,6 +404,7 @@ extern "C" frg_status frg_dcoll_merge(frg_dcoll* c, const double* roots, int32_t
                                       double resid_max, const int32_t* keys, int64_t n, void* stream) {
   if (!c || n < 0 || (n > 0 && (!roots || !codes))) return FRG_ERR_ARG;
   if (n == 0) return FRG_OK;
+  if (n > kMost) return FRG_ERR_ALLOC;
   if (cudaSetDevice(c->device) != cudaSuccess) return FRG_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream;
   if (n > c->bn) {
