@@ -8,7 +8,7 @@ import subprocess
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "..", "finite_root_generation_gb300", "csrc")
 
-MAIN = """
+MAIN = r"""
 #include "cuda_runtime.h"
 static char* base = nullptr;
 static size_t held = 0;
@@ -46,7 +46,7 @@ int main() {
     frg_dcoll* d = nullptr;
     const frg_status s = frg_dcoll_create(&d, 0, c, 1e-6);
     if (outside || s != (c <= kib * kib ? FRG_OK : FRG_ERR_CUDA) || (d != nullptr) != (s == FRG_OK)) {
-      printf("capacity %lld: status %d, outside %d\\n", (long long)c, (int)s, (int)outside);
+      printf("capacity %lld: status %d, outside %d\n", (long long)c, (int)s, (int)outside);
       ++bad;
     }
     outside = false;
