@@ -424,9 +424,8 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   auto launch = [&](int mode) -> cudaError_t {
     if (team) return frg_launch_team(mode, a, team_grid(ctx, mode, N), st);
     const int grid = grid_for(mode, N);
-    const int wcap = warps ? ctx->sm_count * (ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : warp_bps[mode])
-                           : 0;
-    if (by_warp) return frg_launch_warp(mode, a, (int)std::min<int64_t>(wcap, (N + 3) / 4), st);
+    const int wbps = ctx->cfg.blocks_per_sm > 0 ? ctx->cfg.blocks_per_sm : warp_bps[mode];
+    if (by_warp) return frg_launch_warp(mode, a, frg_warp_grid(ctx->sm_count, wbps, N), st);
     if (!warps) return frg_launch_track(mode, a, grid, st);
     frg::TrackArgs b = a;
     b.tail_cap = tail_cap(mode);
@@ -436,7 +435,7 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
     if (e != cudaSuccess) return e;
     b.from_tail = 1;
     b.queue = q + 9 + 2 * mode;
-    return frg_launch_warp(mode, b, (int)std::min<int64_t>(wcap, (b.tail_cap + 3) / 4), st);
+    return frg_launch_warp(mode, b, frg_warp_grid(ctx->sm_count, wbps, b.tail_cap), st);
   };
   if (!mixed) {
     cudaError_t e = launch(0);

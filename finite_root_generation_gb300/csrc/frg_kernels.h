@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include "../../include/frg_gb300.h"
@@ -103,14 +104,20 @@ inline int frg_thread_grid(int sms, int bps, int64_t n) {
 // four warps per SM: one block per SM until its warps are taken, then as many as fit. In
 // the FP32 stage (lo) a block grows with the paths per SM, from 4 warps to 16.
 struct TeamGrid { int blocks, warps; };
-inline TeamGrid frg_team_grid(int sms, int bps, int64_t n, bool lo) {
-  const int64_t most = lo ? (4 * bps < 16 ? 4 * bps : 16) : 4, per_sm = (n + sms - 1) / sms;
+inline TeamGrid frg_team_grid(int sms, int64_t bps, int64_t n, bool lo) {
+  const int64_t most = lo ? (bps < 4 ? 4 * bps : 16) : 4, per_sm = (n + sms - 1) / sms;
   int64_t warps = (per_sm + 3) / 4 * 4;
   warps = warps < 4 ? 4 : (warps < most ? warps : most);
   const int64_t want = n <= sms * warps ? (n < sms ? n : sms) : (n + warps - 1) / warps;
   const int64_t per = 4 * bps / warps, cap = sms * (per < 1 ? 1 : per);
   const int64_t blocks = want < cap ? want : cap;
-  return {(int)(blocks < 1 ? 1 : blocks), (int)warps};
+  return {(int)(blocks < 1 ? 1 : (blocks < INT_MAX ? blocks : INT_MAX)), (int)warps};
+}
+
+// Grid of a warp-per-path launch of a plug-in over at most n paths, four to a block.
+inline int frg_warp_grid(int sms, int64_t bps, int64_t n) {
+  const int64_t want = (n + 3) / 4, cap = sms * bps, blocks = want < cap ? want : cap;
+  return (int)(blocks < INT_MAX ? blocks : INT_MAX);
 }
 
 // A plug-in launch of at most this many paths per SM sub-partition tracks a path per warp,
