@@ -277,6 +277,13 @@ static int mixed_rounds_of(const frg_config& c) {
   return c.kernel_variant == FRG_KERNEL_TEAM ? (c.mixed_rounds > 0 ? c.mixed_rounds : 1) : 1;
 }
 
+// Pieces in which a call's N paths are tracked, and in mixed precision its launches of the
+// FP32 and then the FP64 stage.
+static int pieces_of(const frg_config& c, int64_t N) {
+  return c.system == 0 || N == 0 ? 1 : (int)((N + FRG_PLUGIN_PIECE - 1) / FRG_PLUGIN_PIECE);
+}
+static int launch_rounds(const frg_config& c, int64_t N) { return c.system == 0 ? mixed_rounds_of(c) : pieces_of(c, N); }
+
 static frg_status ensure_events(frg_ctx* ctx, std::vector<cudaEvent_t>& v, size_t n) {
   while (v.size() < n) {
     cudaEvent_t ev;
@@ -307,81 +314,14 @@ static TeamGrid team_grid(const frg_ctx* ctx, int mode, int64_t n) {
   return frg_team_grid(ctx->sm_count, bps, n, mode == 1 || mode == 3);
 }
 
-// One round on a slot: gammas, start values, then the tracking launches, all on `st`.
-// `evs` (2 * mixed rounds + 1 events, mixed precision only) bracket the FP32 and FP64
-// launches. Device pointers only here.
-static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm, int ntasks, const int64_t* ppt,
-                                uint64_t seed, cx<double>* d_roots, int32_t* d_codes, cx<double>* d_yfinal,
-                                double* d_resid, int64_t N, cudaStream_t st, cudaEvent_t* evs) {
+// The tracking launches of a call, or of a piece of one (a.npaths paths), on `st`, with their start
+// values.
+static frg_status enqueue_paths(frg_ctx* ctx, Slot& sl, frg::TrackArgs a, cudaStream_t st, cudaEvent_t* evs) {
   const bool mixed = ctx->cfg.precision == FRG_PREC_MIXED;
+  const int64_t N = a.npaths;
+  unsigned long long* q = (unsigned long long*)sl.queue.p;
   int nv, np;
   dims_of(ctx->cfg, &nv, &np);
-  std::vector<cx<double>> g;
-  task_gammas(ctx->cfg, seed, ntasks, g);
-  std::vector<cx<float>> g_lo(ntasks);
-  std::vector<cx<df>> g_df(ntasks);
-  for (int k = 0; k < ntasks; ++k) {
-    g_lo[k] = cx<float>(g[k]);
-    g_df[k] = cx<df>(df(g[k].re), df(g[k].im));
-  }
-  std::vector<int64_t> starts(ntasks + 1, 0);
-  for (int k = 0; k < ntasks; ++k) starts[k + 1] = starts[k] + ppt[k];
-  FRG_CUDA(ctx, sl.gamma.ensure(sizeof(cx<double>) * ntasks));
-  FRG_CUDA(ctx, sl.gamma_lo.ensure(sizeof(cx<float>) * ntasks));
-  FRG_CUDA(ctx, sl.fpm_lo.ensure(sizeof(cx<float>) * np * ntasks));
-  FRG_CUDA(ctx, sl.fpm_df.ensure(sizeof(cx<df>) * np * ntasks));
-  FRG_CUDA(ctx, sl.gamma_df.ensure(sizeof(cx<df>) * ntasks));
-  FRG_CUDA(ctx, sl.task_start.ensure(sizeof(int64_t) * (ntasks + 1)));
-  FRG_CUDA(ctx, sl.queue.ensure(sizeof(unsigned long long) * FRG_NQUEUE));
-  FRG_CUDA(ctx, sl.counters.ensure(sizeof(unsigned long long) * FRG_NCOUNTERS));
-  // (host-to-device copies from pageable memory are staged before these calls return)
-  FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma_df.p, g_df.data(), sizeof(cx<df>) * ntasks, cudaMemcpyHostToDevice, st));
-  FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma.p, g.data(), sizeof(cx<double>) * ntasks, cudaMemcpyHostToDevice, st));
-  FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma_lo.p, g_lo.data(), sizeof(cx<float>) * ntasks, cudaMemcpyHostToDevice, st));
-  FRG_CUDA(ctx, cudaMemcpyAsync(sl.task_start.p, starts.data(), sizeof(int64_t) * (ntasks + 1),
-                                cudaMemcpyHostToDevice, st));
-  FRG_CUDA(ctx, cudaMemsetAsync(sl.queue.p, 0, sizeof(unsigned long long) * FRG_NQUEUE, st));
-  FRG_CUDA(ctx, cudaMemsetAsync(sl.counters.p, 0, sizeof(unsigned long long) * FRG_NCOUNTERS, st));
-  FRG_CUDA(ctx, frg_launch_to_float(d_fpm, (cx<float>*)sl.fpm_lo.p, np * ntasks, st));
-  FRG_CUDA(ctx, frg_launch_to_df(d_fpm, (cx<df>*)sl.fpm_df.p, np * ntasks, st));
-
-  frg::TrackArgs a;
-  std::memset(&a, 0, sizeof(a));
-  a.cfg = ctx->cfg;
-  a.fpm = d_fpm;
-  a.gamma = (const cx<double>*)sl.gamma.p;
-  a.fpm_lo = (const cx<float>*)sl.fpm_lo.p;
-  a.gamma_lo = (const cx<float>*)sl.gamma_lo.p;
-  a.fpm_df = (const cx<df>*)sl.fpm_df.p;
-  a.gamma_df = (const cx<df>*)sl.gamma_df.p;
-  a.task_start = (const int64_t*)sl.task_start.p;
-  a.ntasks = ntasks;
-  a.sms = ctx->sm_count;
-  a.npaths = N;
-  a.seed = seed;
-  unsigned long long* q = (unsigned long long*)sl.queue.p;
-  a.queue = q;
-  a.roots = d_roots;
-  a.codes = d_codes;
-  a.yfinal = d_yfinal;
-  a.resid = d_resid;
-  a.work = nullptr;
-  a.counters = (unsigned long long*)sl.counters.p;
-  if (ctx->feat_on) {
-    a.feat = (float*)ctx->feat.p;
-    a.nfeat = (int32_t*)ctx->nfeat.p;
-    a.feat_max = ctx->feat_max;
-    a.feat_every = ctx->feat_every;
-    FRG_CUDA(ctx, cudaMemsetAsync(ctx->nfeat.p, 0, sizeof(int32_t) * (size_t)N, st));
-  }
-  if (ctx->mlp_on) {
-    a.mlp.w = (const __nv_bfloat16*)ctx->mlp_w.p;
-    a.mlp.mu = (const float*)ctx->mlp_norm.p;
-    a.mlp.inv_sigma = (const float*)ctx->mlp_norm.p + FRG_MLP_IN;
-    a.mlp.threshold = ctx->mlp_threshold;
-    a.mlp.every = ctx->mlp_every;
-    a.feat_every = ctx->mlp_every;
-  }
   const bool team = ctx->cfg.kernel_variant == FRG_KERNEL_TEAM;
   if (team) {  // start values for every path, generated once up front
     FRG_CUDA(ctx, sl.starts.ensure(sizeof(cx<double>) * frg::FRG_START_STRIDE * (size_t)N));
@@ -482,6 +422,105 @@ static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm,
   return FRG_OK;
 }
 
+// One round on a slot: gammas, start values, then the tracking launches, all on `st`.
+// `evs` (2 * launch_rounds + 1 events, mixed precision only) bracket the FP32 and FP64
+// launches. Device pointers only here.
+static frg_status enqueue_track(frg_ctx* ctx, Slot& sl, const cx<double>* d_fpm, int ntasks, const int64_t* ppt,
+                                uint64_t seed, cx<double>* d_roots, int32_t* d_codes, cx<double>* d_yfinal,
+                                double* d_resid, int64_t N, cudaStream_t st, cudaEvent_t* evs) {
+  const bool mixed = ctx->cfg.precision == FRG_PREC_MIXED;
+  int nv, np;
+  dims_of(ctx->cfg, &nv, &np);
+  std::vector<cx<double>> g;
+  task_gammas(ctx->cfg, seed, ntasks, g);
+  std::vector<cx<float>> g_lo(ntasks);
+  std::vector<cx<df>> g_df(ntasks);
+  for (int k = 0; k < ntasks; ++k) {
+    g_lo[k] = cx<float>(g[k]);
+    g_df[k] = cx<df>(df(g[k].re), df(g[k].im));
+  }
+  // first path of each task, as the paths of each piece of the call are numbered
+  const int pieces = pieces_of(ctx->cfg, N);
+  std::vector<int64_t> starts((size_t)pieces * (ntasks + 1), 0);
+  for (int k = 0; k < ntasks; ++k) starts[k + 1] = starts[k] + ppt[k];
+  for (size_t i = ntasks + 1; i < starts.size(); ++i)
+    starts[i] = std::max<int64_t>(0, starts[i - (ntasks + 1)] - FRG_PLUGIN_PIECE);
+  FRG_CUDA(ctx, sl.gamma.ensure(sizeof(cx<double>) * ntasks));
+  FRG_CUDA(ctx, sl.gamma_lo.ensure(sizeof(cx<float>) * ntasks));
+  FRG_CUDA(ctx, sl.fpm_lo.ensure(sizeof(cx<float>) * np * ntasks));
+  FRG_CUDA(ctx, sl.fpm_df.ensure(sizeof(cx<df>) * np * ntasks));
+  FRG_CUDA(ctx, sl.gamma_df.ensure(sizeof(cx<df>) * ntasks));
+  FRG_CUDA(ctx, sl.task_start.ensure(sizeof(int64_t) * starts.size()));
+  FRG_CUDA(ctx, sl.queue.ensure(sizeof(unsigned long long) * FRG_NQUEUE));
+  FRG_CUDA(ctx, sl.counters.ensure(sizeof(unsigned long long) * FRG_NCOUNTERS));
+  // (host-to-device copies from pageable memory are staged before these calls return)
+  FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma_df.p, g_df.data(), sizeof(cx<df>) * ntasks, cudaMemcpyHostToDevice, st));
+  FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma.p, g.data(), sizeof(cx<double>) * ntasks, cudaMemcpyHostToDevice, st));
+  FRG_CUDA(ctx, cudaMemcpyAsync(sl.gamma_lo.p, g_lo.data(), sizeof(cx<float>) * ntasks, cudaMemcpyHostToDevice, st));
+  FRG_CUDA(ctx, cudaMemcpyAsync(sl.task_start.p, starts.data(), sizeof(int64_t) * starts.size(),
+                                cudaMemcpyHostToDevice, st));
+  FRG_CUDA(ctx, cudaMemsetAsync(sl.queue.p, 0, sizeof(unsigned long long) * FRG_NQUEUE, st));
+  FRG_CUDA(ctx, cudaMemsetAsync(sl.counters.p, 0, sizeof(unsigned long long) * FRG_NCOUNTERS, st));
+  FRG_CUDA(ctx, frg_launch_to_float(d_fpm, (cx<float>*)sl.fpm_lo.p, np * ntasks, st));
+  FRG_CUDA(ctx, frg_launch_to_df(d_fpm, (cx<df>*)sl.fpm_df.p, np * ntasks, st));
+
+  frg::TrackArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.cfg = ctx->cfg;
+  a.fpm = d_fpm;
+  a.gamma = (const cx<double>*)sl.gamma.p;
+  a.fpm_lo = (const cx<float>*)sl.fpm_lo.p;
+  a.gamma_lo = (const cx<float>*)sl.gamma_lo.p;
+  a.fpm_df = (const cx<df>*)sl.fpm_df.p;
+  a.gamma_df = (const cx<df>*)sl.gamma_df.p;
+  a.task_start = (const int64_t*)sl.task_start.p;
+  a.ntasks = ntasks;
+  a.sms = ctx->sm_count;
+  a.npaths = N;
+  a.seed = seed;
+  unsigned long long* q = (unsigned long long*)sl.queue.p;
+  a.queue = q;
+  a.roots = d_roots;
+  a.codes = d_codes;
+  a.yfinal = d_yfinal;
+  a.resid = d_resid;
+  a.work = nullptr;
+  a.counters = (unsigned long long*)sl.counters.p;
+  if (ctx->feat_on) {
+    a.feat = (float*)ctx->feat.p;
+    a.nfeat = (int32_t*)ctx->nfeat.p;
+    a.feat_max = ctx->feat_max;
+    a.feat_every = ctx->feat_every;
+    FRG_CUDA(ctx, cudaMemsetAsync(ctx->nfeat.p, 0, sizeof(int32_t) * (size_t)N, st));
+  }
+  if (ctx->mlp_on) {
+    a.mlp.w = (const __nv_bfloat16*)ctx->mlp_w.p;
+    a.mlp.mu = (const float*)ctx->mlp_norm.p;
+    a.mlp.inv_sigma = (const float*)ctx->mlp_norm.p + FRG_MLP_IN;
+    a.mlp.threshold = ctx->mlp_threshold;
+    a.mlp.every = ctx->mlp_every;
+    a.feat_every = ctx->mlp_every;
+  }
+  if (ctx->cfg.system == 0) return enqueue_paths(ctx, sl, a, st, evs);
+  // a plug-in's call in pieces, one after the other: each is a call of its own on a range of
+  // the paths, with the work buffers of the one before
+  for (int64_t first = 0; first < N; first += FRG_PLUGIN_PIECE) {
+    const int64_t piece = first / FRG_PLUGIN_PIECE;
+    frg::TrackArgs b = a;
+    b.npaths = std::min(N - first, FRG_PLUGIN_PIECE);
+    b.cfg.path_offset += first;
+    b.task_start += piece * (ntasks + 1);
+    b.roots += first * nv;
+    b.codes += first;
+    if (b.yfinal) b.yfinal += first * (nv + 2);
+    if (b.resid) b.resid += first;
+    if (piece > 0) FRG_CUDA(ctx, cudaMemsetAsync(sl.queue.p, 0, sizeof(unsigned long long) * FRG_NQUEUE, st));
+    const frg_status s = enqueue_paths(ctx, sl, b, st, evs + (mixed ? 2 * piece : 0));
+    if (s != FRG_OK) return s;
+  }
+  return FRG_OK;
+}
+
 static frg_status check_track_args(frg_ctx* ctx, const double* fpm, int ntasks, const int64_t* ppt, double* roots,
                                    int32_t* codes, int64_t* N) {
   if (!ctx) return FRG_ERR_ARG;
@@ -507,7 +546,7 @@ extern "C" frg_status frg_track_async(frg_ctx* ctx, const double* fpm, int ntask
   if (!is_device_ptr(fpm) || !is_device_ptr(roots) || !is_device_ptr(codes) || (yfinal && !is_device_ptr(yfinal)) ||
       (resid && !is_device_ptr(resid)))
     return fail(ctx, FRG_ERR_ARG, "frg_track_async takes device pointers only");
-  s = ensure_events(ctx, ctx->round_ev, 2 * mixed_rounds_of(ctx->cfg) + 1);
+  s = ensure_events(ctx, ctx->round_ev, 2 * launch_rounds(ctx->cfg, N) + 1);
   if (s != FRG_OK) return s;
   ctx->last_rounds = 0;  // stage times are not reported for asynchronous calls
   return enqueue_track(ctx, *ctx->slots[0], (const cx<double>*)fpm, ntasks, paths_per_task, seed,
@@ -562,7 +601,7 @@ extern "C" frg_status frg_track(frg_ctx* ctx, const double* fpm, int ntasks, con
   cudaStream_t st = ctx->stream;
   Slot& sl = *ctx->slots[0];
   const bool mixed = ctx->cfg.precision == FRG_PREC_MIXED;
-  const int mr = mixed_rounds_of(ctx->cfg);
+  const int mr = launch_rounds(ctx->cfg, N);
   s = ensure_events(ctx, ctx->round_ev, 2 * mr + 1);
   if (s != FRG_OK) return s;
 
@@ -828,7 +867,7 @@ extern "C" frg_status frg_track_rounds(frg_ctx* ctx, const double* fpm, int ntas
   if (N == 0) return FRG_OK;
   FRG_CUDA(ctx, cudaSetDevice(ctx->device));
   const bool mixed = ctx->cfg.precision == FRG_PREC_MIXED;
-  const int mr = mixed_rounds_of(ctx->cfg);
+  const int mr = launch_rounds(ctx->cfg, N);
   if (depth > nrounds) depth = nrounds;
   while ((int)ctx->slots.size() < depth) {
     Slot* sl = new (std::nothrow) Slot();

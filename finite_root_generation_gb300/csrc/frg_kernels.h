@@ -120,6 +120,13 @@ inline int frg_warp_grid(int sms, int64_t bps, int64_t n) {
   return (int)(blocks < INT_MAX ? blocks : INT_MAX);
 }
 
+// A plug-in's call is tracked in pieces of at most this many paths, so that its start values
+// and endpoints (288 B a path for conic2, 512 B for burmester5; in mixed precision 1.2 KB of
+// records more) never take more than 8.6 GB (29 GB), whatever the call. The last paths of each
+// piece leave the GPU partly idle: 16.8 M conic2 paths in FP64 take 4,454 ms in one piece and 4,510
+// in two, in mixed precision 1,410 and 1,408.
+constexpr int64_t FRG_PLUGIN_PIECE = (int64_t)1 << 24;
+
 // A plug-in launch of at most this many paths per SM sub-partition tracks a path per warp,
 // a larger one a path per thread. GB300 (152 SMs), warp / thread, FP64: conic2 2,432 paths
 // 8.4 / 12.5 ms, 9,728 26.9 / 25.6, 19,456 55.9 / 45.9; burmester5 4,864 52 / 87, 9,728 406 /
