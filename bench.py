@@ -44,6 +44,7 @@ import time
 import numpy as np
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
+WARP_PATHS_PER_SM = 64  # paths per SM up to which a plug-in call runs a warp per path (4 x FRG_WARP_PATHS)
 sys.path.insert(0, ROOT)
 
 METRIC = "distinct finite roots/sec at >=99.5% recall, residual <=1e-10: chosen vs plain FP64"
@@ -824,7 +825,8 @@ def run_plugin(args):
                          "flops_per_solve": fps, "solves": int(solves),
                          "peak_source": "of measured: bench.py's own FP64 FMA kernel"},
             # the parameter copies, starts, tracking (by thread, then the last paths by warp), finishes
-            "gpu_launches": (6 if N > torch.cuda.get_device_properties(0).multi_processor_count * 64 else 5) * k,
+            "gpu_launches": (6 if N > torch.cuda.get_device_properties(0).multi_processor_count * WARP_PATHS_PER_SM
+                             else 5) * k,
             "clocks": clk.summary(),
             "mixed": {"value": round(k * N / (m_ms * 1e-3), 1), "unit": "paths/s",
                       "speedup_vs_plain_fp64": round(ms / m_ms, 3), "recall_vs_plain_fp64": round(hits / max(total, 1), 5),

@@ -128,10 +128,12 @@ inline int frg_warp_grid(int sms, int64_t bps, int64_t n) {
 constexpr int64_t FRG_PLUGIN_PIECE = (int64_t)1 << 24;
 
 // A plug-in launch of at most this many paths per SM sub-partition tracks a path per warp,
-// a larger one a path per thread. GB300 (152 SMs), warp / thread, FP64: conic2 2,432 paths
-// 8.4 / 12.5 ms, 9,728 26.9 / 25.6, 19,456 55.9 / 45.9; burmester5 4,864 52 / 87, 9,728 406 /
-// 433, 19,456 463 / 446. Mixed: conic2 4,864 2.6 / 3.4, 9,728 3.8 / 3.5; burmester5 9,728
-// 383 / 403, 19,456 391 / 411.
+// a larger one a path per thread and its last paths per warp. GB300 (152 SMs), warp / thread,
+// medians of three seeds, FP64: conic2 2,432 paths 14.8 / 18.4 ms, 4,864 25.1 / 25.7, 9,728
+// 28.8 / 27.3, 14,592 33.4 / 28.4; burmester5 4,864 89 / 112, 9,728 402 / 422, 14,592 426 / 429,
+// 19,456 450 / 434. Mixed: conic2 4,864 2.6 / 3.1, 9,728 3.9 / 3.6, 14,592 5.5 / 4.1; burmester5
+// 9,728 379 / 409, 19,456 393 / 414. One line for all: at 9,728 paths conic2 loses a twentieth by
+// it and burmester5 gains as much.
 constexpr int FRG_WARP_PATHS = 16;
 
 // A warp of a thread-per-path launch gives its paths up to a warp-per-path launch when the

@@ -106,8 +106,7 @@ __device__ __forceinline__ void begin_newton(PathState<T, NY_, NP_>& P, int phas
 template <class S>
 __device__ void finish_path(const TrackArgs& a, int64_t id, int task, int code, cd* Yf, const cd* fpm);
 
-// The task arrays in the working precision (FP32 copies are prepared by the host; the
-// FP32 stage exists for Stephenson II only).
+// The task arrays in the working precision (FP32 copies are prepared by the host).
 template <typename T, int NP_> struct TaskFpm;
 template <int NP_> struct TaskFpm<double, NP_> {
   __device__ static const cx<double>* get(const TrackArgs& a, int task) { return a.fpm + (size_t)task * NP_; }

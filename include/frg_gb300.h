@@ -87,7 +87,9 @@ typedef struct frg_config {
                            exceeds this continues its path in FP64 */
   double inf_tol;       /* > 0: |Z0| / |Z| below this at t = 1 marks code 7 */
   int threads_per_block; /* 0 = tuned default */
-  int blocks_per_sm;     /* 0 = tuned default */
+  int blocks_per_sm;     /* most resident blocks per SM, 0 = tuned default: blocks of 64 threads (thread
+                            kernels, a path per thread) or of four warps (team kernels and plug-ins' warp
+                            kernels, a path per warp; the FP32 stage joins up to four of them in one) */
   double newt_tol_lo;    /* mixed: corrector tolerance of the FP32 stage */
   int kernel_variant;    /* FRG_KERNEL_TEAM (a warp per path, default) or FRG_KERNEL_THREAD */
   int mixed_rounds;      /* mixed, team kernels: FP32/FP64 rounds; a path well conditioned again in
@@ -161,9 +163,11 @@ typedef struct frg_stats {
                                 tracks one path) */
   int64_t handbacks;       /* mixed: returns from FP64 to FP32 once well conditioned again */
   int64_t refine_solves;   /* mixed: FP32-stage corrector iterations on double-float residuals */
-  int64_t refine_warp_steps; /* mixed: FP32-stage warp steps whose path refined */
+  int64_t refine_warp_steps; /* mixed: FP32-stage warp steps whose path refined (refine_solves: a warp has
+                                one path) */
   double round_ms[32];     /* mixed: FP32-stage and FP64-stage times, interleaved, of mixed rounds
-                              0..15 (frg_track) or of rounds 0..15 of the call (frg_track_rounds) */
+                              0..15 (frg_track; of a plug-in's call above 16.8 M paths, of its pieces
+                              of that size) or of rounds 0..15 of the call (frg_track_rounds) */
   int64_t fp64_segment_hist[6]; /* mixed: paths leaving an FP64 launch after <100, <300, <1000, <3000,
                                    <10000, >=10000 FP64 solves in it */
   int64_t fp64_segment_max;     /* mixed: most FP64 solves one path spent in one FP64 launch */
