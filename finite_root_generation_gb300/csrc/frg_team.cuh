@@ -31,7 +31,7 @@
 // the four sub-partitions, with 32 lanes on the elimination and equal operations of
 // different quantities in the same instructions, it is about 1,400 on the longest warp,
 // 123k cycles, and 1,150, 105k cycles, while a block has one or two paths (PairCx). The
-// FP32 step went from 105k to 16k. With every SM full the FP64 work per path falls as
+// FP32 step went from 105k to 15k. With every SM full the FP64 work per path falls as
 // well (fewer repeated sums and idle lanes): FP64 rounds of 32,768 paths, three in flight,
 // 6,815 to 3,696 ms a round. Comparisons, maxima and stored negations of FP64 values run
 // on their bit patterns in the integer pipes for the same reason.
@@ -330,36 +330,22 @@ __device__ __forceinline__ T patch_scale(const cx<T>* u, int lane) {
 }
 
 // Pivot search: the row with the largest v (ties: the lowest), as its lane's bit. Row r's
-// value is on lane base + r, v >= 0 or NaN, or -1 for used rows; the other lanes hold -1. As
-// integers the values' bits have their order, with a NaN of negative sign between the
-// used rows and zero; one of positive sign, which would come out above infinity, is put there
-// too, in a search of its own: a used row must never win, or a later part of the elimination
-// finds more unused rows than it has room for.
-__device__ __noinline__ unsigned pivot_lane_nan(float v) {
-  const int key = v == v ? __float_as_int(v) : -1;
-  const unsigned c = __ballot_sync(FULL, key == __reduce_max_sync(FULL, key));
-  return c & (0u - c);
-}
-__device__ __noinline__ unsigned pivot_lane_nan(double v) {
-  const int hi = v == v ? __double2hiint(v) : -1;
-  const unsigned lo = v == v ? (unsigned)__double2loint(v) : 0u;
-  const int m = __reduce_max_sync(FULL, hi);
-  const unsigned ml = __reduce_max_sync(FULL, hi == m ? lo : 0u);
-  const unsigned c = __ballot_sync(FULL, hi == m && lo == ml);
-  return c & (0u - c);
-}
+// value is on lane base + r, v >= 0 or NaN, or -1 for used rows; the other lanes hold -1. The
+// values' bits as integers have their order; a NaN comes out above infinity or, with a
+// negative sign, below zero, but never below the -1 of a used row: such a row must not win, or a
+// later part of the elimination finds more unused rows than it has room for. (Which of the
+// others wins then is all the same, the step has no finite solution.) A branch to a search of
+// its own for infinities and NaN cost 50 cycles a pivot: the FP32 stage of 140 paths 104 -> 100
+// ms, of 2,048 200 -> 191, of 9,600 267 -> 257.
 __device__ __forceinline__ unsigned pivot_lane(float v) {
   const int key = __float_as_int(v);
-  const int m = __reduce_max_sync(FULL, key);
-  if (m > 0x7f800000) return pivot_lane_nan(v);
-  const unsigned c = __ballot_sync(FULL, key == m);
+  const unsigned c = __ballot_sync(FULL, key == __reduce_max_sync(FULL, key));
   return c & (0u - c);
 }
 __device__ __forceinline__ unsigned pivot_lane(double v) {
   const int hi = __double2hiint(v);
   const unsigned lo = (unsigned)__double2loint(v);
   const int m = __reduce_max_sync(FULL, hi);
-  if (m >= 0x7ff00000) return pivot_lane_nan(v);
   unsigned c = __ballot_sync(FULL, hi == m);
   if (c & (c - 1)) {
     const unsigned ml = __reduce_max_sync(FULL, hi == m ? lo : 0u);

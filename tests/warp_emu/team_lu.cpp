@@ -18,7 +18,7 @@ template <typename T> T special(int kind) {
   return kind == 0 ? std::copysign(nan, T(1)) : kind == 1 ? std::copysign(nan, T(-1)) : T(INFINITY);
 }
 
-// The row found is unused, and the first of the largest, NaN being smaller than any number.
+// The row found is unused, and the first of the largest unless there is a NaN.
 template <int RP, typename T>
 void search(const char* type) {
   constexpr int CL = 32 / RP;
@@ -40,14 +40,17 @@ void search(const char* type) {
       bit[lane] = pivot_lane(lane / RP == base / RP ? v[r] : T(-1));
     });
     int want = -1;
-    for (int r = 0; r < RP; ++r)
-      if (!used[r] && (want < 0 || v[r] > v[want] || (v[want] != v[want] && v[r] == v[r]))) want = r;
-    bool nan = v[want] != v[want];
+    bool nan = false;
+    for (int r = 0; r < RP; ++r) {
+      if (used[r]) continue;
+      nan = nan || v[r] != v[r];
+      if (want < 0 || v[r] > v[want]) want = r;
+    }
     for (int l = 0; l < 32; ++l) {
       check(bit[l] == bit[0] && __builtin_popcount(bit[0]) == 1, "one lane", type, k);
       const int row = __builtin_ctz(bit[l]) - base;
       check(row >= 0 && row < RP && !used[row], "an unused row", type, k);
-      if (row >= 0 && row < RP) check(nan ? v[row] != v[row] : row == want, "the first of the largest", type, k);
+      check(nan || row == want, "the first of the largest", type, k);
     }
   }
 }
